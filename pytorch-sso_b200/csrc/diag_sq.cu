@@ -10,7 +10,9 @@
 // accumulates the 64 x 64 per-sample gradient tile over the pixels (operands staged in shared
 // memory, 4x4 register tile per thread), squares it into a second register tile and moves on.
 // Sample ranges go to a workspace and are summed in a fixed order by a finishing kernel
-// (deterministic, no atomics).
+// (deterministic, no atomics).  The bias takes the squares of the gradient values that the CTAs of the
+// first column tile stage anyway and one more row of the workspace (a kernel of its own read the
+// gradient again with one warp per channel: 160 us per layer, 30 % of a step with these curvatures).
 #include "common.cuh"
 
 namespace sso {
@@ -19,7 +21,8 @@ struct DiagSqParams {
   const void* x;        // layer input  [n, c, h, w]   (element strides sxn, sxc, sxh, sxw)
   const void* g;        // output grad  [n, oc, ho, wo] (element strides sgn, sgc, sgh, sgw)
   const float* weight;  // per-sample weights, nullable
-  float* partial;       // [splits][oc][d]
+  float* partial;       // [splits][oc*d + oc]: weight, then bias
+  bool bias;
   int64_t sxn, sxc, sxh, sxw, sgn, sgc, sgh, sgw;
   int n, c, h, w, oc, ho, wo;
   int kh, kw, stride_h, stride_w, pad_h, pad_w, dil_h, dil_w;
@@ -62,6 +65,8 @@ __global__ void __launch_bounds__(256) diag_sq_kernel(const DiagSqParams p) {
     for (int q = 0; q < 4; ++q) sq[i][q] = 0.f;
   // staging map: thread -> (pixel ll = tid / 16, four consecutive tile columns 4*(tid % 16) ..)
   const int ll = tid >> 4, c4 = (tid & 15) * 4;
+  const bool bias = p.bias && blockIdx.y == 0;
+  float bs[4] = {0.f, 0.f, 0.f, 0.f};      // sum over this thread's pixels of w_b g^2, columns c4 ..
   if (ONE_PIXEL) {
     for (int b0 = b_begin; b0 < b_end; b0 += DK) {
       const int b = b0 + ll;
@@ -73,6 +78,7 @@ __global__ void __launch_bounds__(256) diag_sq_kernel(const DiagSqParams p) {
         float gv = 0.f;
         if (bv && o < p.oc) gv = to_f32<T>(__ldg(G + (int64_t)b * p.sgn + (int64_t)o * p.sgc));
         Gs[ll][c4 + q] = wb * gv * gv;
+        bs[q] += wb * gv * gv;
         float uv = 0.f;
         const int64_t off = col_off[c4 + q];
         if (bv && off >= 0) uv = to_f32<T>(__ldg(X + (int64_t)b * p.sxn + off));
@@ -119,8 +125,13 @@ __global__ void __launch_bounds__(256) diag_sq_kernel(const DiagSqParams p) {
         }
       }
     };
+    const float wb = p.weight ? p.weight[b] : 1.f;
     gather(0);
     for (int l0 = 0; l0 < L; l0 += DK) {
+      if (bias) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) bs[q] = fmaf(wb * to_f32<T>(gv[q]), to_f32<T>(gv[q]), bs[q]);
+      }
       *reinterpret_cast<float4*>(&Gs[ll][c4]) = make_float4(to_f32<T>(gv[0]), to_f32<T>(gv[1]), to_f32<T>(gv[2]), to_f32<T>(gv[3]));
       *reinterpret_cast<float4*>(&Us[ll][c4]) = make_float4(to_f32<T>(uv[0]), to_f32<T>(uv[1]), to_f32<T>(uv[2]), to_f32<T>(uv[3]));
       __syncthreads();
@@ -137,13 +148,12 @@ __global__ void __launch_bounds__(256) diag_sq_kernel(const DiagSqParams p) {
       }
       __syncthreads();
     }
-    const float wb = p.weight ? p.weight[b] : 1.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int q = 0; q < 4; ++q) sq[i][q] = fmaf(wb * acc[i][q], acc[i][q], sq[i][q]);
   }
-  float* dst = p.partial + (int64_t)split * p.oc * p.d;
+  float* dst = p.partial + (int64_t)split * p.oc * (p.d + 1);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int o = o0 + ty * 4 + i;
@@ -154,39 +164,28 @@ __global__ void __launch_bounds__(256) diag_sq_kernel(const DiagSqParams p) {
       if (j < p.d) dst[(int64_t)o * p.d + j] = sq[i][q];
     }
   }
+  if (bias) {      // Gs is free: the 16 pixel lanes of a column are summed in order
+    *reinterpret_cast<float4*>(&Gs[ll][c4]) = make_float4(bs[0], bs[1], bs[2], bs[3]);
+    __syncthreads();
+    if (tid < DT && o0 + tid < p.oc) {
+      float t = 0.f;
+#pragma unroll
+      for (int k = 0; k < DK; ++k) t += Gs[k][tid];
+      dst[(int64_t)p.oc * p.d + o0 + tid] = t;
+    }
+  }
 }
 
-__global__ void __launch_bounds__(256) diag_sq_finish_kernel(const float* __restrict__ partial, int splits,
-                                                             int64_t count, float alpha, float beta,
-                                                             float* __restrict__ out) {
+__global__ void __launch_bounds__(256) diag_sq_finish_kernel(const float* __restrict__ partial, int splits, int64_t pitch,
+                                                             int64_t n_w, int64_t count, float alpha, float beta,
+                                                             float* __restrict__ out_w, float* __restrict__ out_b) {
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= count) return;
   float s = 0.f;
-  for (int sp = 0; sp < splits; ++sp) s += partial[(int64_t)sp * count + i];
-  out[i] = (beta == 0.f) ? alpha * s : fmaf(beta, out[i], alpha * s);
-}
-
-// bias: one warp per output channel, samples and pixels summed in a fixed order
-template <typename T>
-__global__ void __launch_bounds__(256) diag_sq_bias_kernel(const DiagSqParams p, float alpha, float beta,
-                                                           float* __restrict__ out_b) {
-  const int o = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (o >= p.oc) return;
-  const T* G = reinterpret_cast<const T*>(p.g);
-  const int L = p.ho * p.wo;
-  float tot = 0.f;
-  for (int b = 0; b < p.n; ++b) {
-    float s = 0.f;
-    for (int l = lane; l < L; l += 32) {
-      const int oy = l / p.wo, ox = l - oy * p.wo;
-      const float v = to_f32<T>(__ldg(G + (int64_t)b * p.sgn + (int64_t)o * p.sgc + (int64_t)oy * p.sgh + (int64_t)ox * p.sgw));
-      s = fmaf(v, v, s);
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    tot = fmaf(p.weight ? p.weight[b] : 1.f, s, tot);
-  }
-  if (lane == 0) out_b[o] = (beta == 0.f) ? alpha * tot : fmaf(beta, out_b[o], alpha * tot);
+#pragma unroll 4
+  for (int sp = 0; sp < splits; ++sp) s += partial[(int64_t)sp * pitch + i];
+  float* o = i < n_w ? out_w + i : out_b + (i - n_w);
+  *o = (beta == 0.f) ? alpha * s : fmaf(beta, *o, alpha * s);
 }
 
 static int diag_sq_splits(int n, int oc, int d) {
@@ -204,13 +203,10 @@ static int diag_sq_typed(DiagSqParams p, float alpha, float beta, float* out_w, 
   else
     diag_sq_kernel<T, false><<<grid, 256, 0, st>>>(p);
   SSO_LAUNCH_OK("diag_sq_kernel");
-  const int64_t count = (int64_t)p.oc * p.d;
-  diag_sq_finish_kernel<<<(unsigned)ceil_div64(count, 256), 256, 0, st>>>(p.partial, splits, count, alpha, beta, out_w);
+  const int64_t n_w = (int64_t)p.oc * p.d, count = n_w + (out_b ? p.oc : 0);
+  diag_sq_finish_kernel<<<(unsigned)ceil_div64(count, 256), 256, 0, st>>>(p.partial, splits, n_w + p.oc, n_w, count, alpha, beta,
+                                                                         out_w, out_b);
   SSO_LAUNCH_OK("diag_sq_finish_kernel");
-  if (out_b) {
-    diag_sq_bias_kernel<T><<<ceil_div(p.oc, 8), 256, 0, st>>>(p, alpha, beta, out_b);
-    SSO_LAUNCH_OK("diag_sq_bias_kernel");
-  }
   return 0;
 }
 
@@ -224,7 +220,7 @@ size_t sso_diag_sq_workspace_bytes(int64_t n, int64_t oc, int64_t d) {
   if (n <= 0 || oc <= 0 || d <= 0) return 0;
   const int splits = diag_sq_splits((int)n, (int)oc, (int)d);
   const int per = ceil_div((int)n, splits);
-  return (size_t)ceil_div((int)n, per) * (size_t)oc * (size_t)d * sizeof(float);
+  return (size_t)ceil_div((int)n, per) * (size_t)oc * (size_t)(d + 1) * sizeof(float);
 }
 
 int sso_diag_sq_im2col(const void* x, const void* g, int dtype, int64_t n, int64_t c, int64_t h, int64_t w,
@@ -246,7 +242,7 @@ int sso_diag_sq_im2col(const void* x, const void* g, int dtype, int64_t n, int64
   SSO_CHECK_ARG(workspace != nullptr && workspace_bytes >= need, "diag_sq: workspace too small: need %zu bytes, got %zu",
                 need, workspace_bytes);
   DiagSqParams p{};
-  p.x = x; p.g = g; p.weight = sample_weight; p.partial = reinterpret_cast<float*>(workspace);
+  p.x = x; p.g = g; p.weight = sample_weight; p.partial = reinterpret_cast<float*>(workspace); p.bias = out_b != nullptr;
   p.sxn = sxn; p.sxc = sxc; p.sxh = sxh; p.sxw = sxw; p.sgn = sgn; p.sgc = sgc; p.sgh = sgh; p.sgw = sgw;
   p.n = (int)n; p.c = (int)c; p.h = (int)h; p.w = (int)w; p.oc = (int)oc; p.ho = (int)ho; p.wo = (int)wo;
   p.kh = kh; p.kw = kw; p.stride_h = stride_h; p.stride_w = stride_w; p.pad_h = pad_h; p.pad_w = pad_w;

@@ -105,6 +105,14 @@ typedef struct {
   float* out;
   int64_t ldo;
 } sso_factor_desc;
+/* One sso_factor_syrk_im2col call with everything that does not change between calls given once: the
+ * description's x may be null, its sample_weight, alpha and beta are ignored.  The handle belongs to the
+ * host only (no device memory); run it with scratch of sso_factor_workspace_bytes bytes. */
+int64_t sso_factor_op_create(const sso_factor_desc* desc, int impl);
+int sso_factor_op_run(int64_t op, const void* x, const float* sample_weight, float alpha, float beta, void* workspace,
+                      size_t workspace_bytes, void* stream);
+int sso_factor_op_destroy(int64_t op);
+
 size_t sso_factor_batch_workspace_bytes(int n, const sso_factor_desc* descs);
 int sso_factor_batch(int n, const sso_factor_desc* descs, void* workspace, size_t workspace_bytes, void* stream);
 
@@ -254,9 +262,24 @@ typedef struct {
   float* ebuf;       /* nullable */
   int64_t count;
   float add, momentum, ema, scale, lr;
-  int32_t pad;
-} sso_tail_rec;
+  int32_t set;       /* sso_optimizer_tail_sets: index of the record's scalars; unused otherwise */
+} sso_tail_rec;    /* count < 2^31 */
 int sso_optimizer_tail(const sso_tail_rec* recs_dev, int n_recs, void* stream);
+
+/* The same with the scalars given at launch: record i uses sets[recs[i].set] (a host array, copied into the
+ * kernel's parameters) in place of its own add .. lr, so that a table outlives a change of learning rate or
+ * regularisation. */
+#define SSO_TAIL_MAX_SETS 128
+typedef struct {
+  float add, momentum, ema, scale, lr;
+} sso_tail_set;
+int sso_optimizer_tail_sets(const sso_tail_rec* recs_dev, int n_recs, const sso_tail_set* sets, int n_sets, void* stream);
+
+/* One draw per row from unnormalised probabilities: out[i] = argmax_c prob[i][c] / q[i][c] over c < classes (the
+ * first one on ties) with q independent Exp(1) numbers.  Entries that are negative or not finite count as
+ * zero; a row that then sums to zero is drawn uniformly.  prob and q are dense [rows, classes].
+ * Replaces: the target sampling of torchsso/curv/fisher/__init__.py:60-64. */
+int sso_sample_classes(const float* prob, const float* q, int64_t rows, int64_t classes, int64_t* out, void* stream);
 
 /* ---------------------------------------------------------------------------------------
  * Tile-task engine.  All dense algebra after factor construction (pi-damped SPD inverse,

@@ -166,6 +166,38 @@ int sso_factor_syrk_im2col(const void* x, int dtype, int64_t n, int64_t c, int64
   return launch_one_factor(p, dtype, workspace, workspace_bytes, impl, reinterpret_cast<cudaStream_t>(stream));
 }
 
+// ---- prepared calls ---------------------------------------------------------------------------
+struct PreparedFactor {
+  FactorParams p;
+  int dtype, impl;
+};
+
+int64_t sso_factor_op_create(const sso_factor_desc* q, int impl) {
+  SSO_CHECK_ARG(q != nullptr, "factor op: null description");
+  PreparedFactor f;
+  const float dummy = 0.f;      // the input's address comes with every call
+  const int rc = make_factor_params(q->x ? q->x : &dummy, q->n, q->c, q->h, q->w, q->sn, q->sc, q->sh, q->sw, q->kh, q->kw,
+                                    q->stride_h, q->stride_w, q->pad_h, q->pad_w, q->dil_h, q->dil_w, q->append_ones, nullptr, 0.f,
+                                    0.f, q->out, q->ldo, f.p);
+  if (rc) return rc;
+  f.dtype = q->dtype; f.impl = impl;
+  return reinterpret_cast<int64_t>(new PreparedFactor(f));
+}
+
+int sso_factor_op_destroy(int64_t op) {
+  delete reinterpret_cast<PreparedFactor*>(op);
+  return 0;
+}
+
+int sso_factor_op_run(int64_t op, const void* x, const float* sample_weight, float alpha, float beta, void* workspace,
+                      size_t workspace_bytes, void* stream) {
+  SSO_CHECK_ARG(op > 0 && x != nullptr, "factor op: null argument");
+  const PreparedFactor* f = reinterpret_cast<const PreparedFactor*>(op);
+  FactorParams p = f->p;
+  p.x = x; p.weight = sample_weight; p.alpha = alpha; p.beta = beta;
+  return launch_one_factor(p, f->dtype, workspace, workspace_bytes, f->impl, reinterpret_cast<cudaStream_t>(stream));
+}
+
 // ---- many factors in one call ----------------------------------------------------------------
 static int batch_params(int n, const sso_factor_desc* descs, std::vector<FactorParams>& ps, std::vector<int>& dts) {
   SSO_CHECK_ARG(n >= 0 && (n == 0 || descs != nullptr), "factor batch: bad argument");

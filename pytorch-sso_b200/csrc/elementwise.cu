@@ -410,23 +410,101 @@ __global__ void __launch_bounds__(256) copy_segments_kernel(const sso_seg_rec* _
   }
 }
 
-__global__ void __launch_bounds__(256) optimizer_tail_kernel(const sso_tail_rec* __restrict__ recs) {
+// One warp per row; the comparison is on the quotients, ties go to the lower class.  Launch bound.
+__global__ void __launch_bounds__(256) sample_classes_kernel(const float* __restrict__ prob, const float* __restrict__ q, int64_t rows,
+                                                             int64_t classes, int64_t* __restrict__ out) {
+  const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const float* p = prob + row * classes;
+  const float* e = q + row * classes;
+  auto clean = [](float v) { return (v > 0.f && v <= 3.402823466e38f) ? v : 0.f; };
+  float best = -1.f, flat = -1.f, sum = 0.f;     // the race over the probabilities, and over a uniform row
+  int64_t best_c = 0, flat_c = 0;
+  for (int64_t c = lane; c < classes; c += 32) {
+    const float v = clean(p[c]), r = v / e[c], u = 1.f / e[c];
+    sum += v;
+    if (r > best) { best = r; best_c = c; }
+    if (u > flat) { flat = u; flat_c = c; }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float b = __shfl_xor_sync(0xffffffffu, best, o), f = __shfl_xor_sync(0xffffffffu, flat, o);
+    const int64_t bc = __shfl_xor_sync(0xffffffffu, best_c, o), fc = __shfl_xor_sync(0xffffffffu, flat_c, o);
+    if (b > best || (b == best && bc < best_c)) { best = b; best_c = bc; }
+    if (f > flat || (f == flat && fc < flat_c)) { flat = f; flat_c = fc; }
+  }
+  if (lane == 0) out[row] = sum > 0.f ? best_c : flat_c;
+}
+
+// Bound: HBM (up to seven streams of 4 bytes per element), at small sizes the launch.  One CTA per record of
+// at most 4096 elements, so that a network of two million parameters already gives every SM several CTAs
+// (with 32768-element records it was 55 CTAs of one scalar load chain each: 65 us for 1.8 M parameters,
+// 8 us now).  Where a record's arrays start on 16 bytes a thread moves float4s, the loads of two of them
+// issued before the first store (source and destination come out of one record, so the compiler must
+// assume that they alias); the scalars travel in kernel parameters, one set per distinct combination, so
+// that a schedule that changes them does not rebuild the table.
+struct TailSets { sso_tail_set s[SSO_TAIL_MAX_SETS]; };
+
+__device__ __forceinline__ void tail_element(const sso_tail_set& q, bool has_m, bool has_e, float& p, float& g, float& m, float& e) {
+  float v = fmaf(q.add, p, g);
+  if (has_m) { v = fmaf(q.momentum, m, v); m = v; }
+  if (has_e) { v = fmaf(q.ema, v, (1.f - q.ema) * e); e = v; }
+  v *= q.scale;
+  g = v;
+  p = fmaf(-q.lr, v, p);
+}
+
+template <bool OWN>
+__global__ void __launch_bounds__(256) optimizer_tail_kernel(const sso_tail_rec* __restrict__ recs,
+                                                             const __grid_constant__ TailSets sets) {
   const sso_tail_rec r = recs[blockIdx.x];
-  for (int64_t i = threadIdx.x; i < r.count; i += 256) {
-    const float pv = r.p[i];
-    float g = r.g[i];
-    g = fmaf(r.add, pv, g);
-    if (r.mbuf) {
-      g = fmaf(r.momentum, r.mbuf[i], g);
-      r.mbuf[i] = g;
+  sso_tail_set q;
+  if (OWN) { q.add = r.add; q.momentum = r.momentum; q.ema = r.ema; q.scale = r.scale; q.lr = r.lr; }
+  else q = sets.s[r.set];
+  const bool has_m = r.mbuf != nullptr, has_e = r.ebuf != nullptr, upd = q.lr != 0.f;
+  const int n = (int)r.count;
+  int done = 0;
+  if (((reinterpret_cast<uintptr_t>(r.p) | reinterpret_cast<uintptr_t>(r.g) | reinterpret_cast<uintptr_t>(r.mbuf) |
+        reinterpret_cast<uintptr_t>(r.ebuf)) & 15) == 0) {
+    const int n4 = n >> 2;
+    done = n4 << 2;
+    auto at = [](float* base, int i) { return reinterpret_cast<float4*>(base) + i; };
+    for (int i0 = threadIdx.x; i0 < n4; i0 += 2 * 256) {
+      float4 p[2], g[2], m[2], e[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = i0 + 256 * u;
+        const bool in = i < n4;
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        p[u] = in ? *at(r.p, i) : z;
+        g[u] = in ? *at(r.g, i) : z;
+        m[u] = in && has_m ? *at(r.mbuf, i) : z;
+        e[u] = in && has_e ? *at(r.ebuf, i) : z;
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = i0 + 256 * u;
+        if (i >= n4) break;
+        tail_element(q, has_m, has_e, p[u].x, g[u].x, m[u].x, e[u].x);
+        tail_element(q, has_m, has_e, p[u].y, g[u].y, m[u].y, e[u].y);
+        tail_element(q, has_m, has_e, p[u].z, g[u].z, m[u].z, e[u].z);
+        tail_element(q, has_m, has_e, p[u].w, g[u].w, m[u].w, e[u].w);
+        *at(r.g, i) = g[u];
+        if (upd) *at(r.p, i) = p[u];
+        if (has_m) *at(r.mbuf, i) = m[u];
+        if (has_e) *at(r.ebuf, i) = e[u];
+      }
     }
-    if (r.ebuf) {
-      g = fmaf(r.ema, g, (1.f - r.ema) * r.ebuf[i]);
-      r.ebuf[i] = g;
-    }
-    g *= r.scale;
+  }
+  for (int i = done + threadIdx.x; i < n; i += 256) {
+    float p = r.p[i], g = r.g[i], m = has_m ? r.mbuf[i] : 0.f, e = has_e ? r.ebuf[i] : 0.f;
+    tail_element(q, has_m, has_e, p, g, m, e);
     r.g[i] = g;
-    if (r.lr != 0.f) r.p[i] = fmaf(-r.lr, g, pv);
+    if (upd) r.p[i] = p;
+    if (has_m) r.mbuf[i] = m;
+    if (has_e) r.ebuf[i] = e;
   }
 }
 
@@ -491,7 +569,26 @@ extern "C" {
 int sso_optimizer_tail(const sso_tail_rec* recs_dev, int n_recs, void* stream) {
   SSO_CHECK_ARG(recs_dev != nullptr && n_recs >= 0, "optimizer_tail: bad argument");
   if (n_recs == 0) return 0;
-  optimizer_tail_kernel<<<n_recs, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(recs_dev);
+  optimizer_tail_kernel<true><<<n_recs, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(recs_dev, TailSets{});
+  SSO_LAUNCH_OK("optimizer_tail_kernel");
+  return 0;
+}
+
+int sso_sample_classes(const float* prob, const float* q, int64_t rows, int64_t classes, int64_t* out, void* stream) {
+  SSO_CHECK_ARG(prob && q && out && rows > 0 && classes > 0, "sample_classes: bad argument");
+  sample_classes_kernel<<<(unsigned)ceil_div64(rows, 8), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(prob, q, rows, classes, out);
+  SSO_LAUNCH_OK("sample_classes_kernel");
+  return 0;
+}
+
+int sso_optimizer_tail_sets(const sso_tail_rec* recs_dev, int n_recs, const sso_tail_set* sets, int n_sets, void* stream) {
+  SSO_CHECK_ARG(recs_dev != nullptr && n_recs >= 0, "optimizer_tail: bad argument");
+  SSO_CHECK_ARG(sets != nullptr && n_sets > 0 && n_sets <= SSO_TAIL_MAX_SETS, "optimizer_tail: %d sets of scalars, at most %d", n_sets,
+                SSO_TAIL_MAX_SETS);
+  if (n_recs == 0) return 0;
+  TailSets all{};
+  for (int i = 0; i < n_sets; ++i) all.s[i] = sets[i];
+  optimizer_tail_kernel<false><<<n_recs, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(recs_dev, all);
   SSO_LAUNCH_OK("optimizer_tail_kernel");
   return 0;
 }

@@ -74,6 +74,9 @@ SIGNATURES = {
                                 c_vp, c_i64, c_vp, c_sz, c_i32, c_vp]),
     'sso_factor_syrk_noalloc': (c_i32, [c_vp, c_i32, c_i64, c_i64, c_i64, c_i64, c_i32, c_vp, c_f32, c_f32,
                                         c_vp, c_i64, c_i32, c_vp]),
+    'sso_factor_op_create': (c_i64, [c_vp, c_i32]),
+    'sso_factor_op_run': (c_i32, [c_i64, c_vp, c_vp, c_f32, c_f32, c_vp, c_sz, c_vp]),
+    'sso_factor_op_destroy': (c_i32, [c_i64]),
     'sso_factor_batch_workspace_bytes': (c_sz, [c_i32, c_vp]),
     'sso_factor_batch': (c_i32, [c_i32, c_vp, c_vp, c_sz, c_vp]),
     'sso_bn_plane_splits': (c_i32, [c_i32, c_i64, c_i64, c_i64, c_i64]),
@@ -108,7 +111,9 @@ SIGNATURES = {
     'sso_plan_num_copy_recs': (c_i32, [c_i64]),
     'sso_plan_copy_copy_recs': (c_i32, [c_i64, c_vp, c_i32]),
     'sso_run_tile_tasks': (c_i32, [c_vp, c_i32, c_i32, c_vp]),
+    'sso_sample_classes': (c_i32, [c_vp, c_vp, c_i64, c_i64, c_vp, c_vp]),
     'sso_optimizer_tail': (c_i32, [c_vp, c_i32, c_vp]),
+    'sso_optimizer_tail_sets': (c_i32, [c_vp, c_i32, c_vp, c_i32, c_vp]),
     'sso_diag_sq_workspace_bytes': (c_sz, [c_i64, c_i64, c_i64]),
     'sso_diag_sq_im2col': (c_i32, [c_vp, c_vp, c_i32] + [c_i64] * 8 + [c_i64] * 5 + [c_i32] * 8 +
                            [c_vp, c_f32, c_f32, c_vp, c_vp, c_vp, c_sz, c_vp]),
@@ -149,8 +154,10 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
+def _stream(_raw=torch._C._cuda_getCurrentRawStream, _device=torch._C._cuda_getDevice):
+    """Handle of the current stream.  Asked for on every launch: torch.cuda.current_stream() builds a
+    Stream object around the same number (3 us against 0.2)."""
+    return _raw(_device())
 
 
 # ---- optional side stream for the curvature kernels of the hooks -----------------------------
@@ -308,7 +315,7 @@ class FactorOp:
     strides, scratch size, output slot) resolved once; the hooks run it ~100 times per step, so
     the per-call Python work is kept to pointer look-ups and one foreign call."""
 
-    __slots__ = ('fn', 'mid', 'out_ptr', 'ldo', 'nbytes', 'device', 'impl', 'flops', 'bytes')
+    __slots__ = ('op', 'run_op', 'mid', 'out_ptr', 'ldo', 'nbytes', 'device', 'flops', 'bytes')
 
     def __init__(self, x: torch.Tensor, kernel_size, stride, padding, dilation, append_ones: bool,
                  out: torch.Tensor, impl: int = IMPL_AUTO):
@@ -326,16 +333,27 @@ class FactorOp:
         assert out.shape == (d, d) and out.dtype == torch.float32 and out.stride(1) == 1, (out.shape, d)
         rows = n * ho * wo
         L = lib()
-        self.fn = L.sso_factor_syrk_im2col
+        self.op = 0
+        self.run_op = L.sso_factor_op_run
         self.mid = (_dtype_code(x), n, c, h, w, sn, sc, sh, sw, kh, kw, stride[0], stride[1],
                     padding[0], padding[1], dilation[0], dilation[1], int(append_ones))
         self.out_ptr, self.ldo = out.data_ptr(), out.stride(0)
         self.nbytes = L.sso_factor_workspace_bytes(rows, d, impl)
-        self.device, self.impl = x.device, impl
+        self.device = x.device
+        desc = FactorDesc()
+        self.fill(desc)
+        self.op = L.sso_factor_op_create(C.byref(desc), impl)
+        if self.op <= 0:
+            _check(int(self.op))
         self.flops = 2.0 * rows * d * d
         self.bytes = x.numel() * x.element_size() + 4 * d * d
 
     def run(self, x: torch.Tensor, weight: Optional[torch.Tensor], alpha: float, beta: float, defer: bool = True):
+        if weight is None and defer:
+            mine = getattr(_collected, 'items', None)
+            if mine is not None:
+                mine.append((self, x, alpha, beta))
+                return
         if _batching and defer and weight is None:
             # wait for the other factors of this pass and go to the device with them in one launch
             if self.out_ptr in _pending_outs:
@@ -348,14 +366,23 @@ class FactorOp:
             a = torch.cuda.Event(enable_timing=True)
             b = torch.cuda.Event(enable_timing=True)
             a.record()
-        rc = self.fn(x.data_ptr(), *self.mid, None if weight is None else weight.data_ptr(), alpha, beta,
-                     self.out_ptr, self.ldo, None if ws is None else ws.data_ptr(),
-                     0 if ws is None else ws.numel(), self.impl, torch.cuda.current_stream().cuda_stream)
+        rc = self.run_op(self.op, x.data_ptr(), None if weight is None else weight.data_ptr(), alpha, beta,
+                         ws.data_ptr(), ws.numel(), _stream())
         if rc < 0:
             _check(rc)
         if FACTOR_TIMING is not None:
             b.record()
             FACTOR_TIMING.append((a, b, self.flops, self.bytes))
+
+    def fill(self, d):
+        """Everything of an sso_factor_desc that does not change between calls."""
+        (d.dtype, d.n, d.c, d.h, d.w, d.sn, d.sc, d.sh, d.sw, d.kh, d.kw, d.stride_h, d.stride_w,
+         d.pad_h, d.pad_w, d.dil_h, d.dil_w, d.append_ones) = self.mid
+        d.out, d.ldo = self.out_ptr, self.ldo
+
+    def __del__(self):
+        if getattr(self, 'op', 0) > 0 and _lib is not None:
+            _lib.sso_factor_op_destroy(self.op)
 
 
 # ---- batched factor construction -------------------------------------------------------------
@@ -397,15 +424,42 @@ def flush_factors():
     items = list(_pending)
     _pending.clear()
     _pending_outs.clear()
+    _launch_factors(items)
+
+
+_collected = threading.local()
+
+
+class collect_factors:
+    """Factor problems of this thread inside the ``with`` block are noted and go to the device in one call
+    at its end, whether batching is on or not: for a caller that holds all inputs of a pass, unmodified."""
+
+    def __enter__(self):
+        self.outer = getattr(_collected, 'items', None)
+        _collected.items = []
+
+    def __exit__(self, kind, value, tb):
+        items, _collected.items = _collected.items, self.outer
+        if kind is None and items:
+            if _pending:
+                flush_factors()
+            outs = [op.out_ptr for op, _, _, _ in items]
+            if len(set(outs)) < len(outs):      # one layer twice in a pass: its problems accumulate, in order
+                for item in items:
+                    _launch_factors([item])
+            else:
+                _launch_factors(items)
+
+
+def _launch_factors(items):
     L = lib()
     key = tuple(id(op) for op, _, _, _ in items)
     ent = _batch_cache.get(key)
     if ent is None:
         arr = (FactorDesc * len(items))()
         for d, (op, x, alpha, beta) in zip(arr, items):
-            (d.dtype, d.n, d.c, d.h, d.w, d.sn, d.sc, d.sh, d.sw, d.kh, d.kw, d.stride_h, d.stride_w,
-             d.pad_h, d.pad_w, d.dil_h, d.dil_w, d.append_ones) = op.mid
-            d.x, d.sample_weight, d.alpha, d.beta, d.out, d.ldo = x.data_ptr(), None, alpha, beta, op.out_ptr, op.ldo
+            op.fill(d)
+            d.x, d.sample_weight = x.data_ptr(), None
         nbytes = L.sso_factor_batch_workspace_bytes(len(items), arr)
         if nbytes == 0:
             _check(-1)
@@ -424,7 +478,7 @@ def flush_factors():
             a = torch.cuda.Event(enable_timing=True)
             b = torch.cuda.Event(enable_timing=True)
             a.record()
-        _check(L.sso_factor_batch(len(items), arr, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
+        _check(L.sso_factor_batch(len(items), arr, ws.data_ptr(), ws.numel(), _stream()))
         if FACTOR_TIMING is not None:
             b.record()
             FACTOR_TIMING.append((a, b, sum(op.flops for op, _, _, _ in items), sum(op.bytes for op, _, _, _ in items)))
@@ -468,6 +522,16 @@ def bn_plane_layout(t: torch.Tensor):
     ok = (st[1] == 1 and t.data_ptr() % 16 == 0 and (st[0] * t.element_size()) % 16 == 0
           and (st[2] * t.element_size()) % 16 == 0)
     return t, st, (splits if ok else 1)
+
+
+def sample_classes(prob: torch.Tensor, q: torch.Tensor) -> torch.Tensor:
+    """[1, n] int64: argmax_c prob[i, c] / q[i, c] of every row, with entries that are negative or not finite
+    counted as zero and rows that then hold nothing as uniform."""
+    _require_cuda(prob, 'probabilities')
+    n, c = prob.shape
+    out = torch.empty((1, n), dtype=torch.int64, device=prob.device)
+    _check(lib().sso_sample_classes(prob.data_ptr(), q.data_ptr(), n, c, out.data_ptr(), _stream()))
+    return out
 
 
 def bn_plane_sums(t: torch.Tensor, is_output: bool, scale, shift, out: torch.Tensor, layout=None) -> int:
@@ -579,26 +643,46 @@ def seg_records(pairs, device, chunk: int = 1 << 14) -> torch.Tensor:
 
 TAIL_REC_DTYPE = np.dtype([('p', np.uint64), ('g', np.uint64), ('mbuf', np.uint64), ('ebuf', np.uint64),
                            ('count', np.int64), ('add', np.float32), ('momentum', np.float32),
-                           ('ema', np.float32), ('scale', np.float32), ('lr', np.float32), ('pad', np.int32)])
+                           ('ema', np.float32), ('scale', np.float32), ('lr', np.float32), ('set', np.int32)])
+TAIL_MAX_SETS = 128
 
 
-def tail_records(items, device, chunk: int = 1 << 15) -> torch.Tensor:
+def tail_records(items, device, chunk: int = 1 << 12) -> torch.Tensor:
     """Device table for sso_optimizer_tail from (p, g, mbuf, ebuf, add, momentum, ema, scale, lr)
     tuples of flat, equally laid out fp32 tensors (mbuf / ebuf may be None)."""
-    recs = []
-    for p, g, mbuf, ebuf, add, momentum, ema, scale, lr in items:
-        n = p.numel()
-        for o in range(0, n, chunk):
-            recs.append((p.data_ptr() + 4 * o, g.data_ptr() + 4 * o,
-                         0 if mbuf is None else mbuf.data_ptr() + 4 * o,
-                         0 if ebuf is None else ebuf.data_ptr() + 4 * o,
-                         min(chunk, n - o), add, momentum, ema, scale, lr, 0))
-    arr = np.array(recs, dtype=TAIL_REC_DTYPE)
-    return torch.from_numpy(arr.view(np.uint8).copy()).to(device)
+    return _tail_table([(p.data_ptr(), g.data_ptr(), 0 if m is None else m.data_ptr(), 0 if e is None else e.data_ptr(),
+                         p.numel(), *scalars, 0) for p, g, m, e, *scalars in items], device, chunk)
+
+
+def tail_set_records(items, device, chunk: int = 1 << 12) -> torch.Tensor:
+    """The same for sso_optimizer_tail_sets from (p, g, mbuf, ebuf, index of the scalars) tuples."""
+    return _tail_table([(p.data_ptr(), g.data_ptr(), 0 if m is None else m.data_ptr(), 0 if e is None else e.data_ptr(),
+                         p.numel(), 0., 0., 0., 0., 0., i) for p, g, m, e, i in items], device, chunk)
+
+
+def _tail_table(rows, device, chunk):
+    whole = np.array(rows, dtype=TAIL_REC_DTYPE)
+    pieces = (whole['count'] + chunk - 1) // chunk
+    arr = np.repeat(whole, pieces)
+    first = np.repeat(np.cumsum(pieces) - pieces, pieces)
+    start = (np.arange(arr.size, dtype=np.int64) - first) * chunk
+    arr['count'] = np.minimum(chunk, arr['count'] - start)
+    for name in ('p', 'g', 'mbuf', 'ebuf'):
+        arr[name] += np.where(arr[name] != 0, 4 * start, 0).astype(np.uint64)
+    return torch.from_numpy(arr.view(np.uint8)).to(device)
 
 
 def optimizer_tail(table: torch.Tensor):
     _check(lib().sso_optimizer_tail(table.data_ptr(), table.numel() // TAIL_REC_DTYPE.itemsize, _stream()))
+
+
+def tail_sets(sets):
+    """Host array of (add, momentum, ema, scale, lr) tuples for optimizer_tail_sets."""
+    return (c_f32 * (5 * len(sets)))(*[v for s in sets for v in s])
+
+
+def optimizer_tail_sets(table: torch.Tensor, sets):
+    _check(lib().sso_optimizer_tail_sets(table.data_ptr(), table.numel() // TAIL_REC_DTYPE.itemsize, sets, len(sets) // 5, _stream()))
 
 
 def copy_segments(table: torch.Tensor, scale: float = 1.0):

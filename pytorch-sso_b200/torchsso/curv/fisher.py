@@ -40,6 +40,11 @@ def sample_targets(prob: torch.Tensor, num_mc: int) -> torch.Tensor:
     # A diverged model produces NaN / all-zero rows, on which the sampling kernel would fail a
     # device-side assertion and take the CUDA context with it: such rows are sampled uniformly
     # instead (the loss is already NaN and says so).
+    if num_mc == 1 and prob.is_cuda and prob.dtype == torch.float32 and prob.dim() == 2 and prob.is_contiguous():
+        # one draw per row is a race of exponential clocks, argmax_c prob_c / q_c with q ~ Exp(1) (what
+        # torch.multinomial does for it, from the same random numbers); one kernel behind the generator
+        # instead of a dozen small ones (110 us of host time for a batch of 16)
+        return nat.sample_classes(prob, torch.empty_like(prob).exponential_())
     prob = torch.nan_to_num(prob, nan=0.0, posinf=0.0, neginf=0.0).clamp_min(0.0)
     dead = prob.sum(dim=1, keepdim=True) <= 0
     prob = torch.where(dead, torch.ones_like(prob), prob)
@@ -53,6 +58,8 @@ def get_closure_for_fisher(optimizer, model, data, target, approx_type=None, num
         raise ValueError('batch_mc_passes needs prune_sampling_pass: the batched walk returns the output '
                          'gradients of the hooked modules instead of running their hooks')
 
+    constant_weight = {}
+
     def set_sampling(on: bool):
         for group in optimizer.param_groups:
             curv = group['curv']
@@ -64,32 +71,46 @@ def get_closure_for_fisher(optimizer, model, data, target, approx_type=None, num
                 for param in group['params']:
                     param.requires_grad = not on
 
-    def sampling_backward(loss, edges):
+    def feed(curvs, grads):
+        """The hooks' work for output gradients that autograd has returned: the factor problems of the pass
+        are only noted, and go to the device together, in one call."""
+        with nat.collect_factors():
+            for curv, g in zip(curvs, grads):
+                if g is not None:
+                    curv.backward_postprocess(curv.module, None, (g,))
+        nat.flush_factors()
+
+    def sampling_backward(loss, curvs, edges):
         if prune_sampling_pass:
-            torch.autograd.grad(loss, edges, retain_graph=True, allow_unused=True)
+            feed(curvs, torch.autograd.grad(loss, edges, retain_graph=True, allow_unused=True))
         else:
             loss.backward(retain_graph=True)
-        # with batched factor construction: this pass's G factors go to the device now, in one launch,
-        # beside whatever the closure does next (the next pass accumulates onto them)
-        nat.flush_factors()
+            nat.flush_factors()
 
     def batched_sampling_backward(output, mc_targets, curvs, edges):
         """All Monte Carlo targets in one walk of the graph, then the hooks' work target by target."""
         losses = torch.stack([F.cross_entropy(output, mc_targets[i]) for i in range(num_mc)])
         seeds = torch.eye(num_mc, device=losses.device, dtype=losses.dtype)
+        grads = torch.autograd.grad(losses, edges, grad_outputs=seeds, is_grads_batched=True,
+                                    retain_graph=True, allow_unused=True)
+        for i in range(num_mc):
+            feed(curvs, [None if g is None else g[i] for g in grads])
+
+    def forward(edges, edge_curvs):
+        """The forward pass.  With pruned sampling passes the hooks only note where the output gradients
+        enter the graph: neither those passes nor the real backward has to call them."""
+        if not prune_sampling_pass:
+            return model(data)
+        curvs = [group['curv'] for group in optimizer.param_groups]
         for curv in curvs:
-            curv.__dict__['_mute_hook'] = True
+            curv._output_edges = []
         try:
-            grads = torch.autograd.grad(losses, edges, grad_outputs=seeds, is_grads_batched=True,
-                                        retain_graph=True, allow_unused=True)
+            return model(data)
         finally:
             for curv in curvs:
-                curv.__dict__['_mute_hook'] = False
-        for i in range(num_mc):
-            for curv, g in zip(curvs, grads):
-                if g is not None:
-                    curv.backward_postprocess(curv.module, None, (g[i],))
-            nat.flush_factors()
+                edges += curv._output_edges
+                edge_curvs += [curv] * len(curv._output_edges)
+                curv._output_edges = None
 
     def closure():
         for group in optimizer.param_groups:
@@ -98,24 +119,20 @@ def get_closure_for_fisher(optimizer, model, data, target, approx_type=None, num
             raise ValueError('Invalid approx type: {}'.format(approx_type))
 
         optimizer.zero_grad()
-        output = model(data)
+        edges, edge_curvs = [], []
+        output = forward(edges, edge_curvs)
         nat.flush_factors()          # batched factor construction: all A factors of the forward pass
         prob = F.softmax(output, dim=1)
-
-        edges, edge_curvs = [], []
-        if prune_sampling_pass:
-            for group in optimizer.param_groups:
-                edge = group['curv'].module.__dict__.pop('output_edge', None)
-                if edge is not None:
-                    edges.append(edge)
-                    edge_curvs.append(group['curv'])
-            if not edges:
-                raise RuntimeError('no hooked module produced an output that requires grad')
+        if prune_sampling_pass and not edges:
+            raise RuntimeError('no hooked module produced an output that requires grad')
 
         set_sampling(True)
         if approx_type == _APPROX_TYPE_MC:
             mc_targets = sample_targets(prob.detach(), num_mc)
-            weight = torch.full_like(prob[:, 0], 1.0 / num_mc).detach()
+            key = (prob.shape[0], prob.dtype, prob.device)
+            weight = constant_weight.get(key)
+            if weight is None:
+                weight = constant_weight[key] = torch.full_like(prob[:, 0], 1.0 / num_mc).detach()
             for group in optimizer.param_groups:
                 group['curv'].prob = weight
                 group['curv'].prob_scale = 1.0 / num_mc
@@ -123,15 +140,17 @@ def get_closure_for_fisher(optimizer, model, data, target, approx_type=None, num
                 batched_sampling_backward(output, mc_targets, edge_curvs, edges)
             else:
                 for i in range(num_mc):
-                    sampling_backward(F.cross_entropy(output, mc_targets[i]), edges)
+                    sampling_backward(F.cross_entropy(output, mc_targets[i]), edge_curvs, edges)
         else:
             for i in range(model.num_classes):
                 weight = prob[:, i].detach().float().contiguous()
                 for group in optimizer.param_groups:
                     group['curv'].prob = weight
                     group['curv'].prob_scale = None
-                sampling_backward(F.cross_entropy(output, torch.full_like(target, i)), edges)
+                sampling_backward(F.cross_entropy(output, torch.full_like(target, i)), edge_curvs, edges)
         set_sampling(False)
+        for curv in edge_curvs:
+            curv.update_in_backward(None)       # what the hooks do in the real backward: close the accumulation
         del edges, edge_curvs
         # every G factor is complete now; the real backward below only produces gradients.  An optimizer
         # with early_inverse set starts its round of inverses here, beside that backward pass.

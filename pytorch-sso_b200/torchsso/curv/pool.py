@@ -69,6 +69,8 @@ class FactorPool:
         self.d_total = off
         self._plans = {}
         self._damp = {}
+        self._mats = {}
+        self._ranges = {}
         self.last_info: Optional[torch.Tensor] = None
         for c in list(self.kron) + list(self.diag):
             c._pool = self
@@ -87,20 +89,38 @@ class FactorPool:
         return (role + ':' + kind) in self._bufs
 
     def mat(self, role: str, curv, which: int) -> torch.Tensor:
-        a_off, da, g_off, dg = self.k_off[id(curv)]
-        off, d = (a_off, da) if which == 0 else (g_off, dg)
-        ld = _ld(d)
-        m = self.buf(role)[off: off + d * ld].view(d, ld)
-        return m if ld == d else m[:, :d]
+        key = (role, id(curv), which)
+        m = self._mats.get(key)
+        if m is None:
+            a_off, da, g_off, dg = self.k_off[id(curv)]
+            off, d = (a_off, da) if which == 0 else (g_off, dg)
+            ld = _ld(d)
+            m = self.buf(role)[off: off + d * ld].view(d, ld)
+            m = self._mats[key] = m if ld == d else m[:, :d]
+        return m
 
     def vec(self, role: str, curv, j: int) -> torch.Tensor:
-        off, shape = self.d_off[id(curv)][j]
-        return self.buf(role, 'd')[off: off + int(math.prod(shape))].view(shape)
+        key = (role, id(curv), j, 'd')
+        v = self._mats.get(key)
+        if v is None:
+            off, shape = self.d_off[id(curv)][j]
+            v = self._mats[key] = self.buf(role, 'd')[off: off + int(math.prod(shape))].view(shape)
+        return v
+
+    def _remembered(self, kind: str, curvs: Sequence, find):
+        key = (kind, *map(id, curvs))
+        r = self._ranges.get(key)
+        if r is None:
+            if len(self._ranges) >= 256:
+                self._ranges.clear()
+            r = self._ranges[key] = find(curvs)
+        return r
 
     def kron_range(self, curvs: Sequence):
         """[lo, hi) element range of the pool covered by `curvs` (must be contiguous in layout)."""
-        if not curvs:
-            return 0, 0
+        return self._remembered('k', curvs, self._find_kron_range) if curvs else (0, 0)
+
+    def _find_kron_range(self, curvs):
         idx = sorted(self.kron.index(c) for c in curvs)
         assert idx == list(range(idx[0], idx[-1] + 1)), 'curvatures are not contiguous in the pool'
         lo = self.k_off[id(self.kron[idx[0]])][0]
@@ -108,8 +128,10 @@ class FactorPool:
         return lo, hi
 
     def diag_range(self, curvs: Sequence):
-        if not curvs:
-            return 0, 0
+        """The same for the diagonal pool."""
+        return self._remembered('d', curvs, self._find_diag_range) if curvs else (0, 0)
+
+    def _find_diag_range(self, curvs):
         idx = sorted(self.diag.index(c) for c in curvs)
         assert idx == list(range(idx[0], idx[-1] + 1)), 'curvatures are not contiguous in the pool'
         lo = self.d_off[id(self.diag[idx[0]])][0][0]

@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import math
 from collections import OrderedDict
+from operator import itemgetter
 from typing import List
 
 import numpy as np
@@ -26,6 +27,10 @@ from torchsso.curv.pool import FactorPool
 from torchsso.utils import TensorAccumulator
 
 _NORM_TYPES = (nn.BatchNorm1d, nn.BatchNorm2d, nn.BatchNorm3d)
+
+
+_TAIL_SETTINGS = itemgetter('lars', 'l2_reg', 'weight_decay', 'momentum', 'momentum_type', 'grad_ema_decay', 'grad_ema_type',
+                            'bias_correction', 'lr')
 
 
 def _is_pooled(curv) -> bool:
@@ -143,12 +148,15 @@ class SecondOrderOptimizer(Optimizer):
         rest = [g for g in groups if id(g) not in taken]
         self.pool = FactorPool([g['curv'] for g in kron], [g['curv'] for g in diag], device)
         # flat fp32 gradient buffer: Kronecker layers, then diagonal layers in the diagonal
-        # pool's own element order, then everything else
+        # pool's own element order, then everything else.  Each Kronecker parameter starts on 256 bytes,
+        # so that the tile tasks and the update kernel can move it in 16-byte pieces whatever came before it.
         views, off = OrderedDict(), 0
         for g in kron:
             for p in g['params']:
+                off = (off + 63) // 64 * 64
                 views[p] = (off, p.numel())
                 off += p.numel()
+        off = (off + 63) // 64 * 64
         self._diag_grad_base = off
         for g in diag:
             for p in g['params']:
@@ -220,8 +228,7 @@ class SecondOrderOptimizer(Optimizer):
     def _after_sampling_passes(self):
         if not (self.early_inverse and self.update_inv):
             return
-        kc = [g['curv'] for g in self.local_param_groups
-              if isinstance(g['curv'], _KronFactors) and _is_pooled(g['curv'])]
+        kc = self._split_groups(self.local_param_groups)[5]
         if not kc:
             return
         nat.flush_factors()
@@ -262,18 +269,18 @@ class SecondOrderOptimizer(Optimizer):
         dsts, srcs = [], []
         for p, v in self._grad_view.items():
             g = p.grad
+            if g is v:
+                continue
             if g is None:
                 v.zero_()
-            elif g.data_ptr() != v.data_ptr() or g.dtype != torch.float32:
-                dsts.append(v)
-                srcs.append(g)
-            if g is not v:
+            else:
+                if g.data_ptr() != v.data_ptr() or g.dtype != torch.float32:
+                    dsts.append(v)
+                    srcs.append(g)
                 p.grad = None
+            p.grad = v
         if dsts:
             torch._foreach_copy_(dsts, srcs)
-        for p, v in self._grad_view.items():
-            if p.grad is None:
-                p.grad = v
 
     def _accumulate(self, scale: float):
         if self._grad_acc is None:
@@ -351,9 +358,24 @@ class SecondOrderOptimizer(Optimizer):
 
     def _fused_tail(self, groups, target, stage):
         """torchsso/optim/secondorder.py:225-283 for all eligible groups in one kernel launch.
-        Returns the ids of the groups it handled."""
+        Returns the ids of the groups it handled.  The device table (addresses) and the sets of scalars are
+        kept: the table until a tensor moves, the scalars until a setting changes."""
         raw = stage == 'raw'
-        items, key, handled = [], [], set()
+        cache = self.__dict__.setdefault('_tail_tables', {})
+        ent = cache.get((target, stage))
+        params = [p for g in groups for p in g[target]]
+        key = ([p.data_ptr() for p in params], [id(p.grad) for p in params], [_TAIL_SETTINGS(g) for g in groups], id(self.state))
+        if ent is None or ent['key'] != key or ent['per_step']:
+            ent = cache[(target, stage)] = self._tail_entry(groups, target, raw, key, ent)
+        for curv, l2 in ent['l2']:
+            curv.l2_reg = l2
+        if ent['table'] is not None:
+            nat.optimizer_tail_sets(ent['table'], ent['sets'])
+        return ent['handled']
+
+    def _tail_entry(self, groups, target, raw, key, old):
+        stage = 'raw' if raw else 'preconditioned'
+        items, rows, handled, sets, l2, per_step = [], [], set(), {}, [], False
         for group in groups:
             if group['lars']:
                 continue                      # needs per-tensor norms: multi-tensor path
@@ -372,47 +394,57 @@ class SecondOrderOptimizer(Optimizer):
                 if getattr(curv, 'use_sqrt_ema', False):
                     bc2 = math.sqrt(bc2)
                 scale = bc2 / bc1
+                per_step = True
             lr = 0.0 if raw else group['lr']
             handled.add(id(group))
             if raw and group['l2_reg'] != 0 and group['curv'] is not None:
-                group['curv'].l2_reg = group['l2_reg']
+                l2.append((group['curv'], group['l2_reg']))
             if raw and add == 0 and not use_m and not use_e:
                 continue                      # nothing to apply at this stage
+            scalars = (float(add), float(group['momentum']), float(group['grad_ema_decay']), float(scale), float(lr))
+            if len(sets) == nat.TAIL_MAX_SETS and scalars not in sets:
+                handled.discard(id(group))    # more distinct settings than one launch carries: multi-tensor path
+                continue
+            index = sets.setdefault(scalars, len(sets))
             for p in params:
                 st = self.state[p]
                 items.append((p.data, p.grad, st['momentum_buffer'] if use_m else None,
-                              st['grad_ema_buffer'] if use_e else None, float(add), float(group['momentum']),
-                              float(group['grad_ema_decay']), float(scale), float(lr)))
-                key.append((p.data.data_ptr(), p.grad.data_ptr(), use_m, use_e, add, group['momentum'],
-                            group['grad_ema_decay'], scale, lr))
+                              st['grad_ema_buffer'] if use_e else None, index))
+                rows.append((p.data_ptr(), p.grad.data_ptr(), *[0 if b is None else b.data_ptr() for b in items[-1][2:4]], index))
+        table = None
         if items:
-            cache = self.__dict__.setdefault('_tail_tables', {})
-            ent = cache.get((target, stage))
-            key = tuple(key)
-            if ent is None or ent[0] != key:
-                ent = (key, nat.tail_records(items, items[0][0].device))
-                cache[(target, stage)] = ent
-            nat.optimizer_tail(ent[1])
-        return handled
+            table = old['table'] if old is not None and old['rows'] == rows else nat.tail_set_records(items, items[0][0].device)
+        # the gradients are kept: their ids are part of the key
+        return {'key': key, 'grads': [it[1] for it in items], 'per_step': per_step, 'handled': handled, 'l2': l2, 'rows': rows,
+                'table': table, 'sets': nat.tail_sets(sets) if sets else None}
+
+    def _split_groups(self, groups):
+        """What never changes about a list of groups: its pooled curvatures by kind and the gradient views of
+        the Kronecker layers."""
+        ent = self.__dict__.get('_split')
+        if ent is None or ent[0] is not groups or ent[1] != len(groups):
+            pooled = [g for g in groups if g['curv'] is not None and _is_pooled(g['curv'])]
+            kron = [g for g in pooled if isinstance(g['curv'], _KronFactors)]
+            diag = [g for g in pooled if isinstance(g['curv'], _DiagBatchNorm)]
+            rest = [g for g in groups if g['curv'] is not None and not _is_pooled(g['curv'])]
+            grads = [[self._grad_view[p] for p in g['params']] for g in kron]
+            ent = self.__dict__['_split'] = (groups, len(groups), [g['curv'] for g in pooled], kron, diag, rest, grads,
+                                             [g['curv'] for g in kron], [g['curv'] for g in diag])
+        return ent[2:]
 
     def _curvature_step(self, groups, target, update_inv, update_std):
-        pooled = [g for g in groups if g['curv'] is not None and _is_pooled(g['curv'])]
-        kron = [g for g in pooled if isinstance(g['curv'], _KronFactors)]
-        diag = [g for g in pooled if isinstance(g['curv'], _DiagBatchNorm)]
-        curvs = [g['curv'] for g in pooled]
+        curvs, kron, diag, others, kron_grads, kc, dc = self._split_groups(groups)
         uniform = len({(c.ema_decay, 'ema' in c._have) for c in curvs}) <= 1
-        if pooled and uniform:
+        if curvs and uniform:
             firsts = [c._ema_bookkeeping() for c in curvs]
             if not self.fuse_ema:        # else the hooks' kernels have already written the average
-                self.pool.update_ema(curvs[0].ema_decay, firsts[0], [g['curv'] for g in kron],
-                                     [g['curv'] for g in diag])
+                self.pool.update_ema(curvs[0].ema_decay, firsts[0], kc, dc)
             for c in curvs:
                 c._have.add('ema')
         else:
             for c in curvs:
                 c.update_ema()
         early = self.__dict__.pop('_early_inverse_done', False)     # consumed by this step whatever it does
-        kc = [g['curv'] for g in kron]
         if kc:
             want_std = [bool(update_std(g)) if update_std else False for g in kron]
             if update_inv:
@@ -423,10 +455,8 @@ class SecondOrderOptimizer(Optimizer):
                     if any(want_std):
                         c._have.add('std')
             if self.precondition_grad or target != 'params':
-                grads = [[self._grad_view[p] for p in g['params']] for g in kron]
-                self.pool.precondition(kc, grads)
+                self.pool.precondition(kc, kron_grads)
         if diag:
-            dc = [g['curv'] for g in diag]
             lo, hi = self.pool.diag_range(dc)
             gflat = None
             if self.precondition_grad or target != 'params':
@@ -446,10 +476,8 @@ class SecondOrderOptimizer(Optimizer):
                     c._have.add('inv')
                     if update_std and update_std(g):
                         c.update_std()
-        for g in groups:
+        for g in others:
             curv = g['curv']
-            if curv is None or _is_pooled(curv):
-                continue
             curv.step(update_inv=bool(update_inv),
                       update_std=bool(update_std(g)) if update_std else False)
             if self.precondition_grad or target != 'params':

@@ -35,12 +35,14 @@ namespace sso {
 int factor_tma_set_wait_controls(long long cycles, int stall);
 int factor_tc_set_wait_controls(long long cycles, int stall);
 int engine_tc_set_wait_controls(long long cycles, int stall);
+int factor_f32_set_wait_controls(long long cycles, int stall);
 static long long g_wait_kcycles = 0;   // 0 = default limit
 static int g_stall = 0;
 static int apply_wait_controls() {
   const long long cycles = g_wait_kcycles * 1024;
   int rc = factor_tma_set_wait_controls(cycles, g_stall);
   if (!rc) rc = factor_tc_set_wait_controls(cycles, 0);
+  if (!rc) rc = factor_f32_set_wait_controls(cycles, 0);
   if (!rc) rc = engine_tc_set_wait_controls(cycles, g_stall);
   return rc;
 }
@@ -49,6 +51,11 @@ int factor_simt_launch(FactorParams p, int dtype, void* workspace, size_t worksp
 size_t factor_tc_workspace_bytes(int64_t rows, int64_t d);
 bool factor_tc_supported(const FactorParams& p, int dtype);
 int factor_tc_launch(FactorParams p, int dtype, void* workspace, size_t workspace_bytes, cudaStream_t st);
+bool factor_direct_supported(const FactorParams& p, int dtype);
+int factor_direct_launch(const FactorParams& p, int dtype, cudaStream_t st);
+bool factor_f32_supported(const FactorParams& p, size_t workspace_bytes);
+size_t factor_f32_workspace_bytes(const FactorParams& p);
+int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, cudaStream_t st);
 void factor_tc_set_flush(int stages);
 int factor_tc_flush_setting();
 bool factor_tma_supported(const FactorParams& p, int dtype);
@@ -138,19 +145,33 @@ static int make_factor_params(const void* x, int64_t n, int64_t c, int64_t h, in
 
 static int launch_one_factor(const FactorParams& p, int dtype, void* workspace, size_t workspace_bytes, int impl,
                              cudaStream_t st) {
+  if (impl == SSO_IMPL_AUTO && g_tc_auto && factor_direct_supported(p, dtype)) return factor_direct_launch(p, dtype, st);
   if (impl == SSO_IMPL_TMA) {
     SSO_CHECK_ARG(factor_tma_supported(p, dtype), "factor: shape not supported by the TMA-fed tcgen05 path");
     return factor_tma_launch(p, dtype, workspace, workspace_bytes, factor_tc_flush_setting(), st);
   }
   if (impl == SSO_IMPL_AUTO && g_tc_auto && g_tma_auto && factor_tma_supported(p, dtype))
     return factor_tma_launch(p, dtype, workspace, workspace_bytes, factor_tc_flush_setting(), st);
-  if (impl == SSO_IMPL_TCGEN05) {
+  if (dtype == SSO_F32 && (impl == SSO_IMPL_TCGEN05 || (impl == SSO_IMPL_AUTO && g_tc_auto))) {
+    const bool fits = factor_f32_supported(p, workspace ? workspace_bytes : 0);
+    // asked for by name, the tensor-core path takes what it can gather without changing the layout
+    if (impl == SSO_IMPL_TCGEN05)
+      SSO_CHECK_ARG(p.sc == 1 && fits, "factor: shape not supported by the tcgen05 path, or scratch too small (%zu bytes)", workspace_bytes);
+    if (fits) return factor_f32_launch(p, workspace, workspace_bytes, st);
+  } else if (impl == SSO_IMPL_TCGEN05) {
     SSO_CHECK_ARG(factor_tc_supported(p, dtype), "factor: shape not supported by the tcgen05 path");
     return factor_tc_launch(p, dtype, workspace, workspace_bytes, st);
-  }
-  if (impl == SSO_IMPL_AUTO && g_tc_auto && factor_tc_supported(p, dtype))
+  } else if (impl == SSO_IMPL_AUTO && g_tc_auto && factor_tc_supported(p, dtype)) {
     return factor_tc_launch(p, dtype, workspace, workspace_bytes, st);
+  }
   return factor_simt_launch(p, dtype, workspace, workspace_bytes, st);
+}
+
+// Scratch that lets a problem run at its best (the minimum is sso_factor_workspace_bytes).
+static size_t preferred_bytes(const FactorParams& p, int dtype, int impl) {
+  size_t b = sso_factor_workspace_bytes(p.rows, p.d, impl);
+  if (dtype == SSO_F32 && impl != SSO_IMPL_SIMT) b = std::max(b, factor_f32_workspace_bytes(p));
+  return b;
 }
 
 int sso_factor_syrk_im2col(const void* x, int dtype, int64_t n, int64_t c, int64_t h, int64_t w,
@@ -172,13 +193,22 @@ struct PreparedFactor {
   int dtype, impl;
 };
 
+static int desc_params(const sso_factor_desc& q, FactorParams& p) {
+  const float dummy = 0.f;      // descriptions of prepared calls carry no input
+  return make_factor_params(q.x ? q.x : &dummy, q.n, q.c, q.h, q.w, q.sn, q.sc, q.sh, q.sw, q.kh, q.kw, q.stride_h, q.stride_w, q.pad_h,
+                            q.pad_w, q.dil_h, q.dil_w, q.append_ones, q.sample_weight, q.alpha, q.beta, q.out, q.ldo, p);
+}
+
+size_t sso_factor_desc_workspace_bytes(const sso_factor_desc* q, int impl) {
+  FactorParams p;
+  if (q == nullptr || desc_params(*q, p) != 0) return 0;
+  return preferred_bytes(p, q->dtype, impl);
+}
+
 int64_t sso_factor_op_create(const sso_factor_desc* q, int impl) {
   SSO_CHECK_ARG(q != nullptr, "factor op: null description");
   PreparedFactor f;
-  const float dummy = 0.f;      // the input's address comes with every call
-  const int rc = make_factor_params(q->x ? q->x : &dummy, q->n, q->c, q->h, q->w, q->sn, q->sc, q->sh, q->sw, q->kh, q->kw,
-                                    q->stride_h, q->stride_w, q->pad_h, q->pad_w, q->dil_h, q->dil_w, q->append_ones, nullptr, 0.f,
-                                    0.f, q->out, q->ldo, f.p);
+  const int rc = desc_params(*q, f.p);
   if (rc) return rc;
   f.dtype = q->dtype; f.impl = impl;
   return reinterpret_cast<int64_t>(new PreparedFactor(f));
@@ -205,9 +235,8 @@ static int batch_params(int n, const sso_factor_desc* descs, std::vector<FactorP
   dts.resize(n);
   for (int i = 0; i < n; ++i) {
     const sso_factor_desc& q = descs[i];
-    const int rc = make_factor_params(q.x, q.n, q.c, q.h, q.w, q.sn, q.sc, q.sh, q.sw, q.kh, q.kw, q.stride_h, q.stride_w,
-                                      q.pad_h, q.pad_w, q.dil_h, q.dil_w, q.append_ones, q.sample_weight, q.alpha, q.beta,
-                                      q.out, q.ldo, ps[i]);
+    SSO_CHECK_ARG(q.x != nullptr, "factor: null pointer");
+    const int rc = desc_params(q, ps[i]);
     if (rc) return rc;
     dts[i] = q.dtype;
   }
@@ -221,7 +250,7 @@ size_t sso_factor_batch_workspace_bytes(int n, const sso_factor_desc* descs) {
   std::vector<int> dts;
   if (batch_params(n, descs, ps, dts) != 0) return 0;
   size_t single = 0;
-  for (int i = 0; i < n; ++i) single = std::max(single, sso_factor_workspace_bytes(ps[i].rows, ps[i].d, SSO_IMPL_AUTO));
+  for (int i = 0; i < n; ++i) single = std::max(single, preferred_bytes(ps[i], dts[i], SSO_IMPL_AUTO));
   const size_t batched = (g_tc_auto && g_tma_auto) ? factor_batch_scratch_bytes(ps.data(), dts.data(), n) : 256;
   return align256(batched) + align256(single);
 }

@@ -1,0 +1,851 @@
+// Kronecker-factor construction from fp32 inputs on the tensor cores (three-way bf16 split, fused im2col gather).
+//
+//   partial[tile][split] = sum over this split's rows r of  w_r u_r[I] u_r[J]^T
+//
+// x = hi + mid + lo in bf16, exact to fp32's 24 bits; the six products down to 2^-16 (lo*hi, hi*lo, mid*mid, mid*hi,
+// hi*mid, hi*hi; what is dropped is below 2^-24) go into one TMEM accumulator that is drained into fp32 registers
+// every FLUSH stages (the tensor core's own running sum truncates).  Two kernels:
+//
+// split_kernel writes the three parts of the input once, as pixel rows [part][pixel][C8] of 16-bit values with the
+// channels padded to a multiple of eight (a 1x1 window's ones column is one of them).  Every activation is converted
+// once instead of once per kernel position and tile, and whatever layout the input has (NCHW, odd channel counts,
+// unaligned rows) the gather sees 16-byte chunks of channels.  Bound: memory, 4 bytes in and 6 out per element.
+//
+// factor_f32_kernel gathers im2col rows of the parts with cp.async straight into the operand layout (MN-major
+// SWIZZLE_128B: 64 columns = 128 bytes of one row, zero-filled outside the image), in one of two shapes:
+//   PAIR   a cluster of two CTAs computes a 256x256 block with tcgen05.mma.cta_group::2; each CTA gathers the
+//          128 columns of either side that its half of the operands needs (factors wider than 128);
+//   single one CTA, one 128x128 tile (narrow factors, where a pair would compute padding).
+// Bound: the copies.  Per stage of 32 rows the twelve MMAs of a pair take 1536 cycles per SM (0.98 us as measured with
+// the gather taken out); 48 KB of parts per stage come in at 1.4 us whatever the number of stages in flight, MMAs or
+// not (5 TB/s over the chip: what the load/store path of an SM keeps outstanding).  Columns of a 5x5 window over 64
+// channels, d = 1601 from 65536 rows: 1.13 ms against 1.81 ms for 3xTF32 on 128x128 tiles, d = 4608 from 8192 rows
+// 1.06 against 1.71 ms.  Measured alternatives: splitting in the gather warps is bound by their instructions (650 per
+// warp and stage, 2.3 us per stage, in bf16 as in 3xTF32), and 32-bit MN-major operands are read at half the rate.
+// The input is processed in runs of whole images whose parts fit the scratch; each run adds to the partial tiles of
+// the one before.
+// Partial tiles, tickets and the finishing kernels are those of the other factor kernels.
+#include <algorithm>
+
+#include "common.cuh"
+#include "factor_finish.cuh"
+#include "factor_params.cuh"
+#include "tc_pair.cuh"
+
+namespace sso {
+
+int factor_tc_run_reduce(const FactorParams& p, int tiles, cudaStream_t st);
+
+namespace f32 {
+
+using namespace tc;
+
+constexpr int TILE = 128, KS = 32, STAGES = 4, LAG = 2, FLUSH = 2;
+// five warpgroups: 0-1 accumulate (128 sums per thread of a pair), 2 issues the MMAs (one thread), 3-4 gather; they
+// share the block's 640 x 96 registers as 168 + 168 + 24 + 56 + 56 per thread
+constexpr int EPI_WARPS = 8, MMA_WARP = 8, LOAD_WARP0 = 12, LOAD_WARPS = 8;
+constexpr int THREADS = 640;
+constexpr uint32_t BLK = KS * 128u;              // 64 columns of one stage, one part
+constexpr uint32_t OPB = 2 * BLK;                // 128 columns
+constexpr uint32_t SIDE = 3 * OPB;               // hi mid lo
+constexpr uint32_t SLOT_BYTES = 2 * SIDE;        // both sides
+constexpr size_t SMEM = STAGES * SLOT_BYTES + 1024;
+
+struct Parts {
+  const __nv_bfloat16* a;      // hi part of the (weighted) row side, the other two `stride` elements apart
+  const __nv_bfloat16* b;      // of the column side; equal to a without weights
+  int64_t stride;
+  int c8;                      // channels per pixel, a multiple of eight
+};
+
+// two fp32 values -> their parts, packed (first value in the low half)
+__device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  auto pack = [](float a, float b) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
+  };
+  hi = pack(x, y);
+  x -= __uint_as_float(hi << 16); y -= __uint_as_float(hi & 0xFFFF0000u);
+  mid = pack(x, y);
+  x -= __uint_as_float(mid << 16); y -= __uint_as_float(mid & 0xFFFF0000u);
+  lo = pack(x, y);
+}
+
+// First kernel of a factor: let the next one set itself up meanwhile (it waits for this one's end before it touches
+// memory), clear the status word and the tickets that it will use.
+__device__ __forceinline__ void begin_factor(const FactorParams& p, int header_words) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (blockIdx.x == 0 && blockIdx.y == 0)
+    for (int i = threadIdx.x; i < header_words; i += blockDim.x) p.status[i] = 0;
+}
+
+// A CTA turns 32 pixels x 64 channels: read with the lanes along whichever of the two is contiguous, staged in shared
+// memory, written as 16-byte chunks of eight channels.  With few channels the kernel's columns are folded into them:
+// channel kx*c + ch of pixel (y, ox) is x[ch][y][ox*stride + kx*dil - pad], so that three channels under a 7x7 window
+// are 7 x 24 columns and not 49 x 8.
+__global__ void __launch_bounds__(256) split_kernel(const FactorParams p, uint32_t pixels, int width, int fold, int ones_at, int header_words,
+                                                    Parts out_a, Parts out_b) {
+  __shared__ __align__(16) float t[32][68];
+  begin_factor(p, header_words);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t px0 = blockIdx.x * 32u;
+  const int c0 = blockIdx.y * 64;
+  const float* x = reinterpret_cast<const float*>(p.x);
+  const int hw = p.h * width;      // pixels of an image
+  auto offset = [&](uint32_t px) {
+    const uint32_t n = px / (uint32_t)hw;
+    const int rem = (int)(px - n * hw), y = rem / width;
+    return n * p.sn + y * p.sh + (rem - y * width) * p.sw;
+  };
+  if (fold) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t px = px0 + lane;
+      const int cf = c0 + warp + 8 * i, kx = cf / p.c, ch = cf - kx * p.c;
+      float v = 0.f;
+      if (px < pixels && kx < fold) {
+        const uint32_t n = px / (uint32_t)hw;
+        const int rem = (int)(px - n * hw), y = rem / width, ix = (rem - y * width) * p.stride_w + kx * p.dil_w - p.pad_w;
+        if ((unsigned)ix < (unsigned)p.w) v = __ldg(x + n * p.sn + y * p.sh + ix * p.sw + ch * p.sc);
+      }
+      t[lane][warp + 8 * i] = v;
+    }
+  } else if (p.sc <= (p.w > 1 ? p.sw : p.h > 1 ? p.sh : p.sn)) {      // lanes along the channels
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t px = px0 + warp + 8 * i;
+      if (px >= pixels) break;
+      const float* row = x + offset(px);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int c = c0 + lane + 32 * u;
+        t[warp + 8 * i][lane + 32 * u] = c < p.c ? __ldg(row + c * p.sc) : (c == ones_at ? 1.f : 0.f);
+      }
+    }
+  } else {                         // lanes along the pixels
+    const uint32_t px = px0 + lane;
+    const float* col = x + (px < pixels ? offset(px) : 0);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int c = c0 + warp + 8 * i;
+      t[lane][warp + 8 * i] = c < p.c ? (px < pixels ? __ldg(col + c * p.sc) : 0.f) : (c == ones_at ? 1.f : 0.f);
+    }
+  }
+  __syncthreads();
+  const int r = tid >> 3, o = (tid & 7) * 8;
+  const uint32_t px = px0 + r;
+  if (px >= pixels || c0 + o >= out_a.c8) return;
+  const float w = p.weight ? p.weight[px / hw] : 1.f;
+  for (int side = 0; side < (p.weight ? 2 : 1); ++side) {
+    const float f = side == 0 ? w : 1.f;
+    uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float4 v = *reinterpret_cast<const float4*>(&t[r][o + 4 * i]);
+      split2(f * v.x, f * v.y, hi[2 * i], mid[2 * i], lo[2 * i]);
+      split2(f * v.z, f * v.w, hi[2 * i + 1], mid[2 * i + 1], lo[2 * i + 1]);
+    }
+    __nv_bfloat16* d = const_cast<__nv_bfloat16*>(side == 0 ? out_a.a : out_b.b) + (int64_t)px * out_a.c8 + c0 + o;
+    *reinterpret_cast<uint4*>(d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(d + out_a.stride) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+    *reinterpret_cast<uint4*>(d + 2 * out_a.stride) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+}
+
+// The same where the channels are contiguous, 16-byte aligned and a multiple of four: a thread takes eight channels of
+// a pixel straight from global memory to global memory.
+__global__ void __launch_bounds__(256) split_direct_kernel(const FactorParams p, uint32_t pixels, int ones_at, int header_words, Parts out_a, Parts out_b) {
+  begin_factor(p, header_words);
+  const int oct = out_a.c8 / 8, hw = p.h * p.w;
+  const uint32_t i = blockIdx.x * 256u + threadIdx.x, px = i / (uint32_t)oct;
+  if (px >= pixels) return;
+  const int c = (int)(i - px * oct) * 8;
+  const uint32_t n = px / (uint32_t)hw;
+  const int rem = (int)(px - n * hw), y = rem / p.w;
+  const float* src = reinterpret_cast<const float*>(p.x) + (n * p.sn + y * p.sh + (rem - y * p.w) * p.sw + c);
+  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 u = c < p.c ? __ldg(reinterpret_cast<const float4*>(src)) : z, v = c + 4 < p.c ? __ldg(reinterpret_cast<const float4*>(src) + 1) : z;
+  if (ones_at == c) u.x = 1.f;      // a multiple of four, so the first of either half
+  if (ones_at == c + 4) v.x = 1.f;
+  const float w = p.weight ? p.weight[n] : 1.f;
+  for (int side = 0; side < (p.weight ? 2 : 1); ++side) {
+    const float f = side == 0 ? w : 1.f;
+    uint32_t hi[4], mid[4], lo[4];
+    split2(f * u.x, f * u.y, hi[0], mid[0], lo[0]);
+    split2(f * u.z, f * u.w, hi[1], mid[1], lo[1]);
+    split2(f * v.x, f * v.y, hi[2], mid[2], lo[2]);
+    split2(f * v.z, f * v.w, hi[3], mid[3], lo[3]);
+    __nv_bfloat16* d = const_cast<__nv_bfloat16*>(side == 0 ? out_a.a : out_b.b) + (int64_t)px * out_a.c8 + c;
+    *reinterpret_cast<uint4*>(d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(d + out_a.stride) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+    *reinterpret_cast<uint4*>(d + 2 * out_a.stride) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+}
+
+// The loads of one thread: 16-byte chunk l8 of the four 64-column blocks (A0 A1 B0 B1) of one row of every stage; a warp
+// instruction covers four rows of one block and part, i.e. four whole lines.
+struct Gather {
+  int koff[4];             // element offset of this thread's chunk in block b
+  int kpos[4];             // kernel position dh | dw << 16; -1: the ones column; -2: nothing
+  int left;                // rows of the split that remain from this one on (<= 0: past the end)
+  int n, y, x;             // image and output pixel
+
+  __device__ __forceinline__ void init(const FactorParams& p, int col_a, int col_b, int64_t r_begin, int rows, int k, int l8) {
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int j0 = (b < 2 ? col_a : col_b) + (b & 1) * 64 + l8 * 8;
+      koff[b] = 0;
+      kpos[b] = (j0 == p.dcols && j0 < p.d) ? -1 : -2;
+      if (j0 < p.dcols) {
+        const int pos = j0 / p.c, c0 = j0 - pos * p.c;
+        const int ky = pos / p.kw, kx = pos - ky * p.kw;
+        const int dh = ky * p.dil_h, dw = kx * p.dil_w;
+        koff[b] = (int)(dh * p.sh + dw * p.sw) + c0;
+        kpos[b] = dh | (dw << 16);
+      }
+    }
+    const int hw = p.ho * p.wo;
+    left = rows - k;
+    const int64_t r = r_begin + k;
+    n = (int)(r / hw);
+    const int rem = (int)(r - (int64_t)n * hw);
+    y = rem / p.wo;
+    x = rem - y * p.wo;
+  }
+  // copies of this row of one stage, then on to the row 32 further
+  __device__ __forceinline__ void stage(const FactorParams& p, const Parts& q, uint32_t dst, uint32_t blocks, bool no_halo, int step_n, int step_y, int step_x) {
+    const bool rvalid = left > 0;
+    const int ih = y * p.stride_h - p.pad_h, iw = x * p.stride_w - p.pad_w;
+    const int64_t pix = n * p.sn + ih * p.sh + iw * p.sw;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      if (!((blocks >> b) & 1u)) continue;
+      const int kp = kpos[b];
+      const uint32_t d = dst + (b >> 1) * SIDE + (b & 1) * BLK;
+      if (kp == -1) {
+#pragma unroll
+        for (int t = 0; t < 3; ++t)
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%2,%2};" ::"r"(d + t * OPB), "r"(t == 0 && rvalid ? 0x3F80u : 0u), "r"(0u) : "memory");
+        continue;
+      }
+      bool in = rvalid && kp >= 0;
+      if (!no_halo) in = in && (unsigned)(ih + (kp & 0xFFFF)) < (unsigned)p.h && (unsigned)(iw + (kp >> 16)) < (unsigned)p.w;
+      const __nv_bfloat16* src = (b < 2 ? q.a : q.b) + (in ? pix + koff[b] : 0);
+      const int bytes = in ? 16 : 0;
+#pragma unroll
+      for (int t = 0; t < 3; ++t)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d + t * OPB), "l"(src + t * q.stride), "r"(bytes) : "memory");
+    }
+    left -= KS;
+    x += step_x;
+    if (x >= p.wo) { x -= p.wo; ++y; }
+    y += step_y;
+    if (y >= p.ho) { y -= p.ho; ++n; }
+    n += step_n;
+  }
+};
+
+template <bool PAIR>
+__global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorParams p, const Parts parts) {
+  constexpr int NACC = PAIR ? 128 : 64;          // accumulator columns per accumulate warp
+  constexpr int ACC_COLS = 2 * NACC;             // TMEM columns of one accumulator
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t bars[2 * STAGES + 4];
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ int fin_flag;
+
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // uniform, for setmaxnreg
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+  int bI, bJ;                                    // block (PAIR: 256 wide) row and column
+  tri_decode(PAIR ? blockIdx.x >> 1 : blockIdx.x, bI, bJ);
+  const bool share = (bI == bJ) && (p.weight == nullptr);
+  const bool fused = p.tickets != nullptr;
+  const int split = blockIdx.y;
+  const int64_t r_begin = (int64_t)split * p.rows_per_split;
+  const int nrows = (int)max((int64_t)0, min((int64_t)p.rows_per_split, p.rows - r_begin));
+  const int nstages = ceil_div(nrows, KS);
+  const int nchunks = ceil_div(nstages, FLUSH);
+  int* status = p.status;
+  const int col_a = bI * (PAIR ? 256 : 128) + (int)rank * TILE, col_b = bJ * (PAIR ? 256 : 128) + (int)rank * TILE;
+  // 64-column blocks A0 A1 B0 B1 that hold columns of the matrix and are needed
+  uint32_t blocks = 0;
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+    if ((b < 2 ? col_a : col_b) + (b & 1) * 64 < p.d && !(share && b >= 2)) blocks |= 1u << b;
+
+  const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t bar0 = smem_u32(bars);
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (STAGES + s); };
+  auto accfull_bar = [&](int b) { return bar0 + 8u * (2 * STAGES + b); };
+  auto accempty_bar = [&](int b) { return bar0 + 8u * (2 * STAGES + 2 + b); };
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full_bar(s), (PAIR ? 2 : 1) * LOAD_WARPS);       // a pair's gather warps all arrive at the leader
+      mbar_init(empty_bar(s), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(accfull_bar(b), 1);
+      mbar_init(accempty_bar(b), (PAIR ? 2 : 1) * EPI_WARPS);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // blocks past the matrix edge are never written: they stay zero
+  const uint32_t idle = ~blocks & (share ? 3u : 15u);
+  if (idle) {
+    for (int b = 0; b < 4; ++b) {
+      if (!((idle >> b) & 1u)) continue;
+      for (uint32_t o = tid * 16u; o < 3 * STAGES * BLK; o += THREADS * 16u) {
+        const uint32_t part = o / BLK;
+        const uint32_t at = smem0 + (part / 3) * SLOT_BYTES + (b >> 1) * SIDE + (part % 3) * OPB + (b & 1) * BLK + o % BLK;
+        asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(at), "r"(0u) : "memory");
+      }
+    }
+  }
+  fence_async_smem();
+  if (warp == MMA_WARP) {
+    if (PAIR) tmem_alloc2(smem_u32(&tmem_base_slot), 2 * ACC_COLS);
+    else tmem_alloc(smem_u32(&tmem_base_slot), 2 * ACC_COLS);
+  }
+  tc_fence_before();
+  if (PAIR) cluster_sync_all();
+  else __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_slot;
+  asm volatile("griddepcontrol.wait;" ::: "memory");                 // the parts are written, the header is clear
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  if (warp < EPI_WARPS) {
+    // ------------------------------------------------------------------ accumulate warps
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+    // warp = 4*half + q: rows 32q.. of the CTA's 128, columns [NACC*half, +NACC)
+    const int q = warp & 3, half = warp >> 2;
+    float acc[NACC];
+#pragma unroll
+    for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
+    const uint32_t accempty0 = PAIR ? map_to_cta(accempty_bar(0), 0u) : accempty_bar(0);
+    for (int c = 0; c < nchunks; ++c) {
+      const int b = c & 1;
+      if (!mbar_wait(accfull_bar(b), (c >> 1) & 1, status, 63)) break;
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * ACC_COLS + half * NACC);
+#pragma unroll
+      for (int part = 0; part < NACC / 32; ++part) {
+        uint32_t v[32];
+        tmem_ld32(taddr + part * 32, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc[part * 32 + i] += __uint_as_float(v[i]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster(accempty0 + 8u * b);
+        else mbar_arrive(accempty0 + 8u * b);
+      }
+    }
+    const int ti = PAIR ? 2 * bI + (int)rank : bI, tj = PAIR ? 2 * bJ + half : bJ;
+    const int col0 = PAIR ? 0 : half * NACC;     // first column inside the 128x128 tile
+    if (ti < ceil_div(p.d, TILE) && tj <= ti) {
+      float* dst = p.partial + ((int64_t)(ti * (ti + 1) / 2 + tj) * p.splits + split) * (TILE * TILE) + part_at(q * 32 + lane, col0);
+      if (p.accumulate) {
+#pragma unroll
+        for (int i = 0; i < NACC; i += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(dst + i * TILE);
+          acc[i] += v.x; acc[i + 1] += v.y; acc[i + 2] += v.z; acc[i + 3] += v.w;
+        }
+      }
+      if (fused && p.splits == 1) {
+        // shared memory is free: every MMA has read its operands before the last accumulator was published
+        float* ct = reinterpret_cast<float*>(smem_raw + (smem0 - smem_u32(smem_raw))) + (PAIR ? half * (TILE * fin::CT_LD) : 0) +
+                    (q * 32 + lane) * fin::CT_LD + col0;
+#pragma unroll
+        for (int i = 0; i < NACC; ++i) ct[i] = acc[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < NACC; i += 4)
+          *reinterpret_cast<float4*>(dst + i * TILE) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+        if (fused) __threadfence();
+      }
+    }
+    // the common tail has equal shares again; nobody may take registers back before these warps have given theirs
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+    asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");
+  } else if (warp < LOAD_WARP0) {
+    // ------------------------------------------------------------------ MMA issuer (of a pair: the leader's)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+    if (warp == MMA_WARP && lane == 0 && rank == 0) {
+      // a narrow tile multiplies only the columns that exist (N in steps of 16)
+      const int n_cols = min(TILE, (p.d - bJ * TILE + 15) / 16 * 16);
+      const uint32_t idesc = PAIR ? instr_desc_pair(1u, 1u)
+                                  : ((instr_desc(1u, 1u) & ~(0x3Fu << 17)) | ((uint32_t)(n_cols >> 3) << 17));
+      bool ok = true;
+      for (int s = 0; s < nstages && ok; ++s) {
+        const int slot = s % STAGES, c = s / FLUSH, b = c & 1;
+        const bool first_of_chunk = (s % FLUSH) == 0;
+        if (first_of_chunk && c >= 2) ok = mbar_wait(accempty_bar(b), ((c >> 1) - 1) & 1, status, 62);
+        if (!ok) break;
+        ok = mbar_wait(full_bar(slot), (s / STAGES) & 1, status, 61);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t a0 = smem0 + slot * SLOT_BYTES, b0 = share ? a0 : a0 + SIDE;
+        const uint32_t d_tmem = tmem_base + (uint32_t)(b * ACC_COLS);
+        uint32_t on = first_of_chunk ? 0u : 1u;
+        for (int ks = 0; ks < KS / 16; ++ks) {
+          // 16 rows = two 1024-byte swizzle atoms; the next 64 columns start BLK further on
+          const uint64_t a_d = smem_desc_sw128(a0 + ks * 2048u, BLK, 1024u), b_d = smem_desc_sw128(b0 + ks * 2048u, BLK, 1024u);
+          constexpr uint64_t P = OPB >> 4;       // from one part to the next, in descriptor units
+          auto mma = [&](int pa, int pb) {
+            if (PAIR) umma2<false>(d_tmem, a_d + pa * P, b_d + pb * P, idesc, on);
+            else umma<false>(d_tmem, a_d + pa * P, b_d + pb * P, idesc, on);
+            on = 1u;
+          };
+          mma(2, 0); mma(0, 2); mma(1, 1); mma(1, 0); mma(0, 1); mma(0, 0);
+        }
+        const bool publish = (s % FLUSH) == FLUSH - 1 || s == nstages - 1;
+        if (PAIR) {
+          umma2_commit_both(empty_bar(slot));
+          if (publish) umma2_commit_both(accfull_bar(b));
+        } else {
+          umma_commit(empty_bar(slot));
+          if (publish) umma_commit(accfull_bar(b));
+        }
+      }
+    }
+    __syncwarp();
+    asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
+  } else {
+    // ------------------------------------------------------------------ gather warps
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    const int w = warp - LOAD_WARP0;
+    const int l8 = lane & 7, row = 4 * w + (lane >> 3);
+    Gather g;
+    g.init(p, col_a, col_b, r_begin, nrows, row, l8);
+    const uint32_t dst0 = smem0 + (uint32_t)row * 128u + (uint32_t)((l8 ^ (row & 7)) << 4);
+    const uint32_t full0 = PAIR ? map_to_cta(full_bar(0), 0u) : full_bar(0);
+    const bool no_halo = p.kh == 1 && p.kw == 1 && p.pad_h == 0 && p.pad_w == 0;
+    const int step_n = KS / (p.ho * p.wo), step_rem = KS - step_n * (p.ho * p.wo);
+    const int step_y = step_rem / p.wo, step_x = step_rem - step_y * p.wo;
+    for (int s = 0; s < nstages + LAG; ++s) {
+      // a stage is handed over before the wait for the next free slot, which depends on an MMA further back
+      if (s >= LAG) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(LAG - 1) : "memory");
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          const uint32_t bar = full0 + 8u * ((s - LAG) % STAGES);
+          if (PAIR) mbar_arrive_cluster(bar);
+          else mbar_arrive(bar);
+        }
+      }
+      if (s < nstages) {
+        const int slot = s % STAGES;
+        if (s >= STAGES && !mbar_wait(empty_bar(slot), ((s / STAGES) - 1) & 1, status, 64)) break;
+        g.stage(p, parts, dst0 + slot * SLOT_BYTES, blocks, no_halo, step_n, step_y, step_x);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
+  }
+  tc_fence_before();
+  if (PAIR) cluster_sync_all();          // neither CTA leaves while its peer's MMAs may still read its shared memory
+  else __syncthreads();
+  if (warp == MMA_WARP) {
+    __syncwarp();
+    tc_fence_after();
+    if (PAIR) tmem_dealloc2(tmem_base, 2 * ACC_COLS);
+    else tmem_dealloc(tmem_base, 2 * ACC_COLS);
+  }
+  if (fused) {
+    const int nb = ceil_div(p.d, TILE);
+    const int ti = PAIR ? 2 * bI + (int)rank : bI;
+    float* ct0 = reinterpret_cast<float*>(smem_raw + (smem0 - smem_u32(smem_raw)));
+    for (int hh = 0; hh < (PAIR ? 2 : 1); ++hh) {
+      const int tj = PAIR ? 2 * bJ + hh : bJ;
+      if (ti < nb && tj <= ti)
+        fin::finish_tile<THREADS>(p, ti * (ti + 1) / 2 + tj, ti, tj, split, ct0 + (p.splits == 1 ? hh * (TILE * fin::CT_LD) : 0),
+                                  &fin_flag, tid);
+      __syncthreads();
+    }
+  }
+}
+
+// Blocks x splits of the rows over the 74 pairs (148 SMs), with measured costs: a stage, the fixed cost of a CTA
+// (set-up, pipeline fill, drain, tile), a partial tile's way to memory and back.
+static int choose_splits(int64_t rows, int units, int slots, int tiles, double stage_us, int max_splits, int& rows_per_split) {
+  const int64_t stages = ceil_div64(rows, KS);
+  const int most = (int)std::max<int64_t>(1, std::min<int64_t>({stages / 4, 148, max_splits}));
+  double best = 1e30;
+  int64_t best_sps = stages;
+  for (int s = 1; s <= most; ++s) {
+    const int64_t sps = ceil_div64(stages, s), real = ceil_div64(stages, sps);
+    const double cost = (double)ceil_div64(units * real, slots) * ((double)sps * stage_us + 5.0) + 0.03 * (double)(tiles * real);
+    if (cost < best - 1e-9) { best = cost; best_sps = sps; }
+  }
+  rows_per_split = (int)(best_sps * KS);
+  return (int)ceil_div64(stages, best_sps);
+}
+
+template <bool PAIR>
+static int launch(const FactorParams& p, const Parts& parts, int units, int splits, cudaStream_t st) {
+  SSO_ENSURE_SMEM(factor_f32_kernel<PAIR>, SMEM);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(PAIR ? 2 * units : units, splits);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = PAIR ? 2 : 1;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
+  cudaLaunchKernelEx(&cfg, factor_f32_kernel<PAIR>, p, parts);
+  SSO_LAUNCH_OK("factor_f32_kernel");
+  return 0;
+}
+
+// ------------------------------------------------------------------------------------------------
+// Tall and narrow: rows of at most 128 columns at one stride (Linear layers, 1x1 factors of channels_last
+// activations).  There is one tile, so an element is converted once wherever that happens, and a pass over memory
+// for the parts would cost more than the factor: the raw rows come into shared memory with cp.async (three stages of
+// 32 KB in flight per SM), the warp that loaded a row splits it into the operand slots.  A stage is 64 rows of 128
+// columns or 128 rows of 64.  Bound: instructions of the split (d = 64 from 802816 rows: 105 us against 355 us
+// through the parts and 434 us for 3xTF32 with one stage of loads).
+// ------------------------------------------------------------------------------------------------
+namespace narrow {
+constexpr int RAW = 4, SLOTS = 2, CHUNK = 64;      // rows between drains of the accumulator
+constexpr uint32_t RAW_BYTES = 32768, SLOT_BYTES = 49152;
+constexpr size_t SMEM = RAW * RAW_BYTES + SLOTS * SLOT_BYTES + 1024;
+
+template <int NBLK, bool VEC>
+__global__ void __launch_bounds__(THREADS, 1) narrow_kernel(const FactorParams p, int64_t row_stride) {
+  constexpr int K = 128 / NBLK, R = K / LOAD_WARPS;            // rows of a stage, of a warp
+  constexpr uint32_t PBLK = K * 128u, PART = NBLK * PBLK;      // 64 columns, one part
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t bars[2 * SLOTS + 4];
+  __shared__ uint32_t tmem_base_slot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t r_begin = (int64_t)blockIdx.x * p.rows_per_split;
+  const int nrows = (int)max((int64_t)0, min((int64_t)p.rows_per_split, p.rows - r_begin));
+  const int nstages = ceil_div(nrows, K), nchunks = nstages * (K / CHUNK);
+  int* status = p.status;
+  const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t raw0 = smem0 + SLOTS * SLOT_BYTES;
+  const uint32_t bar0 = smem_u32(bars);
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (SLOTS + s); };
+  auto accfull_bar = [&](int b) { return bar0 + 8u * (2 * SLOTS + b); };
+  auto accempty_bar = [&](int b) { return bar0 + 8u * (2 * SLOTS + 2 + b); };
+  if (tid == 0) {
+    for (int s = 0; s < SLOTS; ++s) {
+      mbar_init(full_bar(s), LOAD_WARPS);
+      mbar_init(empty_bar(s), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(accfull_bar(b), 1);
+      mbar_init(accempty_bar(b), EPI_WARPS);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == MMA_WARP) tmem_alloc(smem_u32(&tmem_base_slot), 256);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_slot;
+
+  if (warp < EPI_WARPS) {
+    const int q = warp & 3, half = warp >> 2;
+    float acc[64];
+#pragma unroll
+    for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+    for (int c = 0; c < nchunks; ++c) {
+      const int b = c & 1;
+      if (!mbar_wait(accfull_bar(b), (c >> 1) & 1, status, 73)) break;
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 128 + half * 64);
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        uint32_t v[32];
+        tmem_ld32(taddr + part * 32, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc[part * 32 + i] += __uint_as_float(v[i]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(accempty_bar(b));
+    }
+    if (half < NBLK && q < 2 * NBLK) {
+      float* dst = p.partial + (int64_t)blockIdx.x * (TILE * TILE) + part_at(q * 32 + lane, half * 64);
+#pragma unroll
+      for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(dst + i * TILE) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+    }
+  } else if (warp == MMA_WARP) {
+    if (lane == 0) {
+      const int n_cols = (p.d + 15) / 16 * 16;
+      const uint32_t idesc = (instr_desc(1u, 1u) & ~(0x3Fu << 17)) | ((uint32_t)(n_cols >> 3) << 17);
+      bool ok = true;
+      int c = 0;
+      for (int s = 0; s < nstages && ok; ++s) {
+        const int slot = s % SLOTS;
+        ok = mbar_wait(full_bar(slot), (s / SLOTS) & 1, status, 71);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t a0 = smem0 + slot * SLOT_BYTES;
+        for (int ks = 0; ks < K / 16; ++ks) {
+          const int b = c & 1;
+          uint32_t on = (ks % (CHUNK / 16)) == 0 ? 0u : 1u;
+          if (!on && c >= 2) ok = mbar_wait(accempty_bar(b), ((c >> 1) - 1) & 1, status, 72);
+          if (!ok) break;
+          const uint32_t d_tmem = tmem_base + (uint32_t)(b * 128);
+          // with one block the 64 rows behind it (M is 128) are whatever follows in shared memory: they only reach
+          // accumulator rows that nobody reads
+          const uint64_t desc = smem_desc_sw128(a0 + ks * 2048u, PBLK, 1024u);
+          constexpr uint64_t P = PART >> 4;
+          auto mma = [&](int pa, int pb) { umma<false>(d_tmem, desc + pa * P, desc + pb * P, idesc, on); on = 1u; };
+          mma(2, 0); mma(0, 2); mma(1, 1); mma(1, 0); mma(0, 1); mma(0, 0);
+          if ((ks % (CHUNK / 16)) == CHUNK / 16 - 1) {
+            if (ks == K / 16 - 1) umma_commit(empty_bar(slot));
+            umma_commit(accfull_bar(b));
+            ++c;
+          }
+        }
+      }
+    }
+  } else if (warp >= LOAD_WARP0) {
+    const int w = warp - LOAD_WARP0;
+    // 16-byte chunk c of a row's 256 bytes sits at position c ^ (c >> 3): the copies of consecutive chunks and the
+    // loads of every other chunk below both touch eight different bank groups
+    auto pos = [](int c) { return (uint32_t)(c ^ (c >> 3)) * 16u; };
+    const int chunk = lane & 15, row_l = w * R + (lane >> 4);
+    const uint32_t raw_w = raw0 + (uint32_t)row_l * 256u + pos(chunk);
+    const float* src0 = reinterpret_cast<const float*>(p.x) + (r_begin + row_l) * row_stride + chunk * 4;
+    int have[NBLK];
+#pragma unroll
+    for (int b = 0; b < NBLK; ++b) have[b] = max(0, min(4, p.dcols - b * 64 - chunk * 4));
+    auto load = [&](int s) {
+      const float* src = src0 + (int64_t)s * K * row_stride;
+      const uint32_t dst = raw_w + (s % RAW) * RAW_BYTES;
+#pragma unroll
+      for (int j = 0; j < R / 2; ++j) {
+        const bool rv = s * K + row_l + 2 * j < nrows;
+#pragma unroll
+        for (int b = 0; b < NBLK; ++b) {
+          const float* g = src + (int64_t)(2 * j) * row_stride + b * 64;
+          const uint32_t d = dst + b * (K * 256u) + j * 512u;
+          if (VEC) {
+            const bool in = rv && have[b] > 0;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(in ? g : reinterpret_cast<const float*>(p.x)), "r"(in ? 16 : 0) : "memory");
+          } else {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              const bool in = rv && t < have[b];
+              asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 4 * t), "l"(in ? g + t : reinterpret_cast<const float*>(p.x)), "r"(in ? 4 : 0) : "memory");
+            }
+          }
+        }
+      }
+    };
+    const int l8 = lane & 7, k0 = w * R + (lane >> 3);           // this lane splits columns 8*l8 .. of rows k0, k0 + 4, ..
+    const int ones = p.d > p.dcols ? p.dcols - 8 * l8 : -1;      // the ones column, relative to this lane's first
+    for (int s = 0; s < RAW - 1; ++s) {
+      if (s < nstages) load(s);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int s = 0; s < nstages; ++s) {
+      if (s + RAW - 1 < nstages) load(s + RAW - 1);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group %0;" ::"n"(RAW - 1) : "memory");
+      __syncwarp();                              // the whole warp's copies of stage s have landed
+      const int slot = s % SLOTS;
+      if (s >= SLOTS && !mbar_wait(empty_bar(slot), ((s / SLOTS) - 1) & 1, status, 74)) break;
+#pragma unroll
+      for (int j = 0; j < R / 4; ++j)
+#pragma unroll
+        for (int b = 0; b < NBLK; ++b) {
+          const int k = k0 + 4 * j;
+          float v[8];
+          const uint32_t src = raw0 + (s % RAW) * RAW_BYTES + (uint32_t)(b * K + k) * 256u;
+          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(src + pos(2 * l8)) : "memory");
+          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(src + pos(2 * l8 + 1)) : "memory");
+          const int at = ones - 64 * b;
+          if (ones >= 0 && at >= 0 && at < 8) {
+            const float one = s * K + k < nrows ? 1.f : 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              if (i == at) v[i] = one;
+          }
+          uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) split2(v[2 * i], v[2 * i + 1], hi[i], mid[i], lo[i]);
+          const uint32_t dst = smem0 + slot * SLOT_BYTES + b * PBLK + (uint32_t)k * 128u + (uint32_t)((l8 ^ (k & 7)) << 4);
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + PART), "r"(mid[0]), "r"(mid[1]), "r"(mid[2]), "r"(mid[3]) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 2 * PART), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
+        }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full_bar(slot));
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == MMA_WARP) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 256);
+  }
+}
+}  // namespace narrow
+
+// What a problem looks like to the gather: its channels padded (or folded) to c8, its factor of width d.
+struct Shape {
+  int fold, c8, width, dcols, d, tiles, blocks;
+  int64_t image_bytes;       // parts of one image
+};
+static Shape shape_of(const FactorParams& p) {
+  Shape s;
+  const int kk = p.kh * p.kw, ones = p.d - p.dcols;
+  s.fold = (p.c < 8 && p.kw > 1) ? p.kw : 0;
+  s.c8 = ceil_div(s.fold ? p.c * p.kw : p.c + (kk == 1 ? ones : 0), 8) * 8;
+  s.width = s.fold ? p.wo : p.w;
+  s.dcols = kk == 1 ? p.d : s.c8 * (s.fold ? p.kh : kk);
+  s.d = kk == 1 ? p.d : s.dcols + ones;
+  const int nb = ceil_div(s.d, 128), nb2 = ceil_div(s.d, 256);
+  s.tiles = nb * (nb + 1) / 2;
+  s.blocks = nb2 * (nb2 + 1) / 2;
+  s.image_bytes = (int64_t)p.h * s.width * s.c8 * 6 * (p.weight ? 2 : 1);
+  return s;
+}
+constexpr int64_t PARTS_TARGET = (int64_t)256 << 20;     // parts of one run of images
+constexpr int64_t PARTIAL_TARGET = (int64_t)148 * 2 * 65536;
+
+}  // namespace f32
+
+// Scratch: header, partial tiles (at least one split), parts of at least one image.
+static size_t f32_min_bytes(const FactorParams& p, const f32::Shape& s) {
+  return factor_header_bytes(s.tiles) + (size_t)s.tiles * 65536 + (size_t)s.image_bytes + 512;
+}
+size_t factor_f32_workspace_bytes(const FactorParams& p) {
+  const f32::Shape s = f32::shape_of(p);
+  const int64_t all = s.image_bytes * p.n;
+  const int64_t partial = std::max<int64_t>(f32::PARTIAL_TARGET, 4 * (int64_t)s.tiles * 65536);
+  return factor_header_bytes(s.tiles) + (size_t)partial + (size_t)std::max<int64_t>(s.image_bytes, std::min<int64_t>(all, f32::PARTS_TARGET)) + 512;
+}
+
+bool factor_f32_supported(const FactorParams& p, size_t workspace_bytes) {
+  const f32::Shape s = f32::shape_of(p);
+  return (int64_t)p.h * s.width * s.c8 < ((int64_t)1 << 30) && (int64_t)p.n * p.h * s.width < ((int64_t)1 << 31) && workspace_bytes >= f32_min_bytes(p, s);
+}
+
+// Rows at one stride with contiguous columns, at most 128 of them: the stride, else 0.
+static int64_t narrow_stride(const FactorParams& p) {
+  if (p.d > 128 || p.kh != 1 || p.kw != 1 || p.pad_h || p.pad_w || p.stride_h != 1 || p.stride_w != 1 || p.weight || (p.sc != 1 && p.c > 1)) return 0;
+  const int64_t rs = p.w > 1 ? p.sw : p.h > 1 ? p.sh : p.sn;
+  const bool even = (p.w == 1 || p.h == 1 || p.sh == p.w * p.sw) && (p.h * p.w == 1 || p.n == 1 || p.sn == (int64_t)p.h * p.w * rs);
+  return even && rs > 0 ? rs : 0;
+}
+
+template <int NBLK, bool VEC>
+static int narrow_launch(const FactorParams& p, int64_t row_stride, cudaStream_t st) {
+  SSO_ENSURE_SMEM((f32::narrow::narrow_kernel<NBLK, VEC>), f32::narrow::SMEM);
+  f32::narrow::narrow_kernel<NBLK, VEC><<<p.splits, f32::THREADS, f32::narrow::SMEM, st>>>(p, row_stride);
+  SSO_LAUNCH_OK("narrow_kernel");
+  return factor_tc_run_reduce(p, 1, st);
+}
+
+static int factor_narrow_launch(FactorParams p, int64_t row_stride, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  const size_t hdr = factor_header_bytes(1);
+  const int64_t stages = ceil_div64(p.rows, 128);      // a CTA needs about four to pay for its set-up
+  const int64_t most = std::max<int64_t>(1, std::min<int64_t>({148, stages / 4, (int64_t)((workspace_bytes - hdr) / 65536)}));
+  p.rows_per_split = (int)(ceil_div64(stages, most) * 128);
+  p.splits = (int)ceil_div64(p.rows, p.rows_per_split);
+  p.status = reinterpret_cast<int*>(workspace);
+  p.partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + hdr);
+  p.perm_c = 0; p.perm_kk = 1; p.tickets = nullptr;
+  SSO_CUDA_OK(cudaMemsetAsync(p.status, 0, sizeof(int), st));
+  const bool vec = p.c % 4 == 0 && row_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0;
+  if (p.d <= 64) return vec ? narrow_launch<1, true>(p, row_stride, st) : narrow_launch<1, false>(p, row_stride, st);
+  return vec ? narrow_launch<2, true>(p, row_stride, st) : narrow_launch<2, false>(p, row_stride, st);
+}
+
+int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  if (const int64_t rs = narrow_stride(p)) return factor_narrow_launch(p, rs, workspace, workspace_bytes, st);
+  const f32::Shape s = f32::shape_of(p);
+  SSO_CHECK_ARG(workspace != nullptr && workspace_bytes >= f32_min_bytes(p, s), "factor workspace too small: need %zu bytes, got %zu",
+                f32_min_bytes(p, s), workspace_bytes);
+  // images per run: as many as their parts fit next to one split's partial tiles, at most PARTS_TARGET
+  const size_t hdr = factor_header_bytes(s.tiles);
+  const int64_t room = (int64_t)(workspace_bytes - hdr - 512) - (int64_t)s.tiles * 65536;
+  const int64_t per_run = std::max<int64_t>(1, std::min<int64_t>({(int64_t)p.n, f32::PARTS_TARGET / std::max<int64_t>(1, s.image_bytes), room / std::max<int64_t>(1, s.image_bytes)}));
+  const int runs = (int)ceil_div64(p.n, per_run);
+  const int n_run = (int)ceil_div64(p.n, runs);
+  const int64_t parts_bytes = n_run * s.image_bytes;
+  const int max_splits = (int)(((int64_t)(workspace_bytes - hdr - 512) - (parts_bytes + 255) / 256 * 256) / ((int64_t)s.tiles * 65536));
+  char* base = reinterpret_cast<char*>(workspace);
+  FactorParams q = p;
+  q.status = reinterpret_cast<int*>(base);
+  f32::Parts parts;
+  parts.a = reinterpret_cast<const __nv_bfloat16*>(base + (hdr + 255) / 256 * 256);
+  parts.stride = (int64_t)n_run * p.h * s.width * s.c8;
+  parts.b = p.weight ? parts.a + 3 * parts.stride : parts.a;
+  parts.c8 = s.c8;
+  q.partial = reinterpret_cast<float*>(base + (hdr + 255) / 256 * 256 + (parts_bytes + 255) / 256 * 256);
+  // a pair's block is 256 wide: up to 128 columns one CTA's tile is all there is to compute
+  const bool pair = s.d > 128;
+  const int64_t hw = (int64_t)p.ho * p.wo;
+  int rps = 0;
+  q.splits = f32::choose_splits(n_run * hw, pair ? s.blocks : s.tiles, pair ? 74 : 148, s.tiles, pair ? 0.85 : 0.6, max_splits, rps);
+  q.rows_per_split = rps;
+  const int kk = p.kh * p.kw;
+  q.perm_c = kk > 1 ? s.c8 : 0;
+  q.perm_kk = kk;
+  q.perm_pub = kk > 1 ? p.c : 0;
+  q.perm_fold = s.fold;
+  q.c = s.c8; q.dcols = s.dcols; q.d = s.d; q.w = s.width;
+  q.sn = (int64_t)p.h * s.width * s.c8; q.sh = (int64_t)s.width * s.c8; q.sw = s.c8; q.sc = 1;
+  if (s.fold) { q.kw = 1; q.stride_w = 1; q.pad_w = 0; q.dil_w = 1; }
+  const bool fused = kk == 1 && q.splits == 1;
+  q.ticket_tiles = s.tiles;
+  const bool direct = !s.fold && p.sc == 1 && p.c % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 && p.sn % 4 == 0 &&
+                      (p.h == 1 || p.sh % 4 == 0) && (p.w == 1 || p.sw % 4 == 0) && (int64_t)n_run * p.h * s.width * (s.c8 / 8) < ((int64_t)1 << 31);
+  const int header_words = fused ? (int)(hdr / sizeof(int)) : 1;
+  for (int r = 0, n0 = 0; r < runs; ++r, n0 += n_run) {
+    const int n = std::min(n_run, p.n - n0);
+    FactorParams in = p;
+    in.x = reinterpret_cast<const float*>(p.x) + n0 * p.sn;
+    in.status = q.status;
+    in.weight = p.weight ? p.weight + n0 : nullptr;
+    const int64_t pixels = (int64_t)n * p.h * s.width;
+    const int ones_at = kk == 1 && p.d > p.dcols ? p.c : -1;
+    if (direct)
+      f32::split_direct_kernel<<<(unsigned)ceil_div64(pixels * (s.c8 / 8), 256), 256, 0, st>>>(in, (uint32_t)pixels, ones_at,
+                                                                                                            r == 0 ? header_words : 0, parts, parts);
+    else
+      f32::split_kernel<<<dim3((unsigned)ceil_div64(pixels, 32), ceil_div(s.c8, 64)), 256, 0, st>>>(in, (uint32_t)pixels, s.width, s.fold, ones_at,
+                                                                                                  r == 0 ? header_words : 0, parts, parts);
+    SSO_LAUNCH_OK("split_kernel");
+    q.n = n;
+    q.rows = n * hw;
+    q.accumulate = r > 0;
+    q.tickets = fused && r == runs - 1 ? reinterpret_cast<int*>(base + 256) : nullptr;
+    const int rc = pair ? f32::launch<true>(q, parts, s.blocks, q.splits, st) : f32::launch<false>(q, parts, s.tiles, q.splits, st);
+    if (rc) return rc;
+  }
+  if (fused) return 0;
+  return factor_tc_run_reduce(q, s.tiles, st);
+}
+
+int factor_f32_set_wait_controls(long long cycles, int stall) { return tc::set_wait_controls(cycles, stall); }
+
+}  // namespace sso

@@ -39,9 +39,10 @@ __host__ __device__ inline int group_size(int splits) {
 template <int NT>
 __device__ __forceinline__ void sum_tiles(const float* __restrict__ first, int count, int64_t stride_floats,
                                           int vr, float* __restrict__ ct, float* __restrict__ gdst, int tid) {
-  for (int e = tid; e < vr * (T / 4); e += NT) {
-    const int r = e / (T / 4), c4 = (e % (T / 4)) * 4;
-    const float* src = first + r * T + c4;
+  for (int e = tid; e < T * (T / 4); e += NT) {
+    const int r = e % T, c4 = e / T * 4;
+    if (r >= vr) continue;
+    const float* src = first + 4 * e;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     // loads in batches of four (independent, all in flight together); the adds keep the index order
     for (int s0 = 0; s0 < count; s0 += 4) {
@@ -54,7 +55,7 @@ __device__ __forceinline__ void sum_tiles(const float* __restrict__ first, int c
       for (int k = 0; k < 4; ++k) { a.x += v[k].x; a.y += v[k].y; a.z += v[k].z; a.w += v[k].w; }
     }
     if (gdst) {
-      *reinterpret_cast<float4*>(gdst + r * T + c4) = a;
+      *reinterpret_cast<float4*>(gdst + 4 * e) = a;
     } else {
       float* d = ct + r * CT_LD + c4;
       d[0] = a.x; d[1] = a.y; d[2] = a.z; d[3] = a.w;

@@ -23,10 +23,31 @@ struct FactorParams {
   int* status;      // device word: 0 ok, else the code of the wait that gave up
   int perm_c;       // > 0: kernel columns are ordered (kh, kw, c) with c < perm_c; 0: natural order
   int perm_kk;      // kh*kw
+  int perm_pub;     // > 0: public channel count (a group's columns past it are padding); 0: perm_c
+  int perm_fold;    // > 0: the columns of a group are kx*perm_pub + c with kx < perm_fold (kernel width), groups are ky
+  int accumulate;   // the partial tiles already hold the sums of earlier launches of this factor
   // finishing inside the producing kernel (factor_finish.cuh); tickets == nullptr: separate kernel
   int* tickets;     // [ticket_tiles] per-tile counters, then [ticket_tiles][16] per-group counters
   int ticket_tiles;
 };
+
+// Element (r, c) of a 128x128 partial tile of the tensor-core kernels: groups of four columns, rows inside a group.  An
+// accumulate warp holds one row per lane, so its 16-byte stores are 512 contiguous bytes per instruction (row by row
+// every store touched 32 lines: 6 us for the two tiles of a CTA).
+__host__ __device__ __forceinline__ int part_at(int r, int c) { return ((c >> 2) * 128 + r) * 4 + (c & 3); }
+
+// Public column of internal column j (the finishing kernels), -1 for padding.
+__device__ __forceinline__ int public_column(const FactorParams& p, int j) {
+  if (p.perm_c <= 0) return j;
+  const int pub = p.perm_pub > 0 ? p.perm_pub : p.perm_c;
+  if (j >= p.dcols) return pub * p.perm_kk;      // the ones column
+  const int grp = j / p.perm_c, r = j - grp * p.perm_c;
+  if (p.perm_fold > 0) {
+    const int kx = r / pub;
+    return kx < p.perm_fold ? (r - kx * pub) * p.perm_kk + grp * p.perm_fold + kx : -1;
+  }
+  return r < pub ? r * p.perm_kk + grp : -1;
+}
 
 // Scratch layout of the tensor-core factor kernels: [status word, 256 bytes][ticket counters]
 // [partial tiles].  The header is cleared on the stream by every launch.

@@ -142,11 +142,10 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
         acc[32 + i] += __uint_as_float(v1[i]);
       }
     }
-    float* dst = p.partial + ((int64_t)blockIdx.x * p.splits + split) * (TILE * TILE) +
-                 (q * 32 + lane) * TILE + half * 64;
+    float* dst = p.partial + ((int64_t)blockIdx.x * p.splits + split) * (TILE * TILE) + part_at(q * 32 + lane, half * 64);
 #pragma unroll
     for (int i = 0; i < 64; i += 4)
-      *reinterpret_cast<float4*>(dst + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+      *reinterpret_cast<float4*>(dst + i * TILE) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
   } else if (warp == MMA_WARP) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
@@ -378,7 +377,7 @@ constexpr int RED_ROWS = 32, RED_CB = 8, RED_W = 32;
 // independent partial sums keep several loads in flight, combined in a fixed order
 __device__ __forceinline__ float reduce_fetch(const float* __restrict__ partial, int nsplit, int r, int c) {
   const int bi = r >> 7, bj = c >> 7;
-  const float* src = partial + ((int64_t)(bi * (bi + 1) / 2 + bj) * nsplit) * (TILE * TILE) + (r & 127) * TILE + (c & 127);
+  const float* src = partial + ((int64_t)(bi * (bi + 1) / 2 + bj) * nsplit) * (TILE * TILE) + part_at(r & 127, c & 127);
   constexpr int64_t S = TILE * TILE;
   float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
   int sp = 0;
@@ -394,13 +393,14 @@ __device__ __forceinline__ float reduce_fetch(const float* __restrict__ partial,
 
 __global__ void __launch_bounds__(256) factor_tc_reduce(const FactorParams p, int perm_groups, int pitch) {
   extern __shared__ float rs[];
+  asm volatile("griddepcontrol.wait;" ::: "memory");      // launched early behind the kernel that writes the partial tiles
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int gi0 = blockIdx.x * RED_ROWS;
   const int grp = blockIdx.y;
-  const int kk = p.perm_kk, C = p.perm_c, d = p.d;
-  int ext0, n_ext;
+  const int kk = p.perm_kk, C = p.perm_c, d = p.d, pub = p.perm_pub > 0 ? p.perm_pub : C;
+  int ext0, n_ext;      // public columns of this CTA
   if (grp < perm_groups) {
-    const int c0 = grp * RED_CB, len = min(RED_CB, C - c0);
+    const int c0 = grp * RED_CB, len = min(RED_CB, pub - c0);
     ext0 = c0 * kk;
     n_ext = len * kk;
     // below / on the diagonal: 4 rows x 8 columns per warp; above: 32 rows x 1 column per warp
@@ -418,12 +418,13 @@ __global__ void __launch_bounds__(256) factor_tc_reduce(const FactorParams p, in
       if (doB) rs[rrB * pitch + eB * kk + run] = vB;
     }
   } else {
-    ext0 = (perm_groups > 0 ? p.dcols : 0) + (grp - perm_groups) * RED_W;
-    n_ext = min(RED_W, d - ext0);
+    const int int0 = (perm_groups > 0 ? p.dcols : 0) + (grp - perm_groups) * RED_W;      // internal column of ext0
+    ext0 = perm_groups > 0 ? pub * kk : int0;
+    n_ext = min(RED_W, d - int0);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int rrA = warp + 8 * k, giA = gi0 + rrA, gjA = ext0 + lane;
-      const int eB = warp + 8 * k, giB = gi0 + lane, gjB = ext0 + eB;
+      const int rrA = warp + 8 * k, giA = gi0 + rrA, gjA = int0 + lane;
+      const int eB = warp + 8 * k, giB = gi0 + lane, gjB = int0 + eB;
       const bool doA = lane < n_ext && giA < d && gjA <= giA;
       const bool doB = eB < n_ext && giB < d && gjB > giB;
       float vA = 0.f, vB = 0.f;
@@ -438,7 +439,8 @@ __global__ void __launch_bounds__(256) factor_tc_reduce(const FactorParams p, in
   for (int rr = warp; rr < RED_ROWS; rr += 8) {
     const int gi = gi0 + rr;
     if (gi >= d) break;
-    const int gr = (C > 0 && gi < p.dcols) ? (gi % C) * kk + gi / C : gi;
+    const int gr = public_column(p, gi);
+    if (gr < 0) continue;
     float* orow = p.out + (int64_t)gr * p.ldo + ext0;
     for (int e = lane; e < n_ext; e += 32) {
       float v = p.alpha * rs[rr * pitch + e];
@@ -456,11 +458,12 @@ __global__ void __launch_bounds__(256) factor_tc_reduce(const FactorParams p, in
 // the chains get shorter and SL times more CTAs are in flight.
 __global__ void __launch_bounds__(256) factor_tc_reduce_tiles(const FactorParams p, int sl) {
   int bi, bj;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   tri_decode(blockIdx.x, bi, bj);
   const float* src = p.partial + (int64_t)blockIdx.x * p.splits * (TILE * TILE);
   const int group = (blockIdx.y * 256 + threadIdx.x) / sl, sub = threadIdx.x % sl;
   const int e0 = group * 4;
-  const int r = e0 / TILE, c0 = e0 % TILE;
+  const int r = group % TILE, c0 = group / TILE * 4;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f), s2 = make_float4(0.f, 0.f, 0.f, 0.f);
   int sp = sub;
   for (; sp + sl < p.splits; sp += 2 * sl) {      // two independent chains per lane
@@ -482,19 +485,17 @@ __global__ void __launch_bounds__(256) factor_tc_reduce_tiles(const FactorParams
   }
   if (sub != 0) return;
   const bool bad = p.status && *p.status != 0;
-  auto ext = [&](int j) {
-    if (p.perm_c > 0 && j < p.dcols) return (j % p.perm_c) * p.perm_kk + j / p.perm_c;
-    return j;
-  };
   const int gi = bi * TILE + r;
   if (gi >= p.d) return;
-  const int gr = ext(gi);
+  const int gr = public_column(p, gi);
+  if (gr < 0) return;
   const float vals[4] = {s.x, s.y, s.z, s.w};
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int gj = bj * TILE + c0 + q;
     if (gj >= p.d || gj > gi) continue;   // diagonal tiles: lower triangle only, mirrored below
-    const int gc = ext(gj);
+    const int gc = public_column(p, gj);
+    if (gc < 0) continue;
     float v = p.alpha * vals[q];
     if (bad) v = __int_as_float(0x7fc00000);
     float* o = p.out + (int64_t)gr * p.ldo + gc;
@@ -545,15 +546,15 @@ size_t factor_tc_workspace_bytes(int64_t rows, int64_t d) {
 }
 
 bool factor_tc_supported(const FactorParams& p, int dtype) {
-  const int ch = (dtype == SSO_F32) ? 4 : 8;
-  const int esz = (dtype == SSO_F32) ? 4 : 2;
+  if (dtype == SSO_F32) return false;      // factor_f32.cu
+  const int ch = 8, esz = 2;
   if (p.sc != 1) return false;
   if (p.c % ch != 0) return false;
   if ((reinterpret_cast<uintptr_t>(p.x) & 15) != 0) return false;
   if ((p.sn * esz) % 16 != 0) return false;
   if (p.h > 1 && (p.sh * esz) % 16 != 0) return false;
   if (p.w > 1 && (p.sw * esz) % 16 != 0) return false;
-  if (p.weight != nullptr && dtype != SSO_F32) return false;  // weights would round 16-bit operands
+  if (p.weight != nullptr) return false;  // weights would round 16-bit operands
   return true;
 }
 
@@ -583,7 +584,6 @@ int factor_tc_launch(FactorParams p, int dtype, void* workspace, size_t workspac
   p.perm_c = (p.kh * p.kw > 1) ? p.c : 0;
   p.perm_kk = p.kh * p.kw;
   switch (dtype) {
-    case SSO_F32: return tc_launch_typed<float>(p, tiles, st);
     case SSO_BF16: return tc_launch_typed<__nv_bfloat16>(p, tiles, st);
     case SSO_F16: return tc_launch_typed<__half>(p, tiles, st);
   }
@@ -596,20 +596,36 @@ int factor_tc_launch(FactorParams p, int dtype, void* workspace, size_t workspac
 static int g_rowwise_max_splits = 8;
 void factor_tc_set_rowwise_max_splits(int s) { g_rowwise_max_splits = s; }
 
+// A finishing kernel may be set up while its producer still runs (it waits for the producer's end itself).
+template <typename... Args>
+static void launch_early(void (*kernel)(Args...), dim3 grid, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 int factor_tc_run_reduce(const FactorParams& p, int tiles, cudaStream_t st) {
   // a large permuted factor with not too many splits: the output dominates, write it in whole rows
-  if (!(p.perm_c > 0 && p.splits <= g_rowwise_max_splits && p.d >= 1024)) {
+  if (!(p.perm_c > 0 && p.perm_fold == 0 && p.splits <= g_rowwise_max_splits && p.d >= 1024)) {
     // lanes per element group: enough CTAs to fill the GPU when there are few tiles, and chains
     // of at most ~8 partial tiles per lane
     int sl = 1;
     while (sl < 8 && (tiles * 16 * sl < 2 * 148 || p.splits > 8 * sl) && p.splits >= 4 * sl) sl <<= 1;
-    tc::factor_tc_reduce_tiles<<<dim3(tiles, 16 * sl), 256, 0, st>>>(p, sl);
+    launch_early(tc::factor_tc_reduce_tiles, dim3(tiles, 16 * sl), 0, st, FactorParams(p), sl);
     SSO_LAUNCH_OK("factor_tc_reduce_tiles");
     return 0;
   }
   int perm_groups = 0, width = tc::RED_W;
   if (p.perm_c > 0) {
-    perm_groups = ceil_div(p.perm_c, tc::RED_CB);
+    perm_groups = ceil_div(p.perm_pub > 0 ? p.perm_pub : p.perm_c, tc::RED_CB);
     width = std::max(tc::RED_CB * p.perm_kk, 1);
   }
   const int plain_groups = p.perm_c > 0 ? (p.d > p.dcols ? 1 : 0) : ceil_div(p.d, tc::RED_W);
@@ -617,7 +633,7 @@ int factor_tc_run_reduce(const FactorParams& p, int tiles, cudaStream_t st) {
   const size_t smem = (size_t)tc::RED_ROWS * pitch * sizeof(float);
   SSO_CHECK_ARG(smem <= 200 * 1024, "factor: kernel window too large for the finishing kernel");
   SSO_ENSURE_SMEM(tc::factor_tc_reduce, 200 * 1024);
-  tc::factor_tc_reduce<<<dim3(ceil_div(p.d, tc::RED_ROWS), perm_groups + plain_groups), 256, smem, st>>>(p, perm_groups, pitch);
+  launch_early(tc::factor_tc_reduce, dim3(ceil_div(p.d, tc::RED_ROWS), perm_groups + plain_groups), smem, st, FactorParams(p), perm_groups, pitch);
   SSO_LAUNCH_OK("factor_tc_reduce");
   return 0;
 }

@@ -74,6 +74,7 @@ SIGNATURES = {
                                 c_vp, c_i64, c_vp, c_sz, c_i32, c_vp]),
     'sso_factor_syrk_noalloc': (c_i32, [c_vp, c_i32, c_i64, c_i64, c_i64, c_i64, c_i32, c_vp, c_f32, c_f32,
                                         c_vp, c_i64, c_i32, c_vp]),
+    'sso_factor_desc_workspace_bytes': (c_sz, [c_vp, c_i32]),
     'sso_factor_op_create': (c_i64, [c_vp, c_i32]),
     'sso_factor_op_run': (c_i32, [c_i64, c_vp, c_vp, c_f32, c_f32, c_vp, c_sz, c_vp]),
     'sso_factor_op_destroy': (c_i32, [c_i64]),
@@ -272,6 +273,15 @@ def _dtype_code(t: torch.Tensor) -> int:
         raise RuntimeError('unsupported dtype %s (fp32, bf16, fp16 only)' % t.dtype)
 
 
+def _factor_scratch(x, n, c, h, w, strides, geometry, append_ones, weight, out, impl):
+    d = FactorDesc()
+    d.dtype, d.append_ones, d.n, d.c, d.h, d.w = _dtype_code(x), int(append_ones), n, c, h, w
+    d.sn, d.sc, d.sh, d.sw = strides
+    (d.kh, d.kw), (d.stride_h, d.stride_w), (d.pad_h, d.pad_w), (d.dil_h, d.dil_w) = geometry
+    d.x, d.sample_weight, d.out, d.ldo = x.data_ptr(), _ptr(weight), out.data_ptr(), out.stride(0)
+    return workspace(x.device, lib().sso_factor_desc_workspace_bytes(C.byref(d), impl))
+
+
 def factor_im2col(x: torch.Tensor, kernel_size, stride, padding, dilation, append_ones: bool,
                   sample_weight: Optional[torch.Tensor], alpha: float, beta: float,
                   out: torch.Tensor, impl: int = IMPL_AUTO):
@@ -285,8 +295,8 @@ def factor_im2col(x: torch.Tensor, kernel_size, stride, padding, dilation, appen
     assert out.shape == (d, d) and out.dtype == torch.float32 and out.stride(1) == 1, (out.shape, d)
     rows = n * ho * wo
     L = lib()
-    ws = workspace(x.device, L.sso_factor_workspace_bytes(rows, d, impl))
     sn, sc, sh, sw = x.stride()
+    ws = _factor_scratch(x, n, c, h, w, x.stride(), (kernel_size, stride, padding, dilation), append_ones, sample_weight, out, impl)
     _timed_factor(lambda: _check(L.sso_factor_syrk_im2col(
         x.data_ptr(), _dtype_code(x), n, c, h, w, sn, sc, sh, sw, kh, kw, stride[0], stride[1],
         padding[0], padding[1], dilation[0], dilation[1], int(append_ones), _ptr(sample_weight),
@@ -302,7 +312,8 @@ def factor_rows(x: torch.Tensor, append_ones: bool, row_weight: Optional[torch.T
     d = cols + (1 if append_ones else 0)
     assert out.shape == (d, d) and out.dtype == torch.float32 and out.stride(1) == 1
     L = lib()
-    ws = workspace(x.device, L.sso_factor_workspace_bytes(rows, d, impl))
+    ws = _factor_scratch(x, rows, cols, 1, 1, (x.stride(0), x.stride(1), 0, 0), ((1, 1), (1, 1), (0, 0), (1, 1)), append_ones,
+                         row_weight, out, impl)
     _timed_factor(lambda: _check(L.sso_factor_syrk(
         x.data_ptr(), _dtype_code(x), rows, cols, x.stride(0), x.stride(1), int(append_ones),
         _ptr(row_weight), alpha, beta, out.data_ptr(), out.stride(0), _ptr(ws),
@@ -338,10 +349,10 @@ class FactorOp:
         self.mid = (_dtype_code(x), n, c, h, w, sn, sc, sh, sw, kh, kw, stride[0], stride[1],
                     padding[0], padding[1], dilation[0], dilation[1], int(append_ones))
         self.out_ptr, self.ldo = out.data_ptr(), out.stride(0)
-        self.nbytes = L.sso_factor_workspace_bytes(rows, d, impl)
         self.device = x.device
         desc = FactorDesc()
         self.fill(desc)
+        self.nbytes = L.sso_factor_desc_workspace_bytes(C.byref(desc), impl)
         self.op = L.sso_factor_op_create(C.byref(desc), impl)
         if self.op <= 0:
             _check(int(self.op))

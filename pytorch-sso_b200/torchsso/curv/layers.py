@@ -86,10 +86,11 @@ def _fused_ema_coefficients(curv):
 # Kronecker-factored
 # ---------------------------------------------------------------------------------------------
 def _channels_last_if_worthwhile(t, d):
-    """NCHW activations (channel stride != 1) can only use the exact-fp32 SIMT factor kernel; the
+    """16-bit NCHW activations (channel stride != 1) can only use the exact-fp32 SIMT factor kernel; the
     tensor-core kernels gather whole 16-byte runs of channels.  For anything but tiny problems one
-    extra pass over the activation (a layout copy to channels_last) is far cheaper than that."""
-    if t.dim() != 4 or t.stride(1) == 1 or t.shape[1] == 1:
+    extra pass over the activation (a layout copy to channels_last) is far cheaper than that.  fp32
+    activations are split into 16-bit parts on the way, from whatever layout they have."""
+    if t.dtype == torch.float32 or t.dim() != 4 or t.stride(1) == 1 or t.shape[1] == 1:
         return t
     rows = t.shape[0] * t.shape[2] * t.shape[3]
     if 2.0 * rows * d * d < 5e8:
@@ -195,10 +196,10 @@ class KronCovConv2d(_KronFactors):
         if m.groups != 1 or isinstance(m.padding, str):
             raise NotImplementedError('grouped / string-padded convolutions have no Kronecker curvature here')
         n, c = x.shape[0], x.shape[1]
-        vec = 4 if x.dtype == torch.float32 else 8
+        vec = 8
         x = _channels_last_if_worthwhile(x, c * m.kernel_size[0] * m.kernel_size[1])
-        if x.stride(1) == 1 and c % vec != 0 and c < 64:
-            # Channels-last input whose channel count is not a whole number of 16-byte chunks (the
+        if x.dtype != torch.float32 and x.stride(1) == 1 and c % vec != 0 and c < 64:
+            # 16-bit channels-last input whose channel count is not a whole number of 16-byte chunks (the
             # 3-channel stem): zero-pad the channels so the tensor-core kernel applies, then keep
             # the rows / columns of the real channels.  Columns are ordered (c, kh, kw), so the
             # padding channels are a trailing block (followed by the ones column when there is a bias).
@@ -233,7 +234,7 @@ class KronCovConv2d(_KronFactors):
 
     def _factor_G(self, g, weight, scale, beta, out):
         n, c, h, w = g.shape
-        if c % (4 if g.dtype == torch.float32 else 8) == 0:
+        if c % 8 == 0:
             g = _channels_last_if_worthwhile(g, c)
         self._op(g, self._PLAIN, False, out).run(g, weight, scale / (n * h * w), beta)
 

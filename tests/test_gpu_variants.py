@@ -67,3 +67,81 @@ def test_precondition_grad_of_moving_gradients(nat):
         keep.append(params)
         got = torch.cat([params[0].grad, params[1].grad[:, None]], 1)
         assert rel(got, want) < (1e-4 if dtype == torch.float32 else 1e-2)
+
+
+# ---------------------------------------------------------------------------------- fp32 factors
+def conv_ref(x, k, s, p, d, bias, weight=None):
+    """sum_r w_r u_r u_r^T over the im2col rows in fp64, columns (c, kh, kw) and the ones column."""
+    import torch.nn.functional as F
+    u = F.unfold(x.double(), k, dilation=d, padding=p, stride=s).transpose(1, 2)
+    if bias:
+        u = torch.cat([u, torch.ones_like(u[..., :1])], -1)
+    w = torch.ones(x.shape[0], dtype=torch.float64, device=x.device) if weight is None else weight.double()
+    return torch.einsum('n,nri,nrj->ij', w, u, u)
+
+
+# channels below eight (folded), not a multiple of eight, one tile / one pair / several pairs, strides, dilation
+F32_CONVS = [(5, 3, 20, 19, (7, 7), (2, 2), (3, 3), (1, 1), False), (3, 1, 9, 9, (3, 3), (1, 1), (1, 1), (1, 1), True),
+             (4, 7, 12, 10, (3, 2), (1, 2), (1, 0), (2, 1), True), (6, 11, 9, 9, (3, 3), (1, 1), (1, 1), (1, 1), True),
+             (3, 64, 8, 8, (3, 3), (1, 1), (1, 1), (1, 1), True), (2, 26, 13, 13, (5, 5), (1, 1), (2, 2), (1, 1), False),
+             (40, 33, 6, 6, (1, 1), (2, 2), (0, 0), (1, 1), True), (16, 130, 5, 7, (1, 1), (1, 1), (0, 0), (1, 1), True)]
+
+
+@pytest.mark.parametrize('cfg', F32_CONVS)
+@pytest.mark.parametrize('channels_last', [False, True])
+def test_factor_f32_conv(nat, cfg, channels_last):
+    n, c, h, w, k, s, p, d, bias = cfg
+    x = torch.randn(n, c, h, w, device='cuda')
+    x = x.contiguous(memory_format=torch.channels_last) if channels_last else x
+    ref = conv_ref(x, k, s, p, d, bias)
+    out = torch.randn_like(ref, dtype=torch.float32)
+    want = 0.5 * ref + 2.0 * out.double()
+    nat.factor_im2col(x, k, s, p, d, bias, None, 0.5, 2.0, out)
+    assert rel(out, want) < 1e-6
+    weight = torch.rand(n, device='cuda')
+    nat.factor_im2col(x, k, s, p, d, bias, weight, 1.0, 0.0, out)
+    assert rel(out, conv_ref(x, k, s, p, d, bias, weight)) < 1e-6
+    assert torch.equal(out, out.t())
+
+
+@pytest.mark.parametrize('rows,cols,bias', [(1, 1, False), (31, 5, True), (129, 63, True), (700, 64, False), (5000, 64, True), (33000, 128, False),
+                                            (20001, 97, True), (40000, 13, False), (257, 300, True), (1500, 1021, True), (33, 4100, False)])
+@pytest.mark.parametrize('layout', ['rows', 'strided', 'columns'])
+def test_factor_f32_rows(nat, rows, cols, bias, layout):
+    x = torch.randn(rows, cols, device='cuda') + 0.25
+    if layout == 'strided':
+        x = torch.randn(rows, cols + 3, device='cuda')[:, 1:cols + 1]
+    elif layout == 'columns':
+        x = x.t().contiguous().t()
+    u = x.double()
+    if bias:
+        u = torch.cat([u, torch.ones_like(u[:, :1])], 1)
+    d = cols + int(bias)
+    out = torch.full((d, d), float('nan'), device='cuda')
+    nat.factor_rows(x, bias, None, 1.0 / rows, 0.0, out)
+    assert rel(out, u.t() @ u / rows) < 1e-6 and torch.equal(out, out.t())
+
+
+def test_factor_f32_in_runs(nat):
+    """Scratch for a few images at a time: the runs add to the same partial tiles."""
+    n, c = 37, 40
+    x = torch.randn(n, c, 10, 10, device='cuda')
+    ref = conv_ref(x, (3, 3), (1, 1), (1, 1), (1, 1), True)
+    d = ref.shape[0]
+    for space in (900_000, 2_000_000, 64_000_000):
+        out = torch.empty(d, d, device='cuda')
+        ws = torch.empty(space, dtype=torch.uint8, device='cuda')
+        nat._check(nat.lib().sso_factor_syrk_im2col(x.data_ptr(), nat.F32, n, c, 10, 10, *x.stride(), 3, 3, 1, 1, 1, 1, 1, 1, 1, None, 1.0, 0.0,
+                                                    out.data_ptr(), d, ws.data_ptr(), space, nat.IMPL_AUTO, nat._stream()))
+        assert rel(out, ref) < 1e-6
+
+
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize('rows,cols,bias', [(16, 20, True), (50, 65, False), (100, 129, True)])
+def test_factor_direct_16bit(nat, rows, cols, bias, dtype):
+    x = torch.randn(rows, cols, device='cuda').to(dtype)
+    u = torch.cat([x.double(), torch.ones(rows, int(bias), device='cuda', dtype=torch.float64)], 1)
+    d = cols + int(bias)
+    out = torch.empty(d, d, device='cuda')
+    nat.factor_rows(x, bias, None, 1.0, 0.0, out)
+    assert rel(out, u.t() @ u) < 1e-6

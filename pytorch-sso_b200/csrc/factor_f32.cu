@@ -223,10 +223,12 @@ struct Gather {
       if (!((blocks >> b) & 1u)) continue;
       const int kp = kpos[b];
       const uint32_t d = dst + (b >> 1) * SIDE + (b & 1) * BLK;
-      if (kp == -1) {
+      if (kp == -1) {                              // like any other column, the row side takes the weight
+        uint32_t one[3];
+        split2(!rvalid ? 0.f : b < 2 && p.weight ? __ldg(p.weight + n) : 1.f, 0.f, one[0], one[1], one[2]);
 #pragma unroll
         for (int t = 0; t < 3; ++t)
-          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%2,%2};" ::"r"(d + t * OPB), "r"(t == 0 && rvalid ? 0x3F80u : 0u), "r"(0u) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%2,%2};" ::"r"(d + t * OPB), "r"(one[t]), "r"(0u) : "memory");
         continue;
       }
       bool in = rvalid && kp >= 0;
@@ -836,6 +838,7 @@ int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, c
                                                                                                   r == 0 ? header_words : 0, parts, parts);
     SSO_LAUNCH_OK("split_kernel");
     q.n = n;
+    q.weight = in.weight;
     q.rows = n * hw;
     q.accumulate = r > 0;
     q.tickets = fused && r == runs - 1 ? reinterpret_cast<int*>(base + 256) : nullptr;

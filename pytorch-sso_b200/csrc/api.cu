@@ -36,6 +36,7 @@ int factor_tma_set_wait_controls(long long cycles, int stall);
 int factor_tc_set_wait_controls(long long cycles, int stall);
 int engine_tc_set_wait_controls(long long cycles, int stall);
 int factor_f32_set_wait_controls(long long cycles, int stall);
+int flow_set_wait_controls(long long cycles, int stall);
 static long long g_wait_kcycles = 0;   // 0 = default limit
 static int g_stall = 0;
 static int apply_wait_controls() {
@@ -43,6 +44,7 @@ static int apply_wait_controls() {
   int rc = factor_tma_set_wait_controls(cycles, g_stall);
   if (!rc) rc = factor_tc_set_wait_controls(cycles, 0);
   if (!rc) rc = factor_f32_set_wait_controls(cycles, 0);
+  if (!rc) rc = flow_set_wait_controls(cycles, g_stall);
   if (!rc) rc = engine_tc_set_wait_controls(cycles, g_stall);
   return rc;
 }
@@ -75,7 +77,7 @@ static int g_tma_auto = 1;   // whether SSO_IMPL_AUTO may pick the TMA-fed tcgen
 
 using namespace sso;
 
-namespace sso { extern int g_engine_tma; extern int g_chol_ksplit; extern int g_phase_lpt; extern int g_chol_panel; }
+namespace sso { extern int g_flow; extern int g_engine_tma; extern int g_chol_ksplit; extern int g_phase_lpt; extern int g_chol_panel; }
 
 extern "C" {
 
@@ -95,6 +97,7 @@ int sso_configure(const char* key, int value) {
   if (k == "fused_finish") { factor_tma_set_fused_finish(value); return 0; }
   if (k == "tma_pair_min_d") { factor_tma_set_pair_min_d(value); return 0; }
   if (k == "engine_tma") { g_engine_tma = value != 0; return 0; }
+  if (k == "flow") { g_flow = value != 0; return 0; }
   if (k == "phase_lpt") { g_phase_lpt = value != 0; return 0; }
   if (k == "chol_ksplit") { g_chol_ksplit = (int)value; return 0; }
   if (k == "chol_panel") { g_chol_panel = value != 0; return 0; }

@@ -129,13 +129,22 @@ __device__ __forceinline__ void doubling_product(float* __restrict__ S, float* _
   }
 }
 
-template <int SZ>
+// Barrier of the 256 threads that factorise a block: the whole CTA, or eight warps of a larger one.
+struct CtaSync {
+  __device__ __forceinline__ static void sync() { __syncthreads(); }
+};
+template <int ID>
+struct NamedSync {
+  __device__ __forceinline__ static void sync() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory"); }
+};
+
+template <int SZ, typename Sync>
 __device__ __forceinline__ void doubling_level(float* S, float* V, int cols, int ty, int tx) {
   // ranges whose second half lies past the matrix (identity padding) keep Inv21 = 0
   for (int lo = 0; lo + SZ < cols; lo += 2 * SZ) doubling_product<SZ>(S, V, lo, 0, ty, tx);
-  __syncthreads();
+  Sync::sync();
   for (int lo = 0; lo + SZ < cols; lo += 2 * SZ) doubling_product<SZ>(S, V, lo, 1, ty, tx);
-  __syncthreads();
+  Sync::sync();
 }
 
 // Panel K of the thread's elements goes to shared memory (rows >= 16 K).
@@ -181,29 +190,16 @@ __device__ __forceinline__ void update_trailing(float (&a)[8][8], const float* _
   }
 }
 
-__global__ void __launch_bounds__(THREADS, 1) diag_panel_kernel(const sso_diag_rec* __restrict__ recs,
-                                                               int* __restrict__ info) {
-  extern __shared__ __align__(16) float psm[];
-  float* S = psm;               // panels of the block as they are published, then L (lower triangle)
-  float* V = psm + PN * PP;     // L^-1
-  float* dinv = V + PN * PP;    // 1 / L_jj
-  const sso_diag_rec rec = recs[blockIdx.x];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// The factorisation itself, by 256 threads: a[i][j] of thread (ty, tx) is the block's element (ty + 16 i, tx + 16 j), j <= i,
+// rows and columns past n an identity.  Leaves L in S (lower triangle) and L^-1, with zeros above the diagonal and an
+// identity past n, in V.  `info` (nullable) receives the 1-based number row0 + pivot + 1 of the first bad pivot.
+template <typename Sync>
+__device__ __forceinline__ void factor_block(float (&a)[8][8], float* __restrict__ S, float* __restrict__ V, float* __restrict__ dinv, int n,
+                                             int* __restrict__ info, int row0, int tid) {
+  const int lane = tid & 31, warp = tid >> 5;
   const int ty = tid >> 4, tx = tid & 15;
-  const int n = rec.size;
   const int np = (n + PK - 1) / PK;     // panels that hold columns of the matrix
   const int cols = np * PK;
-
-  float a[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j <= i; ++j) {
-      const int r = ty + 16 * i, c = tx + 16 * j;
-      float v = (r == c) ? 1.f : 0.f;
-      if (r < n && c <= r) v = rec.L[(int64_t)r * rec.ld_l + c];
-      a[i][j] = v;
-    }
   for (int e = tid; e < PN * PP / 4; e += THREADS) st4(V + 4 * e, 0.f, 0.f, 0.f, 0.f);
   if (tid < PN) dinv[tid] = 1.f;
 
@@ -220,7 +216,7 @@ __global__ void __launch_bounds__(THREADS, 1) diag_panel_kernel(const sso_diag_r
       case 6: publish_panel<6>(a, S, ty, tx); break;
       default: publish_panel<7>(a, S, ty, tx); break;
     }
-    __syncthreads();
+    Sync::sync();
     // ---- 16x16 diagonal block by warp 0: lane l (and its twin l + 16) holds row l.  One exchange per pivot:
     // every lane fetches the raw column j (pivot included) from the lanes that own it, takes the rsqrt of
     // the pivot itself and applies the rank-1 update to its own row.
@@ -264,8 +260,7 @@ __global__ void __launch_bounds__(THREADS, 1) diag_panel_kernel(const sso_diag_r
           pv = fmaf(-x, x, d1);
         }
       }
-      if (first_bad >= 0 && lane == 0 && info && c0 + first_bad < n)
-        atomicCAS(info + 2 * rec.mat + rec.info_slot, 0, rec.row0 + c0 + first_bad + 1);
+      if (first_bad >= 0 && lane == 0 && info && c0 + first_bad < n) atomicCAS(info, 0, row0 + c0 + first_bad + 1);
       if (lane < PK) {
 #pragma unroll
         for (int q = 0; q < PK; q += 4)
@@ -273,7 +268,7 @@ __global__ void __launch_bounds__(THREADS, 1) diag_panel_kernel(const sso_diag_r
               q + 3 <= l ? r[q + 3] : 0.f);
       }
     }
-    __syncthreads();
+    Sync::sync();
     // ---- rows below the diagonal block: x * L16^T = a, one thread per row, right looking (each finished
     // unknown is subtracted from all later ones at once, so the dependent chain is two operations per step)
     {
@@ -297,7 +292,7 @@ __global__ void __launch_bounds__(THREADS, 1) diag_panel_kernel(const sso_diag_r
         for (int q = 0; q < PK; q += 4) st4(xr + q, x[q], x[q + 1], x[q + 2], x[q + 3]);
       }
     }
-    __syncthreads();
+    Sync::sync();
     // ---- trailing update
     if (k + 1 < np) {
       switch (k) {
@@ -318,7 +313,7 @@ __global__ void __launch_bounds__(THREADS, 1) diag_panel_kernel(const sso_diag_r
 #pragma unroll
       for (int i = j; i < 8; ++i) S[(ty + 16 * i) * PP + 16 * j + tx] = (i == j && ty == tx) ? 1.f : 0.f;
     }
-  __syncthreads();
+  Sync::sync();
   // ---- inverses of the 16x16 diagonal blocks: warp w, lane c = column c of block w
   if (lane < PK) {
     const int b0 = PK * warp, c = lane;
@@ -339,10 +334,34 @@ __global__ void __launch_bounds__(THREADS, 1) diag_panel_kernel(const sso_diag_r
       V[(b0 + c) * PP + b0 + c] = 1.f;
     }
   }
-  __syncthreads();
-  doubling_level<16>(S, V, cols, ty, tx);
-  doubling_level<32>(S, V, cols, ty, tx);
-  doubling_level<64>(S, V, cols, ty, tx);
+  Sync::sync();
+  doubling_level<16, Sync>(S, V, cols, ty, tx);
+  doubling_level<32, Sync>(S, V, cols, ty, tx);
+  doubling_level<64, Sync>(S, V, cols, ty, tx);
+}
+
+static __global__ void __launch_bounds__(THREADS, 1) diag_panel_kernel(const sso_diag_rec* __restrict__ recs,
+                                                               int* __restrict__ info) {
+  extern __shared__ __align__(16) float psm[];
+  float* S = psm;               // panels of the block as they are published, then L (lower triangle)
+  float* V = psm + PN * PP;     // L^-1
+  float* dinv = V + PN * PP;    // 1 / L_jj
+  const sso_diag_rec rec = recs[blockIdx.x];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ty = tid >> 4, tx = tid & 15;
+  const int n = rec.size;
+
+  float a[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j <= i; ++j) {
+      const int r = ty + 16 * i, c = tx + 16 * j;
+      float v = (r == c) ? 1.f : 0.f;
+      if (r < n && c <= r) v = rec.L[(int64_t)r * rec.ld_l + c];
+      a[i][j] = v;
+    }
+  factor_block<CtaSync>(a, S, V, dinv, n, info ? info + 2 * rec.mat + rec.info_slot : nullptr, rec.row0, tid);
   // ---- results: the lower triangle of L, L^-1 with zeros above its diagonal, and optionally the upper
   // triangle of the transpose of L^-1.  Nothing reads L above the diagonal, and the buffer of the transpose
   // is zeroed before the factorisation starts.

@@ -16,10 +16,12 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <queue>
 #include <vector>
 
 #include "common.cuh"
 #include "diag_panel.cuh"
+#include "flow.cuh"
 
 namespace sso {
 
@@ -31,6 +33,7 @@ int g_phase_lpt = 1;    // tasks of a 128-wide phase sorted by decreasing K
 int g_chol_ksplit = 6;  // Cholesky panel updates from this panel index on are cut along K (0: never)
 int g_engine_tma = 1;   // k-contiguous 128-wide tasks fetch their operands with TMA (tensor maps per task)
 int g_engine_tc = 1;    // run 128-wide tile phases on the tensor cores (3xTF32) instead of FFMA
+int g_flow = 1;         // factorisations and inverses run as one dataflow kernel (flow.cu); 0: phases of launches
 int g_chol_panel = 1;   // factorise a 128-column panel's diagonal block in one launch (else two 64-wide halves)
 
 constexpr int NB = 64;  // algorithmic block size of the factorisations
@@ -378,7 +381,19 @@ __global__ void __launch_bounds__(256) copy_kernel(const CopyRec* __restrict__ r
 // ------------------------------------------------------------------------------------------
 // plans
 // ------------------------------------------------------------------------------------------
+struct FlowProgram {
+  std::vector<flow::Task> tasks;
+  std::vector<flow::Mat> mats;
+  int n_flags = 0;
+  flow::Mat* d_mats = nullptr;
+  flow::Task* d_tasks = nullptr;
+  int* d_flags = nullptr;
+  int* d_sync = nullptr;
+  bool ready() const { return d_tasks != nullptr; }
+};
+
 struct Plan {
+  FlowProgram flow_inv, flow_std;
   std::vector<sso_tile_task> tasks;
   std::vector<DiagRec> diags;
   std::vector<CopyRec> copies;
@@ -834,53 +849,227 @@ static Plan* build_kron(int n, const int64_t* dims, float* const* src, float* co
   return p;
 }
 
+// ------------------------------------------------------------------------------------------
+// dataflow programs
+// ------------------------------------------------------------------------------------------
+// Adds the tasks of every matrix in an order in which each of them only depends on earlier ones and the CTAs, taking
+// them in that order, wait as little as possible: a list schedule on 148 workers with rough durations (a
+// 32-column stage 1 us, a tile's fixed cost 3 us, a diagonal block 22 us), longest remaining chain first among the tasks
+// that could run through without waiting.
+static void schedule_flow(FlowProgram& f, bool with_inverse) {
+  struct Node {
+    flow::Task t;
+    int deps[3];
+    int waiting = 0;          // dependencies not scheduled yet
+    float work, tail;         // whole duration; what is left to do once the last dependency is there
+    float chain = 0.f;        // longest chain from this task's start of tail to the end
+    float done = 0.f;         // simulated end
+    std::vector<int> next;
+  };
+  std::vector<Node> nodes;
+  for (size_t mi = 0; mi < f.mats.size(); ++mi) {
+    const int np = f.mats[mi].np;
+    std::vector<int> diag(np), panel(np * np, -1), invt(np * np, -1);
+    auto add = [&](int kind, int a, int b, std::initializer_list<int> deps, float stages, float last, float fixed) {
+      Node n;
+      n.t.kind = (int16_t)kind; n.t.mat = (int16_t)mi; n.t.a = (int16_t)a; n.t.b = (int16_t)b;
+      n.deps[0] = n.deps[1] = n.deps[2] = -1;
+      int k = 0;
+      for (int q : deps) if (q >= 0) n.deps[k++] = q;
+      n.work = stages + fixed;
+      n.tail = last + fixed;
+      nodes.push_back(n);
+      return (int)nodes.size() - 1;
+    };
+    for (int p = 0; p < np; ++p) {
+      diag[p] = add(flow::DIAG, p, p, {p > 0 ? panel[p * np + p - 1] : -1}, 4.f * p, 4.f, 25.f);
+      for (int i = p + 1; i < np; ++i)
+        panel[i * np + p] = add(flow::PANEL, i, p, {diag[p], p > 0 ? panel[i * np + p - 1] : -1, p > 0 ? panel[p * np + p - 1] : -1}, 4.f * p + 4.f, 4.f, 3.f);
+    }
+    if (with_inverse) {
+      for (int i = 1; i < np; ++i)
+        for (int j = 0; j < i; ++j)
+          invt[j * np + i] = add(flow::INVT, j, i, {j == i - 1 ? diag[j] : invt[j * np + i - 1], panel[i * np + i - 1], diag[i]}, 4.f * (i - j) + 4.f, 8.f, 3.f);
+      for (int i = np - 1; i >= 0; --i)
+        for (int j = 0; j <= i; ++j)
+          add(flow::PROD, i, j, {i == np - 1 ? diag[i] : invt[i * np + np - 1], j == np - 1 ? diag[j] : invt[j * np + np - 1]}, 4.f * (np - i), 4.f, 3.f);
+    }
+  }
+  const int n = (int)nodes.size();
+  for (int i = n - 1; i >= 0; --i) {
+    nodes[i].chain += nodes[i].tail;
+    for (int q : nodes[i].deps)
+      if (q >= 0) {
+        nodes[q].next.push_back(i);
+        ++nodes[i].waiting;
+        nodes[q].chain = std::max(nodes[q].chain, nodes[i].chain);
+      }
+  }
+  using Entry = std::pair<float, int>;
+  std::priority_queue<Entry> ready;                                                     // longest chain first
+  std::priority_queue<Entry, std::vector<Entry>, std::greater<Entry>> later, workers;   // by time
+  auto release = [&](int i) {
+    float last = 0.f;
+    for (int q : nodes[i].deps)
+      if (q >= 0) last = std::max(last, nodes[q].done);
+    later.push({std::max(0.f, last - (nodes[i].work - nodes[i].tail)), i});
+  };
+  for (int w = 0; w < 148; ++w) workers.push({0.f, w});
+  for (int i = 0; i < n; ++i)
+    if (nodes[i].waiting == 0) release(i);
+  f.tasks.reserve(n);
+  while (!ready.empty() || !later.empty()) {
+    Entry w = workers.top();
+    workers.pop();
+    while (!later.empty() && later.top().first <= w.first) { ready.push({nodes[later.top().second].chain, later.top().second}); later.pop(); }
+    int i;
+    float start = w.first;
+    if (!ready.empty()) { i = ready.top().second; ready.pop(); }
+    else { i = later.top().second; start = later.top().first; later.pop(); }
+    Node& nd = nodes[i];
+    float last = 0.f;
+    for (int q : nd.deps)
+      if (q >= 0) last = std::max(last, nodes[q].done);
+    nd.done = std::max(start + nd.work, last + nd.tail);
+    workers.push({nd.done, w.second});
+    f.tasks.push_back(nd.t);
+    for (int q : nd.next)
+      if (--nodes[q].waiting == 0) release(q);
+  }
+}
+
+static size_t flow_task_count(int np, bool with_inverse) { return np + (size_t)np * (np - 1) / 2 + (with_inverse ? (size_t)np * np : 0); }
+static size_t flow_bytes(size_t tasks, size_t mats, size_t flags) {
+  return align_up(mats * sizeof(flow::Mat)) + align_up(tasks * sizeof(flow::Task)) + align_up(flags * sizeof(int)) + 256;
+}
+
+static int upload_flow(FlowProgram& f, char*& q) {
+  f.d_mats = reinterpret_cast<flow::Mat*>(q); q += align_up(f.mats.size() * sizeof(flow::Mat));
+  f.d_tasks = reinterpret_cast<flow::Task*>(q); q += align_up(f.tasks.size() * sizeof(flow::Task));
+  f.d_flags = reinterpret_cast<int*>(q); q += align_up(f.n_flags * sizeof(int));
+  f.d_sync = reinterpret_cast<int*>(q); q += 256;
+  SSO_CUDA_OK(cudaMemset(f.d_flags, 0, reinterpret_cast<char*>(f.d_sync) + 256 - reinterpret_cast<char*>(f.d_flags)));
+  SSO_CUDA_OK(cudaMemcpy(f.d_mats, f.mats.data(), f.mats.size() * sizeof(flow::Mat), cudaMemcpyHostToDevice));
+  SSO_CUDA_OK(cudaMemcpy(f.d_tasks, f.tasks.data(), f.tasks.size() * sizeof(flow::Task), cudaMemcpyHostToDevice));
+  return 0;
+}
+
+static int run_flow(const Plan& p, const FlowProgram& f, const float* damp_r, int* info, int clear_info, bool with_traces, cudaStream_t st) {
+  flow::Args a;
+  a.mats = f.d_mats; a.tasks = f.d_tasks; a.n_tasks = (int)f.tasks.size();
+  a.sync = f.d_sync; a.flags = f.d_flags; a.traces = p.d_traces; a.damp_r = damp_r;
+  a.info = info; a.status = p.d_status;
+  return flow_launch(a, (int)f.mats.size(), clear_info, with_traces, st);
+}
+
 }  // namespace sso
 
 using namespace sso;
 
 extern "C" {
 
-static size_t kron_scratch_bytes(int n_mats, const int64_t* dims) {
-  size_t b = 0;
-  for (int i = 0; i < n_mats; ++i) b += align_up((size_t)dims[i] * (size_t)padded_ld((int)dims[i]) * sizeof(float));
-  return b;
+// Scratch at the head of a plan's memory, per matrix: X (L^-T; its lower blocks hold L in the dataflow program) and the
+// inverses of the diagonal blocks.
+struct KronScratch {
+  size_t x, li;      // offsets
+};
+static size_t kron_scratch(int n_mats, const int64_t* dims, std::vector<KronScratch>* out) {
+  size_t at = 0;
+  for (int i = 0; i < n_mats; ++i) {
+    KronScratch k;
+    k.x = at; at += align_up((size_t)dims[i] * (size_t)padded_ld((int)dims[i]) * sizeof(float));
+    k.li = at; at += (size_t)((dims[i] + 127) / 128) * 65536;
+    if (out) out->push_back(k);
+  }
+  return at;
 }
+
+static bool flow_enabled() { return g_flow && g_engine_tma && g_engine_tc && g_chol_panel; }
 
 size_t sso_kron_plan_dev_bytes(int n_mats, const int64_t* dims, int with_std) {
   if (n_mats <= 0 || !dims) return 0;
+  size_t bytes = kron_scratch(n_mats, dims, nullptr) + 256;
+  if (flow_enabled()) {
+    size_t ti = 0, ts = 0, flags = 0;
+    for (int i = 0; i < n_mats; ++i) {
+      const int np = (int)((dims[i] + 127) / 128);
+      ti += flow_task_count(np, true);
+      ts += flow_task_count(np, false);
+      flags += 2 * (size_t)np * np + np;
+    }
+    return bytes + flow_bytes(ti, n_mats, flags) + (with_std ? flow_bytes(ts, n_mats, flags) : 0) + plan_table_bytes(0, 0, 0, n_mats);
+  }
   std::vector<float*> fake(n_mats, nullptr);
   std::vector<float*> fake_x(n_mats, reinterpret_cast<float*>(4096));   // non-null: the scratch matrices exist
   Plan* p = build_kron(n_mats, dims, fake.data(), fake.data(), fake.data(),
                        with_std ? fake.data() : nullptr, nullptr, nullptr, fake_x.data(), nullptr);
-  const size_t bytes = plan_table_bytes(p->tasks.size(), p->diags.size(), p->copies.size(), p->mats.size());
+  bytes += plan_table_bytes(p->tasks.size(), p->diags.size(), p->copies.size(), p->mats.size());
   delete p;
-  return kron_scratch_bytes(n_mats, dims) + 256 + bytes;
+  return bytes;
 }
 
 int64_t sso_kron_plan_create(int n_mats, const int64_t* dims, float* const* src, float* const* dst,
                              float* const* work, float* const* std_out, const int32_t* partner,
                              const int32_t* role, void* dev_mem, size_t dev_mem_bytes, int host_only,
                              const int64_t* lds) {
-  SSO_CHECK_ARG(n_mats > 0 && dims && src && dst && work, "kron plan: null argument");
+  SSO_CHECK_ARG(n_mats > 0 && n_mats < 32768 && dims && src && dst && work, "kron plan: null argument");
   for (int i = 0; i < n_mats; ++i) {
     SSO_CHECK_ARG(dims[i] > 0 && dims[i] <= 32768, "kron plan: bad dim %lld", (long long)dims[i]);
     SSO_CHECK_ARG(src[i] && dst[i] && work[i], "kron plan: null matrix pointer at %d", i);
     if (partner && partner[i] >= 0) SSO_CHECK_ARG(partner[i] < n_mats, "kron plan: bad partner");
   }
-  // the head of the plan's memory holds one scratch matrix per factor (the transposed triangular
-  // inverse); the tables follow.  A host-only plan needs (host) memory for the scratch part only.
-  const size_t scratch = kron_scratch_bytes(n_mats, dims) + 256;
+  // the head of the plan's memory holds the scratch matrices; the tables follow.  A host-only plan needs (host)
+  // memory for the scratch part only.
+  std::vector<KronScratch> where;
+  const size_t scratch = kron_scratch(n_mats, dims, &where) + 256;
   SSO_CHECK_ARG(dev_mem != nullptr && dev_mem_bytes >= scratch, "kron plan: plan memory too small for the scratch matrices");
-  std::vector<float*> xb(n_mats);
-  {
-    char* q = reinterpret_cast<char*>(align_up(reinterpret_cast<uintptr_t>(dev_mem)));
-    for (int i = 0; i < n_mats; ++i) {
-      xb[i] = reinterpret_cast<float*>(q);
-      q += align_up((size_t)dims[i] * (size_t)padded_ld((int)dims[i]) * sizeof(float));
-    }
-  }
+  char* head = reinterpret_cast<char*>(align_up(reinterpret_cast<uintptr_t>(dev_mem)));
   if (lds)
     for (int i = 0; i < n_mats; ++i) SSO_CHECK_ARG(lds[i] >= dims[i], "kron plan: leading dimension %lld < dim %lld", (long long)lds[i], (long long)dims[i]);
+  std::vector<float*> xb(n_mats);
+  for (int i = 0; i < n_mats; ++i) xb[i] = reinterpret_cast<float*>(head + where[i].x);
+  if (!host_only && flow_enabled()) {
+    Plan* p = new Plan();
+    bool ok = true;
+    auto fill = [&](FlowProgram& f, bool inverse) {
+      for (int i = 0; i < n_mats; ++i) {
+        const int d = (int)dims[i], ld = lds ? (int)lds[i] : d;
+        flow::Mat m{};
+        m.d = d; m.np = (d + 127) / 128; m.mat = i;
+        m.src = inverse ? src[i] : dst[i]; m.ld_src = ld;
+        m.W = xb[i]; m.ldw = padded_ld(d);
+        m.Li = reinterpret_cast<float*>(head + where[i].li);
+        m.X = inverse ? xb[i] : nullptr;
+        m.T = inverse ? dst[i] : nullptr; m.ldt = ld;
+        m.U = inverse ? nullptr : std_out[i]; m.ldu = ld;
+        m.shifted = inverse; m.partner = partner ? partner[i] : -1; m.role = role ? role[i] : 0;
+        m.d_partner = m.partner >= 0 ? (int)dims[m.partner] : 0;
+        m.info_slot = inverse ? 0 : 1;
+        m.flag_w = f.n_flags; m.flag_x = m.flag_w + m.np * m.np; m.flag_d = m.flag_x + m.np * m.np;
+        f.n_flags += 2 * m.np * m.np + m.np;
+        ok = ok && tma_encode_f32_rows(m.map_w, m.W, d, d, m.ldw) &&
+             tma_encode_f32_rows(m.map_li, m.Li, (int64_t)m.np * 128, 128, 128);
+        f.mats.push_back(m);
+      }
+      if (ok) schedule_flow(f, inverse);
+    };
+    fill(p->flow_inv, true);
+    if (std_out && ok) fill(p->flow_std, false);
+    p->mats.resize(n_mats);
+    const size_t tables = plan_table_bytes(0, 0, 0, n_mats);
+    const size_t need = scratch + tables + flow_bytes(p->flow_inv.tasks.size(), n_mats, p->flow_inv.n_flags) +
+                        (std_out ? flow_bytes(p->flow_std.tasks.size(), n_mats, p->flow_std.n_flags) : 0);
+    if (ok) {
+      if (dev_mem_bytes < need) { delete p; return fail(-1, "kron plan: plan memory too small: need %zu, got %zu", need, dev_mem_bytes); }
+      int rc = upload(*p, head + scratch - 256, tables);
+      char* q = head + scratch - 256 + align_up(tables);
+      if (!rc) rc = upload_flow(p->flow_inv, q);
+      if (!rc && std_out) rc = upload_flow(p->flow_std, q);
+      if (rc) { delete p; return rc; }
+      return register_plan(p);
+    }
+    delete p;      // no tensor maps to be had: phases of launches
+  }
   Plan* p = build_kron(n_mats, dims, src, dst, work, std_out, partner, role, xb.data(), lds);
   p->host_only = host_only != 0;
   if (!p->host_only) {
@@ -897,9 +1086,16 @@ int sso_kron_plan_run(int64_t plan, const float* damp_r_dev, int* info_dev, int 
   SSO_CHECK_ARG(!p->host_only, "plan %lld was built host-only", (long long)plan);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int n = (int)p->mats.size();
+  SSO_CHECK_ARG(!do_inverse || damp_r_dev != nullptr, "kron run: damping table is null");
+  if (p->flow_inv.ready()) {
+    SSO_CHECK_ARG(!do_std || p->flow_std.ready(), "plan %lld has no std program", (long long)plan);
+    int rc = 0;
+    if (do_inverse) rc = run_flow(*p, p->flow_inv, damp_r_dev, info_dev, 1, true, st);
+    if (!rc && do_std) rc = run_flow(*p, p->flow_std, damp_r_dev, info_dev, !do_inverse, false, st);
+    return rc;
+  }
   if (info_dev) SSO_CUDA_OK(cudaMemsetAsync(info_dev, 0, 2 * n * sizeof(int), st));
   if (do_inverse) {
-    SSO_CHECK_ARG(damp_r_dev != nullptr, "kron run: damping table is null");
     trace_kernel<<<n, 256, 0, st>>>(p->d_mats, p->d_traces);
     SSO_LAUNCH_OK("trace_kernel");
     shift_kernel<<<ceil_div(n, 128), 128, 0, st>>>(p->d_mats, p->d_traces, damp_r_dev, p->d_shift, n);

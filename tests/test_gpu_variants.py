@@ -145,3 +145,58 @@ def test_factor_direct_16bit(nat, rows, cols, bias, dtype):
     out = torch.empty(d, d, device='cuda')
     nat.factor_rows(x, bias, None, 1.0, 0.0, out)
     assert rel(out, u.t() @ u) < 1e-6
+
+
+# ----------------------------------------------------------------------- factorisation and inverse
+FLOW_DIMS = [[1], [10, 127], [128], [129, 128], [256, 1, 257], [300, 640, 64, 31, 385, 512], [1153]]
+
+
+def spd(d, ld, seed):
+    g = torch.Generator(device='cuda').manual_seed(seed)
+    x = torch.randn(3 * d + 8, d, device='cuda', generator=g)
+    out = torch.full((d, ld), float('nan'), device='cuda')
+    out[:, :d] = x.t() @ x / x.shape[0]
+    return out[:, :d]
+
+
+@pytest.mark.parametrize('std', [False, True])
+@pytest.mark.parametrize('pad', [0, 3])
+@pytest.mark.parametrize('dims', FLOW_DIMS)
+def test_kron_plan_in_one_kernel(nat, dims, pad, std):
+    """Tile edges, several matrices, odd row strides; the same bits from a second run."""
+    src = [spd(d, d + pad, i) for i, d in enumerate(dims)]
+    dst, work, sd = ([torch.full((d, d + pad), float('nan'), device='cuda')[:, :d] for d in dims] for _ in range(3))
+    sd = sd if std else None
+    n = len(dims)
+    plan = nat.kron_plan(dims, src, dst, work, sd, [-1] * n, [0] * n, torch.device('cuda'))
+    damp = torch.full((n,), 0.02, device='cuda')
+    info = torch.zeros(2 * n, dtype=torch.int32, device='cuda')
+    nat.kron_plan_run(plan, damp, info, True, std)
+    first = [t.clone() for t in dst + (sd or [])]
+    nat.kron_plan_run(plan, damp, info, True, std)
+    assert not info.any()
+    for t, f in zip(dst + (sd or []), first):
+        assert torch.equal(t, f)
+    for i, (m, out) in enumerate(zip(src, dst)):
+        want = torch.linalg.inv(m.double() + 0.02 * torch.eye(dims[i], device='cuda', dtype=torch.float64))
+        assert rel(out, want) < 1e-5 and torch.equal(out, out.t())
+        if std:
+            assert rel(sd[i], torch.linalg.cholesky(out.double(), upper=True)) < 1e-5
+            assert torch.equal(sd[i], sd[i].triu())
+
+
+@pytest.mark.parametrize('at', [0, 127, 128, 290])
+def test_kron_plan_reports_the_bad_pivot(nat, at):
+    """One matrix of three is not positive definite: its pivot is named and the others are as they would be without it."""
+    dims = [130, 300, 64]
+    src = [spd(d, d, i) for i, d in enumerate(dims)]
+    src[1] = torch.eye(300, device='cuda')
+    src[1][at, at] = -5.0
+    dst = [torch.zeros(d, d, device='cuda') for d in dims]
+    plan = nat.kron_plan(dims, src, dst, [torch.empty_like(m) for m in dst], None, [-1] * 3, [0] * 3, torch.device('cuda'))
+    info = torch.zeros(6, dtype=torch.int32, device='cuda')
+    nat.kron_plan_run(plan, torch.full((3,), 0.02, device='cuda'), info, True, False)
+    assert info.tolist() == [0, 0, at + 1, 0, 0, 0]
+    for i in (0, 2):
+        want = torch.linalg.inv(src[i].double() + 0.02 * torch.eye(dims[i], device='cuda', dtype=torch.float64))
+        assert rel(dst[i], want) < 1e-5

@@ -45,8 +45,7 @@ uint64_t sso_launch_count(void);
  * the TMA-fed one), "engine_tc" (0/1: 128-wide tile phases of the engine on tcgen05 3xTF32 or fp32 FFMA),
  * "tc_flush" (stages of tensor-core accumulation between drains into fp32 registers),
  * "chol_ksplit" (first 128-column panel of the blocked Cholesky whose update tasks are cut along K;
- * 0 = never; read when a plan is built), "rowwise_max_splits" (column-permuted factors of >= 1024 columns with
- * at most this many row splits are finished by the kernel that writes whole output rows), "chol_panel" (0/1: a panel's 128x128 diagonal block is factorised
+ * 0 = never; read when a plan is built), "chol_panel" (0/1: a panel's 128x128 diagonal block is factorised
  * and inverted by one launch, or as two 64-wide halves; read when a plan is built), "phase_lpt" (0/1: tasks
  * of a 128-wide phase ordered by decreasing K, so that the longest tasks of a launch start first; read when
  * a plan is built) */
@@ -162,6 +161,19 @@ int sso_bn_plane_sums(const void* y, const void* g, int dtype, int64_t n, int64_
 int sso_bn_diag_finish(const float* sx, const float* sg, const float* sample_weight,
                        int64_t n, int64_t c, int splits_x, int splits_g, float alpha, float beta,
                        float* w_out, float* b_out, void* stream);
+
+/* The gradient half and the finishing call of many layers in one call; sx of every layer holds its sums over the output. */
+typedef struct {
+  const void* g;                  /* [n, c, hw] */
+  int32_t dtype, splits_g, splits_x;
+  float alpha, beta;
+  int64_t n, c, hw, sn, sc, sp;   /* strides of g in elements */
+  float* sg;                      /* [n, splits_g, c] scratch */
+  const float* sx;                /* [n, splits_x, c] */
+  const float* sample_weight;     /* nullable */
+  float *w_out, *b_out;           /* b_out nullable */
+} sso_bn_desc;
+int sso_bn_batch(int n, const sso_bn_desc* descs, void* stream);
 
 /* ---------------------------------------------------------------------------------------
  * Streaming kernels over flat fp32 buffers.  The Python side keeps every factor of every

@@ -10,13 +10,11 @@
 //               MN-major canonical layout without swizzle) and commits to mbarriers;
 //   warps 9-16  gather: fused im2col.  16-byte global loads of consecutive channels
 //               (channels-contiguous inputs: channels_last activations, row-major matrices),
-//               conversion in registers, 16-byte shared stores straight into the UMMA operand
-//               layout, fence.proxy.async, mbarrier arrive.
-// bf16/fp16 inputs: one kind::f16 pass (products of 16-bit values are exact in fp32).
-// fp32 inputs: 3xTF32 -- x = hi + lo with hi = rna_tf32(x); hi*hi + hi*lo + lo*hi as three
-// kind::tf32 MMAs per k-slice into the same accumulator.
+//               copied (cp.async) straight into the UMMA operand layout, fence.proxy.async,
+//               mbarrier arrive.
+// bf16/fp16 inputs (fp32: factor_f32.cu): one kind::f16 pass (products of 16-bit values are exact in fp32).
 // Column order inside the kernel is (kh, kw, c) so that 16 bytes are one chunk of channels; the
-// finishing kernel (factor_tc_reduce) permutes to the (c, kh, kw) order of the public result,
+// finishing kernel (factor_units.cuh) permutes to the (c, kh, kw) order of the public result,
 // sums the splits in a fixed order and applies alpha / beta and the mirror.
 //
 // Every wait is bounded: on a timeout the role records a code in the status word, leaves its
@@ -25,6 +23,7 @@
 
 #include "common.cuh"
 #include "factor_params.cuh"
+#include "factor_units.cuh"
 #include "tc_common.cuh"
 
 namespace sso {
@@ -46,26 +45,17 @@ struct Cfg;
 //  16-bit inputs, MN-major: 16 bytes = 8 consecutive columns (channels) of one row k;
 //      addr(chunk, k) = chunk*SBO + (k/8)*LBO + (k%8)*16.  The 16 bytes a gather thread fetches
 //      are stored as they are.
-//  fp32 inputs, K-major (tf32 operands are transposed on the way in): 16 bytes = 4 consecutive
-//      rows k of one column;  addr(col, k) = (col/8)*SBO + (k/4)*LBO + (col%8)*16 + (k%4)*4.
-//  LBO = 128 and SBO = 1040 = 8*128 + 16 in both: the 16 extra bytes rotate consecutive chunks /
-//  column groups across the banks, so the 8 chunks of one 128-byte global line (16-bit) and the
-//  32 scalar stores of a warp (fp32) are bank-conflict free.
-template <>
-struct Cfg<float> {
-  static constexpr int KS = 32, CH = 4, STAGES = 3, PARTS = 2, LAG = 0, FLUSH = 2;
-  static constexpr uint32_t FMT = 2, MAJOR = 0;  // tf32, K-major
-  static constexpr uint32_t LBO = 128, SBO = 1040, OPB = 16 * 1040, KSTEP = 2 * 128;
-};
+//  LBO = 128 and SBO = 1040 = 8*128 + 16: the 16 extra bytes rotate consecutive chunks across the
+//  banks, so the 8 chunks of one 128-byte global line are bank-conflict free.
 template <>
 struct Cfg<__nv_bfloat16> {
-  static constexpr int KS = 64, CH = 8, STAGES = 6, PARTS = 1, LAG = 4, FLUSH = 8;
+  static constexpr int KS = 64, CH = 8, STAGES = 6, LAG = 4, FLUSH = 8;
   static constexpr uint32_t FMT = 1, MAJOR = 1;  // bf16, MN-major
   static constexpr uint32_t LBO = 128, SBO = 1040, OPB = 16 * 1040, KSTEP = 2 * 128;
 };
 template <>
 struct Cfg<__half> {
-  static constexpr int KS = 64, CH = 8, STAGES = 6, PARTS = 1, LAG = 4, FLUSH = 8;
+  static constexpr int KS = 64, CH = 8, STAGES = 6, LAG = 4, FLUSH = 8;
   static constexpr uint32_t FMT = 0, MAJOR = 1;  // f16, MN-major
   static constexpr uint32_t LBO = 128, SBO = 1040, OPB = 16 * 1040, KSTEP = 2 * 128;
 };
@@ -73,9 +63,9 @@ struct Cfg<__half> {
 template <typename T>
 __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParams p, int flush) {
   using C = Cfg<T>;
-  constexpr int KS = C::KS, CH = C::CH, STAGES = C::STAGES, PARTS = C::PARTS;
+  constexpr int KS = C::KS, CH = C::CH, STAGES = C::STAGES;
   constexpr uint32_t OPB = C::OPB, SBO = C::SBO, LBO = C::LBO, KSTEP = C::KSTEP;
-  constexpr uint32_t STAGE_BYTES = 2 * PARTS * OPB;
+  constexpr uint32_t STAGE_BYTES = 2 * OPB;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * STAGES + 4];
   __shared__ uint32_t tmem_base_slot;
@@ -83,7 +73,7 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int bi, bj;
   tri_decode(blockIdx.x, bi, bj);
-  const bool share = (bi == bj) && (p.weight == nullptr);
+  const bool share = bi == bj;
   const int split = blockIdx.y;
   const int64_t r_begin = (int64_t)split * p.rows_per_split;
   const int64_t r_end = min(p.rows, r_begin + (int64_t)p.rows_per_split);
@@ -162,24 +152,13 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
         const uint32_t sb = smem0 + slot * STAGE_BYTES;
         const uint32_t d_tmem = tmem_base + (uint32_t)(b * TILE);
         if (dbg_no_mma && s > 0) {
-        } else if (PARTS == 1) {
+        } else {
           const uint32_t a0 = sb, b0 = share ? sb : sb + OPB;
 #pragma unroll
           for (int ks = 0; ks < KS / 16; ++ks) {
             const uint64_t ad = smem_desc(a0 + ks * KSTEP, LBO, SBO);
             const uint64_t bd = smem_desc(b0 + ks * KSTEP, LBO, SBO);
             umma<false>(d_tmem, ad, bd, idesc, (first_of_chunk && ks == 0) ? 0u : 1u);
-          }
-        } else {
-          const uint32_t ah = sb, al = sb + OPB;
-          const uint32_t bh = share ? ah : sb + 2 * OPB, bl = share ? al : sb + 3 * OPB;
-#pragma unroll
-          for (int ks = 0; ks < KS / 8; ++ks) {
-            const uint64_t adh = smem_desc(ah + ks * KSTEP, LBO, SBO), adl = smem_desc(al + ks * KSTEP, LBO, SBO);
-            const uint64_t bdh = smem_desc(bh + ks * KSTEP, LBO, SBO), bdl = smem_desc(bl + ks * KSTEP, LBO, SBO);
-            umma<true>(d_tmem, adl, bdh, idesc, (first_of_chunk && ks == 0) ? 0u : 1u);
-            umma<true>(d_tmem, adh, bdl, idesc, 1u);
-            umma<true>(d_tmem, adh, bdh, idesc, 1u);
           }
         }
         umma_commit(empty_bar(slot));
@@ -194,8 +173,8 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
     // 128 -> one conflict-free wavefront per line.  A warp instruction covers 4 consecutive rows.
     const int lt = tid - 32 * (MMA_WARP + 1);      // 0 .. 255
     const int l8 = lt & 7, q = lt >> 3;            // chunk within its group, item slot 0..31
-    constexpr int GROUPS = TILE / (8 * CH);        // chunk groups per operand (2 or 4)
-    constexpr int ROWS_PER_THREAD = KS / 32;       // rows q, q+32, ... of the stage: 1 (fp32) or 2 (16-bit)
+    constexpr int GROUPS = TILE / (8 * CH);        // chunk groups per operand
+    constexpr int ROWS_PER_THREAD = KS / 32;       // rows q, q+32, ... of the stage
     constexpr int G_PER_ROW = GROUPS;              // a thread covers chunk l8 of every group of its rows
     const T* xp = reinterpret_cast<const T*>(p.x);
     const int Cc = p.c;
@@ -244,110 +223,53 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
       wn[j] += step_n;
     };
     bool ok = true;
-    if (PARTS == 1) {
-      // 16-bit inputs need no conversion: cp.async copies 16 bytes global -> shared straight
-      // into the operand layout (zero-filling where the patch leaves the image), with LAG
-      // stages in flight per thread; a stage is handed to the MMA warp once its copies landed.
-      constexpr int LAG = C::LAG;
-      for (int s = 0; s < nstages + LAG && ok; ++s) {
-        if (s < nstages) {
-          const int slot = s % STAGES;
-          if (s >= STAGES) ok = mbar_wait(empty_bar(slot), ((s / STAGES) - 1) & 1, status, 4);
-          if (!ok) break;
-          const uint32_t sb = smem0 + slot * STAGE_BYTES;
-#pragma unroll
-          for (int j = 0; j < ROWS_PER_THREAD; ++j) {
-            const int krow = q + 32 * j;
-            const bool rvalid = rr[j] < r_end;
-            const int ih0 = wy[j] * p.stride_h - p.pad_h, iw0 = wx[j] * p.stride_w - p.pad_w;
-            const T* pix = xp + ((int64_t)wn[j] * p.sn + (int64_t)ih0 * p.sh + (int64_t)iw0 * p.sw);
-            const uint32_t arow = sb + l8 * SBO + (krow >> 3) * LBO + (krow & 7) * 16;
-#pragma unroll
-            for (int op = 0; op < 2; ++op) {
-              if (op >= nops) continue;
-#pragma unroll
-              for (int g = 0; g < G_PER_ROW; ++g) {
-                const uint32_t a = arow + op * OPB + g * 8 * SBO;
-                const int kp = kpos[op][g];
-                if (kp == -1) {
-                  const uint32_t one = !rvalid ? 0u : (C::FMT == 1 ? 0x3F80u : 0x3C00u);
-                  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%2,%2};" ::"r"(a), "r"(one), "r"(0u) : "memory");
-                } else {
-                  bool in = rvalid && kp >= 0;
-                  if (!no_halo)
-                    in = in && (unsigned)(ih0 + (kp & 0xFFFF)) < (unsigned)p.h &&
-                         (unsigned)(iw0 + (kp >> 16)) < (unsigned)p.w;
-                  if (dbg_no_gather) continue;
-                  const T* src = in ? pix + koff[op][g] : xp;
-                  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(src), "r"(in ? 16 : 0) : "memory");
-                }
-              }
-            }
-            advance(j);
-          }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (s >= LAG) {
-          asm volatile("cp.async.wait_group %0;" ::"n"(LAG) : "memory");
-          fence_async_smem();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(full_bar((s - LAG) % STAGES));   // one arrival per warp
-        }
-      }
-    } else {
-      // fp32 inputs: 16-byte loads into registers, split into tf32 hi / lo, transposing scalar
-      // stores into the K-major operand layout (bank-conflict free thanks to the padded SBO)
-      for (int s = 0; s < nstages && ok; ++s) {
+    // 16-bit inputs need no conversion: cp.async copies 16 bytes global -> shared straight
+    // into the operand layout (zero-filling where the patch leaves the image), with LAG
+    // stages in flight per thread; a stage is handed to the MMA warp once its copies landed.
+    constexpr int LAG = C::LAG;
+    for (int s = 0; s < nstages + LAG && ok; ++s) {
+      if (s < nstages) {
         const int slot = s % STAGES;
-        const int krow = q;
-        const bool rvalid = rr[0] < r_end;
-        const int ih0 = wy[0] * p.stride_h - p.pad_h, iw0 = wx[0] * p.stride_w - p.pad_w;
-        const T* pix = xp + ((int64_t)wn[0] * p.sn + (int64_t)ih0 * p.sh + (int64_t)iw0 * p.sw);
-        const float wgt = (p.weight && rvalid) ? p.weight[wn[0]] : 1.f;
-        uint4 v[2][G_PER_ROW];
-#pragma unroll
-        for (int op = 0; op < 2; ++op)
-#pragma unroll
-          for (int g = 0; g < G_PER_ROW; ++g) {
-            v[op][g] = make_uint4(0u, 0u, 0u, 0u);
-            if (op < nops && rvalid) {
-              const int kp = kpos[op][g];
-              if (kp >= 0) {
-                if (no_halo || ((unsigned)(ih0 + (kp & 0xFFFF)) < (unsigned)p.h &&
-                                (unsigned)(iw0 + (kp >> 16)) < (unsigned)p.w))
-                  v[op][g] = __ldg(reinterpret_cast<const uint4*>(pix + koff[op][g]));
-              } else if (kp == -1) {
-                v[op][g].x = __float_as_uint(1.f);
-              }
-            }
-          }
-        advance(0);
         if (s >= STAGES) ok = mbar_wait(empty_bar(slot), ((s / STAGES) - 1) & 1, status, 4);
         if (!ok) break;
-        const uint32_t sb = smem0 + slot * STAGE_BYTES + (krow >> 2) * LBO + (krow & 3) * 4;
+        const uint32_t sb = smem0 + slot * STAGE_BYTES;
 #pragma unroll
-        for (int op = 0; op < 2; ++op) {
-          if (op >= nops) continue;
+        for (int j = 0; j < ROWS_PER_THREAD; ++j) {
+          const int krow = q + 32 * j;
+          const bool rvalid = rr[j] < r_end;
+          const int ih0 = wy[j] * p.stride_h - p.pad_h, iw0 = wx[j] * p.stride_w - p.pad_w;
+          const T* pix = xp + ((int64_t)wn[j] * p.sn + (int64_t)ih0 * p.sh + (int64_t)iw0 * p.sw);
+          const uint32_t arow = sb + l8 * SBO + (krow >> 3) * LBO + (krow & 7) * 16;
 #pragma unroll
-          for (int g = 0; g < G_PER_ROW; ++g) {
-            float f[4] = {__uint_as_float(v[op][g].x), __uint_as_float(v[op][g].y), __uint_as_float(v[op][g].z),
-                          __uint_as_float(v[op][g].w)};
-            const int col0 = (g * 8 + l8) * 4;
+          for (int op = 0; op < 2; ++op) {
+            if (op >= nops) continue;
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              if (op == 0) f[t] *= wgt;
-              const uint32_t hi = rna_tf32(f[t]);
-              const uint32_t lo = __float_as_uint(f[t] - __uint_as_float(hi));
-              const int col = col0 + t;
-              const uint32_t a = sb + op * (PARTS * OPB) + (col >> 3) * SBO + (col & 7) * 16;
-              asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(hi) : "memory");
-              asm volatile("st.shared.b32 [%0], %1;" ::"r"(a + OPB), "r"(lo) : "memory");
+            for (int g = 0; g < G_PER_ROW; ++g) {
+              const uint32_t a = arow + op * OPB + g * 8 * SBO;
+              const int kp = kpos[op][g];
+              if (kp == -1) {
+                const uint32_t one = !rvalid ? 0u : (C::FMT == 1 ? 0x3F80u : 0x3C00u);
+                asm volatile("st.shared.v4.b32 [%0], {%1,%2,%2,%2};" ::"r"(a), "r"(one), "r"(0u) : "memory");
+              } else {
+                bool in = rvalid && kp >= 0;
+                if (!no_halo)
+                  in = in && (unsigned)(ih0 + (kp & 0xFFFF)) < (unsigned)p.h &&
+                       (unsigned)(iw0 + (kp >> 16)) < (unsigned)p.w;
+                if (dbg_no_gather) continue;
+                const T* src = in ? pix + koff[op][g] : xp;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(src), "r"(in ? 16 : 0) : "memory");
+              }
             }
           }
+          advance(j);
         }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      if (s >= LAG) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(LAG) : "memory");
         fence_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(full_bar(slot));
+        if (lane == 0) mbar_arrive(full_bar((s - LAG) % STAGES));   // one arrival per warp
       }
     }
   }
@@ -360,102 +282,19 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
   }
 }
 
-// Sum the splits (fixed order), permute internal (kh,kw,c) columns to (c,kh,kw), apply
-// alpha / beta, mirror.  A non-zero status (a wait gave up) poisons the result with NaN.
-//
-// One CTA produces 32 output rows x one group of columns that is CONTIGUOUS in the output:
-// for permuted factors a block of up to 8 channels at all kernel positions (8*kk columns), else
-// 32 consecutive columns.  Inside the partial tiles such a group is kk runs of 8 consecutive
-// columns.  Elements on or below the diagonal are read from their own tile with the lanes along
-// the run; elements above it are read from the mirrored position with the lanes along the rows,
-// so global reads come in whole 32-byte sectors, writes in whole rows of the group, and both
-// halves of the symmetric result come from the same numbers (bitwise symmetric).  The block is
-// staged in shared memory.
-constexpr int RED_ROWS = 32, RED_CB = 8, RED_W = 32;
-
-// sum over the splits of element (r, c), r >= c, of the lower-triangle partial tiles; four
-// independent partial sums keep several loads in flight, combined in a fixed order
-__device__ __forceinline__ float reduce_fetch(const float* __restrict__ partial, int nsplit, int r, int c) {
-  const int bi = r >> 7, bj = c >> 7;
-  const float* src = partial + ((int64_t)(bi * (bi + 1) / 2 + bj) * nsplit) * (TILE * TILE) + part_at(r & 127, c & 127);
-  constexpr int64_t S = TILE * TILE;
-  float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-  int sp = 0;
-  for (; sp + 4 <= nsplit; sp += 4) {
-    a0 += src[sp * S];
-    a1 += src[(sp + 1) * S];
-    a2 += src[(sp + 2) * S];
-    a3 += src[(sp + 3) * S];
-  }
-  for (; sp < nsplit; ++sp) a0 += src[sp * S];
-  return (a0 + a1) + (a2 + a3);
+// launched early behind the kernel that writes the partial tiles: it waits for that one's end itself
+__global__ void __launch_bounds__(1024) factor_finish_units(const units::Problem u, const int* status) {
+  extern __shared__ float unit_smem[];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  units::finish(u, blockIdx.x, unit_smem, status);
 }
 
-__global__ void __launch_bounds__(256) factor_tc_reduce(const FactorParams p, int perm_groups, int pitch) {
-  extern __shared__ float rs[];
-  asm volatile("griddepcontrol.wait;" ::: "memory");      // launched early behind the kernel that writes the partial tiles
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int gi0 = blockIdx.x * RED_ROWS;
-  const int grp = blockIdx.y;
-  const int kk = p.perm_kk, C = p.perm_c, d = p.d, pub = p.perm_pub > 0 ? p.perm_pub : C;
-  int ext0, n_ext;      // public columns of this CTA
-  if (grp < perm_groups) {
-    const int c0 = grp * RED_CB, len = min(RED_CB, pub - c0);
-    ext0 = c0 * kk;
-    n_ext = len * kk;
-    // below / on the diagonal: 4 rows x 8 columns per warp; above: 32 rows x 1 column per warp
-    const int rrA = warp * 4 + (lane >> 3), eA = lane & 7, giA = gi0 + rrA;
-    const int rrB = lane, eB = warp, giB = gi0 + rrB;
-    const bool okA = eA < len && giA < d, okB = eB < len && giB < d;
-#pragma unroll 3
-    for (int run = 0; run < kk; ++run) {
-      const int gjA = run * C + c0 + eA, gjB = run * C + c0 + eB;
-      float vA = 0.f, vB = 0.f;
-      const bool doA = okA && gjA <= giA, doB = okB && gjB > giB;
-      if (doA) vA = reduce_fetch(p.partial, p.splits, giA, gjA);
-      if (doB) vB = reduce_fetch(p.partial, p.splits, gjB, giB);
-      if (doA) rs[rrA * pitch + eA * kk + run] = vA;
-      if (doB) rs[rrB * pitch + eB * kk + run] = vB;
-    }
-  } else {
-    const int int0 = (perm_groups > 0 ? p.dcols : 0) + (grp - perm_groups) * RED_W;      // internal column of ext0
-    ext0 = perm_groups > 0 ? pub * kk : int0;
-    n_ext = min(RED_W, d - int0);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int rrA = warp + 8 * k, giA = gi0 + rrA, gjA = int0 + lane;
-      const int eB = warp + 8 * k, giB = gi0 + lane, gjB = int0 + eB;
-      const bool doA = lane < n_ext && giA < d && gjA <= giA;
-      const bool doB = eB < n_ext && giB < d && gjB > giB;
-      float vA = 0.f, vB = 0.f;
-      if (doA) vA = reduce_fetch(p.partial, p.splits, giA, gjA);
-      if (doB) vB = reduce_fetch(p.partial, p.splits, gjB, giB);
-      if (doA) rs[rrA * pitch + lane] = vA;
-      if (doB) rs[lane * pitch + eB] = vB;
-    }
-  }
-  __syncthreads();
-  const bool bad = p.status && *p.status != 0;
-  for (int rr = warp; rr < RED_ROWS; rr += 8) {
-    const int gi = gi0 + rr;
-    if (gi >= d) break;
-    const int gr = public_column(p, gi);
-    if (gr < 0) continue;
-    float* orow = p.out + (int64_t)gr * p.ldo + ext0;
-    for (int e = lane; e < n_ext; e += 32) {
-      float v = p.alpha * rs[rr * pitch + e];
-      if (bad) v = __int_as_float(0x7fc00000);
-      orow[e] = (p.beta == 0.f) ? v : fmaf(p.beta, orow[e], v);
-    }
-  }
-}
-
-// Tile-wise variant of the finishing kernel: a CTA sums 1024/SL elements of one partial tile with
-// 16-byte loads and scatters them (and their mirror) to the output.  It wins when many splits
-// make the partial tiles, not the output, the bulk of the traffic.  With many splits and few
-// tiles, SL = 2, 4 or 8 neighbouring lanes share an element group: lane l sums splits l, l+SL, ...
+// Tile-wise variant of the finishing kernel, for permutations units do not cover: a CTA sums 1024/SL
+// elements of one partial tile with 16-byte loads and scatters them (and their mirror) to the output.
+// SL = 2, 4 or 8 neighbouring lanes share an element group: lane l sums splits l, l+SL, ...
 // and the lanes are combined by shuffles in a fixed tree, so the sum stays deterministic while
-// the chains get shorter and SL times more CTAs are in flight.
+// the chains get shorter and SL times more CTAs are in flight.  A non-zero status (a wait gave up)
+// poisons the result with NaN, here and in the units.
 __global__ void __launch_bounds__(256) factor_tc_reduce_tiles(const FactorParams p, int sl) {
   int bi, bj;
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -534,7 +373,7 @@ size_t factor_tc_workspace_bytes(int64_t rows, int64_t d) {
   const int nb = (int)ceil_div64(d, 128);
   const int tiles = nb * (nb + 1) / 2;
   int splits, rps;
-  tc::choose_splits(rows, tiles, 32, splits, rps);   // the fp32 stage depth gives the larger count
+  tc::choose_splits(rows, tiles, 32, splits, rps);   // fp32 stages
   int s2, r2;
   tc::choose_splits(rows, tiles, 64, s2, r2);
   if (s2 > splits) splits = s2;
@@ -562,7 +401,7 @@ template <typename T>
 static int tc_launch_typed(FactorParams p, int tiles, cudaStream_t st) {
   using C = tc::Cfg<T>;
   tc::choose_splits(p.rows, tiles, C::KS, p.splits, p.rows_per_split);
-  const size_t smem = (size_t)C::STAGES * 2 * C::PARTS * C::OPB + 128;
+  const size_t smem = (size_t)C::STAGES * 2 * C::OPB + 128;
   SSO_ENSURE_SMEM((tc::factor_tc_kernel<T>), smem);
   tc::factor_tc_kernel<T><<<dim3(tiles, p.splits), tc::THREADS, smem, st>>>(
       p, g_flush_stages > 0 ? g_flush_stages : C::FLUSH);
@@ -590,18 +429,12 @@ int factor_tc_launch(FactorParams p, int dtype, void* workspace, size_t workspac
   return fail(-1, "unknown dtype %d", dtype);
 }
 
-// Permuted factors of at least 1024 columns with at most this many splits are finished row-wise (whole
-// output rows through shared memory); the tile-wise kernel scatters 4-byte stores when columns are permuted.
-// 8 instead of 3: VGG-16-style step 59.5 -> 58.3 ms, 5x5 ConvNet step unchanged.
-static int g_rowwise_max_splits = 8;
-void factor_tc_set_rowwise_max_splits(int s) { g_rowwise_max_splits = s; }
-
 // A finishing kernel may be set up while its producer still runs (it waits for the producer's end itself).
 template <typename... Args>
-static void launch_early(void (*kernel)(Args...), dim3 grid, size_t smem, cudaStream_t st, Args... args) {
+static void launch_early(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(256);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
@@ -613,28 +446,20 @@ static void launch_early(void (*kernel)(Args...), dim3 grid, size_t smem, cudaSt
 }
 
 int factor_tc_run_reduce(const FactorParams& p, int tiles, cudaStream_t st) {
-  // a large permuted factor with not too many splits: the output dominates, write it in whole rows
-  if (!(p.perm_c > 0 && p.perm_fold == 0 && p.splits <= g_rowwise_max_splits && p.d >= 1024)) {
-    // lanes per element group: enough CTAs to fill the GPU when there are few tiles, and chains
-    // of at most ~8 partial tiles per lane
-    int sl = 1;
-    while (sl < 8 && (tiles * 16 * sl < 2 * 148 || p.splits > 8 * sl) && p.splits >= 4 * sl) sl <<= 1;
-    launch_early(tc::factor_tc_reduce_tiles, dim3(tiles, 16 * sl), 0, st, FactorParams(p), sl);
-    SSO_LAUNCH_OK("factor_tc_reduce_tiles");
+  if (units::supported(p)) {
+    const units::Problem u = units::plan(p, 148);
+    SSO_ENSURE_SMEM(tc::factor_finish_units, units::SMEM_MAX);
+    launch_early(tc::factor_finish_units, dim3(u.units), units::threads(u), units::smem_bytes(u), st, units::Problem(u), (const int*)p.status);
+    SSO_LAUNCH_OK("factor_finish_units");
     return 0;
   }
-  int perm_groups = 0, width = tc::RED_W;
-  if (p.perm_c > 0) {
-    perm_groups = ceil_div(p.perm_pub > 0 ? p.perm_pub : p.perm_c, tc::RED_CB);
-    width = std::max(tc::RED_CB * p.perm_kk, 1);
-  }
-  const int plain_groups = p.perm_c > 0 ? (p.d > p.dcols ? 1 : 0) : ceil_div(p.d, tc::RED_W);
-  const int pitch = width | 1;
-  const size_t smem = (size_t)tc::RED_ROWS * pitch * sizeof(float);
-  SSO_CHECK_ARG(smem <= 200 * 1024, "factor: kernel window too large for the finishing kernel");
-  SSO_ENSURE_SMEM(tc::factor_tc_reduce, 200 * 1024);
-  launch_early(tc::factor_tc_reduce, dim3(ceil_div(p.d, tc::RED_ROWS), perm_groups + plain_groups), smem, st, FactorParams(p), perm_groups, pitch);
-  SSO_LAUNCH_OK("factor_tc_reduce");
+  // windows folded into the channels (few channels) or too large for a unit: tile by tile with scattered stores.
+  // Lanes per element group: enough CTAs to fill the GPU when there are few tiles, and chains of at most ~8 partial
+  // tiles per lane
+  int sl = 1;
+  while (sl < 8 && (tiles * 16 * sl < 2 * 148 || p.splits > 8 * sl) && p.splits >= 4 * sl) sl <<= 1;
+  launch_early(tc::factor_tc_reduce_tiles, dim3(tiles, 16 * sl), 256, 0, st, FactorParams(p), sl);
+  SSO_LAUNCH_OK("factor_tc_reduce_tiles");
   return 0;
 }
 

@@ -11,8 +11,10 @@
 // memory, 4x4 register tile per thread), squares it into a second register tile and moves on.
 // Sample ranges go to a workspace and are summed in a fixed order by a finishing kernel
 // (deterministic, no atomics).  The bias takes the squares of the gradient values that the CTAs of the
-// first column tile stage anyway and one more row of the workspace (a kernel of its own read the
-// gradient again with one warp per channel: 160 us per layer, 30 % of a step with these curvatures).
+// first column tile stage anyway: a sum per sample and channel, over 32 pixel lanes and a tree of them, and
+// the finishing kernel runs over the samples in order.  (A kernel of its own did these sums in the same
+// order, but read the gradient again with one warp per channel: 160 us per layer, 30 % of a step with these
+// curvatures.  The order stays because a posterior draw feeds its rounding back into the network.)
 #include "common.cuh"
 
 namespace sso {
@@ -21,7 +23,7 @@ struct DiagSqParams {
   const void* x;        // layer input  [n, c, h, w]   (element strides sxn, sxc, sxh, sxw)
   const void* g;        // output grad  [n, oc, ho, wo] (element strides sgn, sgc, sgh, sgw)
   const float* weight;  // per-sample weights, nullable
-  float* partial;       // [splits][oc*d + oc]: weight, then bias
+  float* partial;       // [splits][oc*d], then the bias' sums [n][oc]
   bool bias;
   int64_t sxn, sxc, sxh, sxw, sgn, sgc, sgh, sgw;
   int n, c, h, w, oc, ho, wo;
@@ -38,6 +40,7 @@ template <typename T, bool ONE_PIXEL>
 __global__ void __launch_bounds__(256) diag_sq_kernel(const DiagSqParams p) {
   __shared__ __align__(16) float Gs[DK][DT + 4];   // row pitch 68 floats: float4 rows stay 16-byte aligned
   __shared__ __align__(16) float Us[DK][DT + 4];
+  __shared__ __align__(16) float Bs[DK][DT];       // squares of a sample's gradients, pixel lanes l and l + 16 added
   __shared__ int64_t col_off[DT];
   __shared__ int col_dh[DT], col_dw[DT];
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
@@ -66,7 +69,7 @@ __global__ void __launch_bounds__(256) diag_sq_kernel(const DiagSqParams p) {
   // staging map: thread -> (pixel ll = tid / 16, four consecutive tile columns 4*(tid % 16) ..)
   const int ll = tid >> 4, c4 = (tid & 15) * 4;
   const bool bias = p.bias && blockIdx.y == 0;
-  float bs[4] = {0.f, 0.f, 0.f, 0.f};      // sum over this thread's pixels of w_b g^2, columns c4 ..
+  float* bias_sums = p.partial + (int64_t)gridDim.z * p.oc * p.d;
   if (ONE_PIXEL) {
     for (int b0 = b_begin; b0 < b_end; b0 += DK) {
       const int b = b0 + ll;
@@ -78,7 +81,7 @@ __global__ void __launch_bounds__(256) diag_sq_kernel(const DiagSqParams p) {
         float gv = 0.f;
         if (bv && o < p.oc) gv = to_f32<T>(__ldg(G + (int64_t)b * p.sgn + (int64_t)o * p.sgc));
         Gs[ll][c4 + q] = wb * gv * gv;
-        bs[q] += wb * gv * gv;
+        if (bias && bv && o < p.oc) bias_sums[(int64_t)b * p.oc + o] = gv * gv;
         float uv = 0.f;
         const int64_t off = col_off[c4 + q];
         if (bv && off >= 0) uv = to_f32<T>(__ldg(X + (int64_t)b * p.sxn + off));
@@ -127,10 +130,15 @@ __global__ void __launch_bounds__(256) diag_sq_kernel(const DiagSqParams p) {
     };
     const float wb = p.weight ? p.weight[b] : 1.f;
     gather(0);
+    float even[4] = {0.f, 0.f, 0.f, 0.f}, odd[4] = {0.f, 0.f, 0.f, 0.f};      // pixels ll + 32 i, ll + 16 + 32 i
     for (int l0 = 0; l0 < L; l0 += DK) {
       if (bias) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) bs[q] = fmaf(wb * to_f32<T>(gv[q]), to_f32<T>(gv[q]), bs[q]);
+        for (int q = 0; q < 4; ++q) {
+          const float v = to_f32<T>(gv[q]);
+          if (l0 & DK) odd[q] = fmaf(v, v, odd[q]);
+          else even[q] = fmaf(v, v, even[q]);
+        }
       }
       *reinterpret_cast<float4*>(&Gs[ll][c4]) = make_float4(to_f32<T>(gv[0]), to_f32<T>(gv[1]), to_f32<T>(gv[2]), to_f32<T>(gv[3]));
       *reinterpret_cast<float4*>(&Us[ll][c4]) = make_float4(to_f32<T>(uv[0]), to_f32<T>(uv[1]), to_f32<T>(uv[2]), to_f32<T>(uv[3]));
@@ -152,8 +160,22 @@ __global__ void __launch_bounds__(256) diag_sq_kernel(const DiagSqParams p) {
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int q = 0; q < 4; ++q) sq[i][q] = fmaf(wb * acc[i][q], acc[i][q], sq[i][q]);
+    if (bias) {      // the next sample writes Bs behind the barriers of its own pixels
+      *reinterpret_cast<float4*>(&Bs[ll][c4]) = make_float4(even[0] + odd[0], even[1] + odd[1], even[2] + odd[2], even[3] + odd[3]);
+      __syncthreads();
+      if (tid < DT && o0 + tid < p.oc) {
+        float v[DK];
+#pragma unroll
+        for (int k = 0; k < DK; ++k) v[k] = Bs[k][tid];
+#pragma unroll
+        for (int off = DK / 2; off > 0; off >>= 1)
+#pragma unroll
+          for (int k = 0; k < off; ++k) v[k] += v[k + off];
+        bias_sums[(int64_t)b * p.oc + o0 + tid] = v[0];
+      }
+    }
   }
-  float* dst = p.partial + (int64_t)split * p.oc * (p.d + 1);
+  float* dst = p.partial + (int64_t)split * p.oc * p.d;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int o = o0 + ty * 4 + i;
@@ -164,26 +186,22 @@ __global__ void __launch_bounds__(256) diag_sq_kernel(const DiagSqParams p) {
       if (j < p.d) dst[(int64_t)o * p.d + j] = sq[i][q];
     }
   }
-  if (bias) {      // Gs is free: the 16 pixel lanes of a column are summed in order
-    *reinterpret_cast<float4*>(&Gs[ll][c4]) = make_float4(bs[0], bs[1], bs[2], bs[3]);
-    __syncthreads();
-    if (tid < DT && o0 + tid < p.oc) {
-      float t = 0.f;
-#pragma unroll
-      for (int k = 0; k < DK; ++k) t += Gs[k][tid];
-      dst[(int64_t)p.oc * p.d + o0 + tid] = t;
-    }
-  }
 }
 
-__global__ void __launch_bounds__(256) diag_sq_finish_kernel(const float* __restrict__ partial, int splits, int64_t pitch,
-                                                             int64_t n_w, int64_t count, float alpha, float beta,
+__global__ void __launch_bounds__(256) diag_sq_finish_kernel(const float* __restrict__ partial, int splits, int64_t n_w, int64_t count,
+                                                             const float* __restrict__ weight, int n, float alpha, float beta,
                                                              float* __restrict__ out_w, float* __restrict__ out_b) {
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= count) return;
   float s = 0.f;
+  if (i < n_w) {
 #pragma unroll 4
-  for (int sp = 0; sp < splits; ++sp) s += partial[(int64_t)sp * pitch + i];
+    for (int sp = 0; sp < splits; ++sp) s += partial[(int64_t)sp * n_w + i];
+  } else {
+    const float* src = partial + splits * n_w + (i - n_w);
+#pragma unroll 8
+    for (int b = 0; b < n; ++b) s = fmaf(weight ? weight[b] : 1.f, src[b * (count - n_w)], s);
+  }
   float* o = i < n_w ? out_w + i : out_b + (i - n_w);
   *o = (beta == 0.f) ? alpha * s : fmaf(beta, *o, alpha * s);
 }
@@ -204,7 +222,7 @@ static int diag_sq_typed(DiagSqParams p, float alpha, float beta, float* out_w, 
     diag_sq_kernel<T, false><<<grid, 256, 0, st>>>(p);
   SSO_LAUNCH_OK("diag_sq_kernel");
   const int64_t n_w = (int64_t)p.oc * p.d, count = n_w + (out_b ? p.oc : 0);
-  diag_sq_finish_kernel<<<(unsigned)ceil_div64(count, 256), 256, 0, st>>>(p.partial, splits, n_w + p.oc, n_w, count, alpha, beta,
+  diag_sq_finish_kernel<<<(unsigned)ceil_div64(count, 256), 256, 0, st>>>(p.partial, splits, n_w, count, p.weight, p.n, alpha, beta,
                                                                          out_w, out_b);
   SSO_LAUNCH_OK("diag_sq_finish_kernel");
   return 0;
@@ -220,7 +238,7 @@ size_t sso_diag_sq_workspace_bytes(int64_t n, int64_t oc, int64_t d) {
   if (n <= 0 || oc <= 0 || d <= 0) return 0;
   const int splits = diag_sq_splits((int)n, (int)oc, (int)d);
   const int per = ceil_div((int)n, splits);
-  return (size_t)ceil_div((int)n, per) * (size_t)oc * (size_t)(d + 1) * sizeof(float);
+  return ((size_t)ceil_div((int)n, per) * (size_t)d + (size_t)n) * (size_t)oc * sizeof(float);
 }
 
 int sso_diag_sq_im2col(const void* x, const void* g, int dtype, int64_t n, int64_t c, int64_t h, int64_t w,

@@ -136,15 +136,13 @@ __global__ void __launch_bounds__(256) bn_plane_sums_ccontig(const T* __restrict
 // parallel per block, and the pixel range of one image is cut into `splits` blocks.  Partial sums go
 // to out[(n*splits + split)*c + channel]; the finishing kernel adds the splits.
 template <typename T, bool IS_Y>
-__global__ void __launch_bounds__(256) bn_plane_sums_vec(const T* __restrict__ t, int c, int hw, int64_t sn,
-                                                         int64_t sp, int lp, int splits,
-                                                         const float* __restrict__ scale,
-                                                         const float* __restrict__ shift,
-                                                         float* __restrict__ out) {
+__device__ __forceinline__ void bn_plane_sums_block(const T* __restrict__ t, int c, int hw, int64_t sn, int64_t sp, int lp,
+                                                    int splits, const float* __restrict__ scale,
+                                                    const float* __restrict__ shift, float* __restrict__ out, int in,
+                                                    int split, float* __restrict__ red_) {
   constexpr int V = 16 / sizeof(T);
-  __shared__ float red[256][V + 1];
+  float (*red)[V + 1] = reinterpret_cast<float (*)[V + 1]>(red_);
   const int cv = threadIdx.x % lp, pp = threadIdx.x / lp, npp = 256 / lp;
-  const int in = blockIdx.y, split = blockIdx.x;
   const int per = (hw + splits - 1) / splits;
   const int p0 = split * per, p1 = min(hw, p0 + per);
   const int c0 = cv * V;
@@ -191,16 +189,24 @@ __global__ void __launch_bounds__(256) bn_plane_sums_vec(const T* __restrict__ t
   }
 }
 
+template <typename T, bool IS_Y>
+__global__ void __launch_bounds__(256) bn_plane_sums_vec(const T* __restrict__ t, int c, int hw, int64_t sn, int64_t sp, int lp,
+                                                         int splits, const float* __restrict__ scale,
+                                                         const float* __restrict__ shift, float* __restrict__ out) {
+  __shared__ float red[256 * (16 / sizeof(T) + 1)];
+  bn_plane_sums_block<T, IS_Y>(t, c, hw, sn, sp, lp, splits, scale, shift, out, blockIdx.y, blockIdx.x, red);
+}
+
 // block = 8 channels x 32 image lanes: with the usual 32..256 images a thread owns one to eight
 // images, issues the loads of all their split partials back to back, and the 32 lanes are combined
 // in shared memory (fixed order: deterministic).  Many small blocks keep this latency-bound step short.
-__global__ void __launch_bounds__(256) bn_finish_kernel(const float* __restrict__ sx, const float* __restrict__ sg,
-                                                        const float* __restrict__ weight, int n, int c,
-                                                        int splits_x, int splits_g, float alpha, float beta,
-                                                        float* __restrict__ w_out, float* __restrict__ b_out) {
+__device__ __forceinline__ void bn_finish_block(const float* __restrict__ sx, const float* __restrict__ sg,
+                                                const float* __restrict__ weight, int n, int c, int splits_x, int splits_g,
+                                                float alpha, float beta, float* __restrict__ w_out,
+                                                float* __restrict__ b_out, int block) {
   __shared__ float rw[32][9], rb[32][9];
   const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
-  const int ic = blockIdx.x * 8 + tx;
+  const int ic = block * 8 + tx;
   float aw = 0.f, ab = 0.f;
   if (ic < c) {
     for (int in = ty; in < n; in += 32) {
@@ -228,6 +234,58 @@ __global__ void __launch_bounds__(256) bn_finish_kernel(const float* __restrict_
     w_out[ic] = (beta == 0.f) ? s * tw : fmaf(beta, w_out[ic], s * tw);
     if (b_out) b_out[ic] = (beta == 0.f) ? s * tb : fmaf(beta, b_out[ic], s * tb);
   }
+}
+
+__global__ void __launch_bounds__(256) bn_finish_kernel(const float* __restrict__ sx, const float* __restrict__ sg,
+                                                        const float* __restrict__ weight, int n, int c,
+                                                        int splits_x, int splits_g, float alpha, float beta,
+                                                        float* __restrict__ w_out, float* __restrict__ b_out) {
+  bn_finish_block(sx, sg, weight, n, c, splits_x, splits_g, alpha, beta, w_out, b_out, blockIdx.x);
+}
+
+// The gradient sums of many layers in one launch and their results in a second: a ResNet has a layer of a few
+// microseconds' work per convolution (53 layers at 32 images: 468 + 366 us of launches that each filled the chip for a
+// fraction of their time; BN_MEASURED).  The records travel in the kernel's parameter space.
+constexpr int BN_BATCH = 64;
+struct BnRec {
+  sso_bn_desc d;
+  int lp, sum0, fin0;      // lanes of a pixel; first block of this layer in either launch
+};
+struct BnBatch {
+  int n;
+  BnRec rec[BN_BATCH];
+};
+
+template <bool FINISH>
+__device__ __forceinline__ int bn_find(const BnBatch& b) {
+  int lo = 0, hi = b.n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if ((FINISH ? b.rec[mid].fin0 : b.rec[mid].sum0) <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+__global__ void __launch_bounds__(256) bn_batch_sums_kernel(const __grid_constant__ BnBatch b) {
+  __shared__ float red[256 * 9];
+  const BnRec& r = b.rec[bn_find<false>(b)];
+  const int j = (int)blockIdx.x - r.sum0, in = j / r.d.splits_g, split = j - in * r.d.splits_g;
+  const int c = (int)r.d.c, hw = (int)r.d.hw;
+  if (r.d.dtype == SSO_F32)
+    bn_plane_sums_block<float, false>(reinterpret_cast<const float*>(r.d.g), c, hw, r.d.sn, r.d.sp, r.lp, r.d.splits_g, nullptr,
+                                      nullptr, r.d.sg, in, split, red);
+  else if (r.d.dtype == SSO_BF16)
+    bn_plane_sums_block<__nv_bfloat16, false>(reinterpret_cast<const __nv_bfloat16*>(r.d.g), c, hw, r.d.sn, r.d.sp, r.lp,
+                                              r.d.splits_g, nullptr, nullptr, r.d.sg, in, split, red);
+  else
+    bn_plane_sums_block<__half, false>(reinterpret_cast<const __half*>(r.d.g), c, hw, r.d.sn, r.d.sp, r.lp, r.d.splits_g,
+                                       nullptr, nullptr, r.d.sg, in, split, red);
+}
+
+__global__ void __launch_bounds__(256) bn_batch_finish_kernel(const __grid_constant__ BnBatch b) {
+  const BnRec& r = b.rec[bn_find<true>(b)];
+  bn_finish_block(r.d.sx, r.d.sg, r.d.sample_weight, (int)r.d.n, (int)r.d.c, r.d.splits_x, r.d.splits_g, r.d.alpha, r.d.beta,
+                  r.d.w_out, r.d.b_out, (int)blockIdx.x - r.fin0);
 }
 
 // pixel-range splits of the vectorised kernel for a [n, c, hw] tensor (1 when it is not used)
@@ -641,6 +699,45 @@ int sso_bn_diag_finish(const float* sx, const float* sg, const float* sample_wei
       sx, sg, sample_weight, (int)n, (int)c, splits_x, splits_g, alpha, beta, w_out, b_out);
   SSO_LAUNCH_OK("bn_finish_kernel");
   return 0;
+}
+
+int sso_bn_batch(int n, const sso_bn_desc* descs, void* stream) {
+  SSO_CHECK_ARG(n >= 0 && (n == 0 || descs != nullptr), "bn_batch: bad argument");
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  static thread_local BnBatch b;
+  int sums = 0, blocks = 0;
+  b.n = 0;
+  auto flush = [&]() -> int {
+    if (b.n == 0) return 0;
+    bn_batch_sums_kernel<<<sums, 256, 0, st>>>(b);
+    SSO_LAUNCH_OK("bn_batch_sums_kernel");
+    bn_batch_finish_kernel<<<blocks, 256, 0, st>>>(b);
+    SSO_LAUNCH_OK("bn_batch_finish_kernel");
+    b.n = sums = blocks = 0;
+    return 0;
+  };
+  for (int i = 0; i < n; ++i) {
+    const sso_bn_desc& d = descs[i];
+    SSO_CHECK_ARG(d.g && d.sg && d.sx && d.w_out, "bn_batch: null pointer");
+    SSO_CHECK_ARG(d.n > 0 && d.c > 0 && d.hw > 0 && d.n * d.c < (int64_t)1 << 26 && d.splits_g >= 1 && d.splits_x >= 1,
+                  "bn_batch: bad shape");
+    const int size = d.dtype == SSO_F32 ? 4 : 2, lp = bn_vec_lanes(d.c, 16 / size);
+    if (lp > 0 && d.hw > 1 && d.sc == 1 && (reinterpret_cast<uintptr_t>(d.g) & 15) == 0 && d.sn * size % 16 == 0 && d.sp * size % 16 == 0) {
+      b.rec[b.n] = {d, lp, sums, blocks};
+      ++b.n;
+      sums += (int)(d.n * d.splits_g);
+      blocks += (int)ceil_div64(d.c, 8);
+      if (b.n == BN_BATCH) {
+        const int rc = flush();
+        if (rc) return rc;
+      }
+      continue;
+    }
+    int rc = sso_bn_plane_sums(nullptr, d.g, d.dtype, d.n, d.c, d.hw, 0, 0, 0, d.sn, d.sc, d.sp, nullptr, nullptr, nullptr, d.sg, d.splits_g, stream);
+    if (!rc) rc = sso_bn_diag_finish(d.sx, d.sg, d.sample_weight, d.n, d.c, d.splits_x, d.splits_g, d.alpha, d.beta, d.w_out, d.b_out, stream);
+    if (rc) return rc;
+  }
+  return flush();
 }
 
 int sso_diag_inv_precondition(const float* ema, float* inv, float* grad, int64_t count, float damping,

@@ -58,6 +58,12 @@ class FactorDesc(C.Structure):
                 ('sample_weight', c_vp), ('alpha', c_f32), ('beta', c_f32), ('out', c_vp), ('ldo', c_i64)]
 
 
+class BnDesc(C.Structure):
+    _fields_ = [('g', c_vp), ('dtype', C.c_int32), ('splits_g', C.c_int32), ('splits_x', C.c_int32), ('alpha', c_f32),
+                ('beta', c_f32), ('n', c_i64), ('c', c_i64), ('hw', c_i64), ('sn', c_i64), ('sc', c_i64), ('sp', c_i64),
+                ('sg', c_vp), ('sx', c_vp), ('sample_weight', c_vp), ('w_out', c_vp), ('b_out', c_vp)]
+
+
 TRI_REC_DTYPE = np.dtype([('m', np.uint64), ('packed', np.uint64), ('n', np.int32), ('ld', np.int32),
                           ('row0', np.int32), ('nrows', np.int32)])
 
@@ -83,6 +89,7 @@ SIGNATURES = {
     'sso_bn_plane_splits': (c_i32, [c_i32, c_i64, c_i64, c_i64, c_i64]),
     'sso_bn_plane_sums': (c_i32, [c_vp, c_vp, c_i32] + [c_i64] * 9 + [c_vp] * 4 + [c_i32, c_vp]),
     'sso_bn_diag_finish': (c_i32, [c_vp, c_vp, c_vp, c_i64, c_i64, c_i32, c_i32, c_f32, c_f32, c_vp, c_vp, c_vp]),
+    'sso_bn_batch': (c_i32, [c_i32, c_vp, c_vp]),
     'sso_ema_update': (c_i32, [c_vp, c_vp, c_i64, c_f32, c_i32, c_vp]),
     'sso_axpby': (c_i32, [c_vp, c_vp, c_i64, c_f32, c_f32, c_vp]),
     'sso_diag_inv_precondition': (c_i32, [c_vp, c_vp, c_vp, c_i64, c_f32, c_i32, c_i32, c_vp]),
@@ -446,11 +453,19 @@ class collect_factors:
     at its end, whether batching is on or not: for a caller that holds all inputs of a pass, unmodified."""
 
     def __enter__(self):
-        self.outer = getattr(_collected, 'items', None)
-        _collected.items = []
+        self.outer = getattr(_collected, 'items', None), getattr(_collected, 'norms', None)
+        _collected.items, _collected.norms = [], []
 
     def __exit__(self, kind, value, tb):
-        items, _collected.items = _collected.items, self.outer
+        items, norms = _collected.items, _collected.norms
+        _collected.items, _collected.norms = self.outer
+        if kind is None and norms:
+            outs = [d[2].data_ptr() for d in norms]
+            if len(set(outs)) < len(outs):
+                for item in norms:
+                    _launch_norms([item])
+            else:
+                _launch_norms(norms)
         if kind is None and items:
             if _pending:
                 flush_factors()
@@ -483,7 +498,7 @@ def _launch_factors(items):
         d.x, d.alpha, d.beta = x.data_ptr(), alpha, beta
     device = items[0][0].device
 
-    def launch(_):
+    def launch():
         ws = workspace(device, nbytes, 'batch')
         if FACTOR_TIMING is not None:
             a = torch.cuda.Event(enable_timing=True)
@@ -494,19 +509,47 @@ def _launch_factors(items):
             b.record()
             FACTOR_TIMING.append((a, b, sum(op.flops for op, _, _, _ in items), sum(op.bytes for op, _, _, _ in items)))
 
-    if _curv_enabled:
-        idx = device.index if device.index is not None else torch.cuda.current_device()
-        side = _curv_streams.get(idx)
-        if side is None:
-            side = _curv_streams[idx] = torch.cuda.Stream(device=idx)
-        side.wait_stream(torch.cuda.current_stream(idx))
-        for _, x, _, _ in items:
-            x.record_stream(side)
-        _curv_dirty.add(idx)
-        with torch.cuda.stream(side):
-            launch(None)
-    else:
-        launch(None)
+    _launch_where_enabled(launch, device, [x for _, x, _, _ in items])
+
+
+def _launch_where_enabled(launch, device, inputs):
+    """`launch` on the curvature stream if there is one, else on the current stream."""
+    if not _curv_enabled:
+        launch()
+        return
+    idx = device.index if device.index is not None else torch.cuda.current_device()
+    side = _curv_streams.get(idx)
+    if side is None:
+        side = _curv_streams[idx] = torch.cuda.Stream(device=idx)
+    side.wait_stream(torch.cuda.current_stream(idx))
+    for x in inputs:
+        x.record_stream(side)
+    _curv_dirty.add(idx)
+    with torch.cuda.stream(side):
+        launch()
+
+
+def collect_norm(g, layout, sg, sx, sample_weight, splits_x, alpha, beta, w_out, b_out) -> bool:
+    """Inside ``collect_factors``: the gradient sums and the result of a normalisation layer are noted for one call at
+    its end.  False: not inside, nothing noted."""
+    mine = getattr(_collected, 'norms', None)
+    if mine is None:
+        return False
+    _require_cuda(g, 'batch-norm tensor')
+    mine.append((g, layout, w_out, b_out, sg, sx, sample_weight, splits_x, alpha, beta))
+    return True
+
+
+def _launch_norms(items):
+    arr = (BnDesc * len(items))()
+    for d, (g, layout, w_out, b_out, sg, sx, weight, splits_x, alpha, beta) in zip(arr, items):
+        d.n, d.c = g.shape[0], g.shape[1]
+        d.hw = g.numel() // (d.n * d.c)
+        (d.sn, d.sc, d.sp), d.splits_g = layout
+        d.g, d.dtype, d.splits_x, d.alpha, d.beta = g.data_ptr(), _dtype_code(g), splits_x, alpha, beta
+        d.sg, d.sx, d.sample_weight = sg.data_ptr(), sx.data_ptr(), _ptr(weight)
+        d.w_out, d.b_out = w_out.data_ptr(), _ptr(b_out)
+    _launch_where_enabled(lambda: _check(lib().sso_bn_batch(len(items), arr, _stream())), items[0][0].device, [it[0] for it in items])
 
 
 def _plane_strides(t: torch.Tensor):
@@ -573,6 +616,17 @@ def diag_sq(x: torch.Tensor, g: torch.Tensor, kernel_size, stride, padding, dila
     """out_w <- alpha * sum_b w_b (per-sample weight gradient of sample b)^2 + beta * out_w (and the
     same for the bias) for a convolution with input x [n,c,h,w] and output gradient g [n,oc,ho,wo];
     a Linear layer passes x [n,f_in], g [n,f_out]."""
+    x, g, call = diag_sq_call(x, g, kernel_size, stride, padding, dilation)
+    oc, d, n = call[2], call[3], x.shape[0]
+    assert out_w.is_contiguous() and out_w.dtype == torch.float32 and out_w.numel() == oc * d
+    assert out_b is None or (out_b.is_contiguous() and out_b.numel() == oc)
+    assert sample_weight is None or (sample_weight.dtype == torch.float32 and sample_weight.is_contiguous()
+                                     and sample_weight.numel() == n)
+    diag_sq_run(call, x, g, sample_weight, alpha, beta, out_w.data_ptr(), _ptr(out_b))
+
+
+def diag_sq_call(x, g, kernel_size, stride, padding, dilation):
+    """(x, g, call): the operands as the kernel takes them and what of a call does not change between steps."""
     _require_cuda(x, 'layer input')
     if x.dim() == 2:
         x, g = x[:, :, None, None], g[:, :, None, None]
@@ -582,17 +636,15 @@ def diag_sq(x: torch.Tensor, g: torch.Tensor, kernel_size, stride, padding, dila
     n, c, h, w = x.shape
     oc = g.shape[1]
     d = c * kernel_size[0] * kernel_size[1]
-    assert out_w.is_contiguous() and out_w.dtype == torch.float32 and out_w.numel() == oc * d
-    assert out_b is None or (out_b.is_contiguous() and out_b.numel() == oc)
-    assert sample_weight is None or (sample_weight.dtype == torch.float32 and sample_weight.is_contiguous()
-                                     and sample_weight.numel() == n)
-    L = lib()
-    ws = workspace(x.device, L.sso_diag_sq_workspace_bytes(n, oc, d))
-    _check(L.sso_diag_sq_im2col(x.data_ptr(), g.data_ptr(), _dtype_code(x), n, c, h, w, *x.stride(), oc,
-                                *g.stride(), kernel_size[0], kernel_size[1], stride[0], stride[1],
-                                padding[0], padding[1], dilation[0], dilation[1], _ptr(sample_weight),
-                                alpha, beta, out_w.data_ptr(), _ptr(out_b), _ptr(ws),
-                                0 if ws is None else ws.numel(), _stream()))
+    mid = (_dtype_code(x), n, c, h, w, *x.stride(), oc, *g.stride(), *kernel_size, *stride, *padding, *dilation)
+    return x, g, (mid, lib().sso_diag_sq_workspace_bytes(n, oc, d), oc, d)
+
+
+def diag_sq_run(call, x, g, sample_weight, alpha, beta, w_ptr, b_ptr):
+    mid, nbytes = call[0], call[1]
+    ws = workspace(x.device, nbytes)
+    _check(lib().sso_diag_sq_im2col(x.data_ptr(), g.data_ptr(), *mid, _ptr(sample_weight), alpha, beta, w_ptr, b_ptr,
+                                    _ptr(ws), 0 if ws is None else ws.numel(), _stream()))
 
 
 def ema_update(data: torch.Tensor, ema: torch.Tensor, beta: float, first: bool):

@@ -253,7 +253,14 @@ class DiagCurvature(Curvature):
         FactorPool([], [self], self.device)
 
     def _views(self, role):
-        return [self.pool.vec(role, self, j) for j in range(len(self._get_shape()))]
+        pool = self.pool
+        known = self.__dict__.get('_view_lists')
+        if known is None or known[0] is not pool:
+            known = self.__dict__['_view_lists'] = (pool, {})
+        views = known[1].get(role)
+        if views is None:
+            views = known[1][role] = [pool.vec(role, self, j) for j in range(len(self._get_shape()))]
+        return list(views)
 
     def update_inv(self):
         self.pool.diag_step([self], None, True)

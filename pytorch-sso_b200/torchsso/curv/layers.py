@@ -316,7 +316,6 @@ class _DiagBatchNorm(DiagCurvature):
         n, c = g.shape[0], g.shape[1]
         layout = self._layout(g)
         self._sg = self._buffer(self._sg, n * layout[2] * c, g.device)
-        splits_g = nat.bn_plane_sums(layout[0], False, None, None, self._sg, layout)
         later_pass = fisher and self._passes > 0
         role = 'ema' if self._fuse_ema else 'data'
         views = self.__dict__.get('_bnv')
@@ -326,8 +325,11 @@ class _DiagBatchNorm(DiagCurvature):
         views = views[1]
         w, ws = _weights(self, n, g.device)
         scale, beta = _fused_ema_coefficients(self) if self._fuse_ema else (1.0, 0.0)
-        nat.bn_diag_finish(self._sx, self._sg, w, n, c, self._splits_x, splits_g, scale * ws * float(n) * float(n),
-                           1.0 if later_pass else beta, views[0], views[1] if len(views) > 1 else None)
+        alpha, beta = scale * ws * float(n) * float(n), 1.0 if later_pass else beta
+        b_out = views[1] if len(views) > 1 else None
+        if not nat.collect_norm(layout[0], layout[1:], self._sg, self._sx, w, self._splits_x, alpha, beta, views[0], b_out):
+            splits_g = nat.bn_plane_sums(layout[0], False, None, None, self._sg, layout)
+            nat.bn_diag_finish(self._sx, self._sg, w, n, c, self._splits_x, splits_g, alpha, beta, views[0], b_out)
         if fisher:
             self._passes += 1
         if not self._fuse_ema:
@@ -374,11 +376,21 @@ class _DiagSq(DiagCurvature):
         x, g = self._operands(self._module.data_input, g)
         n = g.shape[0]
         p, ws = _weights(self, n, g.device)
-        views = self._views('data')
         first = not (fisher and self._passes > 0)
+        views = self._views('data')
         # mean over samples, then the n^2 that undoes the mean reduction of the loss
-        nat.diag_sq(x, g, *self._geometry(), p, ws * float(n), 0.0 if first else 1.0,
-                    views[0], views[1] if self.bias else None)
+        alpha, beta = ws * float(n), 0.0 if first else 1.0
+        calls = self.__dict__.setdefault('_calls', {})
+        key = (x.shape, x.stride(), x.dtype, g.shape, g.stride(), g.dtype)
+        call = calls.get(key)
+        if call is not None and p is None:
+            nat.diag_sq_run(call, x, g, None, alpha, beta, views[0].data_ptr(), views[1].data_ptr() if self.bias else None)
+        else:
+            nat.diag_sq(x, g, *self._geometry(), p, alpha, beta, views[0], views[1] if self.bias else None)
+            if call is None and x.dtype == g.dtype:      # checked once for this layout; without a conversion the operands go in as they are
+                while len(calls) >= 16:
+                    calls.pop(next(iter(calls)))
+                calls[key] = nat.diag_sq_call(x, g, *self._geometry())[2]
         if fisher:
             self._passes += 1
         self._have.add('data')

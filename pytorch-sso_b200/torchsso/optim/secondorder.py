@@ -22,7 +22,8 @@ from torch.optim import Optimizer
 
 import torchsso
 from torchsso import _native as nat
-from torchsso.curv.layers import _KronFactors, _DiagBatchNorm
+from torchsso.curv.curvature import DiagCurvature
+from torchsso.curv.layers import _KronFactors, _DiagBatchNorm, _DiagSq
 from torchsso.curv.pool import FactorPool
 from torchsso.utils import TensorAccumulator
 
@@ -34,7 +35,7 @@ _TAIL_SETTINGS = itemgetter('lars', 'l2_reg', 'weight_decay', 'momentum', 'momen
 
 
 def _is_pooled(curv) -> bool:
-    return isinstance(curv, (_KronFactors, _DiagBatchNorm)) and not curv.use_max_ema
+    return isinstance(curv, (_KronFactors, _DiagBatchNorm, _DiagSq)) and not curv.use_max_ema
 
 
 class SecondOrderOptimizer(Optimizer):
@@ -143,7 +144,7 @@ class SecondOrderOptimizer(Optimizer):
         groups = [self.param_groups[i] for i in self._group_order()]
         device = groups[0]['params'][0].device
         kron = [g for g in groups if isinstance(g['curv'], _KronFactors) and _is_pooled(g['curv'])]
-        diag = [g for g in groups if isinstance(g['curv'], _DiagBatchNorm) and _is_pooled(g['curv'])]
+        diag = [g for g in groups if isinstance(g['curv'], DiagCurvature) and _is_pooled(g['curv'])]
         taken = {id(g) for g in kron} | {id(g) for g in diag}
         rest = [g for g in groups if id(g) not in taken]
         self.pool = FactorPool([g['curv'] for g in kron], [g['curv'] for g in diag], device)
@@ -195,7 +196,8 @@ class SecondOrderOptimizer(Optimizer):
             if self.defaults['acc_steps'] != 1 or type(self).backward_postprocess is not SecondOrderOptimizer.backward_postprocess:
                 raise ValueError('fuse_ema needs acc_steps == 1 and a single process: accumulation and the '
                                  'owner-rank exchange carry curv.data')
-            if not all(c is not None and _is_pooled(c) for c in curvs) or len({c.ema_decay for c in curvs}) > 1:
+            fusable = all(isinstance(c, (_KronFactors, _DiagBatchNorm)) and _is_pooled(c) for c in curvs)
+            if not fusable or len({c.ema_decay for c in curvs}) > 1:
                 raise ValueError('fuse_ema needs Kronecker / BatchNorm curvatures with one common ema_decay')
         nat.join_curvature_stream(None)
         for c in curvs:
@@ -425,7 +427,7 @@ class SecondOrderOptimizer(Optimizer):
         if ent is None or ent[0] is not groups or ent[1] != len(groups):
             pooled = [g for g in groups if g['curv'] is not None and _is_pooled(g['curv'])]
             kron = [g for g in pooled if isinstance(g['curv'], _KronFactors)]
-            diag = [g for g in pooled if isinstance(g['curv'], _DiagBatchNorm)]
+            diag = [g for g in pooled if isinstance(g['curv'], DiagCurvature)]
             rest = [g for g in groups if g['curv'] is not None and not _is_pooled(g['curv'])]
             grads = [[self._grad_view[p] for p in g['params']] for g in kron]
             ent = self.__dict__['_split'] = (groups, len(groups), [g['curv'] for g in pooled], kron, diag, rest, grads,
@@ -470,11 +472,16 @@ class SecondOrderOptimizer(Optimizer):
                     gf = None if gflat is None else self._grad_flat[self._diag_grad_base + l:
                                                                      self._diag_grad_base + h]
                     self.pool.diag_step([c], gf, bool(update_inv))
-            for g in diag:
-                c = g['curv']
-                if update_inv:
+            if update_inv:
+                for c in dc:
                     c._have.add('inv')
-                    if update_std and update_std(g):
+                sd = [c for g, c in zip(diag, dc) if update_std and update_std(g)]
+                if len(sd) == len(dc):
+                    torch.sqrt(self.pool.buf('inv', 'd')[lo:hi], out=self.pool.buf('std', 'd')[lo:hi])
+                    for c in dc:
+                        c._have.add('std')
+                else:
+                    for c in sd:
                         c.update_std()
         for g in others:
             curv = g['curv']

@@ -15,7 +15,7 @@ from torchsso import _native as nat
 import torch.nn as nn
 import torch.nn.functional as F
 
-from torchsso.curv.layers import _KronFactors
+from torchsso.curv.layers import _KronFactors, _DiagBatchNorm, _DiagSq
 from torchsso.optim.secondorder import (SecondOrderOptimizer, DistributedSecondOrderOptimizer,
                                         _is_pooled)
 from torchsso.utils import TensorAccumulator
@@ -127,16 +127,25 @@ class VIOptimizer(SecondOrderOptimizer):
         """params <- a draw from the posterior (mean where a layer has no std yet).  Noise is
         drawn layer by layer in param_group order; all Kronecker layers are then transformed in
         one batched plan."""
-        batches = {}
+        batches, diag = {}, {}
         for group in self.param_groups:
             params, mean, curv = group['params'], group['mean'], group['curv']
             if curv is None or curv.std is None:
                 torch._foreach_copy_([p.data for p in params], mean)
                 continue
-            fast = (isinstance(curv, _KronFactors) and _is_pooled(curv) and
+            fast = (isinstance(curv, (_KronFactors, _DiagSq, _DiagBatchNorm)) and _is_pooled(curv) and
                     all(p.data.is_contiguous() and p.dtype == torch.float32 for p in params))
             if not fast:
                 curv.sample_params(params, mean, group['std_scale'])
+                continue
+            if not isinstance(curv, _KronFactors):
+                # drawn tensor by tensor, combined for all layers at once below
+                noise = [curv.pool.vec('noise', curv, j).normal_() for j in range(len(params))]
+                p, m, e, u = diag.setdefault(float(group['std_scale']), ([], [], [], []))
+                p += [t.data for t in params]
+                m += mean
+                e += noise
+                u += curv.std
                 continue
             buf = self._noise_buf(group)
             buf.copy_(torch.randn_like(buf))
@@ -145,6 +154,9 @@ class VIOptimizer(SecondOrderOptimizer):
             c.append(curv)
             t.append([p.data for p in params])
             nz.append(buf)
+        for scale, (p, m, e, u) in diag.items():
+            torch._foreach_copy_(p, m)
+            torch._foreach_addcmul_(p, e, u, value=scale)
         for scale, (c, t, nz) in batches.items():
             self.pool.sample(c, t, nz, scale)
 

@@ -84,7 +84,8 @@ def conv_ref(x, k, s, p, d, bias, weight=None):
 F32_CONVS = [(5, 3, 20, 19, (7, 7), (2, 2), (3, 3), (1, 1), False), (3, 1, 9, 9, (3, 3), (1, 1), (1, 1), (1, 1), True),
              (4, 7, 12, 10, (3, 2), (1, 2), (1, 0), (2, 1), True), (6, 11, 9, 9, (3, 3), (1, 1), (1, 1), (1, 1), True),
              (3, 64, 8, 8, (3, 3), (1, 1), (1, 1), (1, 1), True), (2, 26, 13, 13, (5, 5), (1, 1), (2, 2), (1, 1), False),
-             (40, 33, 6, 6, (1, 1), (2, 2), (0, 0), (1, 1), True), (16, 130, 5, 7, (1, 1), (1, 1), (0, 0), (1, 1), True)]
+             (40, 33, 6, 6, (1, 1), (2, 2), (0, 0), (1, 1), True), (2, 9, 10, 10, (9, 9), (1, 1), (4, 4), (1, 1), True),
+             (3, 21, 9, 8, (4, 4), (1, 1), (1, 1), (1, 1), False), (1, 40, 7, 7, (2, 2), (1, 1), (0, 0), (1, 1), True), (16, 130, 5, 7, (1, 1), (1, 1), (0, 0), (1, 1), True)]
 
 
 @pytest.mark.parametrize('cfg', F32_CONVS)
@@ -200,3 +201,31 @@ def test_kron_plan_reports_the_bad_pivot(nat, at):
     for i in (0, 2):
         want = torch.linalg.inv(src[i].double() + 0.02 * torch.eye(dims[i], device='cuda', dtype=torch.float64))
         assert rel(dst[i], want) < 1e-5
+
+
+# ------------------------------------------------------------------------------- batch normalisation
+@pytest.mark.parametrize('weighted', [False, True])
+def test_bn_batch(nat, weighted):
+    """Layers of every type and layout in one call, more of them than one launch holds."""
+    shapes = [(4, 8, 5, 5), (4, 24, 3, 7), (4, 2048, 2, 2), (4, 64, 1, 1), (4, 7, 4, 4), (4, 12)] + [(4, 16, 9, 9)] * 70
+    w = torch.rand(4, device='cuda') if weighted else None
+    want, keep = [], []
+    with nat.collect_factors():
+        for i, shape in enumerate(shapes):
+            dtype = (torch.float32, torch.bfloat16, torch.float16)[i % 3]
+            g = torch.randn(shape, device='cuda').to(dtype)
+            if len(shape) == 4 and i % 2 == 0:
+                g = g.contiguous(memory_format=torch.channels_last)
+            n, c = shape[:2]
+            t, st, splits = nat.bn_plane_layout(g)
+            sx = torch.rand(n, 2, c, device='cuda')
+            sg = torch.empty(n * splits * c, device='cuda')
+            wo, bo = torch.rand(c, device='cuda'), torch.rand(c, device='cuda') if i % 5 else None
+            gs = g.double().reshape(n, c, -1).square().sum(-1) * (1.0 if w is None else w.double()[:, None])
+            want.append((wo, 0.5 * (sx.double().sum(1) * gs).mean(0) + 2.0 * wo.double()))
+            if bo is not None:
+                want.append((bo, 0.5 * gs.mean(0) + 2.0 * bo.double()))
+            keep.append((sx, sg))
+            assert nat.collect_norm(t, (st, splits), sg, sx, w, 2, 0.5, 2.0, wo, bo)
+    for got, ref in want:
+        assert rel(got, ref) < 1e-5

@@ -1,26 +1,26 @@
-// Diagonal block of a 128-column Cholesky panel, done by one CTA: L = chol(D) and L^-1 for a
-// (<=128)x(<=128) SPD block D, all in fp32 FMA arithmetic.
+// Diagonal block of a 128-column Cholesky panel, done by eight warps: L = chol(D) and L^-1 for a
+// (<=128)x(<=128) SPD block D, all in fp32 FMA arithmetic, in shared memory (pitch 132: the 16-byte loads of
+// eight consecutive rows meet no bank conflict).
 //
-// The block is distributed cyclically over a 16x16 thread grid: thread (ty, tx) holds the elements
-// (ty + 16 i, tx + 16 j), i >= j, in registers, so that every thread owns a piece of every 16-column
-// panel and of every trailing block (the work stays balanced while the trailing matrix shrinks, and
-// the 16 threads of a row of the grid touch 16 consecutive shared-memory rows, which at a pitch of 132
-// floats are 4 banks apart: 16-byte loads without conflicts).  Right-looking over panels of 16 columns:
-//   publish : the owners write panel k (rows >= 16 k) into shared memory
-//   factor  : one warp, lane = row, factorises the 16x16 diagonal block: per pivot one round of shuffles
-//             (the raw column, and the next diagonal element so that the next pivot's rsqrt starts early)
-//   solve   : one thread per row below solves its 16 unknowns against that block (forward substitution)
-//   update  : every thread subtracts the panel's outer product from its registers
-// i.e. three block barriers per 16 columns instead of one per column.  The finished factor sits in shared
-// memory; its inverse follows by the inverses of the eight 16x16 diagonal blocks (one warp each, lane =
-// column) and three levels of doubling, Inv21 = -Inv22 * (L21 * Inv11), with the product L21 * Inv11
-// parked in the (otherwise unused) upper triangle.  Rows and columns past the block's size behave as an
-// identity block.  A pivot that is not a positive normal number (non-positive, denormal or NaN) is recorded
-// once per matrix (LAPACK numbering) and replaced by 1, like the 64-wide kernel does for non-positive ones.
-// Measured (d = 4608, 36 panels): 24 us per launch against 2 x 44 us for the two 64-wide factorisations plus
-// 2 x 14 us of 64-wide panel tasks it replaces; what is left is bound by shared-memory bandwidth (trailing
-// update and doubling products: 16-byte loads cost four cycles each for the whole SM) and by the chain of
-// 128 pivots (86 cycles each).
+// The block is eight panels of 16 columns.  What bounds it is the chain of 128 pivots, so warp 0 does nothing but
+// that chain: of panel k it takes the 16x16 diagonal block, subtracts the panel before, eliminates, and next solves
+// the one 16x16 block that its next diagonal block needs.  The other warps follow half a step behind: trailing update
+// by panel k - 1 and, in the idle half of the matrix, the sums G(k, c) = sum_j L(k, j) Inv(j, c) of row k of the
+// inverse (20 to 28 block products a step, spread over seven warps by a table).  Two barriers a step:
+//   X : panel k's block and its inverse are there, panel k - 1 has been subtracted everywhere
+//       then, one 16x16 product per warp: L(i, k) = A(i, k) Inv_kk^T below, Inv(k, c) = -Inv_kk G(k, c) to the left
+//   Y : those are there (warp 0 only announces its own and goes on)
+// The elimination: lane l of warp 0 holds row l of the block, lane l + 16 row l of an identity that goes through the
+// same steps, which leaves the inverse's column l in it for no further instruction; per pivot one round of shuffles
+// (the raw column, and the next diagonal element so that the next pivot's rsqrt starts early).
+// Rows and columns past the block's size behave as an identity block.  A pivot that is not a positive normal number
+// (non-positive, denormal or NaN) is recorded once per matrix (LAPACK numbering) and replaced by 1, like the 64-wide
+// kernel does for non-positive ones.
+// Measured: 17 us for 128 rows (clocks: 1600 to 3100 per elimination, 750 per round of products, which are bound by
+// the 512 bytes per 16-byte load and warp that shared memory returns); a chain of four barriers per panel with all
+// warps in step and the inverse by three levels of doubling afterwards took 23.  Inside the dataflow kernel, with the
+// inverse of the block announced before the other results are written: 1000 402 -> 307 us, 577+64 264 -> 203, the six
+// factors of 784-1000-1000-10 433 -> 339, 4608+512 2208 -> 1715.
 #pragma once
 #include "common.cuh"
 
@@ -31,7 +31,7 @@ constexpr int PN = 128;        // rows / columns handled by one CTA
 constexpr int PP = 132;        // pitch of the shared-memory matrices (floats)
 constexpr int PK = 16;         // panel width inside the block
 constexpr int THREADS = 256;
-constexpr size_t SMEM_BYTES = (size_t)(2 * PN * PP + PN) * sizeof(float);
+constexpr size_t SMEM_BYTES = (size_t)(2 * PN * PP) * sizeof(float);
 
 // MUFU.RSQ alone (2 ulp); the argument is a positive normal number wherever this is called
 __device__ __forceinline__ float rsqrt_approx(float x) {
@@ -44,324 +44,250 @@ __device__ __forceinline__ void st4(float* p, float x, float y, float z, float w
   *reinterpret_cast<float4*>(p) = make_float4(x, y, z, w);
 }
 
-// One level of the doubling for the range [lo, lo + 2 SZ): first product (stage 0)
-//     Y = L21 * Inv11      -> S rows lo.., columns lo + SZ..  (scratch above the diagonal)
-// then (stage 1)            Inv21 = -Inv22 * Y.
-// Thread (ty, tx) computes the outputs (ty + 16 a, tx + 16 b).  Inv11 and Inv22 are lower triangular: the
-// half of the inner range that only meets zeros of a whole half of the output is skipped.
-template <int SZ>
-__device__ __forceinline__ void doubling_product(float* __restrict__ S, float* __restrict__ V, int lo, int stage,
-                                                 int ty, int tx) {
-  constexpr int NT = SZ / 16;
-  constexpr int NH = NT >= 2 ? NT / 2 : NT;
-  const int mid = lo + SZ;
-  float acc[NT][NT];
+// Barriers 1 and 2 of the eight warps that factorise a block, which may be part of a larger CTA.
+__device__ __forceinline__ void sync_x() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
+__device__ __forceinline__ void sync_y() { asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory"); }
+__device__ __forceinline__ void arrive_y() { asm volatile("bar.arrive 2, %0;" ::"n"(THREADS) : "memory"); }
+
+// A warp's 16x16x16 product: lane (rg, cg) holds rows rg, rg + 8; columns cg + 4 v of A B^T, 4 cg + v of A B.
+struct Acc {
+  float v[2][4];
+  __device__ __forceinline__ void zero() {
 #pragma unroll
-  for (int a = 0; a < NT; ++a)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int b = 0; b < NT; ++b) acc[a][b] = 0.f;
-  if (stage == 0) {
-    // Y[r][c] = sum_q L[mid + r][lo + q] * Inv[lo + q][lo + c], Inv11[q][c] = 0 for q < c
-    const float* Lr = S + (mid + ty) * PP + lo;
-    const float* Vc = V + lo * PP + lo + tx;
-#pragma unroll 8
-    for (int q = 0; q < SZ / 2; ++q) {      // meets the columns of the first half only (all of them if NT == 1)
-      float l[NT];
+      for (int j = 0; j < 4; ++j) v[i][j] = 0.f;
+  }
+  __device__ __forceinline__ void add(int i, float4 a, const float4 (&b)[4]) {      // along q
 #pragma unroll
-      for (int a = 0; a < NT; ++a) l[a] = Lr[16 * a * PP + q];
+    for (int j = 0; j < 4; ++j) v[i][j] = fmaf(a.x, b[j].x, v[i][j]);
 #pragma unroll
-      for (int b = 0; b < NH; ++b) {
-        const float v = Vc[q * PP + 16 * b];
+    for (int j = 0; j < 4; ++j) v[i][j] = fmaf(a.y, b[j].y, v[i][j]);
 #pragma unroll
-        for (int a = 0; a < NT; ++a) acc[a][b] = fmaf(l[a], v, acc[a][b]);
-      }
+    for (int j = 0; j < 4; ++j) v[i][j] = fmaf(a.z, b[j].z, v[i][j]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[i][j] = fmaf(a.w, b[j].w, v[i][j]);
+  }
+  __device__ __forceinline__ void nt(const float* __restrict__ A, const float* __restrict__ B, int rg, int cg) {
+#pragma unroll
+    for (int q = 0; q < PK; q += 4) {
+      const float4 a0 = ld4(A + rg * PP + q), a1 = ld4(A + (rg + 8) * PP + q);
+      float4 b[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = ld4(B + (cg + 4 * j) * PP + q);
+      add(0, a0, b);
+      add(1, a1, b);
     }
-#pragma unroll 8
-    for (int q = SZ / 2; q < SZ; ++q) {
-      float l[NT];
+  }
+  __device__ __forceinline__ void nn(const float* __restrict__ A, const float* __restrict__ B, int rg, int cg) {
 #pragma unroll
-      for (int a = 0; a < NT; ++a) l[a] = Lr[16 * a * PP + q];
+    for (int q = 0; q < PK; q += 4) {
+      const float4 a[2] = {ld4(A + rg * PP + q), ld4(A + (rg + 8) * PP + q)};
+      float4 b[4];
 #pragma unroll
-      for (int b = 0; b < NT; ++b) {
-        const float v = Vc[q * PP + 16 * b];
+      for (int j = 0; j < 4; ++j) b[j] = ld4(B + (q + j) * PP + 4 * cg);
 #pragma unroll
-        for (int a = 0; a < NT; ++a) acc[a][b] = fmaf(l[a], v, acc[a][b]);
-      }
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float x = j == 0 ? a[i].x : j == 1 ? a[i].y : j == 2 ? a[i].z : a[i].w;
+          v[i][0] = fmaf(x, b[j].x, v[i][0]);
+          v[i][1] = fmaf(x, b[j].y, v[i][1]);
+          v[i][2] = fmaf(x, b[j].z, v[i][2]);
+          v[i][3] = fmaf(x, b[j].w, v[i][3]);
+        }
     }
-    float* Y = S + (lo + ty) * PP + mid + tx;
+  }
+};
+
+// What warps 1 to 7 do while warp 0 eliminates panel k >= 1: trailing blocks (i, j) and sums G(k, c), longest first to
+// the warp with the least so far.
+struct Schedule {
+  unsigned char task[8][7][8];      // 0xFF: none; 0x80 | c: G(k, c); else i << 3 | j
+};
+constexpr Schedule make_schedule() {
+  Schedule s{};
+  for (int k = 0; k < 8; ++k) {
+    int load[7] = {}, count[7] = {};
+    for (int w = 0; w < 7; ++w)
+      for (int t = 0; t < 8; ++t) s.task[k][w][t] = 0xFF;
+    if (k == 0) continue;
+    auto give = [&](int code, int cost) {
+      int best = -1;
+      for (int w = 0; w < 7; ++w)
+        if (count[w] < 8 && (best < 0 || load[w] < load[best])) best = w;
+      s.task[k][best][count[best]++] = (unsigned char)code;
+      load[best] += cost;
+    };
+    for (int c = 0; c < k; ++c)
+      if (k - c > 1) give(0x80 | c, 8 * (k - c) + 2);
+    for (int i = k; i < 8; ++i)
+      for (int j = k; j <= i; ++j)
+        if (i != k) give(i << 3 | j, 10);
+    give(0x80 | (k - 1), 10);
+  }
+  return s;
+}
+static __constant__ Schedule c_schedule = make_schedule();
+
+// The elimination of panel k's diagonal block by one warp, after the subtraction of panel k - 1.
+__device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restrict__ V, int k, int n, int* __restrict__ info, int row0, int lane) {
+  const int l = lane & 15, h = lane >> 4, c0 = PK * k;
+  float* D = S + c0 * PP + c0;
+  // row l of the block, columns 8 h ..: both halves of the warp subtract, the lower one collects
+  float d[8];
+  {
+    const float4 u = ld4(D + l * PP + 8 * h), w = ld4(D + l * PP + 8 * h + 4);
+    d[0] = u.x; d[1] = u.y; d[2] = u.z; d[3] = u.w; d[4] = w.x; d[5] = w.y; d[6] = w.z; d[7] = w.w;
+  }
+  if (k > 0) {
+    const float* P = D - PK;
 #pragma unroll
-    for (int a = 0; a < NT; ++a)
+    for (int q = 0; q < PK; q += 4) {
+      const float4 a = ld4(P + l * PP + q);
+      float4 b[8];
 #pragma unroll
-      for (int b = 0; b < NT; ++b) Y[16 * a * PP + 16 * b] = acc[a][b];
+      for (int c = 0; c < 8; ++c) b[c] = ld4(P + (8 * h + c) * PP + q);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) d[c] = fmaf(-a.x, b[c].x, d[c]);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) d[c] = fmaf(-a.y, b[c].y, d[c]);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) d[c] = fmaf(-a.z, b[c].z, d[c]);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) d[c] = fmaf(-a.w, b[c].w, d[c]);
+    }
+  }
+  float v[PK];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const float up = __shfl_down_sync(0xffffffffu, d[c], 16);
+    v[c] = h ? (c == l ? 1.f : 0.f) : (c <= l ? d[c] : 0.f);
+    v[c + 8] = h ? (c + 8 == l ? 1.f : 0.f) : (c + 8 <= l ? up : 0.f);
+  }
+  float pv = __shfl_sync(0xffffffffu, v[0], 0);
+  int first_bad = -1;
+#pragma unroll
+  for (int j = 0; j < PK; ++j) {
+    float t[PK];
+#pragma unroll
+    for (int c = j + 1; c < PK; ++c) t[c] = __shfl_sync(0xffffffffu, v[j], c);      // a[c][j]
+    float d1 = 0.f;
+    if (j + 1 < PK) d1 = __shfl_sync(0xffffffffu, v[j + 1], j + 1);                 // a[j+1][j+1] before this step
+    const bool bad = !(pv >= 1.17549435e-38f);
+    if (bad && first_bad < 0) first_bad = j;
+    const float rs = bad ? 1.f : rsqrt_approx(pv);
+    const float w = v[j] * (rs * rs);
+#pragma unroll
+    for (int c = j + 1; c < PK; ++c) v[c] = fmaf(-w, t[c], v[c]);
+    v[j] = lane == j ? (bad ? 1.f : pv) * rs : v[j] * rs;
+    if (j + 1 < PK) {
+      const float x = t[j + 1] * rs;
+      pv = fmaf(-x, x, d1);
+    }
+  }
+  if (first_bad >= 0 && lane == 0 && info && c0 + first_bad < n) atomicCAS(info, 0, row0 + c0 + first_bad + 1);
+  if (h == 0) {
+#pragma unroll
+    for (int q = 0; q < PK; q += 4)
+      st4(D + l * PP + q, q <= l ? v[q] : 0.f, q + 1 <= l ? v[q + 1] : 0.f, q + 2 <= l ? v[q + 2] : 0.f, q + 3 <= l ? v[q + 3] : 0.f);
   } else {
-    // Inv21[r][c] = -sum_q Inv[mid + r][mid + q] * Y[q][c], Inv22[r][q] = 0 for q > r
-    const float* Vr = V + (mid + ty) * PP + mid;
-    const float* Yc = S + lo * PP + mid + tx;
-#pragma unroll 8
-    for (int q = 0; q < SZ / 2; ++q) {
-      float y[NT];
 #pragma unroll
-      for (int b = 0; b < NT; ++b) y[b] = Yc[q * PP + 16 * b];
-#pragma unroll
-      for (int a = 0; a < NT; ++a) {
-        const float v = Vr[16 * a * PP + q];
-#pragma unroll
-        for (int b = 0; b < NT; ++b) acc[a][b] = fmaf(v, y[b], acc[a][b]);
-      }
-    }
-#pragma unroll 8
-    for (int q = SZ / 2; q < SZ; ++q) {     // meets the rows of the second half only (all of them if NT == 1)
-      float y[NT];
-#pragma unroll
-      for (int b = 0; b < NT; ++b) y[b] = Yc[q * PP + 16 * b];
-#pragma unroll
-      for (int a = NT - NH; a < NT; ++a) {
-        const float v = Vr[16 * a * PP + q];
-#pragma unroll
-        for (int b = 0; b < NT; ++b) acc[a][b] = fmaf(v, y[b], acc[a][b]);
-      }
-    }
-    float* O = V + (mid + ty) * PP + lo + tx;
-#pragma unroll
-    for (int a = 0; a < NT; ++a)
-#pragma unroll
-      for (int b = 0; b < NT; ++b) O[16 * a * PP + 16 * b] = -acc[a][b];
+    for (int r = 0; r < PK; ++r) V[(c0 + r) * PP + c0 + l] = v[r];
   }
 }
 
-// Barrier of the 256 threads that factorise a block: the whole CTA, or eight warps of a larger one.
-struct CtaSync {
-  __device__ __forceinline__ static void sync() { __syncthreads(); }
-};
-template <int ID>
-struct NamedSync {
-  __device__ __forceinline__ static void sync() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory"); }
-};
-
-template <int SZ, typename Sync>
-__device__ __forceinline__ void doubling_level(float* S, float* V, int cols, int ty, int tx) {
-  // ranges whose second half lies past the matrix (identity padding) keep Inv21 = 0
-  for (int lo = 0; lo + SZ < cols; lo += 2 * SZ) doubling_product<SZ>(S, V, lo, 0, ty, tx);
-  Sync::sync();
-  for (int lo = 0; lo + SZ < cols; lo += 2 * SZ) doubling_product<SZ>(S, V, lo, 1, ty, tx);
-  Sync::sync();
-}
-
-// Panel K of the thread's elements goes to shared memory (rows >= 16 K).
-template <int K>
-__device__ __forceinline__ void publish_panel(const float (&a)[8][8], float* __restrict__ S, int ty, int tx) {
-#pragma unroll
-  for (int i = K; i < 8; ++i) S[(ty + 16 * i) * PP + PK * K + tx] = a[i][K];
-}
-
-// a[i][j] -= sum_q L[row_i][16 K + q] * L[col_j][16 K + q] for K < j <= i, four q at a time.  K is a template
-// parameter so that the loop body is straight-line code: a branch per block column costs a single warp
-// more than the multiply-adds it guards.  Rows past the matrix hold zeros in the published panel.
-template <int K>
-__device__ __forceinline__ void update_trailing(float (&a)[8][8], const float* __restrict__ S, int ty, int tx) {
-  if (K >= 7) return;
-  const float* rbase = S + ty * PP + PK * K;
-  const float* cbase = S + tx * PP + PK * K;
-#pragma unroll 1
-  for (int qc = 0; qc < PK / 4; ++qc) {
-    float4 rv[8], cv[8];
-#pragma unroll
-    for (int i = K + 1; i < 8; ++i) {
-      rv[i] = ld4(rbase + 16 * i * PP + 4 * qc);
-      cv[i] = ld4(cbase + 16 * i * PP + 4 * qc);
-    }
-    // one component of the four at a time over all pairs: consecutive multiply-adds are independent
-#pragma unroll
-    for (int j = K + 1; j < 8; ++j)
-#pragma unroll
-      for (int i = j; i < 8; ++i) a[i][j] = fmaf(-rv[i].x, cv[j].x, a[i][j]);
-#pragma unroll
-    for (int j = K + 1; j < 8; ++j)
-#pragma unroll
-      for (int i = j; i < 8; ++i) a[i][j] = fmaf(-rv[i].y, cv[j].y, a[i][j]);
-#pragma unroll
-    for (int j = K + 1; j < 8; ++j)
-#pragma unroll
-      for (int i = j; i < 8; ++i) a[i][j] = fmaf(-rv[i].z, cv[j].z, a[i][j]);
-#pragma unroll
-    for (int j = K + 1; j < 8; ++j)
-#pragma unroll
-      for (int i = j; i < 8; ++i) a[i][j] = fmaf(-rv[i].w, cv[j].w, a[i][j]);
-  }
-}
-
-// The factorisation itself, by 256 threads: a[i][j] of thread (ty, tx) is the block's element (ty + 16 i, tx + 16 j), j <= i,
-// rows and columns past n an identity.  Leaves L in S (lower triangle) and L^-1, with zeros above the diagonal and an
-// identity past n, in V.  `info` (nullable) receives the 1-based number row0 + pivot + 1 of the first bad pivot.
-template <typename Sync>
-__device__ __forceinline__ void factor_block(float (&a)[8][8], float* __restrict__ S, float* __restrict__ V, float* __restrict__ dinv, int n,
-                                             int* __restrict__ info, int row0, int tid) {
-  const int lane = tid & 31, warp = tid >> 5;
-  const int ty = tid >> 4, tx = tid & 15;
+// The factorisation itself, by 256 threads (barriers 1 and 2).  S holds the lower triangle on entry, visible to all of
+// them, with an identity past the first n rows and columns; on return (behind a barrier) L in its lower triangle and
+// L^-1, with zeros above the diagonal and the identity past n, in V.  `info` (nullable) receives the 1-based number
+// row0 + pivot + 1 of the first bad pivot.
+__device__ __forceinline__ void factor_block(float* __restrict__ S, float* __restrict__ V, int n, int* __restrict__ info, int row0, int tid) {
+  const int lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int rg = lane >> 2, cg = lane & 3;
   const int np = (n + PK - 1) / PK;     // panels that hold columns of the matrix
-  const int cols = np * PK;
-  for (int e = tid; e < PN * PP / 4; e += THREADS) st4(V + 4 * e, 0.f, 0.f, 0.f, 0.f);
-  if (tid < PN) dinv[tid] = 1.f;
-
+  auto at = [](float* m, int i, int j) { return m + (PK * i) * PP + PK * j; };
   for (int k = 0; k < np; ++k) {
-    const int c0 = PK * k;
-    // ---- publish panel k
-    switch (k) {
-      case 0: publish_panel<0>(a, S, ty, tx); break;
-      case 1: publish_panel<1>(a, S, ty, tx); break;
-      case 2: publish_panel<2>(a, S, ty, tx); break;
-      case 3: publish_panel<3>(a, S, ty, tx); break;
-      case 4: publish_panel<4>(a, S, ty, tx); break;
-      case 5: publish_panel<5>(a, S, ty, tx); break;
-      case 6: publish_panel<6>(a, S, ty, tx); break;
-      default: publish_panel<7>(a, S, ty, tx); break;
-    }
-    Sync::sync();
-    // ---- 16x16 diagonal block by warp 0: lane l (and its twin l + 16) holds row l.  One exchange per pivot:
-    // every lane fetches the raw column j (pivot included) from the lanes that own it, takes the rsqrt of
-    // the pivot itself and applies the rank-1 update to its own row.
     if (warp == 0) {
-      const int l = lane & 15;
-      float* row = S + (c0 + l) * PP + c0;
-      float r[PK];
-#pragma unroll
-      for (int q = 0; q < PK; q += 4) {
-        const float4 v = ld4(row + q);
-        r[q] = v.x; r[q + 1] = v.y; r[q + 2] = v.z; r[q + 3] = v.w;
+      eliminate(S, V, k, n, info, row0, lane);
+    } else if (k == 0) {
+      // the inverse's upper half, and its identity past the matrix
+      for (int e = tid - 32; e < PN * PN / 4; e += THREADS - 32) {
+        const int r = e / (PN / 4), c = e % (PN / 4) * 4;
+        if (c / PK > r / PK || r >= PK * np) st4(V + r * PP + c, c == r ? 1.f : 0.f, c + 1 == r ? 1.f : 0.f, c + 2 == r ? 1.f : 0.f, c + 3 == r ? 1.f : 0.f);
       }
-#pragma unroll
-      for (int c = 0; c < PK; ++c)
-        if (c > l) r[c] = 0.f;
-      // The pivot of step j + 1 is formed inside step j from the next raw diagonal element (fetched with
-      // the column) by the same multiply-add its owner applies to it: the rsqrt of the next pivot then runs
-      // while the shuffles of the next column are in flight, instead of after them.
-      float pv = __shfl_sync(0xffffffffu, r[0], 0);
-      int first_bad = -1;
-#pragma unroll
-      for (int j = 0; j < PK; ++j) {
-        float t[PK];
-#pragma unroll
-        for (int c = j + 1; c < PK; ++c) t[c] = __shfl_sync(0xffffffffu, r[j], c);     // a[c][j], c > j
-        float d1 = 0.f;
-        if (j + 1 < PK) d1 = __shfl_sync(0xffffffffu, r[j + 1], j + 1);                // a[j+1][j+1] before this step
-        // a pivot that is not a positive normal number (or is NaN) is remembered and replaced by 1; no branch
-        // here: the chain from one pivot to the next is what bounds this kernel
-        const bool bad = !(pv >= 1.17549435e-38f);
-        if (bad && first_bad < 0) first_bad = j;
-        pv = bad ? 1.f : pv;
-        const float rs = rsqrt_approx(pv);
-        const float lj = (l == j) ? pv * rs : r[j] * rs;      // L[l][j]; rows above the pivot hold 0
-#pragma unroll
-        for (int c = j + 1; c < PK; ++c) r[c] = fmaf(-lj, t[c] * rs, r[c]);            // kept for c <= l only
-        r[j] = lj;
-        if (lane == j) dinv[c0 + j] = rs;
-        if (j + 1 < PK) {
-          const float x = t[j + 1] * rs;
-          pv = fmaf(-x, x, d1);
-        }
-      }
-      if (first_bad >= 0 && lane == 0 && info && c0 + first_bad < n) atomicCAS(info, 0, row0 + c0 + first_bad + 1);
-      if (lane < PK) {
-#pragma unroll
-        for (int q = 0; q < PK; q += 4)
-          st4(row + q, q <= l ? r[q] : 0.f, q + 1 <= l ? r[q + 1] : 0.f, q + 2 <= l ? r[q + 2] : 0.f,
-              q + 3 <= l ? r[q + 3] : 0.f);
-      }
-    }
-    Sync::sync();
-    // ---- rows below the diagonal block: x * L16^T = a, one thread per row, right looking (each finished
-    // unknown is subtracted from all later ones at once, so the dependent chain is two operations per step)
-    {
-      const int rowi = c0 + PK + tid;
-      if (rowi < cols) {
-        float* xr = S + rowi * PP + c0;
-        const float* lblk = S + c0 * PP + c0;            // same addresses in every lane: broadcast
-        float x[PK];
-#pragma unroll
-        for (int q = 0; q < PK; q += 4) {
-          const float4 v = ld4(xr + q);
-          x[q] = v.x; x[q + 1] = v.y; x[q + 2] = v.z; x[q + 3] = v.w;
-        }
-#pragma unroll
-        for (int c = 0; c < PK; ++c) {
-          x[c] *= dinv[c0 + c];
-#pragma unroll
-          for (int c2 = c + 1; c2 < PK; ++c2) x[c2] = fmaf(-x[c], lblk[c2 * PP + c], x[c2]);
-        }
-#pragma unroll
-        for (int q = 0; q < PK; q += 4) st4(xr + q, x[q], x[q + 1], x[q + 2], x[q + 3]);
-      }
-    }
-    Sync::sync();
-    // ---- trailing update
-    if (k + 1 < np) {
-      switch (k) {
-        case 0: update_trailing<0>(a, S, ty, tx); break;
-        case 1: update_trailing<1>(a, S, ty, tx); break;
-        case 2: update_trailing<2>(a, S, ty, tx); break;
-        case 3: update_trailing<3>(a, S, ty, tx); break;
-        case 4: update_trailing<4>(a, S, ty, tx); break;
-        case 5: update_trailing<5>(a, S, ty, tx); break;
-        default: update_trailing<6>(a, S, ty, tx); break;
-      }
-    }
-  }
-  // ---- identity padding of the factor (columns that hold no matrix column were never published)
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-    if (j >= np) {
-#pragma unroll
-      for (int i = j; i < 8; ++i) S[(ty + 16 * i) * PP + 16 * j + tx] = (i == j && ty == tx) ? 1.f : 0.f;
-    }
-  Sync::sync();
-  // ---- inverses of the 16x16 diagonal blocks: warp w, lane c = column c of block w
-  if (lane < PK) {
-    const int b0 = PK * warp, c = lane;
-    if (warp < np) {
-      float x[PK];
-#pragma unroll
-      for (int r = 0; r < PK; ++r) {
-        const float* lrow = S + (b0 + r) * PP + b0;
-        float s = 0.f;
-#pragma unroll
-        for (int q = 0; q < r; ++q) s = fmaf(lrow[q], x[q], s);     // x[q] = 0 for q < c
-        const float d = dinv[b0 + r];
-        x[r] = (r < c) ? 0.f : (r == c ? d : -s * d);
-      }
-#pragma unroll
-      for (int r = 0; r < PK; ++r) V[(b0 + r) * PP + b0 + c] = x[r];
     } else {
-      V[(b0 + c) * PP + b0 + c] = 1.f;
+#pragma unroll 1
+      for (int slot = 0; slot < 8; ++slot) {
+        const int code = c_schedule.task[k][warp - 1][slot];
+        if (code == 0xFF) break;
+        Acc acc;
+        acc.zero();
+        if (code & 0x80) {
+          const int c = code & 7;
+#pragma unroll 1
+          for (int j = c; j < k; ++j) acc.nn(at(S, k, j), at(V, j, c), rg, cg);
+          float* G = at(S, c, k);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) st4(G + (rg + 8 * i) * PP + 4 * cg, acc.v[i][0], acc.v[i][1], acc.v[i][2], acc.v[i][3]);
+        } else {
+          const int i0 = code >> 3, j0 = code & 7;
+          if (i0 >= np) continue;
+          acc.nt(at(S, i0, k - 1), at(S, j0, k - 1), rg, cg);
+          float* C = at(S, i0, j0) + rg * PP + cg;
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) C[8 * i * PP + 4 * j] -= acc.v[i][j];
+        }
+      }
+    }
+    sync_x();
+    // warp 0: the block below the diagonal one; the others: k blocks of the inverse's row, then the blocks further below
+    const int m = warp - 1;
+    const bool left = warp != 0 && m < k;
+    const int i = warp == 0 ? k + 1 : k + 2 + (m - k);
+    Acc acc;
+    acc.zero();
+    if (left) {
+      acc.nn(at(V, k, k), at(S, m, k), rg, cg);
+      float* O = at(V, k, m);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) st4(O + (rg + 8 * r) * PP + 4 * cg, -acc.v[r][0], -acc.v[r][1], -acc.v[r][2], -acc.v[r][3]);
+    } else if (i < np) {
+      acc.nt(at(S, i, k), at(V, k, k), rg, cg);
+      __syncwarp();
+      float* O = at(S, i, k) + rg * PP + cg;
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) O[8 * r * PP + 4 * j] = acc.v[r][j];
+    }
+    if (warp == 0) {
+      __syncwarp();
+      if (k + 1 < np) arrive_y();
+      else sync_y();
+    } else {
+      sync_y();
     }
   }
-  Sync::sync();
-  doubling_level<16, Sync>(S, V, cols, ty, tx);
-  doubling_level<32, Sync>(S, V, cols, ty, tx);
-  doubling_level<64, Sync>(S, V, cols, ty, tx);
 }
 
 static __global__ void __launch_bounds__(THREADS, 1) diag_panel_kernel(const sso_diag_rec* __restrict__ recs,
                                                                int* __restrict__ info) {
   extern __shared__ __align__(16) float psm[];
-  float* S = psm;               // panels of the block as they are published, then L (lower triangle)
+  float* S = psm;               // the block, then L (lower triangle)
   float* V = psm + PN * PP;     // L^-1
-  float* dinv = V + PN * PP;    // 1 / L_jj
   const sso_diag_rec rec = recs[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ty = tid >> 4, tx = tid & 15;
   const int n = rec.size;
-
-  float a[8][8];
+  for (int r = warp; r < PN; r += THREADS / 32)
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j <= i; ++j) {
-      const int r = ty + 16 * i, c = tx + 16 * j;
-      float v = (r == c) ? 1.f : 0.f;
-      if (r < n && c <= r) v = rec.L[(int64_t)r * rec.ld_l + c];
-      a[i][j] = v;
+    for (int u = 0; u < 4; ++u) {
+      const int c = lane + 32 * u;
+      if (c <= r) S[r * PP + c] = r < n ? rec.L[(int64_t)r * rec.ld_l + c] : (r == c ? 1.f : 0.f);
     }
-  factor_block<CtaSync>(a, S, V, dinv, n, info ? info + 2 * rec.mat + rec.info_slot : nullptr, rec.row0, tid);
+  __syncthreads();
+  factor_block(S, V, n, info ? info + 2 * rec.mat + rec.info_slot : nullptr, rec.row0, tid);
   // ---- results: the lower triangle of L, L^-1 with zeros above its diagonal, and optionally the upper
   // triangle of the transpose of L^-1.  Nothing reads L above the diagonal, and the buffer of the transpose
   // is zeroed before the factorisation starts.

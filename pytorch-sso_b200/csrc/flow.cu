@@ -4,8 +4,8 @@
 // start (engine.cu simulates the schedule); one CTA per SM takes the next task from a counter, so a task only ever
 // waits for tasks that running CTAs have taken before it.  A tile is announced by a flag in global memory, and a task
 // waits for its operands block by block along K: all but the last 128 columns of a panel update run before the
-// previous panel is done.  The chain from one panel to the next is then one diagonal block, one multiplication by
-// its inverse and the last 128 columns of one update, without a kernel boundary in it; as phases of launches every one
+// previous panel is done.  The chain from one panel to the next is then one diagonal block (its inverse is
+// announced before its other results are written), one multiplication by that inverse and the last 128 columns of one update, without a kernel boundary in it; as phases of launches every one
 // of these was a kernel of at least 11 us (4608: 36 panels of three launches, 20 more for the inverse).
 //
 // Inside a CTA (16 warps): 0-7 accumulate, store and factor diagonal blocks; 8 issues MMAs; 9 takes tasks, waits for flags
@@ -16,9 +16,9 @@
 // warps write it into the raw slots of four more stages.
 //
 // Bound: for one large matrix the chain of diagonal blocks, for many the shared-memory traffic of the 3xTF32 stages
-// (as tile_task_tma_kernel).  Against one launch per phase (us): 577+64 508 -> 264, 1000 637 -> 402, six factors of an
-// 784-1000-1000-10 network 1196 -> 433, 4608+512 3363 -> 2208, the 106 factors of ResNet-50 8970 -> 4630, those of VGG-16
-// with sampling factors 19416 -> 8915.
+// (as tile_task_tma_kernel).  Against one launch per phase (us): 577+64 508 -> 203, 1000 637 -> 307, six factors of an
+// 784-1000-1000-10 network 1196 -> 339, 4608+512 3363 -> 1715, the 106 factors of ResNet-50 8970 -> 4350, those of VGG-16
+// with sampling factors 19416 -> 8610.
 // Every wait is bounded; a CTA whose wait gives up sets the status word and writes NaN for this and all further tasks.
 #include "common.cuh"
 #include "diag_panel.cuh"
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         const Shape sh = shape_of(t, m.d);
         const bool over_x = t.kind == INVT || t.kind == PROD;      // A operand of the sum: X (else L); B: L, X for PROD
         const uint64_t map_w = reinterpret_cast<uint64_t>(m.map_w);
-        auto x_flag = [&](int j, int k) { return g.flags + (k == j ? m.flag_d + j : m.flag_x + j * m.np + k); };
+        auto x_flag = [&](int j, int k) { return g.flags + m.flag_x + j * m.np + k; };
         auto w_flag = [&](int i, int k) { return g.flags + m.flag_w + i * m.np + k; };
         auto issue = [&](uint64_t ma, int row_a, int ka, uint64_t mb, int row_b, int kb, bool a_on, bool b_on) {
           const uint32_t s = stage % RAW;
@@ -437,25 +437,24 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         // ---------------------------------------------------------------- diagonal block, in the operand ring
         float* S = ring;
         float* V = S + dpanel::PN * dpanel::PP;
-        float* dinv = V + dpanel::PN * dpanel::PP;
+        if (row < nr) {
 #pragma unroll
-        for (int i = 0; i < 64; i += 4) dpanel::st4(S + row * dpanel::PP + col0 + i, acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-        dpanel::NamedSync<1>::sync();
-        const int ty = tid >> 4, tx = tid & 15;
-        float a[8][8];
+          for (int i = 0; i < 64; i += 4) dpanel::st4(S + row * dpanel::PP + col0 + i, acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+        } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j <= i; ++j) {
-            const int r = ty + 16 * i, c = tx + 16 * j;
-            a[i][j] = (r < nr && c <= r) ? S[r * dpanel::PP + c] : (r == c ? 1.f : 0.f);
-          }
-        dpanel::NamedSync<1>::sync();
-        dpanel::factor_block<dpanel::NamedSync<1>>(a, S, V, dinv, nr, g.info ? g.info + 2 * m.mat + m.info_slot : nullptr, r0, tid);
+          for (int i = 0; i < 64; ++i) S[row * dpanel::PP + col0 + i] = col0 + i == row ? 1.f : 0.f;
+        }
+        dpanel::sync_x();
+        dpanel::factor_block(S, V, nr, g.info ? g.info + 2 * m.mat + m.info_slot : nullptr, r0, tid);
         float* li = m.Li + (int64_t)t.a * (TILE * TILE);
         for (int e = tid; e < TILE * TILE / 4; e += 256) {
           const int r = e / (TILE / 4), c = e % (TILE / 4) * 4;
           reinterpret_cast<float4*>(li)[e] = dpanel::ld4(V + r * dpanel::PP + c);
+        }
+        dpanel::sync_x();                        // the next panel waits for this alone: announced before the other results
+        if (tid == 0) {
+          __threadfence();
+          store_release(g.flags + m.flag_d + t.a, epoch);
         }
         for (int r = warp; r < nr; r += ACC_WARPS) {
 #pragma unroll
@@ -466,13 +465,13 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
             if (m.U) m.U[(int64_t)(r0 + r) * m.ldu + r0 + c] = c >= r ? S[c * dpanel::PP + r] : 0.f;
           }
         }
-        flag = g.flags + m.flag_d + t.a;
+        if (m.X) flag = g.flags + m.flag_x + t.a * m.np + t.a;
         fence_async_smem();                      // the ring goes back to TMA
         __syncwarp();
         if (lane == 0) mbar_arrive(ddone);
       }
       if (flag) {
-        dpanel::NamedSync<1>::sync();            // the tile is stored by all eight warps
+        dpanel::sync_x();                        // the tile is stored by all eight warps
         if (tid == 0) {
           __threadfence();
           store_release(flag, epoch);
@@ -514,7 +513,9 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
     __syncthreads();
     if (tid == 0 && t.kind != PROD) {
       __threadfence();
-      store_release(g.flags + (t.kind == DIAG ? m.flag_d + t.a : (t.kind == PANEL ? m.flag_w : m.flag_x) + t.a * m.np + t.b), epoch);
+      if (t.kind == DIAG) store_release(g.flags + m.flag_d + t.a, epoch);
+      if (t.kind == PANEL) store_release(g.flags + m.flag_w + t.a * m.np + t.b, epoch);
+      else if (m.X) store_release(g.flags + m.flag_x + t.a * m.np + (t.kind == DIAG ? t.a : t.b), epoch);
     }
   };
   for (uint32_t n = acc_at; n < pushed; ++n)

@@ -11,21 +11,26 @@
 // once instead of once per kernel position and tile, and whatever layout the input has (NCHW, odd channel counts,
 // unaligned rows) the gather sees 16-byte chunks of channels.  Bound: memory, 4 bytes in and 6 out per element.
 //
-// factor_f32_kernel gathers im2col rows of the parts with cp.async straight into the operand layout (MN-major
-// SWIZZLE_128B: 64 columns = 128 bytes of one row, zero-filled outside the image), in one of two shapes:
-//   PAIR   a cluster of two CTAs computes a 256x256 block with tcgen05.mma.cta_group::2; each CTA gathers the
-//          128 columns of either side that its half of the operands needs (factors wider than 128);
-//   single one CTA, one 128x128 tile (narrow factors, where a pair would compute padding).
-// Bound: the copies.  Per stage of 32 rows the twelve MMAs of a pair take 1536 cycles per SM (0.98 us as measured with
-// the gather taken out); 48 KB of parts per stage come in at 1.4 us whatever the number of stages in flight, MMAs or
-// not (5 TB/s over the chip: what the load/store path of an SM keeps outstanding).  Columns of a 5x5 window over 64
-// channels, d = 1601 from 65536 rows: 1.13 ms against 1.81 ms for 3xTF32 on 128x128 tiles, d = 4608 from 8192 rows
-// 1.06 against 1.71 ms.  Measured alternatives: splitting in the gather warps is bound by their instructions (650 per
-// warp and stage, 2.3 us per stage, in bf16 as in 3xTF32), and 32-bit MN-major operands are read at half the rate.
+// factor_f32_kernel brings im2col rows of the parts straight into the operand layout (MN-major SWIZZLE_128B: 64 columns =
+// 128 bytes of one row, zero-filled outside the image), in one of three shapes:
+//   PAIR, BOX  a cluster of two CTAs computes a 256x256 block with tcgen05.mma.cta_group::2; a stage is a box of 32 whole
+//              pixels, fetched by one thread with TMA, the three parts of 64 columns in one piece;
+//   PAIR       the same where no box covers the output exactly: eight warps gather with cp.async;
+//   single     one CTA, one 128x128 tile (narrow factors, where a pair would compute padding), gathered.
+// Bound: with boxes the MMAs, twelve per stage of 32 rows and pair (1536 cycles per SM, 0.98 us as measured without any
+// loads; 1.1 with them); gathered, the copies: 48 KB of parts per stage come in at 1.4 us whatever the number of stages
+// in flight, MMAs or not (5 TB/s over the chip: what the load/store path of an SM keeps outstanding).  us, 3xTF32 on
+// 128x128 tiles / gathered / boxes: 5x5 over 64 channels, d = 1601 from 65536 rows 1810 / 1127 / 896; 3x3 over 64,
+// d = 577 from 131072 rows 495 gathered, 391; d = 4608 from 8192 rows 1710 / 1016 / 876.  Measured alternatives:
+// splitting in the gather warps is bound by their instructions (650 per warp and stage, 2.3 us per stage, in bf16 as in
+// 3xTF32), and 32-bit MN-major operands are read at half the rate.
 // The input is processed in runs of whole images whose parts fit the scratch; each run adds to the partial tiles of
 // the one before.
 // Partial tiles, tickets and the finishing kernels are those of the other factor kernels.
+#include <cuda.h>
+
 #include <algorithm>
+#include <numeric>
 
 #include "common.cuh"
 #include "factor_finish.cuh"
@@ -35,6 +40,7 @@
 namespace sso {
 
 int factor_tc_run_reduce(const FactorParams& p, int tiles, cudaStream_t st);
+decltype(&cuTensorMapEncodeTiled) tensor_map_encoder();      // factor_tma.cu; null if the driver has none
 
 namespace f32 {
 
@@ -71,6 +77,12 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t&
   x -= __uint_as_float(mid << 16); y -= __uint_as_float(mid & 0xFFFF0000u);
   lo = pack(x, y);
 }
+
+// Stages as boxes of whole pixels (32 = bw * bh * bn), fetched by TMA: a view {c8, width, h, n, part} of the parts.
+struct alignas(64) Boxes {
+  CUtensorMap map;
+  int bw, bh, bn, across, down;      // a box; boxes per image in either direction
+};
 
 // First kernel of a factor: let the next one set itself up meanwhile (it waits for this one's end before it touches
 // memory), clear the status word and the tickets that it will use.
@@ -248,8 +260,11 @@ struct Gather {
   }
 };
 
-template <bool PAIR>
-__global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorParams p, const Parts parts) {
+template <bool PAIR, bool BOX>
+__global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorParams p, const Parts parts, const __grid_constant__ Boxes boxes) {
+  static_assert(PAIR || !BOX, "one CTA gathers");
+  // a box brings the three parts of 64 columns in one piece; the gather keeps the 128 columns of a part together
+  constexpr uint32_t BLK_STRIDE = BOX ? 3 * BLK : BLK, PART_STRIDE = BOX ? BLK : OPB;
   constexpr int NACC = PAIR ? 128 : 64;          // accumulator columns per accumulate warp
   constexpr int ACC_COLS = 2 * NACC;             // TMEM columns of one accumulator
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -270,11 +285,13 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
   const int nchunks = ceil_div(nstages, FLUSH);
   int* status = p.status;
   const int col_a = bI * (PAIR ? 256 : 128) + (int)rank * TILE, col_b = bJ * (PAIR ? 256 : 128) + (int)rank * TILE;
-  // 64-column blocks A0 A1 B0 B1 that hold columns of the matrix and are needed
+  // 64-column blocks A0 A1 B0 B1 that hold columns of the matrix and are needed; a box leaves the ones column of a
+  // k x k window out (it has a block to itself, written once below)
+  const int loaded_cols = BOX ? p.dcols : p.d;
   uint32_t blocks = 0;
 #pragma unroll
   for (int b = 0; b < 4; ++b)
-    if ((b < 2 ? col_a : col_b) + (b & 1) * 64 < p.d && !(share && b >= 2)) blocks |= 1u << b;
+    if ((b < 2 ? col_a : col_b) + (b & 1) * 64 < loaded_cols && !(share && b >= 2)) blocks |= 1u << b;
 
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t bar0 = smem_u32(bars);
@@ -284,7 +301,9 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
   auto accempty_bar = [&](int b) { return bar0 + 8u * (2 * STAGES + 2 + b); };
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full_bar(s), (PAIR ? 2 : 1) * LOAD_WARPS);       // a pair's gather warps all arrive at the leader
+      // a pair's gather warps all arrive at the leader; of boxes the leader's producer, which announces the bytes of both
+      // CTAs, and the peer's once it has issued its own
+      mbar_init(full_bar(s), BOX ? 2 : (PAIR ? 2 : 1) * LOAD_WARPS);
       mbar_init(empty_bar(s), 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -300,8 +319,11 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
       if (!((idle >> b) & 1u)) continue;
       for (uint32_t o = tid * 16u; o < 3 * STAGES * BLK; o += THREADS * 16u) {
         const uint32_t part = o / BLK;
-        const uint32_t at = smem0 + (part / 3) * SLOT_BYTES + (b >> 1) * SIDE + (part % 3) * OPB + (b & 1) * BLK + o % BLK;
-        asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(at), "r"(0u) : "memory");
+        const uint32_t at = smem0 + (part / 3) * SLOT_BYTES + (b >> 1) * SIDE + (part % 3) * PART_STRIDE + (b & 1) * BLK_STRIDE + o % BLK;
+        // the ones column, first of its block: hi is 1, in chunk 0 of every row (at its swizzled place)
+        const bool one = BOX && p.d > p.dcols && (b < 2 ? col_a : col_b) + (b & 1) * 64 == p.dcols && part % 3 == 0 &&
+                         ((o >> 4) & 7u) == ((o >> 7) & 7u);
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%2,%2};" ::"r"(at), "r"(one ? 0x3F80u : 0u), "r"(0u) : "memory");
       }
     }
   }
@@ -396,8 +418,8 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
         uint32_t on = first_of_chunk ? 0u : 1u;
         for (int ks = 0; ks < KS / 16; ++ks) {
           // 16 rows = two 1024-byte swizzle atoms; the next 64 columns start BLK further on
-          const uint64_t a_d = smem_desc_sw128(a0 + ks * 2048u, BLK, 1024u), b_d = smem_desc_sw128(b0 + ks * 2048u, BLK, 1024u);
-          constexpr uint64_t P = OPB >> 4;       // from one part to the next, in descriptor units
+          const uint64_t a_d = smem_desc_sw128(a0 + ks * 2048u, BLK_STRIDE, 1024u), b_d = smem_desc_sw128(b0 + ks * 2048u, BLK_STRIDE, 1024u);
+          constexpr uint64_t P = PART_STRIDE >> 4;       // from one part to the next, in descriptor units
           auto mma = [&](int pa, int pb) {
             if (PAIR) umma2<false>(d_tmem, a_d + pa * P, b_d + pb * P, idesc, on);
             else umma<false>(d_tmem, a_d + pa * P, b_d + pb * P, idesc, on);
@@ -421,6 +443,47 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
   } else {
     // ------------------------------------------------------------------ gather warps
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (BOX) {
+      if (warp == LOAD_WARP0 && lane == 0 && !g_inject_stall) {
+        int c0[4], x0[4], y0[4];
+        uint32_t pair_blocks = 0;      // blocks that both CTAs load
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const int j0 = (b < 2 ? col_a : col_b) + (b & 1) * 64, pos = j0 / p.c, ky = pos / p.kw;
+          c0[b] = j0 - pos * p.c;
+          x0[b] = (pos - ky * p.kw) * p.dil_w - p.pad_w;
+          y0[b] = ky * p.dil_h - p.pad_h;
+          const int first = j0 - (int)rank * TILE;
+          if (!(share && b >= 2)) pair_blocks += (first < loaded_cols ? 1u : 0u) + (first + TILE < loaded_cols ? 1u : 0u);
+        }
+        const uint64_t map = reinterpret_cast<uint64_t>(&boxes.map);
+        const uint32_t fulls = map_to_cta(full_bar(0), 0u);
+        const int first_box = (int)(r_begin / KS), per_image = boxes.across * boxes.down;
+        int n = first_box / per_image, iy = (first_box - n * per_image) / boxes.across;
+        int ix = first_box - n * per_image - iy * boxes.across;
+        for (int s = 0; s < nstages; ++s) {
+          const int slot = s % STAGES;
+          if (s >= STAGES && !mbar_wait(empty_bar(slot), ((s / STAGES) - 1) & 1, status, 64)) break;
+          const uint32_t fb = fulls + 8u * slot;
+          if (rank == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full_bar(slot)), "r"(pair_blocks * 3 * BLK) : "memory");
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            if (!((blocks >> b) & 1u)) continue;
+            const uint32_t dst = smem0 + slot * SLOT_BYTES + (b >> 1) * SIDE + (b & 1) * BLK_STRIDE;
+            asm volatile(
+                "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+                ::"r"(dst), "l"(map), "r"(c0[b]), "r"(ix * boxes.bw + x0[b]), "r"(iy * boxes.bh + y0[b]), "r"(n * boxes.bn), "r"(0), "r"(fb)
+                : "memory");
+          }
+          if (rank != 0) mbar_arrive_cluster(fb);
+          if (++ix == boxes.across) { ix = 0; if (++iy == boxes.down) { iy = 0; ++n; } }
+        }
+      }
+      __syncwarp();
+      asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
+    } else {
     const int w = warp - LOAD_WARP0;
     const int l8 = lane & 7, row = 4 * w + (lane >> 3);
     Gather g;
@@ -453,6 +516,7 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
     __syncwarp();
     asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");
     asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
+    }
   }
   tc_fence_before();
   if (PAIR) cluster_sync_all();          // neither CTA leaves while its peer's MMAs may still read its shared memory
@@ -493,9 +557,9 @@ static int choose_splits(int64_t rows, int units, int slots, int tiles, double s
   return (int)ceil_div64(stages, best_sps);
 }
 
-template <bool PAIR>
-static int launch(const FactorParams& p, const Parts& parts, int units, int splits, cudaStream_t st) {
-  SSO_ENSURE_SMEM(factor_f32_kernel<PAIR>, SMEM);
+template <bool PAIR, bool BOX>
+static int launch(const FactorParams& p, const Parts& parts, const Boxes& boxes, int units, int splits, cudaStream_t st) {
+  SSO_ENSURE_SMEM((factor_f32_kernel<PAIR, BOX>), SMEM);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(PAIR ? 2 * units : units, splits);
   cfg.blockDim = dim3(THREADS);
@@ -510,7 +574,7 @@ static int launch(const FactorParams& p, const Parts& parts, int units, int spli
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 2;
-  cudaLaunchKernelEx(&cfg, factor_f32_kernel<PAIR>, p, parts);
+  cudaLaunchKernelEx(&cfg, factor_f32_kernel<PAIR, BOX>, p, parts, boxes);
   SSO_LAUNCH_OK("factor_f32_kernel");
   return 0;
 }
@@ -729,6 +793,27 @@ static Shape shape_of(const FactorParams& p) {
   s.image_bytes = (int64_t)p.h * s.width * s.c8 * 6 * (p.weight ? 2 : 1);
   return s;
 }
+// Boxes of 32 whole pixels that cover the output exactly: no pixel is computed twice or for padding, and no row of a
+// stage is left to be cleared.  Every other geometry (strides, odd image sizes, per-sample weights, channel counts
+// below 64 columns of one kernel position) keeps the gather, which takes any.
+static bool choose_boxes(const FactorParams& p, const Shape& s, Boxes& b) {
+  if (p.weight || s.fold || p.stride_h != 1 || p.stride_w != 1 || (p.kh * p.kw > 1 && s.c8 % 64 != 0)) return false;
+  b.bw = std::gcd(p.wo, KS);
+  b.bh = std::gcd(p.ho, KS / b.bw);
+  b.bn = KS / (b.bw * b.bh);
+  b.across = p.wo / b.bw;
+  b.down = p.ho / b.bh;
+  return p.n % b.bn == 0 && tensor_map_encoder() != nullptr;
+}
+static bool encode_boxes(Boxes& b, const Parts& parts, const Shape& s, int h, int n) {
+  const cuuint64_t row = (cuuint64_t)s.c8 * 2;
+  const cuuint64_t dims[5] = {(cuuint64_t)s.c8, (cuuint64_t)s.width, (cuuint64_t)h, (cuuint64_t)n, 3};
+  const cuuint64_t strides[4] = {row, row * s.width, row * s.width * h, (cuuint64_t)parts.stride * 2};
+  const cuuint32_t box[5] = {64, (cuuint32_t)b.bw, (cuuint32_t)b.bh, (cuuint32_t)b.bn, 3}, step[5] = {1, 1, 1, 1, 1};
+  return tensor_map_encoder()(&b.map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16*>(parts.a), dims, strides, box, step,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 constexpr int64_t PARTS_TARGET = (int64_t)256 << 20;     // parts of one run of images
 constexpr int64_t PARTIAL_TARGET = (int64_t)148 * 2 * 65536;
 
@@ -790,8 +875,13 @@ int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, c
   const size_t hdr = factor_header_bytes(s.tiles);
   const int64_t room = (int64_t)(workspace_bytes - hdr - 512) - (int64_t)s.tiles * 65536;
   const int64_t per_run = std::max<int64_t>(1, std::min<int64_t>({(int64_t)p.n, f32::PARTS_TARGET / std::max<int64_t>(1, s.image_bytes), room / std::max<int64_t>(1, s.image_bytes)}));
-  const int runs = (int)ceil_div64(p.n, per_run);
-  const int n_run = (int)ceil_div64(p.n, runs);
+  // a pair's block is 256 wide: up to 128 columns one CTA's tile is all there is to compute
+  const bool pair = s.d > 128;
+  f32::Boxes boxes{};
+  bool box = pair && f32::choose_boxes(p, s, boxes) && per_run >= boxes.bn;
+  const int whole = box ? boxes.bn : 1;      // images per run are a multiple of a box's
+  const int runs = (int)ceil_div64(p.n, per_run / whole * whole);
+  const int n_run = (int)ceil_div64(ceil_div64(p.n, runs), whole) * whole;
   const int64_t parts_bytes = n_run * s.image_bytes;
   const int max_splits = (int)(((int64_t)(workspace_bytes - hdr - 512) - (parts_bytes + 255) / 256 * 256) / ((int64_t)s.tiles * 65536));
   char* base = reinterpret_cast<char*>(workspace);
@@ -803,11 +893,9 @@ int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, c
   parts.b = p.weight ? parts.a + 3 * parts.stride : parts.a;
   parts.c8 = s.c8;
   q.partial = reinterpret_cast<float*>(base + (hdr + 255) / 256 * 256 + (parts_bytes + 255) / 256 * 256);
-  // a pair's block is 256 wide: up to 128 columns one CTA's tile is all there is to compute
-  const bool pair = s.d > 128;
   const int64_t hw = (int64_t)p.ho * p.wo;
   int rps = 0;
-  q.splits = f32::choose_splits(n_run * hw, pair ? s.blocks : s.tiles, pair ? 74 : 148, s.tiles, pair ? 0.85 : 0.6, max_splits, rps);
+  q.splits = f32::choose_splits(n_run * hw, pair ? s.blocks : s.tiles, pair ? 74 : 148, s.tiles, box ? 0.65 : pair ? 0.85 : 0.6, max_splits, rps);
   q.rows_per_split = rps;
   const int kk = p.kh * p.kw;
   q.perm_c = kk > 1 ? s.c8 : 0;
@@ -842,7 +930,10 @@ int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, c
     q.rows = n * hw;
     q.accumulate = r > 0;
     q.tickets = fused && r == runs - 1 ? reinterpret_cast<int*>(base + 256) : nullptr;
-    const int rc = pair ? f32::launch<true>(q, parts, s.blocks, q.splits, st) : f32::launch<false>(q, parts, s.tiles, q.splits, st);
+    if (box && !f32::encode_boxes(boxes, parts, s, p.h, n)) return fail(-5, "cuTensorMapEncodeTiled failed for the parts of a factor");
+    const int rc = box    ? f32::launch<true, true>(q, parts, boxes, s.blocks, q.splits, st)
+                   : pair ? f32::launch<true, false>(q, parts, boxes, s.blocks, q.splits, st)
+                          : f32::launch<false, false>(q, parts, boxes, s.tiles, q.splits, st);
     if (rc) return rc;
   }
   if (fused) return 0;

@@ -85,7 +85,9 @@ F32_CONVS = [(5, 3, 20, 19, (7, 7), (2, 2), (3, 3), (1, 1), False), (3, 1, 9, 9,
              (4, 7, 12, 10, (3, 2), (1, 2), (1, 0), (2, 1), True), (6, 11, 9, 9, (3, 3), (1, 1), (1, 1), (1, 1), True),
              (3, 64, 8, 8, (3, 3), (1, 1), (1, 1), (1, 1), True), (2, 26, 13, 13, (5, 5), (1, 1), (2, 2), (1, 1), False),
              (40, 33, 6, 6, (1, 1), (2, 2), (0, 0), (1, 1), True), (2, 9, 10, 10, (9, 9), (1, 1), (4, 4), (1, 1), True),
-             (3, 21, 9, 8, (4, 4), (1, 1), (1, 1), (1, 1), False), (1, 40, 7, 7, (2, 2), (1, 1), (0, 0), (1, 1), True), (16, 130, 5, 7, (1, 1), (1, 1), (0, 0), (1, 1), True)]
+             (3, 21, 9, 8, (4, 4), (1, 1), (1, 1), (1, 1), False), (1, 40, 7, 7, (2, 2), (1, 1), (0, 0), (1, 1), True), (6, 128, 4, 4, (3, 3), (1, 1), (1, 1), (1, 1), True),
+             (16, 64, 2, 2, (3, 3), (1, 1), (1, 1), (1, 1), False), (2, 64, 16, 33, (3, 2), (1, 1), (1, 0), (1, 1), True),
+             (2, 64, 12, 24, (5, 5), (1, 1), (4, 4), (2, 2), True), (4, 200, 32, 32, (1, 1), (1, 1), (0, 0), (1, 1), True), (16, 130, 5, 7, (1, 1), (1, 1), (0, 0), (1, 1), True)]
 
 
 @pytest.mark.parametrize('cfg', F32_CONVS)
@@ -106,7 +108,7 @@ def test_factor_f32_conv(nat, cfg, channels_last):
 
 
 @pytest.mark.parametrize('rows,cols,bias', [(1, 1, False), (31, 5, True), (129, 63, True), (700, 64, False), (5000, 64, True), (33000, 128, False),
-                                            (20001, 97, True), (40000, 13, False), (257, 300, True), (1500, 1021, True), (33, 4100, False)])
+                                            (20001, 97, True), (40000, 13, False), (257, 300, True), (256, 300, True), (1024, 1021, False), (1500, 1021, True), (33, 4100, False)])
 @pytest.mark.parametrize('layout', ['rows', 'strided', 'columns'])
 def test_factor_f32_rows(nat, rows, cols, bias, layout):
     x = torch.randn(rows, cols, device='cuda') + 0.25
@@ -229,3 +231,31 @@ def test_bn_batch(nat, weighted):
             assert nat.collect_norm(t, (st, splits), sg, sx, w, 2, 0.5, 2.0, wo, bo)
     for got, ref in want:
         assert rel(got, ref) < 1e-5
+
+
+# ------------------------------------------------------------------------------------------- sampling
+@pytest.mark.parametrize('bias', [False, True])
+@pytest.mark.parametrize('shapes', [[(1, 1)], [(128, 128)], [(129, 127), (130, 1)], [(2, 257), (641, 130), (388, 4)]])
+def test_sample_plan_along_k(nat, shapes, bias):
+    """[w | b] += s U_G E U_A with rows of the factors padded, and noise rows that do or do not start on 16 bytes."""
+    shapes = [(a + int(bias), g) for a, g in shapes]
+
+    def factor(d):
+        ld = (d + 3) // 4 * 4
+        u = torch.zeros(d, ld, device='cuda')
+        u[:, :d] = torch.randn(d, d, device='cuda').triu()
+        return u[:, :d]
+    UA, UG = [factor(a) for a, _ in shapes], [factor(g) for _, g in shapes]
+    E = [torch.randn(g, a, device='cuda') for a, g in shapes]
+    w = [torch.randn(g, a - int(bias), device='cuda') for a, g in shapes]
+    b = [torch.randn(g, device='cuda') if bias else None for _, g in shapes]
+    tmp = [torch.empty(a * g, device='cuda') for a, g in shapes]
+    want = []
+    for i in range(len(shapes)):
+        mean = w[i] if b[i] is None else torch.cat([w[i], b[i][:, None]], 1)
+        want.append(mean.double() + 0.25 * UG[i].double() @ E[i].double() @ UA[i].double())
+    plan = nat.sample_plan([a for a, _ in shapes], [g for _, g in shapes], UA, UG, E, w, b, tmp, torch.device('cuda'))
+    nat.sample_plan_run(plan, 0.25)
+    for i in range(len(shapes)):
+        got = w[i] if b[i] is None else torch.cat([w[i], b[i][:, None]], 1)
+        assert rel(got, want[i]) < 2e-6

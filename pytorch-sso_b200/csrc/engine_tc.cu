@@ -474,18 +474,23 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_kc_kernel(const sso_tile
       const int rs = s % RAW_SLOTS, ls = s % LO_SLOTS;
       if (s >= LO_SLOTS && !mbar_wait(lofree_bar(ls), ((s / LO_SLOTS) - 1) & 1, status, 25)) break;
       const uint32_t hi = smem0 + rs * PART + so0, lo = lo0 + ls * PART + so0;
+      // all loads before the first store: one chunk at a time, each would wait for the one before
+      float4 v[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const uint32_t off = (uint32_t)(j & 3) * 4096u + (uint32_t)(j >> 2) * OPB;
-        float4 v;
-        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(hi + off) : "memory");
+        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w) : "r"(hi + off));
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t off = (uint32_t)(j & 3) * 4096u + (uint32_t)(j >> 2) * OPB;
         // hi is rounded to nearest and written back in place.  Leaving the raw word as hi (the MMA
         // reads only its top 19 bits) saves this store and 10-15 % of the kernel, but a truncated hi
         // doubles |lo| and makes the dropped lo*lo term one-signed: on ill-conditioned factors the
         // preconditioned gradient then misses the 1e-4 bound (3.7e-4 measured against 2e-4).
-        const uint32_t h0 = rna_tf32(v.x), h1 = rna_tf32(v.y), h2 = rna_tf32(v.z), h3 = rna_tf32(v.w);
-        const uint32_t l0 = __float_as_uint(v.x - __uint_as_float(h0)), l1 = __float_as_uint(v.y - __uint_as_float(h1));
-        const uint32_t l2 = __float_as_uint(v.z - __uint_as_float(h2)), l3 = __float_as_uint(v.w - __uint_as_float(h3));
+        const uint32_t h0 = rna_tf32(v[j].x), h1 = rna_tf32(v[j].y), h2 = rna_tf32(v[j].z), h3 = rna_tf32(v[j].w);
+        const uint32_t l0 = __float_as_uint(v[j].x - __uint_as_float(h0)), l1 = __float_as_uint(v[j].y - __uint_as_float(h1));
+        const uint32_t l2 = __float_as_uint(v[j].z - __uint_as_float(h2)), l3 = __float_as_uint(v[j].w - __uint_as_float(h3));
         asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(hi + off), "r"(h0), "r"(h1), "r"(h2), "r"(h3) : "memory");
         asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(lo + off), "r"(l0), "r"(l1), "r"(l2), "r"(l3) : "memory");
       }
@@ -616,18 +621,23 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
       if (!mbar_wait(rawfull_bar(rs), (s / RAW_SLOTS) & 1, status, 46)) break;
       if (s >= LO_SLOTS && !mbar_wait(lofree_bar(ls), ((s / LO_SLOTS) - 1) & 1, status, 45)) break;
       const uint32_t hi = smem0 + rs * PART + so0, lo = lo0 + ls * PART + so0;
+      // all loads before the first store: one chunk at a time, each would wait for the one before
+      float4 v[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const uint32_t off = (uint32_t)(j & 3) * 4096u + (uint32_t)(j >> 2) * OPB;
-        float4 v;
-        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(hi + off) : "memory");
+        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w) : "r"(hi + off));
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t off = (uint32_t)(j & 3) * 4096u + (uint32_t)(j >> 2) * OPB;
         // hi is rounded to nearest and written back in place.  Leaving the raw word as hi (the MMA
         // reads only its top 19 bits) saves this store and 10-15 % of the kernel, but a truncated hi
         // doubles |lo| and makes the dropped lo*lo term one-signed: on ill-conditioned factors the
         // preconditioned gradient then misses the 1e-4 bound (3.7e-4 measured against 2e-4).
-        const uint32_t h0 = rna_tf32(v.x), h1 = rna_tf32(v.y), h2 = rna_tf32(v.z), h3 = rna_tf32(v.w);
-        const uint32_t l0 = __float_as_uint(v.x - __uint_as_float(h0)), l1 = __float_as_uint(v.y - __uint_as_float(h1));
-        const uint32_t l2 = __float_as_uint(v.z - __uint_as_float(h2)), l3 = __float_as_uint(v.w - __uint_as_float(h3));
+        const uint32_t h0 = rna_tf32(v[j].x), h1 = rna_tf32(v[j].y), h2 = rna_tf32(v[j].z), h3 = rna_tf32(v[j].w);
+        const uint32_t l0 = __float_as_uint(v[j].x - __uint_as_float(h0)), l1 = __float_as_uint(v[j].y - __uint_as_float(h1));
+        const uint32_t l2 = __float_as_uint(v[j].z - __uint_as_float(h2)), l3 = __float_as_uint(v[j].w - __uint_as_float(h3));
         asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(hi + off), "r"(h0), "r"(h1), "r"(h2), "r"(h3) : "memory");
         asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(lo + off), "r"(l0), "r"(l1), "r"(l2), "r"(l3) : "memory");
       }

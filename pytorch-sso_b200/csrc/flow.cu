@@ -286,22 +286,24 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         if (ok && stage >= LO) ok = mbar_wait(lofree(ls), ((stage / LO) - 1) & 1, status, 93);
         if (!ok) break;
         const uint32_t hi = smem0 + rs * PART + so0, lo = lo0 + ls * PART + so0;
-        auto split = [&](uint32_t off) {
-          float4 v;
-          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(hi + off) : "memory");
-          // hi rounded to nearest, written back in place (see tile_task_tma_kernel)
-          const uint32_t h0 = rna_tf32(v.x), h1 = rna_tf32(v.y), h2 = rna_tf32(v.z), h3 = rna_tf32(v.w);
-          const uint32_t l0 = __float_as_uint(v.x - __uint_as_float(h0)), l1 = __float_as_uint(v.y - __uint_as_float(h1));
-          const uint32_t l2 = __float_as_uint(v.z - __uint_as_float(h2)), l3 = __float_as_uint(v.w - __uint_as_float(h3));
-          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(hi + off), "r"(h0), "r"(h1), "r"(h2), "r"(h3) : "memory");
-          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(lo + off), "r"(l0), "r"(l1), "r"(l2), "r"(l3) : "memory");
+        // all loads of a side before the first store: one chunk at a time, each would wait for the one before
+        auto split = [&](uint32_t side) {
+          float4 v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j)            // sixteen rows further = 2048 bytes
+            asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w) : "r"(hi + side + j * 2048u));
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            // hi rounded to nearest, written back in place (see tile_task_tma_kernel)
+            const uint32_t h0 = rna_tf32(v[j].x), h1 = rna_tf32(v[j].y), h2 = rna_tf32(v[j].z), h3 = rna_tf32(v[j].w);
+            const uint32_t l0 = __float_as_uint(v[j].x - __uint_as_float(h0)), l1 = __float_as_uint(v[j].y - __uint_as_float(h1));
+            const uint32_t l2 = __float_as_uint(v[j].z - __uint_as_float(h2)), l3 = __float_as_uint(v[j].w - __uint_as_float(h3));
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(hi + side + j * 2048u), "r"(h0), "r"(h1), "r"(h2), "r"(h3) : "memory");
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(lo + side + j * 2048u), "r"(l0), "r"(l1), "r"(l2), "r"(l3) : "memory");
+          }
         };
-#pragma unroll
-        for (int j = 0; j < 8; ++j) split(j * 2048u);              // sixteen rows further = 2048 bytes
-        if (!share) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) split(OPB + j * 2048u);
-        }
+        split(0);
+        if (!share) split(OPB);
         fence_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(full(ls));

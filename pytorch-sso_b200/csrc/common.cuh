@@ -71,6 +71,20 @@ __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(
 __host__ __device__ __forceinline__ int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Two fp32 values -> three bf16 parts each whose sum is exact, packed (first value in the low half).
+__device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  auto pack = [](float a, float b) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
+  };
+  hi = pack(x, y);
+  x -= __uint_as_float(hi << 16); y -= __uint_as_float(hi & 0xFFFF0000u);
+  mid = pack(x, y);
+  x -= __uint_as_float(mid << 16); y -= __uint_as_float(mid & 0xFFFF0000u);
+  lo = pack(x, y);
+}
+
 // Lower-triangle tile index t -> (bi, bj) with bi >= bj, t = bi*(bi+1)/2 + bj.
 __device__ __forceinline__ void tri_decode(int t, int& bi, int& bj) {
   int r = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);

@@ -1,26 +1,30 @@
 // Diagonal block of a 128-column Cholesky panel, done by eight warps: L = chol(D) and L^-1 for a
-// (<=128)x(<=128) SPD block D, all in fp32 FMA arithmetic, in shared memory (pitch 132: the 16-byte loads of
+// (<=128)x(<=128) SPD block D, in shared memory (pitch 132: the 16-byte loads of
 // eight consecutive rows meet no bank conflict).
 //
 // The block is eight panels of 16 columns.  What bounds it is the chain of 128 pivots, so warp 0 does nothing but
 // that chain: of panel k it takes the 16x16 diagonal block, subtracts the panel before, eliminates, and next solves
-// the one 16x16 block that its next diagonal block needs.  The other warps follow half a step behind: trailing update
-// by panel k - 1 and, in the idle half of the matrix, the sums G(k, c) = sum_j L(k, j) Inv(j, c) of row k of the
-// inverse (20 to 28 block products a step, spread over seven warps by a table).  Two barriers a step:
+// the one 16x16 block that its next diagonal block needs.  The other warps follow half a step behind with two things
+// that are one and the same update: the trailing matrix (lower blocks), and the rows of an identity that go through
+// the elimination with it and become L^-T (kept in the idle upper blocks).  Two barriers a step:
 //   X : panel k's block and its inverse are there, panel k - 1 has been subtracted everywhere
-//       then, one 16x16 product per warp: L(i, k) = A(i, k) Inv_kk^T below, Inv(k, c) = -Inv_kk G(k, c) to the left
+//       then, one 16x16 product per warp: row block b of the panel, X(b, k) Inv_kk^T
 //   Y : those are there (warp 0 only announces its own and goes on)
+// The products are mma.sync on three bf16 parts of the fp32 operands, six products each as in factor_f32.cu (fp32
+// grade); the parts of a panel are made once, when its row blocks are finished.  In fp32 FMA, with 2x4 outputs per
+// lane, they were bound by the 512 bytes that shared memory returns per 16-byte load and warp, and took the
+// elimination's shuffles along (17 us for 128 rows).
 // The elimination: lane l of warp 0 holds row l of the block, lane l + 16 row l of an identity that goes through the
 // same steps, which leaves the inverse's column l in it for no further instruction; per pivot one round of shuffles
 // (the raw column, and the next diagonal element so that the next pivot's rsqrt starts early).
 // Rows and columns past the block's size behave as an identity block.  A pivot that is not a positive normal number
 // (non-positive, denormal or NaN) is recorded once per matrix (LAPACK numbering) and replaced by 1, like the 64-wide
 // kernel does for non-positive ones.
-// Measured: 17 us for 128 rows (clocks: 1600 to 3100 per elimination, 750 per round of products, which are bound by
-// the 512 bytes per 16-byte load and warp that shared memory returns); a chain of four barriers per panel with all
-// warps in step and the inverse by three levels of doubling afterwards took 23.  Inside the dataflow kernel, with the
-// inverse of the block announced before the other results are written: 1000 402 -> 307 us, 577+64 264 -> 203, the six
-// factors of 784-1000-1000-10 433 -> 339, 4608+512 2208 -> 1715.
+// Measured: 14.4 us for 128 rows (clocks: 1900 to 2900 per elimination with the subtraction before it, 720 for the
+// round of products); a chain of four barriers per panel with all warps in step and the inverse by three levels of
+// doubling afterwards took 23.  Inside the dataflow kernel, with the inverse of the block announced before the other
+// results are written: 1000 402 -> 284 us, 577+64 264 -> 191, the six factors of 784-1000-1000-10 433 -> 315,
+// 4608+512 2208 -> 1544.
 #pragma once
 #include "common.cuh"
 
@@ -31,7 +35,7 @@ constexpr int PN = 128;        // rows / columns handled by one CTA
 constexpr int PP = 132;        // pitch of the shared-memory matrices (floats)
 constexpr int PK = 16;         // panel width inside the block
 constexpr int THREADS = 256;
-constexpr size_t SMEM_BYTES = (size_t)(2 * PN * PP) * sizeof(float);
+constexpr size_t SMEM_BYTES = (size_t)(2 * PN * PP) * sizeof(float) + 3 * PN * 48;      // two matrices, parts of a panel
 
 // MUFU.RSQ alone (2 ulp); the argument is a positive normal number wherever this is called
 __device__ __forceinline__ float rsqrt_approx(float x) {
@@ -49,121 +53,101 @@ __device__ __forceinline__ void sync_x() { asm volatile("bar.sync 1, %0;" ::"n"(
 __device__ __forceinline__ void sync_y() { asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory"); }
 __device__ __forceinline__ void arrive_y() { asm volatile("bar.arrive 2, %0;" ::"n"(THREADS) : "memory"); }
 
-// A warp's 16x16x16 product: lane (rg, cg) holds rows rg, rg + 8; columns cg + 4 v of A B^T, 4 cg + v of A B.
-struct Acc {
-  float v[2][4];
-  __device__ __forceinline__ void zero() {
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) v[i][j] = 0.f;
-  }
-  __device__ __forceinline__ void add(int i, float4 a, const float4 (&b)[4]) {      // along q
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[i][j] = fmaf(a.x, b[j].x, v[i][j]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[i][j] = fmaf(a.y, b[j].y, v[i][j]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[i][j] = fmaf(a.z, b[j].z, v[i][j]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[i][j] = fmaf(a.w, b[j].w, v[i][j]);
-  }
-  __device__ __forceinline__ void nt(const float* __restrict__ A, const float* __restrict__ B, int rg, int cg) {
-#pragma unroll
-    for (int q = 0; q < PK; q += 4) {
-      const float4 a0 = ld4(A + rg * PP + q), a1 = ld4(A + (rg + 8) * PP + q);
-      float4 b[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = ld4(B + (cg + 4 * j) * PP + q);
-      add(0, a0, b);
-      add(1, a1, b);
-    }
-  }
-  __device__ __forceinline__ void nn(const float* __restrict__ A, const float* __restrict__ B, int rg, int cg) {
-#pragma unroll
-    for (int q = 0; q < PK; q += 4) {
-      const float4 a[2] = {ld4(A + rg * PP + q), ld4(A + (rg + 8) * PP + q)};
-      float4 b[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = ld4(B + (q + j) * PP + 4 * cg);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const float x = j == 0 ? a[i].x : j == 1 ? a[i].y : j == 2 ? a[i].z : a[i].w;
-          v[i][0] = fmaf(x, b[j].x, v[i][0]);
-          v[i][1] = fmaf(x, b[j].y, v[i][1]);
-          v[i][2] = fmaf(x, b[j].z, v[i][2]);
-          v[i][3] = fmaf(x, b[j].w, v[i][3]);
-        }
-    }
-  }
-};
+// The bf16 parts of the current panel: [part][row 0..127][16 columns], rows 48 bytes apart (eight consecutive ones on
+// different banks).  Row block b > k holds L(b, k), b <= k column block k of L^-T.
+constexpr uint32_t PL_ROW = 48, PL_PART = PN * PL_ROW;
 
-// What warps 1 to 7 do while warp 0 eliminates panel k >= 1: trailing blocks (i, j) and sums G(k, c), longest first to
-// the warp with the least so far.
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t saddr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr));
+}
+__device__ __forceinline__ void mma16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// A warp's 16x16x16 product A B^T of operands in three parts (six products; what is dropped is below 2^-24): lane
+// (g, t) gets rows g, g + 8, columns 8 h + 2 t, + 1 of half h.  b[..][2 h], b[..][2 h + 1]: half h of B's rows.
+__device__ __forceinline__ void product(float (&out)[2][4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4]) {
+  float small[2][4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[h][i] = small[h][i] = 0.f;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) { mma16(small[h], a[2], b[0][2 * h], b[0][2 * h + 1]); mma16(out[h], a[1], b[0][2 * h], b[0][2 * h + 1]); }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) { mma16(small[h], a[0], b[2][2 * h], b[2][2 * h + 1]); mma16(out[h], a[0], b[1][2 * h], b[1][2 * h + 1]); }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) { mma16(small[h], a[1], b[1][2 * h], b[1][2 * h + 1]); mma16(out[h], a[0], b[0][2 * h], b[0][2 * h + 1]); }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[h][i] += small[h][i];
+}
+// C(i, j) -= P_i P_j^T (C = -P_i P_j^T if `fresh`), C a 16x16 block of S.
+__device__ __forceinline__ void subtract(float* __restrict__ C, uint32_t planes, int i, int j, bool fresh, int lane) {
+  uint32_t a[3][4], b[3][4];
+  const uint32_t ra = planes + (16 * i + (lane & 15)) * PL_ROW + (lane >> 4) * 16;
+  const uint32_t rb = planes + (16 * j + (lane & 7) + (lane >> 4) * 8) * PL_ROW + ((lane >> 3) & 1) * 16;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) { ldmatrix4(a[q], ra + q * PL_PART); ldmatrix4(b[q], rb + q * PL_PART); }
+  float2* c = reinterpret_cast<float2*>(C + (lane >> 2) * PP + 2 * (lane & 3));
+  float2 v[2][2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) v[h][r] = fresh ? make_float2(0.f, 0.f) : c[(8 * r * PP + 8 * h) / 2];
+  float o[2][4];
+  product(o, a, b);
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) c[(8 * r * PP + 8 * h) / 2] = make_float2(v[h][r].x - o[h][2 * r], v[h][r].y - o[h][2 * r + 1]);
+}
+// Three parts of the values at a lane's places (rows g, g + 8; columns 2 t, + 1 and 2 t + 8, + 9) of row block b.
+__device__ __forceinline__ void put_parts(uint32_t planes, int b, const float (&o)[2][4], int lane) {
+  const uint32_t at = planes + (16 * b + (lane >> 2)) * PL_ROW + 4 * (lane & 3);
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      uint32_t q[3];
+      split2(o[h][2 * r], o[h][2 * r + 1], q[0], q[1], q[2]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + i * PL_PART + 8 * r * PL_ROW + 16 * h), "r"(q[i]) : "memory");
+    }
+}
+
+// What warps 1 to 7 do while warp 0 eliminates panel k >= 1, one after the other: the blocks (i, j), j >= k, that panel
+// k - 1 reaches - of the trailing matrix (i >= j, all but (k, k)) and of L^-T (i < k) - with those of column k first.
 struct Schedule {
-  unsigned char task[8][7][8];      // 0xFF: none; 0x80 | c: G(k, c); else i << 3 | j
+  unsigned char count[8], task[8][36];      // i << 3 | j
 };
 constexpr Schedule make_schedule() {
   Schedule s{};
-  for (int k = 0; k < 8; ++k) {
-    int load[7] = {}, count[7] = {};
-    for (int w = 0; w < 7; ++w)
-      for (int t = 0; t < 8; ++t) s.task[k][w][t] = 0xFF;
-    if (k == 0) continue;
-    auto give = [&](int code, int cost) {
-      int best = -1;
-      for (int w = 0; w < 7; ++w)
-        if (count[w] < 8 && (best < 0 || load[w] < load[best])) best = w;
-      s.task[k][best][count[best]++] = (unsigned char)code;
-      load[best] += cost;
-    };
-    for (int c = 0; c < k; ++c)
-      if (k - c > 1) give(0x80 | c, 8 * (k - c) + 2);
-    for (int i = k; i < 8; ++i)
-      for (int j = k; j <= i; ++j)
-        if (i != k) give(i << 3 | j, 10);
-    give(0x80 | (k - 1), 10);
-  }
+  for (int k = 1; k < 8; ++k)
+    for (int j = k; j < 8; ++j)
+      for (int i = 0; i < 8; ++i)
+        if ((i < k || i >= j) && !(i == k && j == k)) s.task[k][s.count[k]++] = (unsigned char)(i << 3 | j);
   return s;
 }
 static __constant__ Schedule c_schedule = make_schedule();
 
 // The elimination of panel k's diagonal block by one warp, after the subtraction of panel k - 1.
-__device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restrict__ V, int k, int n, int* __restrict__ info, int row0, int lane) {
+__device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restrict__ V, uint32_t planes, int k, int n, int* __restrict__ info, int row0, int lane) {
   const int l = lane & 15, h = lane >> 4, c0 = PK * k;
   float* D = S + c0 * PP + c0;
-  // row l of the block, columns 8 h ..: both halves of the warp subtract, the lower one collects
-  float d[8];
-  {
-    const float4 u = ld4(D + l * PP + 8 * h), w = ld4(D + l * PP + 8 * h + 4);
-    d[0] = u.x; d[1] = u.y; d[2] = u.z; d[3] = u.w; d[4] = w.x; d[5] = w.y; d[6] = w.z; d[7] = w.w;
-  }
   if (k > 0) {
-    const float* P = D - PK;
-#pragma unroll
-    for (int q = 0; q < PK; q += 4) {
-      const float4 a = ld4(P + l * PP + q);
-      float4 b[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) b[c] = ld4(P + (8 * h + c) * PP + q);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) d[c] = fmaf(-a.x, b[c].x, d[c]);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) d[c] = fmaf(-a.y, b[c].y, d[c]);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) d[c] = fmaf(-a.z, b[c].z, d[c]);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) d[c] = fmaf(-a.w, b[c].w, d[c]);
-    }
+    subtract(D, planes, k, k, false, lane);
+    __syncwarp();
   }
   float v[PK];
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    const float up = __shfl_down_sync(0xffffffffu, d[c], 16);
-    v[c] = h ? (c == l ? 1.f : 0.f) : (c <= l ? d[c] : 0.f);
-    v[c + 8] = h ? (c + 8 == l ? 1.f : 0.f) : (c + 8 <= l ? up : 0.f);
+  for (int q = 0; q < PK; q += 4) {
+    const float4 u = ld4(D + l * PP + q);
+    const float d[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[q + i] = h ? (q + i == l ? 1.f : 0.f) : (q + i <= l ? d[i] : 0.f);
   }
   float pv = __shfl_sync(0xffffffffu, v[0], 0);
   int first_bad = -1;
@@ -203,12 +187,13 @@ __device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restri
 // row0 + pivot + 1 of the first bad pivot.
 __device__ __forceinline__ void factor_block(float* __restrict__ S, float* __restrict__ V, int n, int* __restrict__ info, int row0, int tid) {
   const int lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  const int rg = lane >> 2, cg = lane & 3;
+  const int g = lane >> 2, t = lane & 3;
   const int np = (n + PK - 1) / PK;     // panels that hold columns of the matrix
+  const uint32_t planes = (uint32_t)__cvta_generic_to_shared(V + PN * PP);
   auto at = [](float* m, int i, int j) { return m + (PK * i) * PP + PK * j; };
   for (int k = 0; k < np; ++k) {
     if (warp == 0) {
-      eliminate(S, V, k, n, info, row0, lane);
+      eliminate(S, V, planes, k, n, info, row0, lane);
     } else if (k == 0) {
       // the inverse's upper half, and its identity past the matrix
       for (int e = tid - 32; e < PN * PN / 4; e += THREADS - 32) {
@@ -216,55 +201,57 @@ __device__ __forceinline__ void factor_block(float* __restrict__ S, float* __res
         if (c / PK > r / PK || r >= PK * np) st4(V + r * PP + c, c == r ? 1.f : 0.f, c + 1 == r ? 1.f : 0.f, c + 2 == r ? 1.f : 0.f, c + 3 == r ? 1.f : 0.f);
       }
     } else {
+      const int count = c_schedule.count[k];
 #pragma unroll 1
-      for (int slot = 0; slot < 8; ++slot) {
-        const int code = c_schedule.task[k][warp - 1][slot];
-        if (code == 0xFF) break;
-        Acc acc;
-        acc.zero();
-        if (code & 0x80) {
-          const int c = code & 7;
-#pragma unroll 1
-          for (int j = c; j < k; ++j) acc.nn(at(S, k, j), at(V, j, c), rg, cg);
-          float* G = at(S, c, k);
-#pragma unroll
-          for (int i = 0; i < 2; ++i) st4(G + (rg + 8 * i) * PP + 4 * cg, acc.v[i][0], acc.v[i][1], acc.v[i][2], acc.v[i][3]);
-        } else {
-          const int i0 = code >> 3, j0 = code & 7;
-          if (i0 >= np) continue;
-          acc.nt(at(S, i0, k - 1), at(S, j0, k - 1), rg, cg);
-          float* C = at(S, i0, j0) + rg * PP + cg;
-#pragma unroll
-          for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) C[8 * i * PP + 4 * j] -= acc.v[i][j];
-        }
+      for (int s = warp - 1; s < count; s += THREADS / 32 - 1) {
+        const int code = c_schedule.task[k][s], i = code >> 3, j = code & 7;
+        if (i < np && j < np) subtract(at(S, i, j), planes, i, j, i == k - 1, lane);
       }
     }
     sync_x();
-    // warp 0: the block below the diagonal one; the others: k blocks of the inverse's row, then the blocks further below
-    const int m = warp - 1;
-    const bool left = warp != 0 && m < k;
-    const int i = warp == 0 ? k + 1 : k + 2 + (m - k);
-    Acc acc;
-    acc.zero();
-    if (left) {
-      acc.nn(at(V, k, k), at(S, m, k), rg, cg);
-      float* O = at(V, k, m);
+    // row block b of the panel: warp 0 the one below the diagonal block, the others the rest
+    const int b = warp == 0 ? k + 1 : warp - 1 <= k ? warp - 1 : warp;
+    const bool more = k + 1 < np;       // a panel follows that needs this one's parts
+    if (b == k) {
+      if (more) {                       // L^-T's own block: the transposed inverse of the diagonal block
+        const float* I = at(V, k, k);
+        float o[2][4];
 #pragma unroll
-      for (int r = 0; r < 2; ++r) st4(O + (rg + 8 * r) * PP + 4 * cg, -acc.v[r][0], -acc.v[r][1], -acc.v[r][2], -acc.v[r][3]);
-    } else if (i < np) {
-      acc.nt(at(S, i, k), at(V, k, k), rg, cg);
-      __syncwarp();
-      float* O = at(S, i, k) + rg * PP + cg;
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int r = 0; r < 2; ++r)
+          for (int i = 0; i < 4; ++i) o[h][i] = I[(8 * h + 2 * t + (i & 1)) * PP + g + 8 * (i >> 1)];
+        put_parts(planes, k, o, lane);
+      }
+    } else if (b < np) {                // X Inv_kk^T, X = S(b, k): below the diagonal a block of L, above one of L^-T
+      float2* X = reinterpret_cast<float2*>(at(S, b, k) + g * PP + 2 * t);
+      const float* I = at(V, k, k) + g * PP + 2 * t;
+      uint32_t xa[3][4], xb[3][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) O[8 * r * PP + 4 * j] = acc.v[r][j];
+      for (int i = 0; i < 4; ++i) {     // operand registers: row + 8 (i & 1), column + 8 (i >> 1); of B the other way round
+        const float2 x = X[(8 * (i & 1) * PP + 8 * (i >> 1)) / 2];
+        split2(x.x, x.y, xa[0][i], xa[1][i], xa[2][i]);
+        const float2 y = *reinterpret_cast<const float2*>(I + 8 * (i >> 1) * PP + 8 * (i & 1));
+        split2(y.x, y.y, xb[0][i], xb[1][i], xb[2][i]);
+      }
+      float o[2][4];
+      product(o, xa, xb);
+      if (b > k) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) X[(8 * r * PP + 8 * h) / 2] = make_float2(o[h][2 * r], o[h][2 * r + 1]);
+      } else {
+        float* O = at(V, k, b) + 2 * t * PP + g;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) O[(8 * h + (i & 1)) * PP + 8 * (i >> 1)] = o[h][i];
+      }
+      if (more) put_parts(planes, b, o, lane);
     }
     if (warp == 0) {
       __syncwarp();
-      if (k + 1 < np) arrive_y();
+      if (more) arrive_y();
       else sync_y();
     } else {
       sync_y();

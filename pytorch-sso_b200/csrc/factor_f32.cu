@@ -64,20 +64,6 @@ struct Parts {
   int c8;                      // channels per pixel, a multiple of eight
 };
 
-// two fp32 values -> their parts, packed (first value in the low half)
-__device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  auto pack = [](float a, float b) {
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
-    return r;
-  };
-  hi = pack(x, y);
-  x -= __uint_as_float(hi << 16); y -= __uint_as_float(hi & 0xFFFF0000u);
-  mid = pack(x, y);
-  x -= __uint_as_float(mid << 16); y -= __uint_as_float(mid & 0xFFFF0000u);
-  lo = pack(x, y);
-}
-
 // Stages as boxes of whole pixels (32 = bw * bh * bn), fetched by TMA: a view {c8, width, h, n, part} of the parts.
 struct alignas(64) Boxes {
   CUtensorMap map;

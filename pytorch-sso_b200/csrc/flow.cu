@@ -4,9 +4,10 @@
 // start (engine.cu simulates the schedule); one CTA per SM takes the next task from a counter, so a task only ever
 // waits for tasks that running CTAs have taken before it.  A tile is announced by a flag in global memory, and a task
 // waits for its operands block by block along K: all but the last 128 columns of a panel update run before the
-// previous panel is done.  The chain from one panel to the next is then one diagonal block (its inverse is
-// announced before its other results are written), one multiplication by that inverse and the last 128 columns of one update, without a kernel boundary in it; as phases of launches every one
-// of these was a kernel of at least 11 us (4608: 36 panels of three launches, 20 more for the inverse).
+// previous panel is done.  The chain from one panel to the next is then one diagonal block (its inverse is announced
+// before its other results are written), one multiplication by that inverse and the last 128 columns of one update,
+// without a kernel boundary in it; as phases of launches every one of these was a kernel of at least 11 us (4608: 36
+// panels of three launches, 20 more for the inverse).
 //
 // Inside a CTA (16 warps): 0-7 accumulate, store and factor diagonal blocks; 8 issues MMAs; 9 takes tasks, waits for flags
 // and issues TMA loads; 12-15 split the landed fp32 stages into tf32 hi (in place) and lo.  Products are 3xTF32
@@ -16,9 +17,9 @@
 // warps write it into the raw slots of four more stages.
 //
 // Bound: for one large matrix the chain of diagonal blocks, for many the shared-memory traffic of the 3xTF32 stages
-// (as tile_task_tma_kernel).  Against one launch per phase (us): 577+64 508 -> 203, 1000 637 -> 307, six factors of an
-// 784-1000-1000-10 network 1196 -> 339, 4608+512 3363 -> 1715, the 106 factors of ResNet-50 8970 -> 4350, those of VGG-16
-// with sampling factors 19416 -> 8610.
+// (as tile_task_tma_kernel).  Against one launch per phase (us): 577+64 508 -> 191, 1000 637 -> 284, six factors of a
+// 784-1000-1000-10 network 1196 -> 315, 4608+512 3363 -> 1544, the 106 factors of ResNet-50 8970 -> 3710, those of VGG-16
+// with sampling factors 19416 -> 7480.
 // Every wait is bounded; a CTA whose wait gives up sets the status word and writes NaN for this and all further tasks.
 #include "common.cuh"
 #include "diag_panel.cuh"

@@ -361,6 +361,8 @@ typedef struct {
  * dev_mem (device, sso_kron_plan_dev_bytes bytes) receives the tables; host_only != 0 builds
  * the plan without touching the device (for inspecting the task program on a CPU).
  * Returns a plan handle > 0, or a negative error. */
+/* whether plans use the caller's `work` matrices (the dataflow kernel does not: `work` may be null) */
+int sso_kron_plan_uses_work(void);
 size_t sso_kron_plan_dev_bytes(int n_mats, const int64_t* dims, int with_std);
 int64_t sso_kron_plan_create(int n_mats, const int64_t* dims, float* const* src, float* const* dst,
                              float* const* work, float* const* std_out /* nullable */,

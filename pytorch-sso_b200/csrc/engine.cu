@@ -19,6 +19,8 @@
 #include <queue>
 #include <vector>
 
+#include <cuda.h>
+
 #include "common.cuh"
 #include "diag_panel.cuh"
 #include "flow.cuh"
@@ -28,6 +30,7 @@ namespace sso {
 int launch_tile_tasks_tc(const sso_tile_task* tasks_dev, int count, int* status_dev, cudaStream_t st);
 int launch_tile_tasks_kc(const sso_tile_task* tasks_dev, int count, int* status_dev, cudaStream_t st);
 int launch_tile_tasks_tma(const sso_tile_task* tasks_dev, const void* maps_dev, int count, int* status_dev, cudaStream_t st);
+decltype(&cuTensorMapEncodeTiled) tensor_map_encoder();
 bool tma_encode_f32_rows(void* out, const float* base, int64_t rows, int64_t cols, int64_t ld);
 int g_phase_lpt = 1;    // tasks of a 128-wide phase sorted by decreasing K
 int g_chol_ksplit = 6;  // Cholesky panel updates from this panel index on are cut along K (0: never)
@@ -995,7 +998,9 @@ static size_t kron_scratch(int n_mats, const int64_t* dims, std::vector<KronScra
   return at;
 }
 
-static bool flow_enabled() { return g_flow && g_engine_tma && g_engine_tc && g_chol_panel; }
+static bool flow_enabled() { return g_flow && g_engine_tma && g_engine_tc && g_chol_panel && tensor_map_encoder() != nullptr; }
+
+int sso_kron_plan_uses_work(void) { return flow_enabled() ? 0 : 1; }
 
 size_t sso_kron_plan_dev_bytes(int n_mats, const int64_t* dims, int with_std) {
   if (n_mats <= 0 || !dims) return 0;
@@ -1023,10 +1028,11 @@ int64_t sso_kron_plan_create(int n_mats, const int64_t* dims, float* const* src,
                              float* const* work, float* const* std_out, const int32_t* partner,
                              const int32_t* role, void* dev_mem, size_t dev_mem_bytes, int host_only,
                              const int64_t* lds) {
-  SSO_CHECK_ARG(n_mats > 0 && n_mats < 32768 && dims && src && dst && work, "kron plan: null argument");
+  const bool flow = !host_only && flow_enabled();
+  SSO_CHECK_ARG(n_mats > 0 && n_mats < 32768 && dims && src && dst && (work || flow), "kron plan: null argument");
   for (int i = 0; i < n_mats; ++i) {
     SSO_CHECK_ARG(dims[i] > 0 && dims[i] <= 32768, "kron plan: bad dim %lld", (long long)dims[i]);
-    SSO_CHECK_ARG(src[i] && dst[i] && work[i], "kron plan: null matrix pointer at %d", i);
+    SSO_CHECK_ARG(src[i] && dst[i] && (flow || work[i]), "kron plan: null matrix pointer at %d", i);
     if (partner && partner[i] >= 0) SSO_CHECK_ARG(partner[i] < n_mats, "kron plan: bad partner");
   }
   // the head of the plan's memory holds the scratch matrices; the tables follow.  A host-only plan needs (host)
@@ -1039,7 +1045,7 @@ int64_t sso_kron_plan_create(int n_mats, const int64_t* dims, float* const* src,
     for (int i = 0; i < n_mats; ++i) SSO_CHECK_ARG(lds[i] >= dims[i], "kron plan: leading dimension %lld < dim %lld", (long long)lds[i], (long long)dims[i]);
   std::vector<float*> xb(n_mats);
   for (int i = 0; i < n_mats; ++i) xb[i] = reinterpret_cast<float*>(head + where[i].x);
-  if (!host_only && flow_enabled()) {
+  if (flow) {
     Plan* p = new Plan();
     bool ok = true;
     auto fill = [&](FlowProgram& f, bool inverse) {
@@ -1079,7 +1085,8 @@ int64_t sso_kron_plan_create(int n_mats, const int64_t* dims, float* const* src,
       if (rc) { delete p; return rc; }
       return register_plan(p);
     }
-    delete p;      // no tensor maps to be had: phases of launches
+    delete p;
+    return fail(-5, "kron plan: no tensor map for a scratch matrix");
   }
   Plan* p = build_kron(n_mats, dims, src, dst, work, std_out, partner, role, xb.data(), lds);
   p->host_only = host_only != 0;

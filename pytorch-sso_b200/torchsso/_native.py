@@ -99,6 +99,7 @@ SIGNATURES = {
     'sso_wire_absmax': (c_i32, [c_vp, c_vp, c_i32, c_vp, c_vp]),
     'sso_wire_encode': (c_i32, [c_vp, c_vp, c_i32, c_vp, c_vp, c_i32, c_vp]),
     'sso_wire_decode': (c_i32, [c_vp, c_vp, c_i32, c_vp, c_vp, c_i32, c_vp]),
+    'sso_kron_plan_uses_work': (c_i32, []),
     'sso_kron_plan_dev_bytes': (c_sz, [c_i32, c_vp, c_i32]),
     'sso_kron_plan_create': (c_i64, [c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_sz, c_i32, c_vp]),
     'sso_kron_plan_run': (c_i32, [c_i64, c_vp, c_vp, c_i32, c_i32, c_vp]),
@@ -865,6 +866,10 @@ def _lds(*lists):
     return _i64(out)
 
 
+def kron_plan_uses_work() -> bool:
+    return bool(lib().sso_kron_plan_uses_work())
+
+
 def kron_plan(dims, src, dst, work, std, partner, role, device, host_only=False, lds=None) -> Plan:
     L = lib()
     n = len(dims)
@@ -881,7 +886,7 @@ def kron_plan(dims, src, dst, work, std, partner, role, device, host_only=False,
     else:
         mem = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
         mem_ptr = mem.data_ptr()
-    h = L.sso_kron_plan_create(n, d, _ptrs(src), _ptrs(dst), _ptrs(work),
+    h = L.sso_kron_plan_create(n, d, _ptrs(src), _ptrs(dst), None if work is None else _ptrs(work),
                                None if std is None else _ptrs(std), _i32(partner), _i32(role),
                                mem_ptr, nbytes, int(host_only), _i64(lds) if lds is not None else _lds(src, dst, work, std))
     plan = Plan(h, mem, (src, dst, work, std, host_mem))

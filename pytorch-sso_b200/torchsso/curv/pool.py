@@ -175,6 +175,7 @@ class FactorPool:
         ent = self._plans.get(key)
         if ent is None:
             dims, src, dst, work, std, partner, role = [], [], [], [], [], [], []
+            uses_work = nat.kron_plan_uses_work()
             for c in curvs:
                 base = len(dims)
                 for which in (0, 1):
@@ -182,13 +183,14 @@ class FactorPool:
                     dims.append(m.shape[0])
                     src.append(m)
                     dst.append(self.mat('inv', c, which))
-                    work.append(self.mat('work', c, which))
+                    if uses_work:
+                        work.append(self.mat('work', c, which))
                     if with_std:
                         std.append(self.mat('std', c, which))
                     tracenorm = getattr(c, 'pi_type', 'tracenorm') == 'tracenorm'
                     partner.append(base + (1 - which) if tracenorm else -1)
                     role.append(which)
-            plan = nat.kron_plan(dims, src, dst, work, std if with_std else None, partner, role, self.device)
+            plan = nat.kron_plan(dims, src, dst, work if uses_work else None, std if with_std else None, partner, role, self.device)
             damp = torch.zeros(len(dims), dtype=torch.float32, device=self.device)
             info = torch.zeros(2 * len(dims), dtype=torch.int32, device=self.device)
             ent = (plan, damp, info)

@@ -17,12 +17,12 @@ def _solo(d: int, device):
     key = (d, device.index)
     ent = _cache.get(key)
     if ent is None:
-        bufs = [torch.empty((d, d), dtype=torch.float32, device=device) for _ in range(4)]
-        src, dst, work, std = bufs
-        plan = nat.kron_plan([d], [src], [dst], [work], [std], [-1], [0], device)
+        src, dst, std = (torch.empty((d, d), dtype=torch.float32, device=device) for _ in range(3))
+        work = [torch.empty_like(src)] if nat.kron_plan_uses_work() else None
+        plan = nat.kron_plan([d], [src], [dst], work, [std], [-1], [0], device)
         zero = torch.zeros(1, dtype=torch.float32, device=device)
         info = torch.zeros(2, dtype=torch.int32, device=device)
-        ent = (plan, src, dst, work, std, zero, info)
+        ent = (plan, src, dst, std, zero, info)
         if len(_cache) > 16:
             _cache.clear()
         _cache[key] = ent
@@ -33,7 +33,7 @@ def inv(m: torch.Tensor) -> torch.Tensor:
     if not m.is_cuda:
         raise RuntimeError('torchsso.utils.inv needs a CUDA tensor (no CPU path in this build)')
     assert m.dim() == 2 and m.shape[0] == m.shape[1]
-    plan, src, dst, work, std, zero, info = _solo(m.shape[0], m.device)
+    plan, src, dst, std, zero, info = _solo(m.shape[0], m.device)
     src.copy_(m)
     nat.kron_plan_run(plan, zero, info, True, False)
     return dst.clone()
@@ -43,7 +43,7 @@ def cholesky(m: torch.Tensor, upper: bool = True) -> torch.Tensor:
     if not m.is_cuda:
         raise RuntimeError('torchsso.utils.cholesky needs a CUDA tensor (no CPU path in this build)')
     assert m.dim() == 2 and m.shape[0] == m.shape[1]
-    plan, src, dst, work, std, zero, info = _solo(m.shape[0], m.device)
+    plan, src, dst, std, zero, info = _solo(m.shape[0], m.device)
     dst.copy_(m)           # the factorisation stage reads the "inverse" slot
     nat.kron_plan_run(plan, zero, info, False, True)
     out = std.clone()

@@ -31,7 +31,7 @@ int launch_tile_tasks_tc(const sso_tile_task* tasks_dev, int count, int* status_
 int launch_tile_tasks_kc(const sso_tile_task* tasks_dev, int count, int* status_dev, cudaStream_t st);
 int launch_tile_tasks_tma(const sso_tile_task* tasks_dev, const void* maps_dev, int count, int* status_dev, cudaStream_t st);
 decltype(&cuTensorMapEncodeTiled) tensor_map_encoder();
-bool tma_encode_f32_rows(void* out, const float* base, int64_t rows, int64_t cols, int64_t ld);
+bool tma_encode_f32_rows(void* out, const float* base, int64_t rows, int64_t cols, int64_t ld, int box_rows = 128);
 int g_phase_lpt = 1;    // tasks of a 128-wide phase sorted by decreasing K
 int g_chol_ksplit = 6;  // Cholesky panel updates from this panel index on are cut along K (0: never)
 int g_engine_tma = 1;   // k-contiguous 128-wide tasks fetch their operands with TMA (tensor maps per task)
@@ -1065,7 +1065,7 @@ int64_t sso_kron_plan_create(int n_mats, const int64_t* dims, float* const* src,
         m.flag_w = f.n_flags; m.flag_x = m.flag_w + m.np * m.np; m.flag_d = m.flag_x + m.np * m.np;
         f.n_flags += 2 * m.np * m.np + m.np;
         ok = ok && tma_encode_f32_rows(m.map_w, m.W, d, d, m.ldw) &&
-             tma_encode_f32_rows(m.map_li, m.Li, (int64_t)m.np * 128, 128, 128);
+             tma_encode_f32_rows(m.map_li, m.Li, (int64_t)m.np * 128, 128, 128) && tma_encode_f32_rows(m.map_box, m.W, d, d, m.ldw, 32);
         f.mats.push_back(m);
       }
       if (ok) schedule_flow(f, inverse);

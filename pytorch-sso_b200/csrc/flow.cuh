@@ -21,6 +21,7 @@ struct Task {
 struct alignas(64) Mat {
   unsigned char map_w[128];      // tensor maps (box 32 columns x 128 rows, SWIZZLE_128B) of the scratch matrix and of Linv
   unsigned char map_li[128];
+  unsigned char map_box[128];    // the scratch matrix again, for stores of 32x32
   const float* src;              // M before damping
   float* W;                      // scratch matrix: L in the blocks below the diagonal
   float* X;                      // the same matrix, L^-T in the others; null: factorisation only

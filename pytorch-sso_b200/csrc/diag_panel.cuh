@@ -149,25 +149,46 @@ __device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restri
 #pragma unroll
     for (int i = 0; i < 4; ++i) v[q + i] = h ? (q + i == l ? 1.f : 0.f) : (q + i <= l ? d[i] : 0.f);
   }
-  float pv = __shfl_sync(0xffffffffu, v[0], 0);
   int first_bad = -1;
 #pragma unroll
-  for (int j = 0; j < PK; ++j) {
-    float t[PK];
+  for (int j0 = 0; j0 < PK; j0 += 8) {
+    if (j0 > 0) {
+      // the first eight columns from the other eight, all at once: rows 8 to 15 of them by way of shared memory (a
+      // shuffle costs more than four cycles, 64 of them more than the sixteen loads)
+      if (lane >= 8 && lane < 16) {
+        st4(D + l * PP, v[0], v[1], v[2], v[3]);
+        st4(D + l * PP + 4, v[4], v[5], v[6], v[7]);
+      }
+      __syncwarp();
 #pragma unroll
-    for (int c = j + 1; c < PK; ++c) t[c] = __shfl_sync(0xffffffffu, v[j], c);      // a[c][j]
-    float d1 = 0.f;
-    if (j + 1 < PK) d1 = __shfl_sync(0xffffffffu, v[j + 1], j + 1);                 // a[j+1][j+1] before this step
-    const bool bad = !(pv >= 1.17549435e-38f);
-    if (bad && first_bad < 0) first_bad = j;
-    const float rs = bad ? 1.f : rsqrt_approx(pv);
-    const float w = v[j] * (rs * rs);
+      for (int c = 8; c < PK; ++c) {
+        const float4 x = ld4(D + c * PP), y = ld4(D + c * PP + 4);
+        float s0 = v[0] * x.x, s1 = v[4] * y.x;
+        s0 = fmaf(v[1], x.y, s0); s1 = fmaf(v[5], y.y, s1);
+        s0 = fmaf(v[2], x.z, s0); s1 = fmaf(v[6], y.z, s1);
+        s0 = fmaf(v[3], x.w, s0); s1 = fmaf(v[7], y.w, s1);
+        v[c] -= s0 + s1;
+      }
+    }
+    float pv = __shfl_sync(0xffffffffu, v[j0], j0);
 #pragma unroll
-    for (int c = j + 1; c < PK; ++c) v[c] = fmaf(-w, t[c], v[c]);
-    v[j] = lane == j ? (bad ? 1.f : pv) * rs : v[j] * rs;
-    if (j + 1 < PK) {
-      const float x = t[j + 1] * rs;
-      pv = fmaf(-x, x, d1);
+    for (int j = j0; j < j0 + 8; ++j) {
+      float t[PK];
+#pragma unroll
+      for (int c = j + 1; c < j0 + 8; ++c) t[c] = __shfl_sync(0xffffffffu, v[j], c);      // a[c][j]
+      float d1 = 0.f;
+      if (j + 1 < j0 + 8) d1 = __shfl_sync(0xffffffffu, v[j + 1], j + 1);                 // a[j+1][j+1] before this step
+      const bool bad = !(pv >= 1.17549435e-38f);
+      if (bad && first_bad < 0) first_bad = j;
+      const float rs = bad ? 1.f : rsqrt_approx(pv);
+      const float w = v[j] * (rs * rs);
+#pragma unroll
+      for (int c = j + 1; c < j0 + 8; ++c) v[c] = fmaf(-w, t[c], v[c]);
+      v[j] = lane == j ? (bad ? 1.f : pv) * rs : v[j] * rs;
+      if (j + 1 < j0 + 8) {
+        const float x = t[j + 1] * rs;
+        pv = fmaf(-x, x, d1);
+      }
     }
   }
   if (first_bad >= 0 && lane == 0 && info && c0 + first_bad < n) atomicCAS(info, 0, row0 + c0 + first_bad + 1);

@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         const uint32_t rs = stage % RAW, ls = stage % LO;
         const bool mult = s >= sh.n1, share = sh.share && !mult;
         if (s == sh.n1) ok = mbar_wait(afull, n_mult & 1, status, 91);      // the sum has been written into the raw slots
-        if (ok) ok = mbar_wait(rawfull(rs), (stage / RAW) & 1, status, 92);
+        if (ok && !mult) ok = mbar_wait(rawfull(rs), (stage / RAW) & 1, status, 92);
         if (ok && stage >= LO) ok = mbar_wait(lofree(ls), ((stage / LO) - 1) & 1, status, 93);
         if (!ok) break;
         const uint32_t hi = smem0 + rs * PART + so0, lo = lo0 + ls * PART + so0;
@@ -304,6 +304,8 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
           }
         };
         split(0);
+        if (mult) ok = mbar_wait(rawfull(rs), (stage / RAW) & 1, status, 92);      // the sum is split while the inverse is awaited
+        if (!ok) break;
         if (!share) split(OPB);
         fence_async_smem();
         __syncwarp();

@@ -20,11 +20,10 @@
 // Rows and columns past the block's size behave as an identity block.  A pivot that is not a positive normal number
 // (non-positive, denormal or NaN) is recorded once per matrix (LAPACK numbering) and replaced by 1, like the 64-wide
 // kernel does for non-positive ones.
-// Measured: 14.4 us for 128 rows (clocks: 1900 to 2900 per elimination with the subtraction before it, 720 for the
-// round of products); a chain of four barriers per panel with all warps in step and the inverse by three levels of
-// doubling afterwards took 23.  Inside the dataflow kernel, with the inverse of the block announced before the other
-// results are written: 1000 402 -> 284 us, 577+64 264 -> 191, the six factors of 784-1000-1000-10 433 -> 315,
-// 4608+512 2208 -> 1544.
+// Measured: 12.5 us for 128 rows (before the elimination went in two steps of eight and took the next block from
+// registers 14.4); a chain of four barriers per panel with all warps in step and the inverse by three levels of
+// doubling afterwards took 23.  Inside the dataflow kernel (1000 columns) 402 us with that one, 265 now; elimination and
+// products are straight-line code that issues an instruction in about four clocks.
 #pragma once
 #include "common.cuh"
 
@@ -104,17 +103,18 @@ __device__ __forceinline__ void subtract(float* __restrict__ C, uint32_t planes,
 #pragma unroll
     for (int r = 0; r < 2; ++r) c[(8 * r * PP + 8 * h) / 2] = make_float2(v[h][r].x - o[h][2 * r], v[h][r].y - o[h][2 * r + 1]);
 }
-// Three parts of the values at a lane's places (rows g, g + 8; columns 2 t, + 1 and 2 t + 8, + 9) of row block b.
-__device__ __forceinline__ void put_parts(uint32_t planes, int b, const float (&o)[2][4], int lane) {
+// Three parts of the values at a lane's places (rows g, g + 8; columns 2 t, + 1 and 2 t + 8, + 9) of row block b: into
+// `q` as the registers of an A operand, and to shared memory.
+__device__ __forceinline__ void put_parts(uint32_t planes, int b, const float (&o)[2][4], uint32_t (&q)[3][4], int lane) {
   const uint32_t at = planes + (16 * b + (lane >> 2)) * PL_ROW + 4 * (lane & 3);
 #pragma unroll
   for (int h = 0; h < 2; ++h)
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      uint32_t q[3];
-      split2(o[h][2 * r], o[h][2 * r + 1], q[0], q[1], q[2]);
+      split2(o[h][2 * r], o[h][2 * r + 1], q[0][2 * h + r], q[1][2 * h + r], q[2][2 * h + r]);
 #pragma unroll
-      for (int i = 0; i < 3; ++i) asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + i * PL_PART + 8 * r * PL_ROW + 16 * h), "r"(q[i]) : "memory");
+      for (int i = 0; i < 3; ++i)
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + i * PL_PART + 8 * r * PL_ROW + 16 * h), "r"(q[i][2 * h + r]) : "memory");
     }
 }
 
@@ -133,14 +133,10 @@ constexpr Schedule make_schedule() {
 }
 static __constant__ Schedule c_schedule = make_schedule();
 
-// The elimination of panel k's diagonal block by one warp, after the subtraction of panel k - 1.
-__device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restrict__ V, uint32_t planes, int k, int n, int* __restrict__ info, int row0, int lane) {
+// The elimination of panel k's diagonal block by one warp.
+__device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restrict__ V, int k, int n, int* __restrict__ info, int row0, int lane) {
   const int l = lane & 15, h = lane >> 4, c0 = PK * k;
   float* D = S + c0 * PP + c0;
-  if (k > 0) {
-    subtract(D, planes, k, k, false, lane);
-    __syncwarp();
-  }
   float v[PK];
 #pragma unroll
   for (int q = 0; q < PK; q += 4) {
@@ -214,7 +210,7 @@ __device__ __forceinline__ void factor_block(float* __restrict__ S, float* __res
   auto at = [](float* m, int i, int j) { return m + (PK * i) * PP + PK * j; };
   for (int k = 0; k < np; ++k) {
     if (warp == 0) {
-      eliminate(S, V, planes, k, n, info, row0, lane);
+      eliminate(S, V, k, n, info, row0, lane);
     } else if (k == 0) {
       // the inverse's upper half, and its identity past the matrix
       for (int e = tid - 32; e < PN * PN / 4; e += THREADS - 32) {
@@ -241,7 +237,8 @@ __device__ __forceinline__ void factor_block(float* __restrict__ S, float* __res
         for (int h = 0; h < 2; ++h)
 #pragma unroll
           for (int i = 0; i < 4; ++i) o[h][i] = I[(8 * h + 2 * t + (i & 1)) * PP + g + 8 * (i >> 1)];
-        put_parts(planes, k, o, lane);
+        uint32_t q[3][4];
+        put_parts(planes, k, o, q, lane);
       }
     } else if (b < np) {                // X Inv_kk^T, X = S(b, k): below the diagonal a block of L, above one of L^-T
       float2* X = reinterpret_cast<float2*>(at(S, b, k) + g * PP + 2 * t);
@@ -268,12 +265,27 @@ __device__ __forceinline__ void factor_block(float* __restrict__ S, float* __res
 #pragma unroll
           for (int i = 0; i < 4; ++i) O[(8 * h + (i & 1)) * PP + 8 * (i >> 1)] = o[h][i];
       }
-      if (more) put_parts(planes, b, o, lane);
+      if (more) put_parts(planes, b, o, xa, lane);
+      if (warp == 0) {
+        __syncwarp();
+        arrive_y();
+        // the next diagonal block minus this panel: both operands are the block just finished, still in registers
+#pragma unroll
+        for (int i = 0; i < 3; ++i) { xb[i][0] = xa[i][0]; xb[i][1] = xa[i][2]; xb[i][2] = xa[i][1]; xb[i][3] = xa[i][3]; }
+        float2* D = reinterpret_cast<float2*>(at(S, b, b) + g * PP + 2 * t);
+        product(o, xa, xb);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            float2& c = D[(8 * r * PP + 8 * h) / 2];
+            c = make_float2(c.x - o[h][2 * r], c.y - o[h][2 * r + 1]);
+          }
+        __syncwarp();
+      }
     }
     if (warp == 0) {
-      __syncwarp();
-      if (more) arrive_y();
-      else sync_y();
+      if (!more) sync_y();
     } else {
       sync_y();
     }

@@ -17,9 +17,9 @@
 // warps write it into the raw slots of four more stages.
 //
 // Bound: for one large matrix the chain of diagonal blocks, for many the shared-memory traffic of the 3xTF32 stages
-// (as tile_task_tma_kernel).  Against one launch per phase (us): 577+64 508 -> 191, 1000 637 -> 284, six factors of a
-// 784-1000-1000-10 network 1196 -> 315, 4608+512 3363 -> 1544, the 106 factors of ResNet-50 8970 -> 3710, those of VGG-16
-// with sampling factors 19416 -> 7480.
+// (as tile_task_tma_kernel).  Against one launch per phase (us): 577+64 508 -> 180, 1000 637 -> 265, six factors of a
+// 784-1000-1000-10 network 1196 -> 296, 4608+512 3363 -> 1424, the 106 factors of ResNet-50 8970 -> 3600, those of VGG-16
+// with sampling factors 19416 -> 7440.
 // Every wait is bounded; a CTA whose wait gives up sets the status word and writes NaN for this and all further tasks.
 #include "common.cuh"
 #include "diag_panel.cuh"

@@ -11,6 +11,7 @@ sm_100a kernels in libsso_b200 (no torch linear algebra, no CPU path).
 from __future__ import annotations
 
 import math
+import weakref
 
 import torch
 import torch.nn as nn
@@ -20,6 +21,27 @@ from .pool import FactorPool
 
 PI_TYPE_TRACENORM = 'tracenorm'
 _NORM_TYPES = (nn.BatchNorm1d, nn.BatchNorm2d, nn.BatchNorm3d)
+
+
+class _ForwardHook:
+    """What a hooked module keeps of its curvature: a weak reference, so that a curvature whose owner is gone gives its
+    buffers back at once instead of at the next cycle collection.  A copy of the module has no curvature."""
+
+    __slots__ = ('ref',)
+
+    def __init__(self, curv=None):
+        self.ref = weakref.ref(curv) if curv is not None else lambda: None
+
+    def __call__(self, module, input, output):
+        curv = self.ref()
+        if curv is not None:
+            curv.forward_postprocess(module, input, output)
+
+    def __deepcopy__(self, memo):
+        return _ForwardHook()
+
+    def __reduce__(self):
+        return _ForwardHook, ()
 
 
 class Curvature(object):
@@ -48,7 +70,7 @@ class Curvature(object):
         self._have = set()          # which of data / ema / inv / std hold values
         self._generic = {}          # storage for curvature shapes the pool does not manage
         self._is_norm = isinstance(module, _NORM_TYPES)
-        module.register_forward_hook(self.forward_postprocess)
+        module.register_forward_hook(_ForwardHook(self))
 
     # ---- identity ---------------------------------------------------------------
     @property

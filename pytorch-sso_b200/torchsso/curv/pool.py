@@ -18,6 +18,7 @@ single code path.
 from __future__ import annotations
 
 import math
+import weakref
 from typing import Dict, List, Optional, Sequence
 
 import torch
@@ -43,13 +44,13 @@ class FactorPool:
 
     def __init__(self, kron: Sequence, diag: Sequence, device):
         self.device = torch.device(device)
-        self.kron = list(kron)
-        self.diag = list(diag)
+        self._kron = [weakref.ref(c) for c in kron]      # the curvatures hold their pool
+        self._diag = [weakref.ref(c) for c in diag]
         self._bufs: Dict[str, torch.Tensor] = {}
         # --- Kronecker layout: [A_0 | G_0 | A_1 | G_1 | ...]
         self.k_off = {}
         off = 0
-        for c in self.kron:
+        for c in kron:
             (da, _), (dg, _) = c._get_shape()
             a_off = off
             off = _round_up(off + da * _ld(da))
@@ -60,7 +61,7 @@ class FactorPool:
         # --- diagonal layout: parameters of each layer back to back, layers back to back
         self.d_off = {}
         off = 0
-        for c in self.diag:
+        for c in diag:
             offs = []
             for p in c.module.parameters():
                 offs.append((off, tuple(p.shape)))
@@ -72,8 +73,16 @@ class FactorPool:
         self._mats = {}
         self._ranges = {}
         self.last_info: Optional[torch.Tensor] = None
-        for c in list(self.kron) + list(self.diag):
+        for c in list(kron) + list(diag):
             c._pool = self
+
+    @property
+    def kron(self) -> List:
+        return [r() for r in self._kron]
+
+    @property
+    def diag(self) -> List:
+        return [r() for r in self._diag]
 
     # ------------------------------------------------------------------ storage
     def buf(self, role: str, kind: str = 'k') -> torch.Tensor:
@@ -121,10 +130,11 @@ class FactorPool:
         return self._remembered('k', curvs, self._find_kron_range) if curvs else (0, 0)
 
     def _find_kron_range(self, curvs):
-        idx = sorted(self.kron.index(c) for c in curvs)
+        kron = self.kron
+        idx = sorted(kron.index(c) for c in curvs)
         assert idx == list(range(idx[0], idx[-1] + 1)), 'curvatures are not contiguous in the pool'
-        lo = self.k_off[id(self.kron[idx[0]])][0]
-        hi = self.k_off[id(self.kron[idx[-1] + 1])][0] if idx[-1] + 1 < len(self.kron) else self.k_total
+        lo = self.k_off[id(kron[idx[0]])][0]
+        hi = self.k_off[id(kron[idx[-1] + 1])][0] if idx[-1] + 1 < len(kron) else self.k_total
         return lo, hi
 
     def diag_range(self, curvs: Sequence):
@@ -132,10 +142,11 @@ class FactorPool:
         return self._remembered('d', curvs, self._find_diag_range) if curvs else (0, 0)
 
     def _find_diag_range(self, curvs):
-        idx = sorted(self.diag.index(c) for c in curvs)
+        diag = self.diag
+        idx = sorted(diag.index(c) for c in curvs)
         assert idx == list(range(idx[0], idx[-1] + 1)), 'curvatures are not contiguous in the pool'
-        lo = self.d_off[id(self.diag[idx[0]])][0][0]
-        hi = self.d_off[id(self.diag[idx[-1] + 1])][0][0] if idx[-1] + 1 < len(self.diag) else self.d_total
+        lo = self.d_off[id(diag[idx[0]])][0][0]
+        hi = self.d_off[id(diag[idx[-1] + 1])][0][0] if idx[-1] + 1 < len(diag) else self.d_total
         return lo, hi
 
     # ------------------------------------------------------------------ streaming ops

@@ -259,3 +259,36 @@ def test_sample_plan_along_k(nat, shapes, bias):
     for i in range(len(shapes)):
         got = w[i] if b[i] is None else torch.cat([w[i], b[i][:, None]], 1)
         assert rel(got, want[i]) < 2e-6
+
+
+# ------------------------------------------------------------------------------------------- lifetime
+def test_an_optimizer_gives_its_buffers_back_when_it_goes(nat):
+    """No reference cycle through hooks and pools; a copy of a hooked model has no curvature."""
+    import copy
+    import gc
+    import torchsso
+    model = torch.nn.Sequential(torch.nn.Linear(300, 200), torch.nn.Unflatten(1, (8, 5, 5)), torch.nn.BatchNorm2d(8), torch.nn.Flatten(),
+                                torch.nn.Linear(200, 10)).cuda()
+    x, y = torch.randn(64, 300, device='cuda'), torch.randint(0, 10, (64,), device='cuda')
+
+    def step():
+        opt = torchsso.optim.SecondOrderOptimizer(model, 'Fisher', {'Linear': 'Kron', 'BatchNorm2d': 'Diag'}, {'damping': 1e-2})
+        opt.step(closure=torchsso.get_closure_for_fisher(opt, model, x, y, approx_type='mc', num_mc=1))
+        copy.deepcopy(model)(x)
+        return opt
+    for p in model.parameters():
+        p.grad = None
+    gc.collect()
+    gc.disable()
+    try:
+        held = []
+        for _ in range(3):
+            opt = step()
+            torch.cuda.synchronize()
+            del opt
+            for p in model.parameters():
+                p.grad = None
+            held.append(torch.cuda.memory_allocated())
+    finally:
+        gc.enable()
+    assert held[2] <= held[1] + (1 << 16), held

@@ -20,8 +20,8 @@
 // Bound: with boxes the MMAs, twelve per stage of 32 rows and pair (1536 cycles per SM, 0.98 us as measured without any
 // loads; 1.1 with them); gathered, the copies: 48 KB of parts per stage come in at 1.4 us whatever the number of stages
 // in flight, MMAs or not (5 TB/s over the chip: what the load/store path of an SM keeps outstanding).  us, 3xTF32 on
-// 128x128 tiles / gathered / boxes: 5x5 over 64 channels, d = 1601 from 65536 rows 1810 / 1127 / 896; 3x3 over 64,
-// d = 577 from 131072 rows 495 gathered, 391; d = 4608 from 8192 rows 1710 / 1016 / 876.  Measured alternatives:
+// 128x128 tiles / gathered / boxes / with narrow last block rows: 5x5 over 64 channels, d = 1601 from 65536 rows 1810 /
+// 1127 / 896 / 840; 3x3 over 64, d = 577 from 131072 rows 495 gathered, 391 / 363; d = 4608 from 8192 rows 1710 / 1016 / 876.  Measured alternatives:
 // splitting in the gather warps is bound by their instructions (650 per warp and stage, 2.3 us per stage, in bf16 as in
 // 3xTF32), and 32-bit MN-major operands are read at half the rate.
 // The input is processed in runs of whole images whose parts fit the scratch; each run adds to the partial tiles of
@@ -68,6 +68,7 @@ struct Parts {
 struct alignas(64) Boxes {
   CUtensorMap map;
   int bw, bh, bn, across, down;      // a box; boxes per image in either direction
+  int narrow;                        // N of the last block row's MMAs (narrow_columns), 0: an ordinary row
 };
 
 // First kernel of a factor: let the next one set itself up meanwhile (it waits for this one's end before it touches
@@ -260,24 +261,46 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // uniform, for setmaxnreg
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
-  int bI, bJ;                                    // block (PAIR: 256 wide) row and column
-  tri_decode(PAIR ? blockIdx.x >> 1 : blockIdx.x, bI, bJ);
-  const bool share = (bI == bJ) && (p.weight == nullptr);
   const bool fused = p.tickets != nullptr;
-  const int split = blockIdx.y;
+  const int last_n = BOX ? boxes.narrow : 0;
+  int bI, bJ;                                    // block (PAIR: 256 wide) row and column
+  int split = blockIdx.y;
+  if (BOX) {
+    // the blocks of a narrow last block row come behind all others, whatever their split: short work last
+    const int nb2 = ceil_div(p.d, 256), units = nb2 * (nb2 + 1) / 2;
+    const int whole = last_n ? units - nb2 : units, narrow = units - whole;
+    int id = blockIdx.x >> 1, unit;
+    if (id < whole * p.splits) {
+      split = id / whole;
+      unit = id - split * whole;
+    } else {
+      id -= whole * p.splits;
+      split = id / narrow;
+      unit = whole + id - split * narrow;
+    }
+    tri_decode(unit, bI, bJ);
+  } else {
+    tri_decode(PAIR ? blockIdx.x >> 1 : blockIdx.x, bI, bJ);
+  }
   const int64_t r_begin = (int64_t)split * p.rows_per_split;
   const int nrows = (int)max((int64_t)0, min((int64_t)p.rows_per_split, p.rows - r_begin));
   const int nstages = ceil_div(nrows, KS);
   const int nchunks = ceil_div(nstages, FLUSH);
   int* status = p.status;
-  const int col_a = bI * (PAIR ? 256 : 128) + (int)rank * TILE, col_b = bJ * (PAIR ? 256 : 128) + (int)rank * TILE;
+  // The last block row, if it is at most 128 wide, takes the column side: N is that width (halves of it per CTA) and the
+  // block it meets fills the 256 rows, so that its MMAs and loads shrink with it.  The tile comes out transposed.
+  const bool ragged = last_n != 0 && bI == (p.d - 1) / 256, swapped = ragged && bI != bJ;
+  const int col_a = (swapped ? bJ : bI) * (PAIR ? 256 : 128) + (int)rank * TILE;
+  const int col_b = !ragged ? bJ * (PAIR ? 256 : 128) + (int)rank * TILE : rank == 0 ? bI * 256 : last_n == 128 ? bI * 256 + 64 : p.d + 255;
   // 64-column blocks A0 A1 B0 B1 that hold columns of the matrix and are needed; a box leaves the ones column of a
   // k x k window out (it has a block to itself, written once below)
   const int loaded_cols = BOX ? p.dcols : p.d;
+  const bool share = bI == bJ && p.weight == nullptr && !ragged;
+  const uint32_t used = share ? 3u : ragged ? 7u : 15u;
   uint32_t blocks = 0;
 #pragma unroll
   for (int b = 0; b < 4; ++b)
-    if ((b < 2 ? col_a : col_b) + (b & 1) * 64 < loaded_cols && !(share && b >= 2)) blocks |= 1u << b;
+    if ((b < 2 ? col_a : col_b) + (b & 1) * 64 < loaded_cols && ((used >> b) & 1u)) blocks |= 1u << b;
 
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t bar0 = smem_u32(bars);
@@ -299,7 +322,7 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // blocks past the matrix edge are never written: they stay zero
-  const uint32_t idle = ~blocks & (share ? 3u : 15u);
+  const uint32_t idle = ~blocks & used;
   if (idle) {
     for (int b = 0; b < 4; ++b) {
       if (!((idle >> b) & 1u)) continue;
@@ -357,7 +380,16 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
     }
     const int ti = PAIR ? 2 * bI + (int)rank : bI, tj = PAIR ? 2 * bJ + half : bJ;
     const int col0 = PAIR ? 0 : half * NACC;     // first column inside the 128x128 tile
-    if (ti < ceil_div(p.d, TILE) && tj <= ti) {
+    if (BOX && swapped) {
+      // column i of the last block row, row jr of this CTA's 128: transposed into tile (2 bI, 2 bJ + rank)
+      const int tr = 2 * bI, tc = 2 * bJ + (int)rank, jr = q * 32 + lane, width = p.d - 256 * bI;
+      float* dst = p.partial + ((int64_t)(tr * (tr + 1) / 2 + tc) * p.splits + split) * (TILE * TILE) + part_at(0, jr);
+      if (half == 0) {
+#pragma unroll
+        for (int i = 0; i < NACC; ++i)
+          if (i < width) dst[4 * i] = p.accumulate ? dst[4 * i] + acc[i] : acc[i];
+      }
+    } else if (ti < ceil_div(p.d, TILE) && tj <= ti) {
       float* dst = p.partial + ((int64_t)(ti * (ti + 1) / 2 + tj) * p.splits + split) * (TILE * TILE) + part_at(q * 32 + lane, col0);
       if (p.accumulate) {
 #pragma unroll
@@ -388,7 +420,7 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
     if (warp == MMA_WARP && lane == 0 && rank == 0) {
       // a narrow tile multiplies only the columns that exist (N in steps of 16)
       const int n_cols = min(TILE, (p.d - bJ * TILE + 15) / 16 * 16);
-      const uint32_t idesc = PAIR ? instr_desc_pair(1u, 1u)
+      const uint32_t idesc = PAIR ? (instr_desc_pair(1u, 1u) & ~(0x3Fu << 17)) | ((uint32_t)((ragged ? last_n : 256) >> 3) << 17)
                                   : ((instr_desc(1u, 1u) & ~(0x3Fu << 17)) | ((uint32_t)(n_cols >> 3) << 17));
       bool ok = true;
       for (int s = 0; s < nstages && ok; ++s) {
@@ -440,7 +472,9 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
           x0[b] = (pos - ky * p.kw) * p.dil_w - p.pad_w;
           y0[b] = ky * p.dil_h - p.pad_h;
           const int first = j0 - (int)rank * TILE;
-          if (!(share && b >= 2)) pair_blocks += (first < loaded_cols ? 1u : 0u) + (first + TILE < loaded_cols ? 1u : 0u);
+          if (!((used >> b) & 1u)) continue;
+          if (ragged && b == 2) pair_blocks += (bI * 256 < loaded_cols ? 1u : 0u) + (last_n == 128 && bI * 256 + 64 < loaded_cols ? 1u : 0u);
+          else pair_blocks += (first < loaded_cols ? 1u : 0u) + (first + TILE < loaded_cols ? 1u : 0u);
         }
         const uint64_t map = reinterpret_cast<uint64_t>(&boxes.map);
         const uint32_t fulls = map_to_cta(full_bar(0), 0u);
@@ -529,14 +563,24 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
 
 // Blocks x splits of the rows over the 74 pairs (148 SMs), with measured costs: a stage, the fixed cost of a CTA
 // (set-up, pipeline fill, drain, tile), a partial tile's way to memory and back.
-static int choose_splits(int64_t rows, int units, int slots, int tiles, double stage_us, int max_splits, int& rows_per_split) {
+// `narrow` of the units take `part` of the others' time and run behind them.
+static int choose_splits(int64_t rows, int units, int narrow, double part, int slots, int tiles, double stage_us, int max_splits,
+                         int& rows_per_split) {
   const int64_t stages = ceil_div64(rows, KS);
   const int most = (int)std::max<int64_t>(1, std::min<int64_t>({stages / 4, 148, max_splits}));
   double best = 1e30;
   int64_t best_sps = stages;
   for (int s = 1; s <= most; ++s) {
     const int64_t sps = ceil_div64(stages, s), real = ceil_div64(stages, sps);
-    const double cost = (double)ceil_div64(units * real, slots) * ((double)sps * stage_us + 5.0) + 0.03 * (double)(tiles * real);
+    const int64_t whole = (units - narrow) * real, rest = whole % slots;
+    double rounds = (double)(whole / slots);
+    int64_t left = narrow * real;
+    if (rest) {
+      rounds += 1.0;
+      left -= (slots - rest) * (int64_t)(1.0 / part);      // beside the last round of the others
+    }
+    if (left > 0) rounds += part * (double)ceil_div64(left, slots);
+    const double cost = rounds * ((double)sps * stage_us + 5.0) + 0.03 * (double)(tiles * real);
     if (cost < best - 1e-9) { best = cost; best_sps = sps; }
   }
   rows_per_split = (int)(best_sps * KS);
@@ -547,7 +591,7 @@ template <bool PAIR, bool BOX>
 static int launch(const FactorParams& p, const Parts& parts, const Boxes& boxes, int units, int splits, cudaStream_t st) {
   SSO_ENSURE_SMEM((factor_f32_kernel<PAIR, BOX>), SMEM);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(PAIR ? 2 * units : units, splits);
+  cfg.gridDim = BOX ? dim3(2 * units * splits) : dim3(PAIR ? 2 * units : units, splits);
   cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = SMEM;
   cfg.stream = st;
@@ -801,6 +845,14 @@ static bool encode_boxes(Boxes& b, const Parts& parts, const Shape& s, int h, in
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 constexpr int64_t PARTS_TARGET = (int64_t)256 << 20;     // parts of one run of images
+// Columns that the MMAs of the last block row compute if it is a narrow one: 32 (at most sixteen columns, all of them
+// from one CTA; a pair's N is a multiple of 32), 128, or 0 for an ordinary block.  Its blocks run behind all others and
+// read the parts once more: from L2 up to this size (d = 333 from 401408 rows, 256 MB a run, 1153 us without, 1267 with).
+constexpr int64_t NARROW_PARTS = (int64_t)96 << 20;
+static int narrow_columns(int d) {
+  const int width = d - (d - 1) / 256 * 256;
+  return d <= 256 || width > 128 ? 0 : width <= 16 ? 32 : 128;
+}
 constexpr int64_t PARTIAL_TARGET = (int64_t)148 * 2 * 65536;
 
 }  // namespace f32
@@ -881,7 +933,9 @@ int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, c
   q.partial = reinterpret_cast<float*>(base + (hdr + 255) / 256 * 256 + (parts_bytes + 255) / 256 * 256);
   const int64_t hw = (int64_t)p.ho * p.wo;
   int rps = 0;
-  q.splits = f32::choose_splits(n_run * hw, pair ? s.blocks : s.tiles, pair ? 74 : 148, s.tiles, box ? 0.65 : pair ? 0.85 : 0.6, max_splits, rps);
+  boxes.narrow = box && parts_bytes <= f32::NARROW_PARTS ? f32::narrow_columns(s.d) : 0;
+  q.splits = f32::choose_splits(n_run * hw, pair ? s.blocks : s.tiles, boxes.narrow ? ceil_div(s.d, 256) : 0, boxes.narrow == 32 ? 0.6 : 0.75,
+                                pair ? 74 : 148, s.tiles, box ? 1.05 : pair ? 0.85 : 0.6, max_splits, rps);
   q.rows_per_split = rps;
   const int kk = p.kh * p.kw;
   q.perm_c = kk > 1 ? s.c8 : 0;
@@ -892,6 +946,7 @@ int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, c
   q.sn = (int64_t)p.h * s.width * s.c8; q.sh = (int64_t)s.width * s.c8; q.sw = s.c8; q.sc = 1;
   if (s.fold) { q.kw = 1; q.stride_w = 1; q.pad_w = 0; q.dil_w = 1; }
   const bool fused = kk == 1 && q.splits == 1;
+  if (fused) boxes.narrow = 0;      // its tiles come out transposed, which the finishing in the kernel does not expect
   q.ticket_tiles = s.tiles;
   const bool direct = !s.fold && p.sc == 1 && p.c % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 && p.sn % 4 == 0 &&
                       (p.h == 1 || p.sh % 4 == 0) && (p.w == 1 || p.sw % 4 == 0) && (int64_t)n_run * p.h * s.width * (s.c8 / 8) < ((int64_t)1 << 31);

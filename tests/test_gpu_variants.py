@@ -87,7 +87,8 @@ F32_CONVS = [(5, 3, 20, 19, (7, 7), (2, 2), (3, 3), (1, 1), False), (3, 1, 9, 9,
              (40, 33, 6, 6, (1, 1), (2, 2), (0, 0), (1, 1), True), (2, 9, 10, 10, (9, 9), (1, 1), (4, 4), (1, 1), True),
              (3, 21, 9, 8, (4, 4), (1, 1), (1, 1), (1, 1), False), (1, 40, 7, 7, (2, 2), (1, 1), (0, 0), (1, 1), True), (6, 128, 4, 4, (3, 3), (1, 1), (1, 1), (1, 1), True),
              (16, 64, 2, 2, (3, 3), (1, 1), (1, 1), (1, 1), False), (2, 64, 16, 33, (3, 2), (1, 1), (1, 0), (1, 1), True),
-             (2, 64, 12, 24, (5, 5), (1, 1), (4, 4), (2, 2), True), (4, 200, 32, 32, (1, 1), (1, 1), (0, 0), (1, 1), True), (16, 130, 5, 7, (1, 1), (1, 1), (0, 0), (1, 1), True)]
+             (2, 64, 12, 24, (5, 5), (1, 1), (4, 4), (2, 2), True), (4, 200, 32, 32, (1, 1), (1, 1), (0, 0), (1, 1), True), (2, 128, 8, 8, (3, 2), (1, 1), (1, 1), (1, 1), True),
+             (2, 256, 8, 8, (3, 3), (1, 1), (1, 1), (1, 1), True), (16, 130, 5, 7, (1, 1), (1, 1), (0, 0), (1, 1), True)]
 
 
 @pytest.mark.parametrize('cfg', F32_CONVS)
@@ -108,7 +109,7 @@ def test_factor_f32_conv(nat, cfg, channels_last):
 
 
 @pytest.mark.parametrize('rows,cols,bias', [(1, 1, False), (31, 5, True), (129, 63, True), (700, 64, False), (5000, 64, True), (33000, 128, False),
-                                            (20001, 97, True), (40000, 13, False), (257, 300, True), (256, 300, True), (1024, 1021, False), (1500, 1021, True), (33, 4100, False)])
+                                            (20001, 97, True), (40000, 13, False), (257, 300, True), (256, 300, True), (1024, 1021, False), (256, 272, False), (288, 264, True), (512, 384, False), (128, 511, True), (320, 520, True), (1500, 1021, True), (33, 4100, False)])
 @pytest.mark.parametrize('layout', ['rows', 'strided', 'columns'])
 def test_factor_f32_rows(nat, rows, cols, bias, layout):
     x = torch.randn(rows, cols, device='cuda') + 0.25
@@ -125,16 +126,16 @@ def test_factor_f32_rows(nat, rows, cols, bias, layout):
     assert rel(out, u.t() @ u / rows) < 1e-6 and torch.equal(out, out.t())
 
 
-def test_factor_f32_in_runs(nat):
+@pytest.mark.parametrize('n,c,size', [(37, 40, 10), (36, 64, 8)])
+def test_factor_f32_in_runs(nat, n, c, size):
     """Scratch for a few images at a time: the runs add to the same partial tiles."""
-    n, c = 37, 40
-    x = torch.randn(n, c, 10, 10, device='cuda')
+    x = torch.randn(n, c, size, size, device='cuda')
     ref = conv_ref(x, (3, 3), (1, 1), (1, 1), (1, 1), True)
     d = ref.shape[0]
-    for space in (900_000, 2_000_000, 64_000_000):
+    for space in (1_100_000, 2_000_000, 64_000_000):
         out = torch.empty(d, d, device='cuda')
         ws = torch.empty(space, dtype=torch.uint8, device='cuda')
-        nat._check(nat.lib().sso_factor_syrk_im2col(x.data_ptr(), nat.F32, n, c, 10, 10, *x.stride(), 3, 3, 1, 1, 1, 1, 1, 1, 1, None, 1.0, 0.0,
+        nat._check(nat.lib().sso_factor_syrk_im2col(x.data_ptr(), nat.F32, n, c, size, size, *x.stride(), 3, 3, 1, 1, 1, 1, 1, 1, 1, None, 1.0, 0.0,
                                                     out.data_ptr(), d, ws.data_ptr(), space, nat.IMPL_AUTO, nat._stream()))
         assert rel(out, ref) < 1e-6
 

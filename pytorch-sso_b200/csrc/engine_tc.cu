@@ -364,6 +364,7 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tc_kernel(const sso_tile
 // value, lo goes to a ring of LO_SLOTS stages) and hand the stage to the MMA warp.
 // ------------------------------------------------------------------------------------------
 constexpr uint32_t PART = 2 * OPB;                       // A and B of one stage, one flavour (raw/hi or lo)
+constexpr uint32_t TS_COLS = 512;                        // two accumulators and the A operands of up to four stages
 constexpr uint32_t KC_SMEM = 7 * PART;                   // RAW_SLOTS + LO_SLOTS = 7 in every variant
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t src_bytes) {
@@ -513,7 +514,11 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_kc_kernel(const sso_tile
 // TMA-fed variant of the k-contiguous kernel: the two operand boxes of a stage (128 rows x 32 k,
 // fp32) are fetched by one thread with cp.async.bulk.tensor into the raw ring (tensor maps made
 // on the host when the plan is built, two per task), so the loads no longer pass through the
-// load/store units.  The load warps only split: hi in place, lo into the second ring.
+// load/store units.  The load warps only split: A into tensor memory (hi and lo, a row per lane, which
+// takes its part of the operand traffic off shared memory), B's hi in place and lo into a second ring.
+// Bound: the MMAs for large tasks (4608 x 512 preconditioned in 152 us, 287 TFLOP/s), set-up, pipeline fill
+// and store of a task (about 10 us) for small ones.  us, with A in shared memory and chunks split one by one / in
+// shared memory / in tensor memory: that layer 175 / 161 / 152, ResNet-50's preconditioning 1122 / 1037 / 1005.
 // ------------------------------------------------------------------------------------------
 struct alignas(128) TaskMaps {
   unsigned char a[128];
@@ -559,7 +564,7 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == MMA_WARP) tmem_alloc(smem_u32(&tmem_base_slot), TMEM_COLS);
+  if (warp == MMA_WARP) tmem_alloc(smem_u32(&tmem_base_slot), TS_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -580,15 +585,15 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
         ok = mbar_wait(full_bar(ls), (s / LO_SLOTS) & 1, status, 41);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t ah = smem0 + rs * PART, bh = ah + OPB, al = lo0 + ls * PART, bl = al + OPB;
+        const uint32_t bh = smem0 + rs * PART + OPB, bl = lo0 + ls * OPB;
+        const uint32_t ah = tmem_base + TMEM_COLS + ls * 2 * KS, al = ah + KS;
         const uint32_t d_tmem = tmem_base + (uint32_t)(b * TILE);
 #pragma unroll
         for (int ks = 0; ks < KS / 8; ++ks) {
-          const uint64_t adh = smem_desc_sw128_kmajor(ah + ks * 32u), adl = smem_desc_sw128_kmajor(al + ks * 32u);
           const uint64_t bdh = smem_desc_sw128_kmajor(bh + ks * 32u), bdl = smem_desc_sw128_kmajor(bl + ks * 32u);
-          umma<true>(d_tmem, adl, bdh, idesc, (first_of_chunk && ks == 0) ? 0u : 1u);
-          umma<true>(d_tmem, adh, bdl, idesc, 1u);
-          umma<true>(d_tmem, adh, bdh, idesc, 1u);
+          umma_tf32_ts(d_tmem, al + ks * 8, bdh, idesc, (first_of_chunk && ks == 0) ? 0u : 1u);
+          umma_tf32_ts(d_tmem, ah + ks * 8, bdl, idesc, 1u);
+          umma_tf32_ts(d_tmem, ah + ks * 8, bdh, idesc, 1u);
         }
         umma_commit(rawfree_bar(rs));
         umma_commit(lofree_bar(ls));
@@ -600,6 +605,7 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
     const int lt = tid - 32 * (MMA_WARP + 1);
     const int q = lt >> 3, l8 = lt & 7;
     const uint32_t so0 = sw_off(q, l8 * 4);
+    const int a_row = 32 * (warp & 3) + lane, a_col = ((lt >> 5) >> 2) * (KS / 2);      // a warp reaches the lanes of its quarter
     const uint64_t map_a = reinterpret_cast<uint64_t>(maps[blockIdx.x].a), map_b = reinterpret_cast<uint64_t>(maps[blockIdx.x].b);
     bool ok = true;
     auto issue = [&](int s) {       // one thread: both boxes of stage s
@@ -620,27 +626,45 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
       const int rs = s % RAW_SLOTS, ls = s % LO_SLOTS;
       if (!mbar_wait(rawfull_bar(rs), (s / RAW_SLOTS) & 1, status, 46)) break;
       if (s >= LO_SLOTS && !mbar_wait(lofree_bar(ls), ((s / LO_SLOTS) - 1) & 1, status, 45)) break;
-      const uint32_t hi = smem0 + rs * PART + so0, lo = lo0 + ls * PART + so0;
-      // all loads before the first store: one chunk at a time, each would wait for the one before
-      float4 v[8];
+      tc_fence_after();                          // the MMAs that read this slot of tensor memory are done
+      // A: a row per lane, half of the stage's columns per warp, into tensor memory; B: hi in place, lo into its ring.
+      // hi is rounded to nearest.  Leaving the raw word as hi (the MMA reads only its top 19 bits) was faster, but a
+      // truncated hi doubles |lo| and makes the dropped lo*lo term one-signed: on ill-conditioned factors the
+      // preconditioned gradient then misses the 1e-4 bound (3.7e-4 measured against 2e-4).
+      // All loads before the first store: one chunk at a time, each would wait for the one before.
+      const uint32_t ra = smem0 + rs * PART, hi = ra + OPB + so0, lo = lo0 + ls * OPB + so0;
+      float4 v[4], u[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t off = (uint32_t)(j & 3) * 4096u + (uint32_t)(j >> 2) * OPB;
-        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w) : "r"(hi + off));
+      for (int j = 0; j < 4; ++j)
+        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w) : "r"(ra + sw_off(a_row, a_col + 4 * j)));
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(u[j].x), "=f"(u[j].y), "=f"(u[j].z), "=f"(u[j].w) : "r"(hi + j * 4096u));
+      {
+        uint32_t h[16], l[16];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float x[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            h[4 * j + i] = rna_tf32(x[i]);
+            l[4 * j + i] = __float_as_uint(x[i] - __uint_as_float(h[4 * j + i]));
+          }
+        }
+        const uint32_t ta = tmem_base + ((uint32_t)(a_row & ~31) << 16) + TMEM_COLS + ls * 2 * KS + a_col;
+        tmem_st16(ta, h);
+        tmem_st16(ta + KS, l);
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t off = (uint32_t)(j & 3) * 4096u + (uint32_t)(j >> 2) * OPB;
-        // hi is rounded to nearest and written back in place.  Leaving the raw word as hi (the MMA
-        // reads only its top 19 bits) saves this store and 10-15 % of the kernel, but a truncated hi
-        // doubles |lo| and makes the dropped lo*lo term one-signed: on ill-conditioned factors the
-        // preconditioned gradient then misses the 1e-4 bound (3.7e-4 measured against 2e-4).
-        const uint32_t h0 = rna_tf32(v[j].x), h1 = rna_tf32(v[j].y), h2 = rna_tf32(v[j].z), h3 = rna_tf32(v[j].w);
-        const uint32_t l0 = __float_as_uint(v[j].x - __uint_as_float(h0)), l1 = __float_as_uint(v[j].y - __uint_as_float(h1));
-        const uint32_t l2 = __float_as_uint(v[j].z - __uint_as_float(h2)), l3 = __float_as_uint(v[j].w - __uint_as_float(h3));
-        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(hi + off), "r"(h0), "r"(h1), "r"(h2), "r"(h3) : "memory");
-        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(lo + off), "r"(l0), "r"(l1), "r"(l2), "r"(l3) : "memory");
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t h0 = rna_tf32(u[j].x), h1 = rna_tf32(u[j].y), h2 = rna_tf32(u[j].z), h3 = rna_tf32(u[j].w);
+        const uint32_t l0 = __float_as_uint(u[j].x - __uint_as_float(h0)), l1 = __float_as_uint(u[j].y - __uint_as_float(h1));
+        const uint32_t l2 = __float_as_uint(u[j].z - __uint_as_float(h2)), l3 = __float_as_uint(u[j].w - __uint_as_float(h3));
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(hi + j * 4096u), "r"(h0), "r"(h1), "r"(h2), "r"(h3) : "memory");
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(lo + j * 4096u), "r"(l0), "r"(l1), "r"(l2), "r"(l3) : "memory");
       }
+      tmem_st_wait();
+      tc_fence_before();
       fence_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(full_bar(ls));
@@ -651,7 +675,7 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
   if (warp == MMA_WARP) {
     __syncwarp();
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    tmem_dealloc(tmem_base, TS_COLS);
   }
 }
 
@@ -660,9 +684,10 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
 int engine_tc_set_wait_controls(long long cycles, int stall) { return tc::set_wait_controls(cycles, stall); }
 
 int launch_tile_tasks_tma(const sso_tile_task* tasks_dev, const void* maps_dev, int count, int* status_dev, cudaStream_t st) {
-  const size_t smem = (size_t)etc::KC_SMEM + 1024;
-  SSO_ENSURE_SMEM((etc::tile_task_tma_kernel<5, 2, 3>), smem);
-  etc::tile_task_tma_kernel<5, 2, 3><<<count, etc::THREADS, smem, st>>>(tasks_dev, reinterpret_cast<const etc::TaskMaps*>(maps_dev), status_dev);
+  constexpr int RAW = 5, LO = 3;
+  const size_t smem = (size_t)RAW * etc::PART + (size_t)LO * etc::OPB + 1024;
+  SSO_ENSURE_SMEM((etc::tile_task_tma_kernel<RAW, LO, 3>), smem);
+  etc::tile_task_tma_kernel<RAW, LO, 3><<<count, etc::THREADS, smem, st>>>(tasks_dev, reinterpret_cast<const etc::TaskMaps*>(maps_dev), status_dev);
   SSO_LAUNCH_OK("tile_task_tma_kernel");
   return 0;
 }

@@ -7,7 +7,7 @@
 // every FLUSH stages (the tensor core's own running sum truncates).  Two kernels:
 //
 // split_kernel writes the three parts of the input once, as pixel rows [part][pixel][C8] of 16-bit values with the
-// channels padded to a multiple of eight (a 1x1 window's ones column is one of them).  Every activation is converted
+// channels padded to a multiple of eight (the ones column of a 1x1 window without padding is one of them).  Every activation is converted
 // once instead of once per kernel position and tile, and whatever layout the input has (NCHW, odd channel counts,
 // unaligned rows) the gather sees 16-byte chunks of channels.  Bound: memory, 4 bytes in and 6 out per element.
 //
@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
   const bool ragged = last_n != 0 && bI == (p.d - 1) / 256, swapped = ragged && bI != bJ;
   const int col_a = (swapped ? bJ : bI) * (PAIR ? 256 : 128) + (int)rank * TILE;
   const int col_b = !ragged ? bJ * (PAIR ? 256 : 128) + (int)rank * TILE : rank == 0 ? bI * 256 : last_n == 128 ? bI * 256 + 64 : p.d + 255;
-  // 64-column blocks A0 A1 B0 B1 that hold columns of the matrix and are needed; a box leaves the ones column of a
-  // k x k window out (it has a block to itself, written once below)
+  // 64-column blocks A0 A1 B0 B1 that hold columns of the matrix and are needed; a box leaves a ones column
+  // that is not among the channels out (it has a block to itself, written once below)
   const int loaded_cols = BOX ? p.dcols : p.d;
   const bool share = bI == bJ && p.weight == nullptr && !ragged;
   const uint32_t used = share ? 3u : ragged ? 7u : 15u;
@@ -807,16 +807,19 @@ __global__ void __launch_bounds__(THREADS, 1) narrow_kernel(const FactorParams p
 // What a problem looks like to the gather: its channels padded (or folded) to c8, its factor of width d.
 struct Shape {
   int fold, c8, width, dcols, d, tiles, blocks;
+  bool plain;                // columns are the channels as they lie, the ones column one of them
   int64_t image_bytes;       // parts of one image
 };
 static Shape shape_of(const FactorParams& p) {
   Shape s;
   const int kk = p.kh * p.kw, ones = p.d - p.dcols;
+  // a row of a padded 1x1 window may lie outside the image, where every channel is zero and the ones column is not
+  s.plain = kk == 1 && (ones == 0 || (p.pad_h == 0 && p.pad_w == 0));
   s.fold = (p.c < 8 && p.kw > 1) ? p.kw : 0;
-  s.c8 = ceil_div(s.fold ? p.c * p.kw : p.c + (kk == 1 ? ones : 0), 8) * 8;
+  s.c8 = ceil_div(s.fold ? p.c * p.kw : p.c + (s.plain ? ones : 0), 8) * 8;
   s.width = s.fold ? p.wo : p.w;
-  s.dcols = kk == 1 ? p.d : s.c8 * (s.fold ? p.kh : kk);
-  s.d = kk == 1 ? p.d : s.dcols + ones;
+  s.dcols = s.plain ? p.d : s.c8 * (s.fold ? p.kh : kk);
+  s.d = s.plain ? p.d : s.dcols + ones;
   const int nb = ceil_div(s.d, 128), nb2 = ceil_div(s.d, 256);
   s.tiles = nb * (nb + 1) / 2;
   s.blocks = nb2 * (nb2 + 1) / 2;
@@ -827,7 +830,7 @@ static Shape shape_of(const FactorParams& p) {
 // stage is left to be cleared.  Every other geometry (strides, odd image sizes, per-sample weights, channel counts
 // below 64 columns of one kernel position) keeps the gather, which takes any.
 static bool choose_boxes(const FactorParams& p, const Shape& s, Boxes& b) {
-  if (p.weight || s.fold || p.stride_h != 1 || p.stride_w != 1 || (p.kh * p.kw > 1 && s.c8 % 64 != 0)) return false;
+  if (p.weight || s.fold || p.stride_h != 1 || p.stride_w != 1 || (!s.plain && s.c8 % 64 != 0)) return false;
   b.bw = std::gcd(p.wo, KS);
   b.bh = std::gcd(p.ho, KS / b.bw);
   b.bn = KS / (b.bw * b.bh);
@@ -938,14 +941,14 @@ int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, c
                                 pair ? 74 : 148, s.tiles, box ? 1.05 : pair ? 0.85 : 0.6, max_splits, rps);
   q.rows_per_split = rps;
   const int kk = p.kh * p.kw;
-  q.perm_c = kk > 1 ? s.c8 : 0;
+  q.perm_c = s.plain ? 0 : s.c8;
   q.perm_kk = kk;
-  q.perm_pub = kk > 1 ? p.c : 0;
+  q.perm_pub = s.plain ? 0 : p.c;
   q.perm_fold = s.fold;
   q.c = s.c8; q.dcols = s.dcols; q.d = s.d; q.w = s.width;
   q.sn = (int64_t)p.h * s.width * s.c8; q.sh = (int64_t)s.width * s.c8; q.sw = s.c8; q.sc = 1;
   if (s.fold) { q.kw = 1; q.stride_w = 1; q.pad_w = 0; q.dil_w = 1; }
-  const bool fused = kk == 1 && q.splits == 1;
+  const bool fused = s.plain && q.splits == 1;
   if (fused) boxes.narrow = 0;      // its tiles come out transposed, which the finishing in the kernel does not expect
   q.ticket_tiles = s.tiles;
   const bool direct = !s.fold && p.sc == 1 && p.c % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 && p.sn % 4 == 0 &&
@@ -958,7 +961,7 @@ int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, c
     in.status = q.status;
     in.weight = p.weight ? p.weight + n0 : nullptr;
     const int64_t pixels = (int64_t)n * p.h * s.width;
-    const int ones_at = kk == 1 && p.d > p.dcols ? p.c : -1;
+    const int ones_at = s.plain && p.d > p.dcols ? p.c : -1;
     if (direct)
       f32::split_direct_kernel<<<(unsigned)ceil_div64(pixels * (s.c8 / 8), 256), 256, 0, st>>>(in, (uint32_t)pixels, ones_at,
                                                                                                             r == 0 ? header_words : 0, parts, parts);

@@ -108,6 +108,22 @@ def test_factor_f32_conv(nat, cfg, channels_last):
     assert torch.equal(out, out.t())
 
 
+@pytest.mark.parametrize('n,c,h,w,stride,pad', [(2, 3, 5, 5, (1, 1), (1, 1)), (5, 20, 9, 9, (1, 1), (1, 1)), (3, 40, 7, 7, (2, 2), (1, 0)),
+                                                (4, 200, 6, 7, (1, 1), (2, 1)), (8, 100, 6, 6, (1, 1), (1, 1)), (16, 192, 6, 6, (1, 1), (1, 1)),
+                                                (16, 256, 6, 6, (1, 1), (1, 1)), (4, 127, 30, 30, (1, 1), (1, 1))])
+@pytest.mark.parametrize('channels_last', [False, True])
+def test_factor_f32_padded_1x1_with_bias(nat, n, c, h, w, stride, pad, channels_last):
+    """Rows in the padding are zero but for the ones column: one tile, gathered pairs, boxes, a narrow last block row."""
+    x = torch.randn(n, c, h, w, device='cuda') + 0.25
+    x = x.contiguous(memory_format=torch.channels_last) if channels_last else x
+    for weight in (None, torch.rand(n, device='cuda')):
+        ref = conv_ref(x, (1, 1), stride, pad, (1, 1), True, weight)
+        out = torch.full_like(ref, float('nan'), dtype=torch.float32)
+        nat.factor_im2col(x, (1, 1), stride, pad, (1, 1), True, weight, 0.5, 0.0, out)
+        assert rel(out, 0.5 * ref) < 1e-6 and torch.equal(out, out.t())
+        assert rel(out[c], 0.5 * ref[c]) < 1e-5
+
+
 @pytest.mark.parametrize('rows,cols,bias', [(1, 1, False), (31, 5, True), (129, 63, True), (700, 64, False), (5000, 64, True), (33000, 128, False),
                                             (20001, 97, True), (40000, 13, False), (257, 300, True), (256, 300, True), (1024, 1021, False), (256, 272, False), (288, 264, True), (512, 384, False), (128, 511, True), (320, 520, True), (1500, 1021, True), (33, 4100, False)])
 @pytest.mark.parametrize('layout', ['rows', 'strided', 'columns'])

@@ -361,12 +361,15 @@ class SecondOrderOptimizer(Optimizer):
     def _fused_tail(self, groups, target, stage):
         """torchsso/optim/secondorder.py:225-283 for all eligible groups in one kernel launch.
         Returns the ids of the groups it handled.  The device table (addresses) and the sets of scalars are
-        kept: the table until a tensor moves, the scalars until a setting changes."""
+        kept: the table while every address and layout in it is still the one that a group's tensors and buffers
+        have, the scalars until a setting changes."""
         raw = stage == 'raw'
+        if raw and not any(g['l2_reg'] != 0 or (g['momentum_type'] == stage and g['momentum'] != 0) or
+                           (g['grad_ema_type'] == stage and g['grad_ema_decay'] != 1) for g in groups):
+            return {id(g) for g in groups if not g['lars']}      # nothing to apply at this stage
         cache = self.__dict__.setdefault('_tail_tables', {})
         ent = cache.get((target, stage))
-        params = [p for g in groups for p in g[target]]
-        key = ([p.data_ptr() for p in params], [id(p.grad) for p in params], [_TAIL_SETTINGS(g) for g in groups], id(self.state))
+        key = self._tail_key(groups, target, stage)
         if ent is None or ent['key'] != key or ent['per_step']:
             ent = cache[(target, stage)] = self._tail_entry(groups, target, raw, key, ent)
         for curv, l2 in ent['l2']:
@@ -374,6 +377,28 @@ class SecondOrderOptimizer(Optimizer):
         if ent['table'] is not None:
             nat.optimizer_tail_sets(ent['table'], ent['sets'])
         return ent['handled']
+
+    def _tail_key(self, groups, target, stage):
+        """Everything a table is built from: the groups, their settings, and of every tensor and buffer that the
+        kernel touches the address and layout as they are now."""
+        state, key = self.state, []
+        for g in groups:
+            key.append((id(g), id(g['curv']), _TAIL_SETTINGS(g)))
+            if g['lars']:
+                continue
+            use_m = g['momentum_type'] == stage and g['momentum'] != 0
+            use_e = g['grad_ema_type'] == stage and g['grad_ema_decay'] != 1
+            for p in g[target]:
+                grad = p.grad
+                if grad is None:
+                    key.append(None)
+                    continue
+                key.append((p.data_ptr(), p.numel(), p.dtype, p.is_contiguous(), grad.data_ptr(), grad.dtype, grad.is_contiguous()))
+                if use_m:
+                    key.append(state[p]['momentum_buffer'].data_ptr())
+                if use_e:
+                    key.append(state[p]['grad_ema_buffer'].data_ptr())
+        return key
 
     def _tail_entry(self, groups, target, raw, key, old):
         stage = 'raw' if raw else 'preconditioned'
@@ -412,12 +437,13 @@ class SecondOrderOptimizer(Optimizer):
                 st = self.state[p]
                 items.append((p.data, p.grad, st['momentum_buffer'] if use_m else None,
                               st['grad_ema_buffer'] if use_e else None, index))
-                rows.append((p.data_ptr(), p.grad.data_ptr(), *[0 if b is None else b.data_ptr() for b in items[-1][2:4]], index))
+                rows.append((p.data_ptr(), p.numel(), p.grad.data_ptr(), *[0 if b is None else b.data_ptr() for b in items[-1][2:4]], index))
         table = None
         if items:
             table = old['table'] if old is not None and old['rows'] == rows else nat.tail_set_records(items, items[0][0].device)
-        # the gradients are kept: their ids are part of the key
-        return {'key': key, 'grads': [it[1] for it in items], 'per_step': per_step, 'handled': handled, 'l2': l2, 'rows': rows,
+        # what the key names by id or address is kept, so that none of it can become another object's
+        held = (list(groups), [g['curv'] for g in groups], items)
+        return {'key': key, 'held': held, 'per_step': per_step, 'handled': handled, 'l2': l2, 'rows': rows,
                 'table': table, 'sets': nat.tail_sets(sets) if sets else None}
 
     def _split_groups(self, groups):

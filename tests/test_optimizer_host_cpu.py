@@ -1,0 +1,97 @@
+"""Host side of the optimizers without a device: what is kept between steps must follow the groups, tensors and
+buffers that the next step finds."""
+import collections
+
+import pytest
+import torch
+import torch.nn as nn
+
+import torchsso
+from torchsso import _native as nat
+
+SHAPES = {'Linear': 'Kron'}
+
+
+def make(seed=0, **kwargs):
+    torch.manual_seed(seed)
+    model = nn.Sequential(nn.Linear(5, 7), nn.Tanh(), nn.Linear(7, 3))
+    kwargs = {'lr': 0.1, 'momentum': 0.9, 'weight_decay': 0.01, **kwargs}
+    return torchsso.optim.SecondOrderOptimizer(model, 'Cov', SHAPES, {'damping': 1e-2}, **kwargs)
+
+
+@pytest.fixture
+def kernel(monkeypatch):
+    """The update kernel on tensors in place of addresses: a table holds on to what it was built from."""
+    def run(table, sets):
+        for p, g, m, e, i in table:
+            add, mom, ema, scale, lr = sets[i]
+            v = g + add * p
+            if m is not None:
+                v = m.copy_(mom * m + v)
+            if e is not None:
+                v = e.copy_(ema * v + (1 - ema) * e)
+            g.copy_(scale * v)
+            p.sub_(lr * g)
+    monkeypatch.setattr(nat, 'tail_set_records', lambda items, device: list(items))
+    monkeypatch.setattr(nat, 'tail_sets', list)
+    monkeypatch.setattr(nat, 'optimizer_tail_sets', run)
+
+
+def step(opt, seed, fused=True):
+    opt._curvature_step = lambda *a: None
+    if not fused:
+        opt._fused_tail = lambda *a: set()
+    g = torch.Generator().manual_seed(seed)
+    for group in opt.param_groups:
+        for p in group['params']:
+            p.grad = torch.randn(p.shape, generator=g)
+    opt._harvest_grads()
+    opt._update_groups(opt.param_groups, 'params', False, None)
+
+
+def reset_buffers(opt):
+    for group in opt.param_groups:
+        opt.init_buffer(group['params'])
+
+
+def rebind_one(opt):
+    p = opt.param_groups[0]['params'][0]
+    opt.state[p]['momentum_buffer'] = torch.ones_like(p)
+
+
+def new_state(opt):
+    for _ in range(3):          # more than once: a state may come to lie where one before it was
+        opt.state = collections.defaultdict(dict)
+        reset_buffers(opt)
+
+
+def copied_groups(opt):
+    opt.param_groups[:] = [dict(g) for g in opt.param_groups]
+
+
+def other_layout(opt):
+    p = opt.param_groups[0]['params'][0]      # same address, another order of its elements
+    p.data = p.data.view(p.shape[1], p.shape[0]).t()
+
+
+def other_curvature(opt):
+    opt.param_groups[0]['curv'] = None
+
+
+@pytest.mark.parametrize('kwargs', [{}, {'l2_reg': 0.1, 'momentum_type': 'raw', 'grad_ema_decay': 0.3}])
+@pytest.mark.parametrize('change', [reset_buffers, rebind_one, new_state, copied_groups, other_layout, other_curvature])
+def test_update_table_follows_what_changed(kernel, kwargs, change):
+    got, want = make(**kwargs), make(**kwargs)
+    for i in range(4):
+        if i == 2:
+            change(got)
+            change(want)
+        step(got, i)
+        step(want, i, fused=False)
+    for a, b in zip(got.param_groups, want.param_groups):
+        for p, q in zip(a['params'], b['params']):
+            torch.testing.assert_close(p, q, rtol=1e-5, atol=1e-6)
+            for name in ('momentum_buffer', 'grad_ema_buffer'):
+                torch.testing.assert_close(got.state[p][name], want.state[q][name], rtol=1e-5, atol=1e-6)
+        if a['curv'] is not None:
+            assert a['curv'].l2_reg == b['curv'].l2_reg

@@ -447,16 +447,18 @@ class SecondOrderOptimizer(Optimizer):
                 'table': table, 'sets': nat.tail_sets(sets) if sets else None}
 
     def _split_groups(self, groups):
-        """What never changes about a list of groups: its pooled curvatures by kind and the gradient views of
-        the Kronecker layers."""
+        """A list of groups by the kind of their curvatures, and the gradient views of the Kronecker layers: kept
+        until a group's curvature, how it is stored, or its parameters change."""
+        key = [(id(g), id(g['curv']), getattr(g['curv'], 'use_max_ema', None), *map(id, g['params'])) for g in groups]
         ent = self.__dict__.get('_split')
-        if ent is None or ent[0] is not groups or ent[1] != len(groups):
+        if ent is None or ent[0] != key:
             pooled = [g for g in groups if g['curv'] is not None and _is_pooled(g['curv'])]
             kron = [g for g in pooled if isinstance(g['curv'], _KronFactors)]
             diag = [g for g in pooled if isinstance(g['curv'], DiagCurvature)]
             rest = [g for g in groups if g['curv'] is not None and not _is_pooled(g['curv'])]
             grads = [[self._grad_view[p] for p in g['params']] for g in kron]
-            ent = self.__dict__['_split'] = (groups, len(groups), [g['curv'] for g in pooled], kron, diag, rest, grads,
+            held = [(g, g['curv'], list(g['params'])) for g in groups]      # no id in the key may become another object's
+            ent = self.__dict__['_split'] = (key, held, [g['curv'] for g in pooled], kron, diag, rest, grads,
                                              [g['curv'] for g in kron], [g['curv'] for g in diag])
         return ent[2:]
 

@@ -95,3 +95,41 @@ def test_update_table_follows_what_changed(kernel, kwargs, change):
                 torch.testing.assert_close(got.state[p][name], want.state[q][name], rtol=1e-5, atol=1e-6)
         if a['curv'] is not None:
             assert a['curv'].l2_reg == b['curv'].l2_reg
+
+
+class Recorder:
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        return lambda *args, **kwargs: self.calls.append((name, *args))
+
+    def given(self, name):
+        return [c[1] for c in self.calls if c[0] == name]
+
+
+def curvature_step(opt, monkeypatch):
+    """(curvatures whose inverses the pool refreshes, those it preconditions with, those that step by themselves)."""
+    opt.pool, alone = Recorder(), []
+    monkeypatch.setattr(torchsso.KronCovLinear, 'step', lambda self, **kw: alone.append(self))
+    monkeypatch.setattr(torchsso.KronCovLinear, 'precondition_grad', lambda self, params: None)
+    opt._curvature_step(opt.param_groups, 'params', True, None)
+    inverted = sum(opt.pool.given('update_inv'), [])
+    return inverted, sum(opt.pool.given('precondition'), []), alone
+
+
+def test_curvature_step_follows_what_changed(monkeypatch):
+    opt = make()
+    first, second = (g['curv'] for g in opt.param_groups)
+    assert curvature_step(opt, monkeypatch) == ([first, second], [first, second], [])
+    second.use_max_ema = True               # the pool does not keep running maxima
+    assert curvature_step(opt, monkeypatch) == ([first], [first], [second])
+    second.use_max_ema = False
+    assert curvature_step(opt, monkeypatch) == ([first, second], [first, second], [])
+    opt.param_groups[0]['curv'] = None
+    assert curvature_step(opt, monkeypatch) == ([second], [second], [])
+    opt.param_groups[0]['curv'] = first
+    opt.param_groups[0]['params'] = opt.param_groups[0]['params'][:1]
+    curvature_step(opt, monkeypatch)
+    grads = next(c[2] for c in opt.pool.calls if c[0] == 'precondition')
+    assert [len(g) for g in grads] == [1, 2]

@@ -43,7 +43,7 @@ static int apply_wait_controls() {
   const long long cycles = g_wait_kcycles * 1024;
   int rc = factor_tma_set_wait_controls(cycles, g_stall);
   if (!rc) rc = factor_tc_set_wait_controls(cycles, 0);
-  if (!rc) rc = factor_f32_set_wait_controls(cycles, 0);
+  if (!rc) rc = factor_f32_set_wait_controls(cycles, g_stall);
   if (!rc) rc = flow_set_wait_controls(cycles, g_stall);
   if (!rc) rc = engine_tc_set_wait_controls(cycles, g_stall);
   return rc;

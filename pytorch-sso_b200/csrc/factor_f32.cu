@@ -481,7 +481,8 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
         const int first_box = (int)(r_begin / KS), per_image = boxes.across * boxes.down;
         int n = first_box / per_image, iy = (first_box - n * per_image) / boxes.across;
         int ix = first_box - n * per_image - iy * boxes.across;
-        for (int s = 0; s < nstages; ++s) {
+        int s = 0;
+        for (; s < nstages; ++s) {
           const int slot = s % STAGES;
           if (s >= STAGES && !mbar_wait(empty_bar(slot), ((s / STAGES) - 1) & 1, status, 64)) break;
           const uint32_t fb = fulls + 8u * slot;
@@ -499,6 +500,8 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
           if (rank != 0) mbar_arrive_cluster(fb);
           if (++ix == boxes.across) { ix = 0; if (++iy == boxes.down) { iy = 0; ++n; } }
         }
+        // the copies of both CTAs complete on the leader's barriers, and the cluster leaves together
+        if (rank == 0) ring_landed<STAGES>(s, full_bar, status, 65);
       }
       __syncwarp();
       asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");
@@ -513,7 +516,7 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
     const bool no_halo = p.kh == 1 && p.kw == 1 && p.pad_h == 0 && p.pad_w == 0;
     const int step_n = KS / (p.ho * p.wo), step_rem = KS - step_n * (p.ho * p.wo);
     const int step_y = step_rem / p.wo, step_x = step_rem - step_y * p.wo;
-    for (int s = 0; s < nstages + LAG; ++s) {
+    for (int s = g_inject_stall ? nstages + LAG : 0; s < nstages + LAG; ++s) {      // stalled: nothing is loaded or handed over
       // a stage is handed over before the wait for the next free slot, which depends on an MMA further back
       if (s >= LAG) {
         asm volatile("cp.async.wait_group %0;" ::"n"(LAG - 1) : "memory");
@@ -757,7 +760,7 @@ __global__ void __launch_bounds__(THREADS, 1) narrow_kernel(const FactorParams p
       if (s < nstages) load(s);
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    for (int s = 0; s < nstages; ++s) {
+    for (int s = g_inject_stall ? nstages : 0; s < nstages; ++s) {      // stalled: no stage is handed over
       if (s + RAW - 1 < nstages) load(s + RAW - 1);
       asm volatile("cp.async.commit_group;" ::: "memory");
       asm volatile("cp.async.wait_group %0;" ::"n"(RAW - 1) : "memory");

@@ -56,6 +56,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
   }
   return true;
 }
+// Bounded wait for the last bulk copies of a ring of SLOTS stages, by the thread that issued `issued` of them: when a wait
+// gave up, nobody else may have waited for these, and they must not land in shared memory that has been given back.
+template <int SLOTS, typename Bar>
+__device__ __forceinline__ void ring_landed(int issued, Bar full_bar, int* status, int code) {
+  for (int s = issued > SLOTS ? issued - SLOTS : 0; s < issued; ++s) mbar_wait(full_bar(s % SLOTS), (s / SLOTS) & 1, status, code);
+}
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }

@@ -51,6 +51,28 @@ def test_factor_kernel_wait_runs_out(nat, channels):
     assert int(ws[:4].view(torch.int32).item()) == 0
 
 
+@pytest.mark.parametrize('n,c,size,k,pad', [(3, 64, 8, 3, 1), (4, 256, 8, 1, 0),      # boxes; finished in the kernel
+                                            (2, 26, 13, 5, 2), (16, 130, 5, 1, 0),    # gathered by pairs
+                                            (4, 7, 10, 3, 1), (40, 33, 6, 1, 0)])     # one CTA; rows of at most 128 columns
+def test_fp32_factor_kernel_wait_runs_out(nat, n, c, size, k, pad):
+    x = cases.make_normal((n, c, size, size), 5).cuda().contiguous(memory_format=torch.channels_last)
+    geo = ((k, k), (1, 1), (pad, pad), (1, 1))
+    d = c * k * k
+    out = torch.zeros((d, d), device='cuda')
+    nat.configure('wait_kcycles', 2000)
+    nat.configure('inject_stall', 1)
+    nat.factor_im2col(x, *geo, False, None, 1.0 / n, 0.0, out, impl=nat.IMPL_TCGEN05)
+    torch.cuda.synchronize()
+    ws = nat._workspaces[('cuda', x.device.index)]
+    assert int(ws[:4].view(torch.int32).item()) != 0
+    assert bool(torch.isnan(out).all())
+    nat.configure('inject_stall', 0)
+    nat.configure('wait_kcycles', 0)
+    nat.factor_im2col(x, *geo, False, None, 1.0 / n, 0.0, out, impl=nat.IMPL_TCGEN05)
+    assert _rel(out, ko.conv_factor_A(x.double().cpu(), *geo, False)) < 1e-5
+    assert int(ws[:4].view(torch.int32).item()) == 0
+
+
 def test_batched_factor_kernel_wait_runs_out(nat):
     """The persistent kernel of sso_factor_batch: with its producers stalled, every role's wait runs out,
     the kernel returns, and the finishing kernel writes NaN for every problem of the batch."""

@@ -608,9 +608,12 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
     const int a_row = 32 * (warp & 3) + lane, a_col = ((lt >> 5) >> 2) * (KS / 2);      // a warp reaches the lanes of its quarter
     const uint64_t map_a = reinterpret_cast<uint64_t>(maps[blockIdx.x].a), map_b = reinterpret_cast<uint64_t>(maps[blockIdx.x].b);
     bool ok = true;
+    int issued = 0;
     auto issue = [&](int s) {       // one thread: both boxes of stage s
       const int rs = s % RAW_SLOTS;
-      if (s >= RAW_SLOTS && !mbar_wait(rawfree_bar(rs), ((s / RAW_SLOTS) - 1) & 1, status, 44)) { ok = false; return; }
+      ok = ok && (s < RAW_SLOTS || mbar_wait(rawfree_bar(rs), ((s / RAW_SLOTS) - 1) & 1, status, 44));
+      if (!ok) return;
+      issued = s + 1;
       const uint32_t fb = rawfull_bar(rs), dst = smem0 + rs * PART;
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(PART) : "memory");
       asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -669,6 +672,7 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
       __syncwarp();
       if (lane == 0) mbar_arrive(full_bar(ls));
     }
+    if (producer) ring_landed<RAW_SLOTS>(issued, rawfull_bar, status, 47);
   }
   tc_fence_before();
   __syncthreads();

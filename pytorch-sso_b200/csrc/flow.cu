@@ -119,9 +119,11 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
   __shared__ uint32_t tmem_base_slot;
   __shared__ Task queue[QUEUE];
   __shared__ volatile int dead;          // a wait of this CTA gave up
-  // for that case: queue entries pushed, the first one not finished, a task taken but not pushed, stages loaded
+  // for that case: queue entries pushed, the first one not finished, stages loaded; the task that the accumulate warps
+  // left (they release its entry when they take it, so that another may lie there by now), one taken but not pushed
   __shared__ volatile uint32_t pushed, acc_at, issued;
-  __shared__ Task lost;
+  __shared__ volatile uint32_t gave_up;  // first queue entry at which one of the accumulate warps gave up
+  __shared__ Task left, lost;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t lo0 = smem0 + RAW * PART;
@@ -142,7 +144,8 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     dead = 0;
     pushed = acc_at = issued = 0;
-    lost.kind = -1;
+    gave_up = 0xffffffffu;
+    left.kind = lost.kind = -1;
   }
   if (warp == MMA_WARP) tmem_alloc(smem_u32(&tmem_base_slot), 256);
   tc_fence_before();
@@ -326,9 +329,21 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
     uint32_t n = 0;
     bool ok = true;
     for (;; ++n) {
+      // Barriers have no limit, so the eight warps leave a task together: a wait may run out for one of them and just not
+      // for another.  Each passes all_well once per task, whatever happens, and reads the same answer behind it (a warp
+      // that is already at the next task may have given up there).
+      auto all_well = [&]() {
+        dpanel::sync_x();
+        return gave_up > n;
+      };
+      auto fail = [&]() {
+        gave_up = n;
+        all_well();
+        ok = false;
+      };
       Task t;
-      if (!take(n, t)) { ok = false; break; }
-      if (t.kind < 0) break;
+      if (!take(n, t)) { fail(); break; }
+      if (t.kind < 0) { ok = all_well(); break; }
       const Mat& m = g.mats[t.mat];
       const int d = m.d;
       const Shape sh = shape_of(t, d);
@@ -381,8 +396,11 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         }
         return true;
       };
-      ok = drain(ceil_div(sh.n1, FLUSH), t.kind == PROD ? 1.f : -1.f);
-      if (!ok) break;
+      auto leave = [&]() {
+        if (lane == 0) left = t;
+        ok = false;
+      };
+      if (!drain(ceil_div(sh.n1, FLUSH), t.kind == PROD ? 1.f : -1.f)) { fail(); leave(); break; }
       stage += sh.n1;
       if (sh.n2) {
         // the sum becomes the A operand of four more stages: 64 columns = two of them (every MMA that read these
@@ -398,8 +416,7 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         stage += sh.n2;
 #pragma unroll
         for (int i = 0; i < 64; ++i) acc[i] = 0.f;
-        ok = drain(ceil_div(sh.n2, FLUSH), 1.f);
-        if (!ok) break;
+        if (!drain(ceil_div(sh.n2, FLUSH), 1.f)) { fail(); leave(); break; }
       }
       const int nr = min(TILE, d - r0), nc = min(TILE, d - c0);
       // rows of `out` (tile origin o) along lanes, through 32 columns of this warp's staging tile at a time
@@ -453,20 +470,23 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         }
       };
       int* flag = nullptr;
-      if (t.kind == PANEL) {
-        store_boxes();
-        if (m.U) {
-          store_columns(m.U + (int64_t)c0 * m.ldu + r0, m.ldu, false);
-          for (int rr = warp; rr < nr; rr += ACC_WARPS)
-            for (int c = lane; c < nc; c += 32) m.U[(int64_t)(r0 + rr) * m.ldu + c0 + c] = 0.f;
+      if (t.kind != DIAG) {
+        if (t.kind == PANEL) {
+          store_boxes();
+          if (m.U) {
+            store_columns(m.U + (int64_t)c0 * m.ldu + r0, m.ldu, false);
+            for (int rr = warp; rr < nr; rr += ACC_WARPS)
+              for (int c = lane; c < nc; c += 32) m.U[(int64_t)(r0 + rr) * m.ldu + c0 + c] = 0.f;
+          }
+          flag = g.flags + m.flag_w + t.a * m.np + t.b;
+        } else if (t.kind == INVT) {
+          store_boxes();
+          flag = g.flags + m.flag_x + t.a * m.np + t.b;
+        } else {
+          store_rows(m.T + (int64_t)r0 * m.ldt + c0, m.ldt, t.a == t.b);
+          store_columns(m.T + (int64_t)c0 * m.ldt + r0, m.ldt, t.a == t.b);
         }
-        flag = g.flags + m.flag_w + t.a * m.np + t.b;
-      } else if (t.kind == INVT) {
-        store_boxes();
-        flag = g.flags + m.flag_x + t.a * m.np + t.b;
-      } else if (t.kind == PROD) {
-        store_rows(m.T + (int64_t)r0 * m.ldt + c0, m.ldt, t.a == t.b);
-        store_columns(m.T + (int64_t)c0 * m.ldt + r0, m.ldt, t.a == t.b);
+        if (!all_well()) { leave(); break; }      // and the tile is stored by all eight warps
       } else {
         // ---------------------------------------------------------------- diagonal block, in the operand ring
         float* S = ring;
@@ -478,7 +498,7 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
 #pragma unroll
           for (int i = 0; i < 64; ++i) S[row * dpanel::PP + col0 + i] = col0 + i == row ? 1.f : 0.f;
         }
-        dpanel::sync_x();
+        if (!all_well()) { leave(); break; }
         dpanel::factor_block(S, V, nr, g.info ? g.info + 2 * m.mat + m.info_slot : nullptr, r0, tid);
         float* li = m.Li + (int64_t)t.a * (TILE * TILE);
         for (int e = tid; e < TILE * TILE / 4; e += 256) {
@@ -503,13 +523,11 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         fence_async_smem();                      // the ring goes back to TMA
         __syncwarp();
         if (lane == 0) mbar_arrive(ddone);
+        if (flag) dpanel::sync_x();
       }
-      if (flag) {
-        dpanel::sync_x();                        // the tile is stored by all eight warps
-        if (tid == 0) {
-          __threadfence();
-          store_release(flag, epoch);
-        }
+      if (flag && tid == 0) {
+        __threadfence();
+        store_release(flag, epoch);
       }
     }
     if (!ok) dead = 1;
@@ -552,7 +570,8 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
       else if (m.X) store_release(g.flags + m.flag_x + t.a * m.np + (t.kind == DIAG ? t.a : t.b), epoch);
     }
   };
-  for (uint32_t n = acc_at; n < pushed; ++n)
+  if (left.kind >= 0) poison(left);
+  for (uint32_t n = acc_at + (left.kind >= 0 ? 1 : 0); n < pushed; ++n)
     if (queue[n % QUEUE].kind >= 0) poison(queue[n % QUEUE]);
   if (lost.kind >= 0) poison(lost);
   for (;;) {

@@ -157,3 +157,25 @@ def test_pool_check_info_reports_a_wait_that_gave_up(nat):
         nat.configure('wait_kcycles', 0)
     with pytest.raises(RuntimeError, match='wait of the inverse plan gave up'):
         curv.pool.check_info()
+
+
+def test_inverse_of_many_small_matrices_wait_runs_out(nat):
+    """Tasks of one stage: by the time the waits run out, the queue entry of the task that was being worked on has
+    been used again.  Every inverse is NaN, none keeps what was in it."""
+    n, d = 600, 8
+    src = [cases.make_normal((2 * d, d), i) for i in range(n)]
+    src = [(x.t() @ x / x.shape[0]).cuda() for x in src]
+    dst = [torch.full((d, d), 7.0, device='cuda') for _ in range(n)]
+    plan = nat.kron_plan([d] * n, src, dst, None, None, [-1] * n, [0] * n, torch.device('cuda'))
+    damp = torch.full((n,), 0.1, device='cuda')
+    info = torch.zeros(2 * n, dtype=torch.int32, device='cuda')
+    nat.configure('wait_kcycles', 2000)
+    nat.configure('inject_stall', 1)
+    try:
+        nat.kron_plan_run(plan, damp, info, True, False)
+        torch.cuda.synchronize()
+    finally:
+        nat.configure('inject_stall', 0)
+        nat.configure('wait_kcycles', 0)
+    assert plan.status() != 0 and int(info[0]) == -(1000 + plan.status())
+    assert bool(torch.isnan(torch.stack(dst)).all())

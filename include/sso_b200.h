@@ -104,12 +104,13 @@ typedef struct {
   float* out;
   int64_t ldo;
 } sso_factor_desc;
-/* One sso_factor_syrk_im2col call with everything that does not change between calls given once: the
- * description's x may be null, its sample_weight, alpha and beta are ignored.  The handle belongs to the
- * host only (no device memory); run it with scratch of sso_factor_workspace_bytes bytes. */
 /* Scratch with which the described problem runs at its best: fp32 inputs are split into 16-bit parts that pass
  * through the scratch, and with the sso_factor_workspace_bytes minimum they do so in smaller pieces. */
 size_t sso_factor_desc_workspace_bytes(const sso_factor_desc* desc, int impl);
+/* One sso_factor_syrk_im2col call with everything that does not change between calls given once: the
+ * description's x may be null, its sample_weight, alpha and beta are ignored.  The handle belongs to the
+ * host only (no device memory); run it with scratch of sso_factor_workspace_bytes bytes.  A handle that has been
+ * destroyed or was never given out is refused. */
 int64_t sso_factor_op_create(const sso_factor_desc* desc, int impl);
 int sso_factor_op_run(int64_t op, const void* x, const float* sample_weight, float alpha, float beta, void* workspace,
                       size_t workspace_bytes, void* stream);

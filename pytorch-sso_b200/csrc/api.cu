@@ -11,6 +11,7 @@ unsigned long long g_launches = 0;
 
 #include <algorithm>
 #include <map>
+#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -193,6 +194,9 @@ struct PreparedFactor {
   FactorParams p;
   int dtype, impl;
 };
+static std::mutex g_ops_mu;
+static std::unordered_map<int64_t, PreparedFactor> g_ops;
+static int64_t g_next_op = 1;
 
 static int desc_params(const sso_factor_desc& q, FactorParams& p) {
   const float dummy = 0.f;      // descriptions of prepared calls carry no input
@@ -212,21 +216,29 @@ int64_t sso_factor_op_create(const sso_factor_desc* q, int impl) {
   const int rc = desc_params(*q, f.p);
   if (rc) return rc;
   f.dtype = q->dtype; f.impl = impl;
-  return reinterpret_cast<int64_t>(new PreparedFactor(f));
+  std::lock_guard<std::mutex> lk(g_ops_mu);
+  g_ops.emplace(g_next_op, f);
+  return g_next_op++;
 }
 
 int sso_factor_op_destroy(int64_t op) {
-  delete reinterpret_cast<PreparedFactor*>(op);
+  std::lock_guard<std::mutex> lk(g_ops_mu);
+  SSO_CHECK_ARG(g_ops.erase(op) == 1, "factor op: unknown handle %lld", (long long)op);
   return 0;
 }
 
 int sso_factor_op_run(int64_t op, const void* x, const float* sample_weight, float alpha, float beta, void* workspace,
                       size_t workspace_bytes, void* stream) {
-  SSO_CHECK_ARG(op > 0 && x != nullptr, "factor op: null argument");
-  const PreparedFactor* f = reinterpret_cast<const PreparedFactor*>(op);
-  FactorParams p = f->p;
-  p.x = x; p.weight = sample_weight; p.alpha = alpha; p.beta = beta;
-  return launch_one_factor(p, f->dtype, workspace, workspace_bytes, f->impl, reinterpret_cast<cudaStream_t>(stream));
+  SSO_CHECK_ARG(x != nullptr, "factor op: null argument");
+  PreparedFactor f;      // a copy: another thread may destroy the handle meanwhile
+  {
+    std::lock_guard<std::mutex> lk(g_ops_mu);
+    auto it = g_ops.find(op);
+    SSO_CHECK_ARG(it != g_ops.end(), "factor op: unknown handle %lld", (long long)op);
+    f = it->second;
+  }
+  f.p.x = x; f.p.weight = sample_weight; f.p.alpha = alpha; f.p.beta = beta;
+  return launch_one_factor(f.p, f.dtype, workspace, workspace_bytes, f.impl, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // ---- many factors in one call ----------------------------------------------------------------

@@ -1,0 +1,37 @@
+"""Entry points of the library that answer without a device: handles and argument checks."""
+import ctypes as C
+
+import pytest
+
+from torchsso import _native as nat
+
+
+def description(**kwargs):
+    d = nat.FactorDesc()
+    d.n, d.c, d.h, d.w, d.sn, d.sc = 4, 8, 1, 1, 8, 1
+    d.kh = d.kw = d.stride_h = d.stride_w = d.dil_h = d.dil_w = 1
+    d.out, d.ldo = 4096, 8
+    for k, v in kwargs.items():
+        setattr(d, k, v)
+    return d
+
+
+def test_factor_op_handles():
+    lib = nat.lib()
+
+    def refused(rc):
+        return rc == -1 and b'unknown handle' in lib.sso_last_error()
+    d = description()
+    a, b = (lib.sso_factor_op_create(C.byref(d), 0) for _ in range(2))
+    assert a > 0 and b > 0 and a != b
+    assert lib.sso_factor_op_run(a, None, None, 1.0, 0.0, None, 0, None) == -1      # no input
+    assert lib.sso_factor_op_destroy(a) == 0
+    for h in (a, 0, -5, b + 1000, 1 << 62):          # destroyed, or never given out
+        assert refused(lib.sso_factor_op_run(h, 4096, None, 1.0, 0.0, None, 0, None))
+        assert refused(lib.sso_factor_op_destroy(h))
+    assert lib.sso_factor_op_destroy(b) == 0
+
+
+@pytest.mark.parametrize('bad', [{'n': 0}, {'kh': 0}, {'ldo': 7}, {'out': None}, {'kw': 2}])
+def test_factor_op_refuses_a_bad_description(bad):
+    assert nat.lib().sso_factor_op_create(C.byref(description(**bad)), 0) < 0

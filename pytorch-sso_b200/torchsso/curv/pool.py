@@ -46,6 +46,7 @@ class FactorPool:
         self.device = torch.device(device)
         self._kron = [weakref.ref(c) for c in kron]      # the curvatures hold their pool
         self._diag = [weakref.ref(c) for c in diag]
+        self._k_ids, self._d_ids = [id(c) for c in kron], [id(c) for c in diag]      # layout order, whoever is left
         self._bufs: Dict[str, torch.Tensor] = {}
         # --- Kronecker layout: [A_0 | G_0 | A_1 | G_1 | ...]
         self.k_off = {}
@@ -78,11 +79,11 @@ class FactorPool:
 
     @property
     def kron(self) -> List:
-        return [r() for r in self._kron]
+        return [c for c in (r() for r in self._kron) if c is not None]
 
     @property
     def diag(self) -> List:
-        return [r() for r in self._diag]
+        return [c for c in (r() for r in self._diag) if c is not None]
 
     # ------------------------------------------------------------------ storage
     def buf(self, role: str, kind: str = 'k') -> torch.Tensor:
@@ -130,51 +131,44 @@ class FactorPool:
         return self._remembered('k', curvs, self._find_kron_range) if curvs else (0, 0)
 
     def _find_kron_range(self, curvs):
-        kron = self.kron
-        idx = sorted(kron.index(c) for c in curvs)
+        first, last = self._places(self._k_ids, curvs)
+        return self.k_off[self._k_ids[first]][0], self.k_off[self._k_ids[last]][0] if last < len(self._k_ids) else self.k_total
+
+    @staticmethod
+    def _places(ids, curvs):
+        idx = sorted(ids.index(id(c)) for c in curvs)
         assert idx == list(range(idx[0], idx[-1] + 1)), 'curvatures are not contiguous in the pool'
-        lo = self.k_off[id(kron[idx[0]])][0]
-        hi = self.k_off[id(kron[idx[-1] + 1])][0] if idx[-1] + 1 < len(kron) else self.k_total
-        return lo, hi
+        return idx[0], idx[-1] + 1
 
     def diag_range(self, curvs: Sequence):
         """The same for the diagonal pool."""
         return self._remembered('d', curvs, self._find_diag_range) if curvs else (0, 0)
 
     def _find_diag_range(self, curvs):
-        diag = self.diag
-        idx = sorted(diag.index(c) for c in curvs)
-        assert idx == list(range(idx[0], idx[-1] + 1)), 'curvatures are not contiguous in the pool'
-        lo = self.d_off[id(diag[idx[0]])][0][0]
-        hi = self.d_off[id(diag[idx[-1] + 1])][0][0] if idx[-1] + 1 < len(diag) else self.d_total
-        return lo, hi
+        first, last = self._places(self._d_ids, curvs)
+        return self.d_off[self._d_ids[first]][0][0], self.d_off[self._d_ids[last]][0][0] if last < len(self._d_ids) else self.d_total
 
     # ------------------------------------------------------------------ streaming ops
     def _flat(self, src_role, dst_role, a, b, kron, diag):
-        lo, hi = self.kron_range(kron)
+        """Over the ranges of the given curvatures; None: the whole pool of a kind."""
+        lo, hi = (0, self.k_total) if kron is None else self.kron_range(kron)
         if hi > lo:
             nat.axpby(self.buf(src_role)[lo:hi], self.buf(dst_role)[lo:hi], a, b)
-        lo, hi = self.diag_range(diag)
+        lo, hi = (0, self.d_total) if diag is None else self.diag_range(diag)
         if hi > lo:
             nat.axpby(self.buf(src_role, 'd')[lo:hi], self.buf(dst_role, 'd')[lo:hi], a, b)
 
     def accumulate(self, scale: float, first: bool, kron=None, diag=None):
         """acc <- scale*data (first) or acc + scale*data."""
-        kron = self.kron if kron is None else kron
-        diag = self.diag if diag is None else diag
         self._flat('data', 'acc', scale, 0.0 if first else 1.0, kron, diag)
 
     def take_accumulated(self, kron=None, diag=None):
         """data <- acc."""
-        kron = self.kron if kron is None else kron
-        diag = self.diag if diag is None else diag
         self._flat('acc', 'data', 1.0, 0.0, kron, diag)
 
     def update_ema(self, beta: float, first: bool, kron=None, diag=None):
         """ema <- data (first use, or beta == 1), else beta*data + (1-beta)*ema, for all given
         layers in one launch per pool (torchsso/curv/curvature.py:174-191)."""
-        kron = self.kron if kron is None else kron
-        diag = self.diag if diag is None else diag
         if first or beta == 1:
             self._flat('data', 'ema', 1.0, 0.0, kron, diag)
         else:

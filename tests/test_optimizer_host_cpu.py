@@ -1,6 +1,8 @@
 """Host side of the optimizers without a device: what is kept between steps must follow the groups, tensors and
 buffers that the next step finds."""
 import collections
+import copy
+import gc
 
 import pytest
 import torch
@@ -133,3 +135,58 @@ def test_curvature_step_follows_what_changed(monkeypatch):
     curvature_step(opt, monkeypatch)
     grads = next(c[2] for c in opt.pool.calls if c[0] == 'precondition')
     assert [len(g) for g in grads] == [1, 2]
+
+
+# ------------------------------------------------------------------------------------------- lifetime
+def hooked(module, width=5):
+    """Whether the module's forward pass reaches a curvature (which has no CPU path)."""
+    try:
+        module(torch.ones(2, width))
+    except RuntimeError as e:
+        assert 'CUDA' in str(e)
+        return True
+    return False
+
+
+@pytest.fixture
+def no_collection():
+    gc.collect()
+    gc.disable()
+    yield
+    gc.enable()
+
+
+def test_a_curvature_by_itself_lives_as_long_as_its_module():
+    layer = nn.Linear(5, 7)
+    torchsso.KronCovLinear(layer, damping=1e-2)
+    gc.collect()
+    assert hooked(layer)
+    assert not hooked(copy.deepcopy(layer))          # a copy of the module has none
+    hook, = layer._forward_hooks.values()
+    curv = copy.deepcopy(hook.keep)                  # a copy of the curvature brings its module
+    assert curv.module is not layer and hooked(curv.module)
+
+
+def test_the_curvatures_of_an_optimizer_go_with_it(no_collection):
+    opt = make()
+    layer, keep = opt.model[0], opt.param_groups[1]['curv']
+    assert hooked(layer)
+    del opt
+    assert not hooked(layer)
+    # one that somebody still holds keeps its place in the pool
+    (da, _), (dg, _) = keep.shape
+    lo, hi = keep.pool.kron_range([keep])
+    assert keep.pool.kron == [keep] and hi - lo >= da * da + dg * dg and hi == keep.pool.k_total
+
+
+def test_pool_ranges_without_a_neighbour(no_collection, monkeypatch):
+    opt = make()
+    first, pool = opt.param_groups[0]['curv'], opt.pool
+    lo, hi = pool.kron_range([first])
+    pool._ranges.clear()
+    opt.param_groups[1]['curv'] = None               # gone, and with it the only strong reference
+    assert len(pool.kron) == 1 and pool.kron_range([first]) == (lo, hi)
+    spans = []
+    monkeypatch.setattr(nat, 'axpby', lambda x, y, a, b: spans.append(x.numel()))
+    pool.accumulate(1.0, True)
+    assert spans == [pool.k_total]

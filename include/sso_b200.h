@@ -279,7 +279,7 @@ typedef struct {
   int64_t count;
   float add, momentum, ema, scale, lr;
   int32_t set;       /* sso_optimizer_tail_sets: index of the record's scalars; unused otherwise */
-} sso_tail_rec;    /* count < 2^31 */
+} sso_tail_rec;
 int sso_optimizer_tail(const sso_tail_rec* recs_dev, int n_recs, void* stream);
 
 /* The same with the scalars given at launch: record i uses sets[recs[i].set] (a host array, copied into the

@@ -533,18 +533,18 @@ __global__ void __launch_bounds__(256) optimizer_tail_kernel(const sso_tail_rec*
   if (OWN) { q.add = r.add; q.momentum = r.momentum; q.ema = r.ema; q.scale = r.scale; q.lr = r.lr; }
   else q = sets.s[r.set];
   const bool has_m = r.mbuf != nullptr, has_e = r.ebuf != nullptr, upd = q.lr != 0.f;
-  const int n = (int)r.count;
-  int done = 0;
+  const int64_t n = r.count;
+  int64_t done = 0;
   if (((reinterpret_cast<uintptr_t>(r.p) | reinterpret_cast<uintptr_t>(r.g) | reinterpret_cast<uintptr_t>(r.mbuf) |
         reinterpret_cast<uintptr_t>(r.ebuf)) & 15) == 0) {
-    const int n4 = n >> 2;
+    const int64_t n4 = n >> 2;
     done = n4 << 2;
-    auto at = [](float* base, int i) { return reinterpret_cast<float4*>(base) + i; };
-    for (int i0 = threadIdx.x; i0 < n4; i0 += 2 * 256) {
+    auto at = [](float* base, int64_t i) { return reinterpret_cast<float4*>(base) + i; };
+    for (int64_t i0 = threadIdx.x; i0 < n4; i0 += 2 * 256) {
       float4 p[2], g[2], m[2], e[2];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const int i = i0 + 256 * u;
+        const int64_t i = i0 + 256 * u;
         const bool in = i < n4;
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
         p[u] = in ? *at(r.p, i) : z;
@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(256) optimizer_tail_kernel(const sso_tail_rec*
       }
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const int i = i0 + 256 * u;
+        const int64_t i = i0 + 256 * u;
         if (i >= n4) break;
         tail_element(q, has_m, has_e, p[u].x, g[u].x, m[u].x, e[u].x);
         tail_element(q, has_m, has_e, p[u].y, g[u].y, m[u].y, e[u].y);
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(256) optimizer_tail_kernel(const sso_tail_rec*
       }
     }
   }
-  for (int i = done + threadIdx.x; i < n; i += 256) {
+  for (int64_t i = done + threadIdx.x; i < n; i += 256) {
     float p = r.p[i], g = r.g[i], m = has_m ? r.mbuf[i] : 0.f, e = has_e ? r.ebuf[i] : 0.f;
     tail_element(q, has_m, has_e, p, g, m, e);
     r.g[i] = g;

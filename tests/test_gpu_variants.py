@@ -49,6 +49,15 @@ def test_optimizer_tail_sets(nat, numel, shift):
             assert rel(got, ref) < 1e-6
 
 
+def test_optimizer_tail_of_a_record_beyond_31_bits(nat):
+    n = (1 << 31) + 5
+    p, g = torch.ones(n, device='cuda'), torch.full((n,), 2.0, device='cuda')
+    nat.optimizer_tail(nat.tail_records([(p, g, None, None, 1.0, 0.0, 1.0, 1.0, 0.5)], p.device, chunk=n))
+    for t, want in ((p, -0.5), (g, 3.0)):
+        lo, hi = torch.aminmax(t)
+        assert (lo.item(), hi.item()) == (want, want)
+
+
 def test_precondition_grad_of_moving_gradients(nat):
     """Gradients at a new address on every call, and of another type and layout."""
     import torchsso

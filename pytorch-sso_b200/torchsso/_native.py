@@ -629,6 +629,7 @@ def diag_sq(x: torch.Tensor, g: torch.Tensor, kernel_size, stride, padding, dila
 def diag_sq_call(x, g, kernel_size, stride, padding, dilation):
     """(x, g, call): the operands as the kernel takes them and what of a call does not change between steps."""
     _require_cuda(x, 'layer input')
+    _require_cuda(g, 'output gradient')
     if x.dim() == 2:
         x, g = x[:, :, None, None], g[:, :, None, None]
         kernel_size, stride, padding, dilation = (1, 1), (1, 1), (0, 0), (1, 1)

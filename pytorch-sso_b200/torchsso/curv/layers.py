@@ -98,6 +98,12 @@ def _channels_last_if_worthwhile(t, d):
     return t.contiguous(memory_format=torch.channels_last)
 
 
+def _flat(geometry):
+    """Kernel size, stride, padding and dilation as part of a key, whatever kind of pair a module keeps them as."""
+    k, s, p, d = geometry
+    return (*k, *s, *p, *d)
+
+
 class _KronFactors(KronCurvature):
     """Shared driver: A in the forward hook, G (optionally prob-weighted and accumulated over
     sampling passes) in the backward hook, both by the fused factor kernel."""
@@ -109,9 +115,9 @@ class _KronFactors(KronCurvature):
         raise NotImplementedError
 
     def _op(self, x, geometry, append_ones, out):
-        """Prepared factor call for this input layout (built on first sight of a shape/stride/dtype)."""
+        """Prepared factor call for this input (built on first sight of its layout, type, device or geometry)."""
         ops = self.__dict__.setdefault('_ops', {})
-        key = (x.shape, x.stride(), x.dtype, out.data_ptr())
+        key = (x.shape, x.stride(), x.dtype, x.device, append_ones, out.data_ptr(), *_flat(geometry))
         op = ops.get(key)
         if op is None:
             while len(ops) >= 16:          # oldest first: a second input shape must not evict the first
@@ -381,16 +387,17 @@ class _DiagSq(DiagCurvature):
         # mean over samples, then the n^2 that undoes the mean reduction of the loss
         alpha, beta = ws * float(n), 0.0 if first else 1.0
         calls = self.__dict__.setdefault('_calls', {})
-        key = (x.shape, x.stride(), x.dtype, g.shape, g.stride(), g.dtype)
+        geometry = self._geometry()
+        key = (x.shape, x.stride(), x.dtype, x.device, g.shape, g.stride(), g.dtype, g.device, *_flat(geometry))
         call = calls.get(key)
         if call is not None and p is None:
             nat.diag_sq_run(call, x, g, None, alpha, beta, views[0].data_ptr(), views[1].data_ptr() if self.bias else None)
         else:
-            nat.diag_sq(x, g, *self._geometry(), p, alpha, beta, views[0], views[1] if self.bias else None)
-            if call is None and x.dtype == g.dtype:      # checked once for this layout; without a conversion the operands go in as they are
+            nat.diag_sq(x, g, *geometry, p, alpha, beta, views[0], views[1] if self.bias else None)
+            if call is None and x.dtype == g.dtype:      # checked once for these operands; without a conversion they go in as they are
                 while len(calls) >= 16:
                     calls.pop(next(iter(calls)))
-                calls[key] = nat.diag_sq_call(x, g, *self._geometry())[2]
+                calls[key] = nat.diag_sq_call(x, g, *geometry)[2]
         if fisher:
             self._passes += 1
         self._have.add('data')

@@ -190,3 +190,61 @@ def test_pool_ranges_without_a_neighbour(no_collection, monkeypatch):
     monkeypatch.setattr(nat, 'axpby', lambda x, y, a, b: spans.append(x.numel()))
     pool.accumulate(1.0, True)
     assert spans == [pool.k_total]
+
+
+# ------------------------------------------------------------------------------------------- prepared calls
+def on_meta(t):
+    return torch.empty_strided(t.shape, t.stride(), dtype=t.dtype, device='meta')
+
+
+def other_padding(m, x, g):
+    m.padding = [0, 2]
+    return x, g
+
+
+CHANGES = [lambda m, x, g: (on_meta(x), g), lambda m, x, g: (x, on_meta(g)), lambda m, x, g: (on_meta(x), on_meta(g)), other_padding]
+
+
+@pytest.mark.parametrize('change', CHANGES)
+def test_squared_gradient_calls_are_prepared_per_device_and_geometry(monkeypatch, change):
+    """An operand on another device has passed no check, whatever was checked for its layout before."""
+    calls = []
+    monkeypatch.setattr(nat, 'diag_sq', lambda *a: calls.append('checked'))
+    monkeypatch.setattr(nat, 'diag_sq_call', lambda x, g, *geometry: (x, g, 'call'))
+    monkeypatch.setattr(nat, 'diag_sq_run', lambda *a: calls.append('prepared'))
+    m = nn.Conv2d(3, 4, 3, padding=1)
+    curv = torchsso.DiagCovConv2d(m)
+    x, g = torch.randn(2, 3, 5, 5), torch.randn(2, 4, 5, 5)
+    for _ in range(2):
+        m.data_input = x
+        curv.update_in_backward(g)
+    m.data_input, g = change(m, x, g)
+    curv.update_in_backward(g)
+    assert calls == ['checked', 'prepared', 'checked']
+
+
+@pytest.mark.parametrize('change', [CHANGES[0], other_padding])
+def test_factor_calls_are_prepared_per_device_and_geometry(monkeypatch, change):
+    made = []
+
+    class Op:
+        def __init__(self, x, kernel_size, stride, padding, dilation, append_ones, out):
+            made.append((x.device.type, tuple(padding)))
+
+        def run(self, *args):
+            pass
+    monkeypatch.setattr(nat, 'FactorOp', Op)
+    m = nn.Conv2d(3, 4, 3, padding=1)
+    curv = torchsso.KronCovConv2d(m)
+    x = torch.randn(2, 3, 5, 5)
+    curv.update_in_forward(x)
+    curv.update_in_forward(x)
+    curv.update_in_forward(change(m, x, None)[0])
+    assert len(made) == 2 and len(set(made)) == 2
+
+
+def test_an_output_gradient_on_the_host_is_refused(monkeypatch):
+    monkeypatch.setattr(nat, '_require_cuda', lambda t, what: calls.append(what))
+    calls = []
+    nat.diag_sq_call(torch.randn(2, 3), torch.randn(2, 4), (1, 1), (1, 1), (0, 0), (1, 1))
+    assert calls == ['layer input', 'output gradient']

@@ -68,6 +68,9 @@ int sso_configure(const char* key, int value);
  *           (prob-weighted variants), the in-place rescale at torchsso/curv/curvature.py:299-300
  *           and the accumulation at torchsso/utils/accumulator.py:23-38 (through alpha/beta).
  * ------------------------------------------------------------------------------------- */
+/* Scratch for a factor of d columns from that many rows, whatever its type and geometry: enough for the kernel that `impl`
+ * chooses, unless the parts of one fp32 image (12 bytes per pixel and channel) exceed 64 MB.
+ * sso_factor_desc_workspace_bytes (below) has the figure for one problem. */
 size_t sso_factor_workspace_bytes(int64_t rows, int64_t d, int impl);
 
 int sso_factor_syrk_im2col(const void* x, int dtype,
@@ -105,7 +108,7 @@ typedef struct {
   int64_t ldo;
 } sso_factor_desc;
 /* Scratch with which the described problem runs at its best: fp32 inputs are split into 16-bit parts that pass
- * through the scratch, and with the sso_factor_workspace_bytes minimum they do so in smaller pieces. */
+ * through the scratch, and with sso_factor_workspace_bytes they may do so in smaller pieces. */
 size_t sso_factor_desc_workspace_bytes(const sso_factor_desc* desc, int impl);
 /* One sso_factor_syrk_im2col call with everything that does not change between calls given once: the
  * description's x may be null, its sample_weight, alpha and beta are ignored.  The handle belongs to the

@@ -109,12 +109,23 @@ int sso_configure(const char* key, int value) {
   return fail(-1, "configure: unknown key %s", key);
 }
 
-size_t sso_factor_workspace_bytes(int64_t rows, int64_t d, int impl) {
+// What the kernels that read the input as it lies need.
+static size_t partial_bytes(int64_t rows, int64_t d, int impl) {
   const size_t a = factor_simt_workspace_bytes(rows, d);
   const size_t b = factor_tc_workspace_bytes(rows, d);
   if (impl == SSO_IMPL_SIMT) return a;
   if (impl == SSO_IMPL_TCGEN05 || impl == SSO_IMPL_TMA) return b;
   return a > b ? a : b;
+}
+
+// That, and room for an fp32 input on its way through 16-bit parts: tiles of channels padded to eight, and the parts of
+// some images (of one at least; 48 bytes per element of the rows covers weights and a stride of two under a 1x1 window).
+size_t sso_factor_workspace_bytes(int64_t rows, int64_t d, int impl) {
+  const size_t least = partial_bytes(rows, d, impl);
+  if (impl == SSO_IMPL_SIMT || impl == SSO_IMPL_TMA || rows <= 0 || d <= 0) return least;
+  const int64_t nb = ceil_div64(d + d / 3 + 16, 128), tiles = nb * (nb + 1) / 2;
+  const int64_t parts = std::min<int64_t>(rows, ((int64_t)1 << 40) / d) * (d + 16) * 48;
+  return std::max(least, factor_header_bytes((int)tiles) + (size_t)tiles * 65536) + (size_t)std::min<int64_t>((int64_t)64 << 20, parts) + 1024;
 }
 
 // Argument checks and launch parameters shared by the single-problem and the batched entry points.
@@ -169,9 +180,9 @@ static int launch_one_factor(const FactorParams& p, int dtype, void* workspace, 
   return factor_simt_launch(p, dtype, workspace, workspace_bytes, st);
 }
 
-// Scratch that lets a problem run at its best (the minimum is sso_factor_workspace_bytes).
+// Scratch that lets a problem run at its best.
 static size_t preferred_bytes(const FactorParams& p, int dtype, int impl) {
-  size_t b = sso_factor_workspace_bytes(p.rows, p.d, impl);
+  size_t b = partial_bytes(p.rows, p.d, impl);
   if (dtype == SSO_F32 && impl != SSO_IMPL_SIMT) b = std::max(b, factor_f32_workspace_bytes(p));
   return b;
 }

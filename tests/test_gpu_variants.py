@@ -287,6 +287,26 @@ def test_sample_plan_along_k(nat, shapes, bias):
         assert rel(got, want[i]) < 2e-6
 
 
+@pytest.mark.parametrize('cfg', [(128, 4096, 1, 1, (1, 1), (1, 1), (0, 0), (1, 1), True), (1, 300, 1, 1, (1, 1), (1, 1), (0, 0), (1, 1), False),
+                                 (4, 512, 7, 7, (3, 3), (1, 1), (1, 1), (1, 1), True), (1, 256, 40, 40, (1, 1), (2, 2), (0, 0), (1, 1), False),
+                                 (2, 4, 30, 30, (11, 11), (4, 4), (2, 2), (1, 1), True), (1, 64, 224, 224, (3, 3), (1, 1), (1, 1), (1, 1), False)])
+@pytest.mark.parametrize('weighted', [False, True])
+def test_factor_f32_with_the_scratch_that_a_caller_asks_for(nat, cfg, weighted):
+    """sso_factor_workspace_bytes knows rows and columns only; the tensor-core path takes what it gives."""
+    n, c, h, w, k, s, p, d, bias = cfg
+    x = torch.randn(n, c, h, w, device='cuda').contiguous(memory_format=torch.channels_last)
+    weight = torch.rand(n, device='cuda') if weighted else None
+    ref = conv_ref(x, k, s, p, d, bias, weight)
+    cols = ref.shape[0]
+    ho, wo = (h + 2 * p[0] - k[0]) // s[0] + 1, (w + 2 * p[1] - k[1]) // s[1] + 1
+    space = nat.lib().sso_factor_workspace_bytes(n * ho * wo, cols, nat.IMPL_TCGEN05)
+    ws, out = torch.empty(space, dtype=torch.uint8, device='cuda'), torch.empty(cols, cols, device='cuda')
+    st = (x.stride(0), 1, x.stride(2), x.stride(3))
+    nat._check(nat.lib().sso_factor_syrk_im2col(x.data_ptr(), nat.F32, n, c, h, w, *st, *k, *s, *p, *d, int(bias), nat._ptr(weight), 1.0, 0.0,
+                                                out.data_ptr(), cols, ws.data_ptr(), space, nat.IMPL_TCGEN05, nat._stream()))
+    assert rel(out, ref) < 1e-6
+
+
 # ------------------------------------------------------------------------------------------- lifetime
 def test_an_optimizer_gives_its_buffers_back_when_it_goes(nat):
     """No reference cycle through hooks and pools; a copy of a hooked model has no curvature."""

@@ -39,8 +39,8 @@ def test_factor_op_refuses_a_bad_description(bad):
 
 def test_factor_scratch_grows_with_the_problem_and_has_an_end():
     size = nat.lib().sso_factor_workspace_bytes
+    assert size(1 << 31, 16384, nat.IMPL_TCGEN05) < 1 << 31
     for impl in (nat.IMPL_AUTO, nat.IMPL_TCGEN05):
         assert size(1, 1, impl) > 65536
-        assert size(1 << 31, 16384, impl) < 1 << 34
         for rows, d in ((1, 300), (128, 4097), (100000, 64)):
             assert size(rows, d, impl) >= size(rows, d, nat.IMPL_TMA)

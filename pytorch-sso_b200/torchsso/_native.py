@@ -585,6 +585,8 @@ def sample_classes(prob: torch.Tensor, q: torch.Tensor) -> torch.Tensor:
     _require_cuda(prob, 'probabilities')
     n, c = prob.shape
     out = torch.empty((1, n), dtype=torch.int64, device=prob.device)
+    if n == 0:
+        return out
     _check(lib().sso_sample_classes(prob.data_ptr(), q.data_ptr(), n, c, out.data_ptr(), _stream()))
     return out
 

@@ -29,6 +29,13 @@ def test_sample_classes_is_the_multinomial_draw(nat, n, c):
     assert 0 <= int(got.min()) and int(got.max()) < c and got[:, 0].unique().numel() > min(c, 20) // 2
 
 
+def test_targets_of_an_empty_batch(nat):
+    from torchsso.curv.fisher import sample_targets
+    for num_mc in (1, 2):
+        t = sample_targets(torch.empty(0, 7, device='cuda'), num_mc)
+        assert t.shape == (num_mc, 0) and t.dtype == torch.int64
+
+
 @pytest.mark.parametrize('numel,shift', [(1, 0), (4095, 0), (4096, 0), (4097, 1), (12300, 2)])
 def test_optimizer_tail_sets(nat, numel, shift):
     """Records of one launch with different scalars; `shift` elements off the 16-byte boundary."""

@@ -58,8 +58,6 @@ def get_closure_for_fisher(optimizer, model, data, target, approx_type=None, num
         raise ValueError('batch_mc_passes needs prune_sampling_pass: the batched walk returns the output '
                          'gradients of the hooked modules instead of running their hooks')
 
-    constant_weight = {}
-
     def set_sampling(on: bool):
         for group in optimizer.param_groups:
             curv = group['curv']
@@ -129,10 +127,7 @@ def get_closure_for_fisher(optimizer, model, data, target, approx_type=None, num
         set_sampling(True)
         if approx_type == _APPROX_TYPE_MC:
             mc_targets = sample_targets(prob.detach(), num_mc)
-            key = (prob.shape[0], prob.dtype, prob.device)
-            weight = constant_weight.get(key)
-            if weight is None:
-                weight = constant_weight[key] = torch.full_like(prob[:, 0], 1.0 / num_mc).detach()
+            weight = prob.new_full((prob.shape[0],), 1.0 / num_mc)
             for group in optimizer.param_groups:
                 group['curv'].prob = weight
                 group['curv'].prob_scale = 1.0 / num_mc

@@ -345,3 +345,18 @@ def test_an_optimizer_gives_its_buffers_back_when_it_goes(nat):
     finally:
         gc.enable()
     assert held[2] <= held[1] + (1 << 16), held
+
+
+# ------------------------------------------------------------------------------------------- closures
+def test_every_closure_call_brings_its_own_weights(nat):
+    import torchsso
+    model = torch.nn.Linear(6, 4).cuda()
+    model.num_classes = 4
+    x, y = torch.randn(8, 6, device='cuda'), torch.randint(0, 4, (8,), device='cuda')
+    opt = torchsso.optim.SecondOrderOptimizer(model, 'Fisher', {'Linear': 'Kron'}, {'damping': 1e-2})
+    closure = torchsso.get_closure_for_fisher(opt, model, x, y, approx_type='mc', num_mc=2)
+    curv = opt.param_groups[0]['curv']
+    for _ in range(2):
+        opt.step(closure=closure)
+        assert torch.equal(curv.prob, torch.full((8,), 0.5, device='cuda'))
+        curv.prob.zero_()

@@ -77,9 +77,6 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
   const int split = blockIdx.y;
   const int64_t r_begin = (int64_t)split * p.rows_per_split;
   const int64_t r_end = min(p.rows, r_begin + (int64_t)p.rows_per_split);
-  // bits 16 / 17 of `flush` are timing experiments: skip the gather's copies / skip the MMAs
-  const bool dbg_no_gather = (flush & 0x10000) != 0, dbg_no_mma = (flush & 0x20000) != 0;
-  flush &= 0xFFFF;
   const int nstages = (int)ceil_div64(max((int64_t)0, r_end - r_begin), KS);
   const int nchunks = ceil_div(nstages, flush);
   int* status = p.status;
@@ -151,15 +148,12 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
         tc_fence_after();
         const uint32_t sb = smem0 + slot * STAGE_BYTES;
         const uint32_t d_tmem = tmem_base + (uint32_t)(b * TILE);
-        if (dbg_no_mma && s > 0) {
-        } else {
-          const uint32_t a0 = sb, b0 = share ? sb : sb + OPB;
+        const uint32_t a0 = sb, b0 = share ? sb : sb + OPB;
 #pragma unroll
-          for (int ks = 0; ks < KS / 16; ++ks) {
-            const uint64_t ad = smem_desc(a0 + ks * KSTEP, LBO, SBO);
-            const uint64_t bd = smem_desc(b0 + ks * KSTEP, LBO, SBO);
-            umma<false>(d_tmem, ad, bd, idesc, (first_of_chunk && ks == 0) ? 0u : 1u);
-          }
+        for (int ks = 0; ks < KS / 16; ++ks) {
+          const uint64_t ad = smem_desc(a0 + ks * KSTEP, LBO, SBO);
+          const uint64_t bd = smem_desc(b0 + ks * KSTEP, LBO, SBO);
+          umma<false>(d_tmem, ad, bd, idesc, (first_of_chunk && ks == 0) ? 0u : 1u);
         }
         umma_commit(empty_bar(slot));
         if ((s % flush) == flush - 1 || s == nstages - 1) umma_commit(accfull_bar(b));
@@ -255,7 +249,6 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
                 if (!no_halo)
                   in = in && (unsigned)(ih0 + (kp & 0xFFFF)) < (unsigned)p.h &&
                        (unsigned)(iw0 + (kp >> 16)) < (unsigned)p.w;
-                if (dbg_no_gather) continue;
                 const T* src = in ? pix + koff[op][g] : xp;
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(src), "r"(in ? 16 : 0) : "memory");
               }
@@ -465,8 +458,8 @@ int factor_tc_run_reduce(const FactorParams& p, int tiles, cudaStream_t st) {
 
 int factor_tc_set_wait_controls(long long cycles, int stall) { return tc::set_wait_controls(cycles, stall); }
 
-int factor_tc_flush_setting() { return g_flush_stages & 0xFFFF; }
+int factor_tc_flush_setting() { return g_flush_stages; }
 
-void factor_tc_set_flush(int stages) { g_flush_stages = stages < 0 ? 0 : stages; }  // see kernel for bits 16/17
+void factor_tc_set_flush(int stages) { g_flush_stages = stages < 0 ? 0 : stages; }
 
 }  // namespace sso

@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
         if (lane == 0) mbar_arrive(full_bar((s - LAG) % STAGES));   // one arrival per warp
       }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");      // also when a wait gave up
   }
   tc_fence_before();
   __syncthreads();

@@ -393,6 +393,8 @@ int sso_precond_plan_run(int64_t plan, void* stream);
 /* Posterior sampling  [W|b] <- [W|b] + s * U_G E U_A  (W, b pre-loaded with the mean by the
  * caller; E is dG x dA standard normal, supplied).  U_* upper triangular.
  * Replaces: torchsso/curv/cov/linear.py:86-100, torchsso/curv/cov/conv.py:94-108. */
+/* whether plans use the caller's `tmp` matrices (where the products run along k they do not: `tmp` may be null) */
+int sso_sample_plan_uses_tmp(void);
 size_t sso_sample_plan_dev_bytes(int n_layers, const int64_t* dA, const int64_t* dG);
 int64_t sso_sample_plan_create(int n_layers, const int64_t* dA, const int64_t* dG,
                                float* const* U_A, float* const* U_G, float* const* noise,

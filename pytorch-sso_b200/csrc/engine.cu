@@ -1370,16 +1370,21 @@ static Plan* build_sample(int n, const int64_t* dA, const int64_t* dG, float* co
   return p;
 }
 
+static bool sample_along_k() { return g_engine_tma && g_engine_tc; }
+
+int sso_sample_plan_uses_tmp(void) { return sample_along_k() ? 0 : 1; }
+
 size_t sso_sample_plan_dev_bytes(int n_layers, const int64_t* dA, const int64_t* dG) {
-  return sso_precond_plan_dev_bytes(n_layers, dA, dG) + (g_engine_tma && g_engine_tc ? sample_scratch_bytes(n_layers, dA, dG) : 0);
+  return sso_precond_plan_dev_bytes(n_layers, dA, dG) + (sample_along_k() ? sample_scratch_bytes(n_layers, dA, dG) : 0);
 }
 
 int64_t sso_sample_plan_create(int n_layers, const int64_t* dA, const int64_t* dG, float* const* U_A,
                                float* const* U_G, float* const* noise, float* const* w,
                                float* const* b, float* const* tmp, void* dev_mem,
                                size_t dev_mem_bytes, int host_only, const int64_t* ldA, const int64_t* ldG) {
-  SSO_CHECK_ARG(n_layers > 0 && dA && dG && U_A && U_G && noise && w && tmp, "sample plan: null argument");
-  if (!host_only && g_engine_tma && g_engine_tc) {
+  const bool along_k = !host_only && sample_along_k();
+  SSO_CHECK_ARG(n_layers > 0 && dA && dG && U_A && U_G && noise && w && (tmp || along_k), "sample plan: null argument");
+  if (along_k) {
     const size_t scratch = sample_scratch_bytes(n_layers, dA, dG);
     SSO_CHECK_ARG(dev_mem != nullptr && dev_mem_bytes >= scratch, "sample plan: plan memory too small");
     char* mem = reinterpret_cast<char*>(align_up(reinterpret_cast<uintptr_t>(dev_mem)));

@@ -106,6 +106,7 @@ SIGNATURES = {
     'sso_precond_plan_dev_bytes': (c_sz, [c_i32, c_vp, c_vp]),
     'sso_precond_plan_create': (c_i64, [c_i32] + [c_vp] * 8 + [c_sz, c_i32, c_vp, c_vp]),
     'sso_precond_plan_run': (c_i32, [c_i64, c_vp]),
+    'sso_sample_plan_uses_tmp': (c_i32, []),
     'sso_sample_plan_dev_bytes': (c_sz, [c_i32, c_vp, c_vp]),
     'sso_sample_plan_create': (c_i64, [c_i32] + [c_vp] * 9 + [c_sz, c_i32, c_vp, c_vp]),
     'sso_sample_plan_run': (c_i32, [c_i64, c_f32, c_vp]),
@@ -918,6 +919,10 @@ def precond_plan_run(plan: Plan):
     _check(lib().sso_precond_plan_run(plan.handle, _stream()))
 
 
+def sample_plan_uses_tmp() -> bool:
+    return bool(lib().sso_sample_plan_uses_tmp())
+
+
 def sample_plan(dA, dG, U_A, U_G, noise, w, b, tmp, device, host_only=False) -> Plan:
     L = lib()
     n = len(dA)
@@ -925,7 +930,7 @@ def sample_plan(dA, dG, U_A, U_G, noise, w, b, tmp, device, host_only=False) -> 
     nbytes = L.sso_sample_plan_dev_bytes(n, a, g)
     mem = None if host_only else torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
     h = L.sso_sample_plan_create(n, a, g, _ptrs(U_A), _ptrs(U_G), _ptrs(noise), _ptrs(w), _ptrs(b),
-                                 _ptrs(tmp), _ptr(mem), nbytes, int(host_only), _lds(U_A), _lds(U_G))
+                                 None if tmp is None else _ptrs(tmp), _ptr(mem), nbytes, int(host_only), _lds(U_A), _lds(U_G))
     return Plan(h, mem, (U_A, U_G, noise, w, b, tmp))
 
 

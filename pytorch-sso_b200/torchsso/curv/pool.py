@@ -283,14 +283,16 @@ class FactorPool:
         plan = self._plans.get(key)
         if plan is None:
             dA, dG, UA, UG, w, b, tmp = [], [], [], [], [], [], []
+            uses_tmp = nat.sample_plan_uses_tmp()
             for c, ps in zip(curvs, params):
                 ua, ug = self.mat('std', c, 0), self.mat('std', c, 1)
                 dA.append(ua.shape[0]); dG.append(ug.shape[0])
                 UA.append(ua); UG.append(ug)
                 assert ps[0].is_contiguous() and ps[0].dtype == torch.float32
                 w.append(ps[0]); b.append(ps[1] if len(ps) > 1 else None)
-                tmp.append(torch.empty(ug.shape[0] * ua.shape[0], dtype=torch.float32, device=self.device))
-            plan = nat.sample_plan(dA, dG, UA, UG, list(noises), w, b, tmp, self.device)
+                if uses_tmp:
+                    tmp.append(torch.empty(ug.shape[0] * ua.shape[0], dtype=torch.float32, device=self.device))
+            plan = nat.sample_plan(dA, dG, UA, UG, list(noises), w, b, tmp if uses_tmp else None, self.device)
             self._trim_plans()
             self._plans[key] = plan
         nat.sample_plan_run(plan, std_scale)

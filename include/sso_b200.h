@@ -365,6 +365,11 @@ typedef struct {
  * dev_mem (device, sso_kron_plan_dev_bytes bytes) receives the tables; host_only != 0 builds
  * the plan without touching the device (for inspecting the task program on a CPU).
  * Returns a plan handle > 0, or a negative error. */
+/* Host only: the tile tasks of the dataflow program for matrices of these dimensions, in the order in which the CTAs
+ * take them (a task waits only for earlier ones).  Four values per task into `out` (nullable, room for `capacity`
+ * tasks): kind (0 diagonal block, 1 panel tile, 2 tile of the transposed triangular inverse, 3 product), matrix, and
+ * the two block indices.  with_inverse == 0: the factorisation alone.  Returns the number of tasks. */
+int sso_flow_tasks(int n_mats, const int64_t* dims, int with_inverse, int16_t* out, int capacity);
 /* whether plans use the caller's `work` matrices (the dataflow kernel does not: `work` may be null) */
 int sso_kron_plan_uses_work(void);
 size_t sso_kron_plan_dev_bytes(int n_mats, const int64_t* dims, int with_std);

@@ -868,8 +868,9 @@ static Plan* build_kron(int n, const int64_t* dims, float* const* src, float* co
 // ------------------------------------------------------------------------------------------
 // Adds the tasks of every matrix in an order in which each of them only depends on earlier ones and the CTAs, taking
 // them in that order, wait as little as possible: a list schedule on 148 workers with rough durations (a
-// 32-column stage 1 us, a tile's fixed cost 3 us, a diagonal block 22 us), longest remaining chain first among the tasks
-// that could run through without waiting.
+// 32-column stage 1 us, a tile's fixed cost 3 us, a diagonal block 25 us), longest remaining chain first among the tasks
+// that could run through without waiting.  The durations only order the list: a diagonal block is counted as it was
+// when they were chosen (it takes 12.5 us now).
 static void schedule_flow(FlowProgram& f, bool with_inverse) {
   struct Node {
     flow::Task t;
@@ -999,6 +1000,24 @@ static size_t kron_scratch(int n_mats, const int64_t* dims, std::vector<KronScra
 }
 
 static bool flow_enabled() { return g_flow && g_engine_tma && g_engine_tc && g_chol_panel && tensor_map_encoder() != nullptr; }
+
+int sso_flow_tasks(int n_mats, const int64_t* dims, int with_inverse, int16_t* out, int capacity) {
+  SSO_CHECK_ARG(n_mats > 0 && n_mats < 32768 && dims, "flow tasks: bad argument");
+  FlowProgram f;
+  for (int i = 0; i < n_mats; ++i) {
+    SSO_CHECK_ARG(dims[i] > 0 && dims[i] <= 32768, "flow tasks: bad dim %lld", (long long)dims[i]);
+    flow::Mat m{};
+    m.d = (int)dims[i]; m.np = (m.d + 127) / 128;
+    f.mats.push_back(m);
+  }
+  schedule_flow(f, with_inverse != 0);
+  for (int i = 0; out && i < std::min(capacity, (int)f.tasks.size()); ++i) {
+    const flow::Task& t = f.tasks[i];
+    int16_t* o = out + 4 * (int64_t)i;
+    o[0] = t.kind; o[1] = t.mat; o[2] = t.a; o[3] = t.b;
+  }
+  return (int)f.tasks.size();
+}
 
 int sso_kron_plan_uses_work(void) { return flow_enabled() ? 0 : 1; }
 

@@ -99,6 +99,7 @@ SIGNATURES = {
     'sso_wire_absmax': (c_i32, [c_vp, c_vp, c_i32, c_vp, c_vp]),
     'sso_wire_encode': (c_i32, [c_vp, c_vp, c_i32, c_vp, c_vp, c_i32, c_vp]),
     'sso_wire_decode': (c_i32, [c_vp, c_vp, c_i32, c_vp, c_vp, c_i32, c_vp]),
+    'sso_flow_tasks': (c_i32, [c_i32, c_vp, c_i32, c_vp, c_i32]),
     'sso_kron_plan_uses_work': (c_i32, []),
     'sso_kron_plan_dev_bytes': (c_sz, [c_i32, c_vp, c_i32]),
     'sso_kron_plan_create': (c_i64, [c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_sz, c_i32, c_vp]),

@@ -360,3 +360,83 @@ def test_every_closure_call_brings_its_own_weights(nat):
         opt.step(closure=closure)
         assert torch.equal(curv.prob, torch.full((8,), 0.5, device='cuda'))
         curv.prob.zero_()
+
+
+# ------------------------------------------------------------------------------------------- variational step
+def test_vi_step_at_fixed_draws(nat, monkeypatch):
+    """The second step of a thirteen-layer stack, which draws its weights, piece by piece against fp64 at the draws that it
+    made: a draw feeds the last digits of a Cholesky factor into the network, so two runs are not comparable."""
+    import torch.nn as nn
+    import torch.nn.functional as F
+    import torchsso
+    torch.manual_seed(0)
+    layers, cin = [], 3
+    for c, count in ((6, 2), (12, 2), (20, 3), (24, 3), (24, 3)):
+        for _ in range(count):
+            layers += [nn.Conv2d(cin, c, 3, padding=1), nn.Tanh()]
+            cin = c
+        layers.append(nn.AvgPool2d(2))
+    model = nn.Sequential(*layers, nn.Flatten(), nn.Linear(24, 10)).cuda()
+    x, y = torch.randn(8, 3, 32, 32, device='cuda'), torch.randint(0, 10, (8,), device='cuda')
+    opt = torchsso.optim.VIOptimizer(model, 500, 'Cov', {'Linear': 'Kron', 'Conv2d': 'Kron'}, {'ema_decay': 0.9, 'damping': 1e-2},
+                                     lr=0.05, num_mc_samples=2)
+    groups, noise, draws, losses = opt.param_groups, [], [], []
+    randn_like = torch.randn_like
+    monkeypatch.setattr(torch, 'randn_like', lambda t: (noise.append(randn_like(t)), noise[-1])[1])
+
+    def closure():
+        opt.zero_grad()
+        draws.append([[p.detach().double() for p in g['params']] for g in groups])
+        out = model(x)
+        loss = F.cross_entropy(out, y)
+        loss.backward()
+        losses.append(loss.detach())
+        return loss, out
+
+    def flat(ts):
+        return torch.cat([ts[0].double().flatten(1)] + [t.double()[:, None] for t in ts[1:]], 1)
+    with torch.backends.cudnn.flags(allow_tf32=False):
+        opt.step(closure=closure)
+        std = [[u.double() for u in g['curv'].std] for g in groups]
+        mean = [flat(g['mean']) for g in groups]
+        for seen in (noise, draws, losses):
+            seen.clear()
+        opt.step(closure=closure)
+    ref = nn.Sequential(*[type(m)(*((m.in_features, m.out_features) if isinstance(m, nn.Linear) else (m.in_channels, m.out_channels, 3, 1, 1)))
+                          if hasattr(m, 'weight') else m for m in model]).double().cuda()
+    ref_layers = [m for m in ref if hasattr(m, 'weight')]
+    grad_sum, a_sum, g_sum = [], [0.0] * len(groups), [0.0] * len(groups)
+    for i, draw in enumerate(draws):
+        for j, (g, (ua, ug)) in enumerate(zip(groups, std)):
+            e = noise[i * len(groups) + j].double()
+            assert rel(flat(draw[j]) - mean[j], g['std_scale'] * ug @ e @ ua) < 1e-5      # of the difference of two fp32 numbers
+            with torch.no_grad():
+                ref_layers[j].weight.copy_(draw[j][0])
+                ref_layers[j].bias.copy_(draw[j][1])
+        h, ins, outs = x.double(), [], []
+        for m in ref:
+            if m in ref_layers:
+                ins.append(h)
+            h = m(h)
+            if m in ref_layers:
+                outs.append(h)
+        loss = F.cross_entropy(h, y)
+        assert abs(losses[i].item() - loss.item()) < 1e-6 * abs(loss.item())
+        params = [p for m in ref_layers for p in (m.weight, m.bias)]
+        got = torch.autograd.grad(loss, params + outs)
+        grad_sum = [a + b / 2 for a, b in zip(grad_sum or [0.0] * len(params), got)]
+        for j, (u, g) in enumerate(zip(ins, got[len(params):])):
+            n = u.shape[0]
+            if u.dim() == 4:
+                a = conv_ref(u, (3, 3), (1, 1), (1, 1), (1, 1), True) / n
+                gg = g.permute(0, 2, 3, 1).reshape(-1, g.shape[1])
+            else:
+                a, gg = conv_ref(u[:, :, None, None], (1, 1), (1, 1), (0, 0), (1, 1), True) / n, g
+            a_sum[j] = a_sum[j] + a / 2
+            g_sum[j] = g_sum[j] + gg.t() @ gg / gg.shape[0] * n * n / 2
+    for j, g in enumerate(groups):
+        a, gg = g['curv'].data
+        assert rel(a, a_sum[j]) < 1e-5 and rel(gg, g_sum[j]) < 1e-4, j
+        ia, ig = (m.double() for m in g['curv'].inv)
+        raw = flat(grad_sum[2 * j:2 * j + 2]) + g['l2_reg'] * mean[j]
+        assert rel(flat(g['mean']) - mean[j], -0.05 * ig @ raw @ ia) < 1e-3, j

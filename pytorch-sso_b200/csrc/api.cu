@@ -331,7 +331,7 @@ int sso_factor_syrk(const void* x, int dtype, int64_t rows, int64_t cols, int64_
 //
 //  * The array is kStaticScratchBytes (16 MiB) per GPU that loads the library and stays
 //    resident until the process exits, whether or not this entry point is ever used.
-//  * Problems whose scratch need (sso_factor_workspace_bytes) exceeds it are rejected with an
+//  * Problems whose partial tiles (partial_bytes) exceed it are rejected with an
 //    error; nothing is launched.
 //  * The first call on each device looks up the array's device address (cudaGetSymbolAddress,
 //    with that device current).  Make that first call before starting any stream capture.  With
@@ -373,7 +373,7 @@ int sso_factor_syrk_noalloc(const void* x, int dtype, int64_t rows, int64_t cols
                             float beta, float* out, int64_t ldo, int impl, void* stream) {
   SSO_CHECK_ARG(rows > 0 && cols > 0, "factor (no-alloc): bad shape");
   const int64_t d = cols + (append_ones ? 1 : 0);
-  const size_t need = sso_factor_workspace_bytes(rows, d, impl);
+  const size_t need = partial_bytes(rows, d, impl);      // parts of an fp32 input take what is left of the array
   SSO_CHECK_ARG(need <= kStaticScratchBytes,
                 "factor (no-alloc): %lld rows x %lld columns needs %zu bytes of scratch but the built-in "
                 "scratch holds %zu; use sso_factor_syrk with caller-provided scratch",

@@ -44,3 +44,11 @@ def test_factor_scratch_grows_with_the_problem_and_has_an_end():
         assert size(1, 1, impl) > 65536
         for rows, d in ((1, 300), (128, 4097), (100000, 64)):
             assert size(rows, d, impl) >= size(rows, d, nat.IMPL_TMA)
+
+
+@pytest.mark.parametrize('rows,cols,fits', [(5000, 300, True), (20000, 64, True), (128, 2000, True), (1568, 4608, False)])
+def test_factor_without_allocation_goes_by_the_partial_tiles(rows, cols, fits):
+    """What is refused for its size is refused before the device is asked for anything."""
+    lib = nat.lib()
+    rc = lib.sso_factor_syrk_noalloc(None, nat.F32, rows, cols, cols, 1, 0, None, 1.0, 0.0, None, cols, nat.IMPL_AUTO, None)
+    assert rc < 0 and (b'built-in scratch' not in lib.sso_last_error()) == fits

@@ -24,15 +24,14 @@ _NORM_TYPES = (nn.BatchNorm1d, nn.BatchNorm2d, nn.BatchNorm3d)
 
 
 class _ForwardHook:
-    """What a hooked module keeps of its curvature.  One that was made by itself lives as long as the module does.  One
-    that has an owner (an optimizer) is only referred to weakly, so that its buffers are given back as soon as the owner
-    goes, and not at the next cycle collection.  A copy of the module alone has no curvature."""
+    """What a hooked module keeps of its curvature: a weak reference, so that a curvature that nobody holds any more gives
+    its buffers back at once instead of at the next cycle collection (held by its layer, a curvature of 4608 x 512 had its
+    successor map new memory: first use 4.1 -> 16.7 ms).  A copy of the module alone has no curvature."""
 
-    __slots__ = ('ref', 'keep')
+    __slots__ = ('ref',)
 
-    def __init__(self, curv=None, keep=False):
+    def __init__(self, curv=None):
         self.ref = weakref.ref(curv) if curv is not None else lambda: None
-        self.keep = curv if keep else None
 
     def __call__(self, module, input, output):
         curv = self.ref()
@@ -40,8 +39,7 @@ class _ForwardHook:
             curv.forward_postprocess(module, input, output)
 
     def __deepcopy__(self, memo):
-        copied = memo.get(id(self.ref()))       # the curvature is being copied together with its module
-        return _ForwardHook(copied, self.keep is not None)
+        return _ForwardHook(memo.get(id(self.ref())))       # with the curvature, if that is being copied too
 
     def __reduce__(self):
         return _ForwardHook, ()
@@ -73,12 +71,7 @@ class Curvature(object):
         self._have = set()          # which of data / ema / inv / std hold values
         self._generic = {}          # storage for curvature shapes the pool does not manage
         self._is_norm = isinstance(module, _NORM_TYPES)
-        self._hook = _ForwardHook(self, keep=True)
-        module.register_forward_hook(self._hook)
-
-    def owned(self):
-        """Called by what owns this curvature: it need not live as long as its module."""
-        self._hook.keep = None
+        module.register_forward_hook(_ForwardHook(self))
 
     # ---- identity ---------------------------------------------------------------
     @property

@@ -107,7 +107,6 @@ class SecondOrderOptimizer(Optimizer):
             if len(params) == 0:
                 continue
             curvature = self.get_curv_class(module)(module, **curv_kwargs)
-            curvature.owned()
             group = {'params': params, 'curv': curvature,
                      'acc_curv': TensorAccumulator(), 'acc_grads': TensorAccumulator()}
             if non_reg_for_bn and isinstance(module, _NORM_TYPES):

@@ -156,15 +156,15 @@ def no_collection():
     gc.enable()
 
 
-def test_a_curvature_by_itself_lives_as_long_as_its_module():
+def test_a_curvature_lives_as_long_as_it_is_held(no_collection):
     layer = nn.Linear(5, 7)
-    torchsso.KronCovLinear(layer, damping=1e-2)
-    gc.collect()
+    curv = torchsso.KronCovLinear(layer, damping=1e-2)
     assert hooked(layer)
     assert not hooked(copy.deepcopy(layer))          # a copy of the module has none
-    hook, = layer._forward_hooks.values()
-    curv = copy.deepcopy(hook.keep)                  # a copy of the curvature brings its module
-    assert curv.module is not layer and hooked(curv.module)
+    copied = copy.deepcopy(curv)                     # a copy of the curvature brings its module
+    assert copied.module is not layer and hooked(copied.module)
+    del curv
+    assert not hooked(layer) and hooked(copied.module)
 
 
 def test_the_curvatures_of_an_optimizer_go_with_it(no_collection):

@@ -44,6 +44,8 @@ uint64_t sso_launch_count(void);
 /* process-wide switches: "tc_auto" / "tma_auto" (0/1: may SSO_IMPL_AUTO choose the tcgen05 kernels /
  * the TMA-fed one), "engine_tc" (0/1: 128-wide tile phases of the engine on tcgen05 3xTF32 or fp32 FFMA),
  * "tc_flush" (stages of tensor-core accumulation between drains into fp32 registers),
+ * "flow" (0/1: factorisations and inverses as one dataflow kernel or as phases of launches, to which alone the next three
+ * apply; read when a plan is built),
  * "chol_ksplit" (first 128-column panel of the blocked Cholesky whose update tasks are cut along K;
  * 0 = never; read when a plan is built), "chol_panel" (0/1: a panel's 128x128 diagonal block is factorised
  * and inverted by one launch, or as two 64-wide halves; read when a plan is built), "phase_lpt" (0/1: tasks

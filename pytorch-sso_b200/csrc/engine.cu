@@ -4,7 +4,9 @@
 // (one kernel launch per phase, covering every matrix of every layer) plus a dense 64x64
 // diagonal-block factorisation done by one CTA in shared memory.
 //
-// Blocked algorithm per SPD matrix M (panels of 128 columns, left looking):
+// Factorisations and inverses run as one dataflow kernel (flow.cu; its task lists are made at the end of this file).  As
+// phases of launches (switch "flow" off, or a plan built without a device) the blocked algorithm per SPD matrix M is
+// (panels of 128 columns, left looking):
 //   Cholesky, panel p:
 //       update : M_ip -= sum_{k<p} L_ik * L_pk^T         for i >= p (128-wide tile tasks, long K)
 //       diag   : L_pp = chol(M_pp), also Linv_pp = L_pp^-1          (diag-panel kernel, one CTA)

@@ -564,9 +564,11 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
   }
 }
 
-// Blocks x splits of the rows over the 74 pairs (148 SMs), with measured costs: a stage, the fixed cost of a CTA
-// (set-up, pipeline fill, drain, tile), a partial tile's way to memory and back.
+// Blocks x splits of the rows over the 74 pairs (148 SMs), with rough costs: a stage (`stage_us`), the fixed cost of a CTA
+// (set-up, pipeline fill, drain, tile: 5 us), a partial tile's way to memory and back (0.03 us).
 // `narrow` of the units take `part` of the others' time and run behind them.
+// Of these only the stage of boxes is a measurement (1.05 of the 1.1 us above); the others are estimates that were not
+// measured by themselves.  They weigh splits against each other, nothing else.
 static int choose_splits(int64_t rows, int units, int narrow, double part, int slots, int tiles, double stage_us, int max_splits,
                          int& rows_per_split) {
   const int64_t stages = ceil_div64(rows, KS);
@@ -853,7 +855,8 @@ static bool encode_boxes(Boxes& b, const Parts& parts, const Shape& s, int h, in
 constexpr int64_t PARTS_TARGET = (int64_t)256 << 20;     // parts of one run of images
 // Columns that the MMAs of the last block row compute if it is a narrow one: 32 (at most sixteen columns, all of them
 // from one CTA; a pair's N is a multiple of 32), 128, or 0 for an ordinary block.  Its blocks run behind all others and
-// read the parts once more: from L2 up to this size (d = 333 from 401408 rows, 256 MB a run, 1153 us without, 1267 with).
+// read the parts once more, from L2 if they are small: the line lies between 50 MB (d = 577 from 131072 rows, 391 us
+// without, 363 with) and 256 MB (d = 333 from 401408 rows, 1153 without, 1267 with), nearer to the size of L2.
 constexpr int64_t NARROW_PARTS = (int64_t)96 << 20;
 static int narrow_columns(int d) {
   const int width = d - (d - 1) / 256 * 256;

@@ -3,10 +3,9 @@ as torchsso/optim/secondorder.py:148-156 does: Kron{Cov,Fisher}{Linear,Conv2d},
 Diag{Cov,Fisher}{Linear,Conv2d}, DiagCovBatchNorm{1d,2d}, DiagFisherBatchNorm2d and the full
 Cov* placeholders.
 
-Hot classes (Kron Linear/Conv2d, Diag BatchNorm) run on libsso_b200 kernels.  The diagonal
-Linear/Conv2d curvatures (per-sample squared gradients, torchsso/curv/cov/linear.py:28-45,
-torchsso/curv/cov/conv.py:15-42) are outside the accelerated path and are computed with plain
-torch ops on the device.
+Kron Linear/Conv2d, Diag BatchNorm and Diag Linear/Conv2d (per-sample squared gradients,
+torchsso/curv/cov/linear.py:28-45, torchsso/curv/cov/conv.py:15-42) run on libsso_b200 kernels.  The full
+covariance of a Linear layer is outside the accelerated path and computed with plain torch ops on the device.
 """
 from __future__ import annotations
 

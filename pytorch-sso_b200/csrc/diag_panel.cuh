@@ -134,7 +134,7 @@ constexpr Schedule make_schedule() {
 static __constant__ Schedule c_schedule = make_schedule();
 
 // The elimination of panel k's diagonal block by one warp.
-__device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restrict__ V, int k, int n, int* __restrict__ info, int row0, int lane) {
+__device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restrict__ V, int k, int n, int* __restrict__ info, int first, int dir, int lane) {
   const int l = lane & 15, h = lane >> 4, c0 = PK * k;
   float* D = S + c0 * PP + c0;
   float v[PK];
@@ -187,7 +187,7 @@ __device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restri
       }
     }
   }
-  if (first_bad >= 0 && lane == 0 && info && c0 + first_bad < n) atomicCAS(info, 0, row0 + c0 + first_bad + 1);
+  if (first_bad >= 0 && lane == 0 && info && c0 + first_bad < n) atomicCAS(info, 0, first + dir * (c0 + first_bad));
   if (h == 0) {
 #pragma unroll
     for (int q = 0; q < PK; q += 4)
@@ -201,8 +201,8 @@ __device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restri
 // The factorisation itself, by 256 threads (barriers 1 and 2).  S holds the lower triangle on entry, visible to all of
 // them, with an identity past the first n rows and columns; on return (behind a barrier) L in its lower triangle and
 // L^-1, with zeros above the diagonal and the identity past n, in V.  `info` (nullable) receives the 1-based number
-// row0 + pivot + 1 of the first bad pivot.
-__device__ __forceinline__ void factor_block(float* __restrict__ S, float* __restrict__ V, int n, int* __restrict__ info, int row0, int tid) {
+// of the first bad pivot, which is first + dir * pivot.
+__device__ __forceinline__ void factor_block(float* __restrict__ S, float* __restrict__ V, int n, int* __restrict__ info, int first, int dir, int tid) {
   const int lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int g = lane >> 2, t = lane & 3;
   const int np = (n + PK - 1) / PK;     // panels that hold columns of the matrix
@@ -210,7 +210,7 @@ __device__ __forceinline__ void factor_block(float* __restrict__ S, float* __res
   auto at = [](float* m, int i, int j) { return m + (PK * i) * PP + PK * j; };
   for (int k = 0; k < np; ++k) {
     if (warp == 0) {
-      eliminate(S, V, k, n, info, row0, lane);
+      eliminate(S, V, k, n, info, first, dir, lane);
     } else if (k == 0) {
       // the inverse's upper half, and its identity past the matrix
       for (int e = tid - 32; e < PN * PN / 4; e += THREADS - 32) {
@@ -307,7 +307,7 @@ static __global__ void __launch_bounds__(THREADS, 1) diag_panel_kernel(const sso
       if (c <= r) S[r * PP + c] = r < n ? rec.L[(int64_t)r * rec.ld_l + c] : (r == c ? 1.f : 0.f);
     }
   __syncthreads();
-  factor_block(S, V, n, info ? info + 2 * rec.mat + rec.info_slot : nullptr, rec.row0, tid);
+  factor_block(S, V, n, info ? info + 2 * rec.mat + rec.info_slot : nullptr, rec.row0 + 1, 1, tid);
   // ---- results: the lower triangle of L, L^-1 with zeros above its diagonal, and optionally the upper
   // triangle of the transpose of L^-1.  Nothing reads L above the diagonal, and the buffer of the transpose
   // is zeroed before the factorisation starts.

@@ -19,7 +19,9 @@
 // Bound: for one large matrix the chain of diagonal blocks, for many the shared-memory traffic of the 3xTF32 stages
 // (as tile_task_tma_kernel).  Against one launch per phase (us): 577+64 508 -> 180, 1000 637 -> 265, six factors of a
 // 784-1000-1000-10 network 1196 -> 296, 4608+512 3363 -> 1424, the 106 factors of ResNet-50 8970 -> 3600, those of VGG-16
-// with sampling factors 19416 -> 7440.
+// with sampling factors 19416 -> 7440, with these out of the same factorisation 6440 -> 4620.
+// Sampling factors: with J the reversal of rows and columns and J M J = L L^T, the lower Cholesky factor of M^-1 is J L^-T J.  A
+// matrix whose factor is wanted is therefore read, and its results are written, in reverse; in between nothing differs.
 // Every wait is bounded; a CTA whose wait gives up sets the status word and writes NaN for this and all further tasks.
 #include "common.cuh"
 #include "diag_panel.cuh"
@@ -93,7 +95,7 @@ __global__ void __launch_bounds__(256) begin_kernel(const Mat* __restrict__ mats
   if (!with_traces) return;
   const Mat& m = mats[blockIdx.x];
   float s = 0.f;
-  for (int i = tid; i < m.d; i += 256) s += m.src[(int64_t)i * m.ld_src + i];
+  for (int i = tid; i < m.pub; i += 256) s += m.src[(int64_t)i * m.ld_src + i];
   red[tid] = s;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
@@ -108,11 +110,13 @@ __device__ __forceinline__ float shift_of(const Mat& m, const float* traces, con
   if (!m.shifted) return 0.f;
   const float r = damp_r[m.mat];
   if (m.partner < 0) return r;
-  const float mine = traces[m.mat] / (float)m.d, other = traces[m.partner] / (float)m.d_partner;
+  const float mine = traces[m.mat] / (float)m.pub, other = traces[m.partner] / (float)m.d_partner;
   const float pi = m.role == 0 ? sqrtf(mine / other) : sqrtf(other / mine);
   return m.role == 0 ? r * pi : r / pi;
 }
 
+// REV: every matrix of the run is taken in reverse (a variant of its own: the addresses of the results cost 2 % of a run otherwise)
+template <bool REV>
 __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * RAW + 2 * LO + 4 + 2 + 2 * QUEUE];
@@ -355,9 +359,30 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
       for (int i = 0; i < 64; ++i) acc[i] = 0.f;
       if (t.kind == DIAG || t.kind == PANEL) {
         const int gr = r0 + row, gc = c0 + col0;
-        if (gr < d) {
+        const bool vec = m.ld_src % 4 == 0 && (reinterpret_cast<uintptr_t>(m.src) & 15) == 0 && gc + 64 <= d;
+        if (REV) {
+          // row and column d - 1 - i; the padding rows come first and are those of an identity
+          const int row_p = d - 1 - gr;
+          if (row_p >= m.pub) {
+#pragma unroll
+            for (int i = 0; i < 64; ++i) acc[i] = gc + i == gr ? 1.f : 0.f;
+          } else if (row_p >= 0) {
+            const float* p = m.src + (int64_t)row_p * m.ld_src + (d - 1 - gc);
+            if (vec && (gc > 0 || d == m.pub)) {
+#pragma unroll
+              for (int i = 0; i < 64; i += 4) {
+                const float4 v = __ldcg(reinterpret_cast<const float4*>(p - i - 3));
+                acc[i] = v.w; acc[i + 1] = v.z; acc[i + 2] = v.y; acc[i + 3] = v.x;
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 64; ++i)
+                if (gc + i < d && d - 1 - gc - i < m.pub) acc[i] = __ldcg(p - i);
+            }
+          }
+        } else if (gr < d) {
           const float* p = m.src + (int64_t)gr * m.ld_src + gc;
-          if (m.ld_src % 4 == 0 && (reinterpret_cast<uintptr_t>(m.src) & 15) == 0 && gc + 64 <= d) {
+          if (vec) {
 #pragma unroll
             for (int i = 0; i < 64; i += 4) {
               const float4 v = __ldcg(reinterpret_cast<const float4*>(p + i));
@@ -373,7 +398,7 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
           const float v = shift_of(m, g.traces, g.damp_r);
 #pragma unroll
           for (int i = 0; i < 64; ++i)
-            if (gc + i == gr) acc[i] += v;
+            if (gc + i == gr && (!REV || gr >= d - m.pub)) acc[i] += v;
         }
       }
       auto drain = [&](int chunks, float sign) {
@@ -419,7 +444,13 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         if (!drain(ceil_div(sh.n2, FLUSH), 1.f)) { fail(); leave(); break; }
       }
       const int nr = min(TILE, d - r0), nc = min(TILE, d - c0);
-      // rows of `out` (tile origin o) along lanes, through 32 columns of this warp's staging tile at a time
+      // Results in the order of M: element (r, c) of the tile at o + r * sr + c * sc, of which the padding is left out.
+      const int pad = REV ? d - m.pub : 0;
+      constexpr int dir = REV ? -1 : 1;
+      auto place = [&](float* base, int ld, int r, int c) {
+        return REV ? base + (int64_t)(d - 1 - r) * ld + (d - 1 - c) : base + (int64_t)r * ld + c;
+      };
+      // rows along lanes, through 32 columns of this warp's staging tile at a time
       auto store_rows = [&](float* o, int ld, bool lower) {
 #pragma unroll
         for (int part = 0; part < 2; ++part) {
@@ -429,7 +460,8 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
           const int c = col0 + part * 32 + lane;
           for (int rr = 0; rr < 32; ++rr) {
             const int r = q * 32 + rr;
-            if (r < nr && c < nc && !(lower && c > r)) o[(int64_t)r * ld + c] = stg[rr * 32 + (lane ^ rr)];
+            if (r < nr && c < nc && r0 + r >= pad && c0 + c >= pad && !(lower && c > r))
+              o[(int64_t)r * (dir * ld) + dir * c] = stg[rr * 32 + (lane ^ rr)];
           }
           __syncwarp();
         }
@@ -463,28 +495,33 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         __syncwarp();
       };
       auto store_columns = [&](float* o, int ld, bool lower) {      // the transposed tile: a column per instruction
+        o += (int64_t)col0 * (dir * ld) + dir * row;
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
+        for (int i = 0; i < 64; ++i, o += dir * ld) {
           const int c = col0 + i;
-          if (row < nr && c < nc && !(lower && c >= row)) o[(int64_t)c * ld + row] = acc[i];
+          if (row < nr && c < nc && r0 + row >= pad && c0 + c >= pad && !(lower && c >= row)) *o = acc[i];
         }
       };
+      // the tile, transposed, as a block of U, and zeros across the diagonal
+      auto store_u = [&]() {
+        store_columns(place(m.U, m.ldu, c0, r0), m.ldu, false);
+        float* z = place(m.U, m.ldu, r0, c0);
+        for (int rr = warp; rr < nr; rr += ACC_WARPS)
+          for (int c = lane; c < nc; c += 32)
+            if (r0 + rr >= pad && c0 + c >= pad) z[(int64_t)rr * (dir * m.ldu) + dir * c] = 0.f;
+      };
+      const bool with_u = m.U && g.with_u;
       int* flag = nullptr;
       if (t.kind != DIAG) {
         if (t.kind == PANEL) {
           store_boxes();
-          if (m.U) {
-            store_columns(m.U + (int64_t)c0 * m.ldu + r0, m.ldu, false);
-            for (int rr = warp; rr < nr; rr += ACC_WARPS)
-              for (int c = lane; c < nc; c += 32) m.U[(int64_t)(r0 + rr) * m.ldu + c0 + c] = 0.f;
-          }
           flag = g.flags + m.flag_w + t.a * m.np + t.b;
         } else if (t.kind == INVT) {
           store_boxes();
           flag = g.flags + m.flag_x + t.a * m.np + t.b;
         } else {
-          store_rows(m.T + (int64_t)r0 * m.ldt + c0, m.ldt, t.a == t.b);
-          store_columns(m.T + (int64_t)c0 * m.ldt + r0, m.ldt, t.a == t.b);
+          store_rows(place(m.T, m.ldt, r0, c0), m.ldt, t.a == t.b);
+          store_columns(place(m.T, m.ldt, c0, r0), m.ldt, t.a == t.b);
         }
         if (!all_well()) { leave(); break; }      // and the tile is stored by all eight warps
       } else {
@@ -499,7 +536,7 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
           for (int i = 0; i < 64; ++i) S[row * dpanel::PP + col0 + i] = col0 + i == row ? 1.f : 0.f;
         }
         if (!all_well()) { leave(); break; }
-        dpanel::factor_block(S, V, nr, g.info ? g.info + 2 * m.mat + m.info_slot : nullptr, r0, tid);
+        dpanel::factor_block(S, V, nr, g.info ? g.info + 2 * m.mat + m.info_slot : nullptr, REV ? d - r0 : r0 + 1, dir, tid);
         float* li = m.Li + (int64_t)t.a * (TILE * TILE);
         for (int e = tid; e < TILE * TILE / 4; e += 256) {
           const int r = e / (TILE / 4), c = e % (TILE / 4) * 4;
@@ -516,7 +553,8 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
             const int c = lane + 32 * u;
             if (c >= nr) continue;
             if (m.X) m.X[(int64_t)(r0 + r) * m.ldw + r0 + c] = V[c * dpanel::PP + r];
-            if (m.U) m.U[(int64_t)(r0 + r) * m.ldu + r0 + c] = c >= r ? S[c * dpanel::PP + r] : 0.f;
+            if (with_u && !m.X) m.U[(int64_t)(r0 + r) * m.ldu + r0 + c] = c >= r ? S[c * dpanel::PP + r] : 0.f;
+            if (with_u && m.X && r0 + r >= pad && r0 + c >= pad) *place(m.U, m.ldu, r0 + r, r0 + c) = c <= r ? V[r * dpanel::PP + c] : 0.f;
           }
         }
         if (m.X) flag = g.flags + m.flag_x + t.a * m.np + t.a;
@@ -529,6 +567,7 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         __threadfence();
         store_release(flag, epoch);
       }
+      if (with_u && t.kind == (m.X ? INVT : PANEL)) store_u();      // nobody waits for U
     }
     if (!ok) dead = 1;
     if (tid == 0) acc_at = n;
@@ -551,8 +590,13 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
     const Mat& m = g.mats[t.mat];
     const int r0 = t.a * TILE, c0 = (t.kind == DIAG ? t.a : t.b) * TILE, nr = min(TILE, m.d - r0), nc = min(TILE, m.d - c0);
     auto fill = [&](float* o, int ld, int rows, int cols) {
-      if (o)
-        for (int e = tid; e < rows * cols; e += THREADS) o[(int64_t)(e / cols) * ld + e % cols] = nan;
+      for (int e = tid; e < rows * cols; e += THREADS) o[(int64_t)(e / cols) * ld + e % cols] = nan;
+    };
+    auto fill_result = [&](float* base, int ld, int row, int col, int rows, int cols) {      // a block in the order of M
+      for (int e = tid; e < rows * cols; e += THREADS) {
+        const int r = row + e / cols, c = col + e % cols, pad = m.d - m.pub;
+        if (r >= pad && c >= pad) base[REV ? (int64_t)(m.d - 1 - r) * ld + (m.d - 1 - c) : (int64_t)r * ld + c] = nan;
+      }
     };
     if (t.kind == DIAG) {
       fill(m.Li + (int64_t)t.a * (TILE * TILE), TILE, TILE, TILE);
@@ -560,8 +604,8 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
     }
     if (t.kind == PANEL) fill(m.W + (int64_t)r0 * m.ldw + c0, m.ldw, nr, nc);
     if (t.kind == INVT) fill(m.X + (int64_t)r0 * m.ldw + c0, m.ldw, nr, nc);
-    if (t.kind == PROD) { fill(m.T + (int64_t)r0 * m.ldt + c0, m.ldt, nr, nc); fill(m.T + (int64_t)c0 * m.ldt + r0, m.ldt, nc, nr); }
-    if (m.U && (t.kind == DIAG || t.kind == PANEL)) fill(m.U + (int64_t)c0 * m.ldu + r0, m.ldu, nc, nr);
+    if (t.kind == PROD) { fill_result(m.T, m.ldt, r0, c0, nr, nc); fill_result(m.T, m.ldt, c0, r0, nc, nr); }
+    if (m.U && g.with_u && (t.kind == DIAG || t.kind == (m.X ? INVT : PANEL))) fill_result(m.U, m.ldu, c0, r0, nc, nr);
     __syncthreads();
     if (tid == 0 && t.kind != PROD) {
       __threadfence();
@@ -593,10 +637,11 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
 int flow_set_wait_controls(long long cycles, int stall) { return tc::set_wait_controls(cycles, stall); }
 
 int flow_launch(const flow::Args& a, int n_mats, int clear_info, int with_traces, cudaStream_t st) {
-  SSO_ENSURE_SMEM(flow::flow_kernel, flow::SMEM);
+  SSO_ENSURE_SMEM(flow::flow_kernel<false>, flow::SMEM);
+  SSO_ENSURE_SMEM(flow::flow_kernel<true>, flow::SMEM);
   flow::begin_kernel<<<n_mats, 256, 0, st>>>(a.mats, n_mats, a.sync, const_cast<float*>(a.traces), a.info, clear_info, with_traces);
   SSO_LAUNCH_OK("flow begin");
-  flow::flow_kernel<<<a.n_tasks < 148 ? a.n_tasks : 148, flow::THREADS, flow::SMEM, st>>>(a);
+  (a.rev ? flow::flow_kernel<true> : flow::flow_kernel<false>)<<<a.n_tasks < 148 ? a.n_tasks : 148, flow::THREADS, flow::SMEM, st>>>(a);
   SSO_LAUNCH_OK("flow_kernel");
   return 0;
 }

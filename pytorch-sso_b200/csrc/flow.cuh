@@ -27,9 +27,10 @@ struct alignas(64) Mat {
   float* X;                      // the same matrix, L^-T in the others; null: factorisation only
   float* Li;                     // [panels][128][128]: inverses of the diagonal blocks
   float* T;                      // the inverse, or null (factorisation only)
-  float* U;                      // upper Cholesky factor, or null
+  float* U;                      // upper Cholesky factor (of M, or with X of the inverse), or null
   int32_t ld_src, ldw, ldt, ldu;
   int32_t d, np;
+  int32_t pub;                   // size of M; d is larger by the padding rows of a reversed matrix
   int32_t mat;                   // index into the shift and info tables
   int32_t shifted;               // whether the damping shift is added
   int32_t partner, role, d_partner;
@@ -47,6 +48,8 @@ struct Args {
   const float* damp_r;
   int* info;                 // nullable
   int* status;
+  int with_u;                // whether U is written
+  int rev;                   // the matrices are taken from the last row and column to the first
 };
 
 }  // namespace flow

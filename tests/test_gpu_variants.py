@@ -221,6 +221,34 @@ def test_kron_plan_in_one_kernel(nat, dims, pad, std):
             assert torch.equal(sd[i], sd[i].triu())
 
 
+@pytest.mark.parametrize('pad', [0, 1, 4])
+def test_kron_plan_with_std_runs_either_half(nat, pad):
+    """Sampling factors come with the inverse, which then goes from the last column to the first: every remainder modulo
+    four columns (its padding), pairs with a shared shift, and the halves by themselves."""
+    dims = [1, 2, 3, 5, 6, 7, 126, 130, 131, 255, 389, 258]
+    n = len(dims)
+    src = [spd(d, d + pad, i) for i, d in enumerate(dims)]
+    dst, work, sd = ([torch.full((d, d + pad), 7.0, device='cuda')[:, :d] for d in dims] for _ in range(3))
+    plan = nat.kron_plan(dims, src, dst, work, sd, [i ^ 1 for i in range(n)], [i & 1 for i in range(n)], torch.device('cuda'))
+    damp = torch.full((n,), 0.1, device='cuda')
+    info = torch.zeros(2 * n, dtype=torch.int32, device='cuda')
+    nat.kron_plan_run(plan, damp, info, True, False)
+    assert all(bool((u == 7.0).all()) for u in sd)
+    nat.kron_plan_run(plan, damp, info, True, True)
+    together = [u.clone() for u in sd]
+    nat.kron_plan_run(plan, damp, info, False, True)
+    assert not info.any()
+    mean = [float(m.double().trace()) / d for m, d in zip(src, dims)]
+    for i, d in enumerate(dims):
+        shift = 0.1 * (mean[i] / mean[i ^ 1]) ** 0.5
+        want = torch.linalg.inv(src[i].double() + shift * torch.eye(d, device='cuda', dtype=torch.float64))
+        u = torch.linalg.cholesky(want, upper=True)
+        assert rel(dst[i], want) < 1e-5 and rel(together[i], u) < 1e-5 and rel(sd[i], u) < 1e-5, d
+        assert torch.equal(together[i], together[i].triu())
+        if pad:      # nothing outside the matrices
+            assert bool((sd[i]._base[:, d:] == 7.0).all()) and bool((dst[i]._base[:, d:] == 7.0).all())
+
+
 @pytest.mark.parametrize('at', [0, 127, 128, 290])
 def test_kron_plan_reports_the_bad_pivot(nat, at):
     """One matrix of three is not positive definite: its pivot is named and the others are as they would be without it."""

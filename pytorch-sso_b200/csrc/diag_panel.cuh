@@ -16,12 +16,13 @@
 // elimination's shuffles along (17 us for 128 rows).
 // The elimination: lane l of warp 0 holds row l of the block, lane l + 16 row l of an identity that goes through the
 // same steps, which leaves the inverse's column l in it for no further instruction; per pivot one round of shuffles
-// (the raw column, and the next diagonal element so that the next pivot's rsqrt starts early).
+// (the raw column, and the next diagonal element so that the next pivot's reciprocal starts early).
 // Rows and columns past the block's size behave as an identity block.  A pivot that is not a positive normal number
 // (non-positive, denormal or NaN) is recorded once per matrix (LAPACK numbering) and replaced by 1, like the 64-wide
 // kernel does for non-positive ones.
-// Measured: 12.5 us for 128 rows (before the elimination went in two steps of eight and took the next block from
-// registers 14.4); a chain of four barriers per panel with all warps in step and the inverse by three levels of
+// Measured: a 16x16 block in 1500 clocks (2280 with a reciprocal square root, a select and the scaling of the column on the
+// chain between two pivots, and with the entries above the diagonal cleared); 128 rows in 12.5 us before that (before the
+// elimination went in two steps of eight and took the next block from registers 14.4); a chain of four barriers per panel with all warps in step and the inverse by three levels of
 // doubling afterwards took 23.  Inside the dataflow kernel (1000 columns) 402 us with that one, 265 now; elimination and
 // products are straight-line code that issues an instruction in about four clocks.
 #pragma once
@@ -40,6 +41,12 @@ constexpr size_t SMEM_BYTES = (size_t)(2 * PN * PP) * sizeof(float) + 3 * PN * 4
 __device__ __forceinline__ float rsqrt_approx(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// MUFU.RCP alone (1 ulp); the same
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -133,7 +140,7 @@ constexpr Schedule make_schedule() {
 }
 static __constant__ Schedule c_schedule = make_schedule();
 
-// The elimination of panel k's diagonal block by one warp.
+// The elimination of panel k's diagonal block by one warp.  The block's entries above the diagonal are not looked at.
 __device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restrict__ V, int k, int n, int* __restrict__ info, int first, int dir, int lane) {
   const int l = lane & 15, h = lane >> 4, c0 = PK * k;
   float* D = S + c0 * PP + c0;
@@ -143,9 +150,9 @@ __device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restri
     const float4 u = ld4(D + l * PP + q);
     const float d[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[q + i] = h ? (q + i == l ? 1.f : 0.f) : (q + i <= l ? d[i] : 0.f);
+    for (int i = 0; i < 4; ++i) v[q + i] = h ? (q + i == l ? 1.f : 0.f) : d[i];
   }
-  int first_bad = -1;
+  uint32_t bad_pivots = 0;
 #pragma unroll
   for (int j0 = 0; j0 < PK; j0 += 8) {
     if (j0 > 0) {
@@ -166,35 +173,41 @@ __device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restri
         v[c] -= s0 + s1;
       }
     }
-    float pv = __shfl_sync(0xffffffffu, v[j0], j0);
+    // Columns stay unscaled (w = a[.][j] / pivot) until all eight are done: on the chain from one pivot to the next are a
+    // reciprocal, a product and a sum, and the two shuffles it waits for go first.
+    float scale[8], pv = __shfl_sync(0xffffffffu, v[j0], j0);
 #pragma unroll
     for (int j = j0; j < j0 + 8; ++j) {
-      float t[PK];
+      float t[PK], d1 = 0.f;
+      if (j + 1 < j0 + 8) {
+        t[j + 1] = __shfl_sync(0xffffffffu, v[j], j + 1);          // a[j+1][j]
+        d1 = __shfl_sync(0xffffffffu, v[j + 1], j + 1);            // a[j+1][j+1] before this step
+      }
 #pragma unroll
-      for (int c = j + 1; c < j0 + 8; ++c) t[c] = __shfl_sync(0xffffffffu, v[j], c);      // a[c][j]
-      float d1 = 0.f;
-      if (j + 1 < j0 + 8) d1 = __shfl_sync(0xffffffffu, v[j + 1], j + 1);                 // a[j+1][j+1] before this step
+      for (int c = j + 2; c < j0 + 8; ++c) t[c] = __shfl_sync(0xffffffffu, v[j], c);
       const bool bad = !(pv >= 1.17549435e-38f);
-      if (bad && first_bad < 0) first_bad = j;
-      const float rs = bad ? 1.f : rsqrt_approx(pv);
-      const float w = v[j] * (rs * rs);
+      if (bad) bad_pivots |= 1u << j;
+      const float pivot = bad ? 1.f : pv;
+      const float inv = rcp_approx(pivot), w = v[j] * inv;
 #pragma unroll
       for (int c = j + 1; c < j0 + 8; ++c) v[c] = fmaf(-w, t[c], v[c]);
-      v[j] = lane == j ? (bad ? 1.f : pv) * rs : v[j] * rs;
-      if (j + 1 < j0 + 8) {
-        const float x = t[j + 1] * rs;
-        pv = fmaf(-x, x, d1);
-      }
+      scale[j - j0] = rsqrt_approx(pivot);
+      if (lane == j) v[j] = pivot;
+      if (j + 1 < j0 + 8) pv = fmaf(-(t[j + 1] * inv), t[j + 1], d1);
     }
-  }
-  if (first_bad >= 0 && lane == 0 && info && c0 + first_bad < n) atomicCAS(info, 0, first + dir * (c0 + first_bad));
-  if (h == 0) {
 #pragma unroll
-    for (int q = 0; q < PK; q += 4)
-      st4(D + l * PP + q, q <= l ? v[q] : 0.f, q + 1 <= l ? v[q + 1] : 0.f, q + 2 <= l ? v[q + 2] : 0.f, q + 3 <= l ? v[q + 3] : 0.f);
-  } else {
+    for (int j = 0; j < 8; ++j) v[j0 + j] *= scale[j];
+  }
+  if (h) {
 #pragma unroll
     for (int r = 0; r < PK; ++r) V[(c0 + r) * PP + c0 + l] = v[r];
+  } else {
+#pragma unroll
+    for (int q = 0; q < PK; q += 4) st4(D + l * PP + q, v[q], v[q + 1], v[q + 2], v[q + 3]);
+  }
+  if (bad_pivots && lane == 0 && info) {
+    const int bad = __ffs(bad_pivots) - 1;
+    if (c0 + bad < n) atomicCAS(info, 0, first + dir * (c0 + bad));
   }
 }
 

@@ -385,6 +385,10 @@ int64_t sso_kron_plan_create(int n_mats, const int64_t* dims, float* const* src,
  * first (the factor comes with the inverse then, and with do_inverse only the first of the two statuses is used). */
 int sso_kron_plan_run(int64_t plan, const float* damp_r_dev, int* info_dev,
                       int do_inverse, int do_std, void* stream);
+/* The inverse (do_inverse) or else the upper Cholesky factor of a matrix that is not the plan's own: `src` instead of src_0 (or
+ * dst_0), the result to `out`, which must not overlap it.  For plans of one matrix that use no `work`. */
+int sso_kron_plan_run_at(int64_t plan, const float* damp_r_dev, int* info_dev, int do_inverse, const float* src, int64_t ld_src,
+                         float* out, int64_t ld_out, void* stream);
 
 /* Kronecker precondition  dW|db <- G^-1 [dW|db] A^-1  for a set of layers, in place.
  * Replaces: torchsso/curv/cov/linear.py:69-84, torchsso/curv/cov/conv.py:76-92 (cat, 2 mm, 2 copies).

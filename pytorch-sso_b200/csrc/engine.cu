@@ -972,8 +972,10 @@ static int upload_flow(FlowProgram& f, char*& q) {
   return 0;
 }
 
-static int run_flow(const Plan& p, const FlowProgram& f, const float* damp_r, int* info, int clear_info, bool with_traces, bool with_u, cudaStream_t st) {
+static int run_flow(const Plan& p, const FlowProgram& f, const float* damp_r, int* info, int clear_info, bool with_traces, bool with_u, cudaStream_t st,
+                    const float* src = nullptr, int64_t ld_src = 0, float* out = nullptr, int64_t ld_out = 0) {
   flow::Args a;
+  a.src = src; a.ld_src = (int)ld_src; a.out = out; a.ld_out = (int)ld_out;
   a.mats = f.d_mats; a.tasks = f.d_tasks; a.n_tasks = (int)f.tasks.size();
   a.sync = f.d_sync; a.flags = f.d_flags; a.traces = p.d_traces; a.damp_r = damp_r;
   a.info = info; a.status = p.d_status; a.with_u = with_u; a.rev = f.rev;
@@ -1159,6 +1161,20 @@ int sso_kron_plan_run(int64_t plan, const float* damp_r_dev, int* info_dev, int 
     SSO_LAUNCH_OK("fold_status_kernel");
   }
   return 0;
+}
+
+int sso_kron_plan_run_at(int64_t plan, const float* damp_r_dev, int* info_dev, int do_inverse, const float* src, int64_t ld_src, float* out,
+                         int64_t ld_out, void* stream) {
+  Plan* p = find_plan(plan);
+  SSO_CHECK_ARG(p != nullptr && !p->host_only, "unknown or host-only plan %lld", (long long)plan);
+  SSO_CHECK_ARG(p->flow_inv.ready() && p->mats.size() == 1, "kron run: operands of its own are for plans of one matrix in one kernel");
+  const int64_t d = p->flow_inv.mats[0].pub;
+  SSO_CHECK_ARG(src && out && ld_src >= d && ld_out >= d && ld_src < ((int64_t)1 << 31) && ld_out < ((int64_t)1 << 31), "kron run: bad operand");
+  SSO_CHECK_ARG(src + (d - 1) * ld_src + d <= out || out + (d - 1) * ld_out + d <= src, "kron run: the result would overwrite the matrix");
+  SSO_CHECK_ARG(!do_inverse || damp_r_dev != nullptr, "kron run: damping table is null");
+  SSO_CHECK_ARG(do_inverse || p->flow_std.ready(), "plan %lld has no std program", (long long)plan);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  return run_flow(*p, do_inverse ? p->flow_inv : p->flow_std, damp_r_dev, info_dev, 1, do_inverse != 0, !do_inverse, st, src, ld_src, out, ld_out);
 }
 
 // ---- precondition --------------------------------------------------------------------------

@@ -87,15 +87,17 @@ __device__ __forceinline__ Shape shape_of(const Task& t, int d) {
 
 // Before a run: next epoch, traces of the matrices, info cleared.
 __global__ void __launch_bounds__(256) begin_kernel(const Mat* __restrict__ mats, int n_mats, int* sync, float* __restrict__ traces, int* info,
-                                                    int clear_info, int with_traces) {
+                                                    int clear_info, int with_traces, const float* src, int ld_src) {
   __shared__ float red[256];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the next kernel sets itself up meanwhile
   const int tid = threadIdx.x;
   if (blockIdx.x == 0 && tid == 0) { sync[1] += 1; sync[2] = sync[0]; }
   if (info && clear_info && tid < 2) info[2 * mats[blockIdx.x].mat + tid] = 0;
   if (!with_traces) return;
   const Mat& m = mats[blockIdx.x];
+  if (!src) { src = m.src; ld_src = m.ld_src; }
   float s = 0.f;
-  for (int i = tid; i < m.pub; i += 256) s += m.src[(int64_t)i * m.ld_src + i];
+  for (int i = tid; i < m.pub; i += 256) s += src[(int64_t)i * ld_src + i];
   red[tid] = s;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
@@ -157,6 +159,7 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   int* status = g.status;
+  asm volatile("griddepcontrol.wait;" ::: "memory");      // begin_kernel, and all before it, are done
   const int epoch = g.sync[1];
   // next entry of the task queue; every consumer warp reads it and arrives on its "empty" barrier
   auto take = [&](uint32_t n, Task& t) -> bool {
@@ -359,7 +362,9 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
       for (int i = 0; i < 64; ++i) acc[i] = 0.f;
       if (t.kind == DIAG || t.kind == PANEL) {
         const int gr = r0 + row, gc = c0 + col0;
-        const bool vec = m.ld_src % 4 == 0 && (reinterpret_cast<uintptr_t>(m.src) & 15) == 0 && gc + 64 <= d;
+        const float* const src = g.src ? g.src : m.src;
+        const int ld_src = g.src ? g.ld_src : m.ld_src;
+        const bool vec = ld_src % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && gc + 64 <= d;
         if (REV) {
           // row and column d - 1 - i; the padding rows come first and are those of an identity
           const int row_p = d - 1 - gr;
@@ -367,7 +372,7 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
 #pragma unroll
             for (int i = 0; i < 64; ++i) acc[i] = gc + i == gr ? 1.f : 0.f;
           } else if (row_p >= 0) {
-            const float* p = m.src + (int64_t)row_p * m.ld_src + (d - 1 - gc);
+            const float* p = src + (int64_t)row_p * ld_src + (d - 1 - gc);
             if (vec && (gc > 0 || d == m.pub)) {
 #pragma unroll
               for (int i = 0; i < 64; i += 4) {
@@ -381,7 +386,7 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
             }
           }
         } else if (gr < d) {
-          const float* p = m.src + (int64_t)gr * m.ld_src + gc;
+          const float* p = src + (int64_t)gr * ld_src + gc;
           if (vec) {
 #pragma unroll
             for (int i = 0; i < 64; i += 4) {
@@ -445,6 +450,9 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
       }
       const int nr = min(TILE, d - r0), nc = min(TILE, d - c0);
       // Results in the order of M: element (r, c) of the tile at o + r * sr + c * sc, of which the padding is left out.
+      float* const T = g.out ? g.out : m.T;
+      float* const U = m.U && g.out ? g.out : m.U;
+      const int ldt = g.out ? g.ld_out : m.ldt, ldu = g.out ? g.ld_out : m.ldu;
       const int pad = REV ? d - m.pub : 0;
       constexpr int dir = REV ? -1 : 1;
       auto place = [&](float* base, int ld, int r, int c) {
@@ -504,13 +512,13 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
       };
       // the tile, transposed, as a block of U, and zeros across the diagonal
       auto store_u = [&]() {
-        store_columns(place(m.U, m.ldu, c0, r0), m.ldu, false);
-        float* z = place(m.U, m.ldu, r0, c0);
+        store_columns(place(U, ldu, c0, r0), ldu, false);
+        float* z = place(U, ldu, r0, c0);
         for (int rr = warp; rr < nr; rr += ACC_WARPS)
           for (int c = lane; c < nc; c += 32)
-            if (r0 + rr >= pad && c0 + c >= pad) z[(int64_t)rr * (dir * m.ldu) + dir * c] = 0.f;
+            if (r0 + rr >= pad && c0 + c >= pad) z[(int64_t)rr * (dir * ldu) + dir * c] = 0.f;
       };
-      const bool with_u = m.U && g.with_u;
+      const bool with_u = U && g.with_u;
       int* flag = nullptr;
       if (t.kind != DIAG) {
         if (t.kind == PANEL) {
@@ -520,8 +528,8 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
           store_boxes();
           flag = g.flags + m.flag_x + t.a * m.np + t.b;
         } else {
-          store_rows(place(m.T, m.ldt, r0, c0), m.ldt, t.a == t.b);
-          store_columns(place(m.T, m.ldt, c0, r0), m.ldt, t.a == t.b);
+          store_rows(place(T, ldt, r0, c0), ldt, t.a == t.b);
+          store_columns(place(T, ldt, c0, r0), ldt, t.a == t.b);
         }
         if (!all_well()) { leave(); break; }      // and the tile is stored by all eight warps
       } else {
@@ -553,8 +561,8 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
             const int c = lane + 32 * u;
             if (c >= nr) continue;
             if (m.X) m.X[(int64_t)(r0 + r) * m.ldw + r0 + c] = V[c * dpanel::PP + r];
-            if (with_u && !m.X) m.U[(int64_t)(r0 + r) * m.ldu + r0 + c] = c >= r ? S[c * dpanel::PP + r] : 0.f;
-            if (with_u && m.X && r0 + r >= pad && r0 + c >= pad) *place(m.U, m.ldu, r0 + r, r0 + c) = c <= r ? V[r * dpanel::PP + c] : 0.f;
+            if (with_u && !m.X) U[(int64_t)(r0 + r) * ldu + r0 + c] = c >= r ? S[c * dpanel::PP + r] : 0.f;
+            if (with_u && m.X && r0 + r >= pad && r0 + c >= pad) *place(U, ldu, r0 + r, r0 + c) = c <= r ? V[r * dpanel::PP + c] : 0.f;
           }
         }
         if (m.X) flag = g.flags + m.flag_x + t.a * m.np + t.a;
@@ -604,8 +612,11 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
     }
     if (t.kind == PANEL) fill(m.W + (int64_t)r0 * m.ldw + c0, m.ldw, nr, nc);
     if (t.kind == INVT) fill(m.X + (int64_t)r0 * m.ldw + c0, m.ldw, nr, nc);
-    if (t.kind == PROD) { fill_result(m.T, m.ldt, r0, c0, nr, nc); fill_result(m.T, m.ldt, c0, r0, nc, nr); }
-    if (m.U && g.with_u && (t.kind == DIAG || t.kind == (m.X ? INVT : PANEL))) fill_result(m.U, m.ldu, c0, r0, nc, nr);
+    float* const T = g.out ? g.out : m.T;
+    float* const U = m.U && g.out ? g.out : m.U;
+    const int ldt = g.out ? g.ld_out : m.ldt, ldu = g.out ? g.ld_out : m.ldu;
+    if (t.kind == PROD) { fill_result(T, ldt, r0, c0, nr, nc); fill_result(T, ldt, c0, r0, nc, nr); }
+    if (m.U && g.with_u && (t.kind == DIAG || t.kind == (m.X ? INVT : PANEL))) fill_result(U, ldu, c0, r0, nc, nr);
     __syncthreads();
     if (tid == 0 && t.kind != PROD) {
       __threadfence();
@@ -639,9 +650,19 @@ int flow_set_wait_controls(long long cycles, int stall) { return tc::set_wait_co
 int flow_launch(const flow::Args& a, int n_mats, int clear_info, int with_traces, cudaStream_t st) {
   SSO_ENSURE_SMEM(flow::flow_kernel<false>, flow::SMEM);
   SSO_ENSURE_SMEM(flow::flow_kernel<true>, flow::SMEM);
-  flow::begin_kernel<<<n_mats, 256, 0, st>>>(a.mats, n_mats, a.sync, const_cast<float*>(a.traces), a.info, clear_info, with_traces);
+  flow::begin_kernel<<<n_mats, 256, 0, st>>>(a.mats, n_mats, a.sync, const_cast<float*>(a.traces), a.info, clear_info, with_traces, a.src, a.ld_src);
   SSO_LAUNCH_OK("flow begin");
-  (a.rev ? flow::flow_kernel<true> : flow::flow_kernel<false>)<<<a.n_tasks < 148 ? a.n_tasks : 148, flow::THREADS, flow::SMEM, st>>>(a);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(a.n_tasks < 148 ? a.n_tasks : 148);
+  cfg.blockDim = dim3(flow::THREADS);
+  cfg.dynamicSmemBytes = flow::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // set-up beside begin_kernel
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, a.rev ? flow::flow_kernel<true> : flow::flow_kernel<false>, a);
   SSO_LAUNCH_OK("flow_kernel");
   return 0;
 }

@@ -49,6 +49,9 @@ struct Args {
   int* info;                 // nullable
   int* status;
   int with_u;                // whether U is written
+  const float* src;          // nullable: the one matrix of the plan lies here this time, and its result goes to out
+  float* out;
+  int ld_src, ld_out;
   int rev;                   // the matrices are taken from the last row and column to the first
 };
 

@@ -104,6 +104,7 @@ SIGNATURES = {
     'sso_kron_plan_dev_bytes': (c_sz, [c_i32, c_vp, c_i32]),
     'sso_kron_plan_create': (c_i64, [c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_sz, c_i32, c_vp]),
     'sso_kron_plan_run': (c_i32, [c_i64, c_vp, c_vp, c_i32, c_i32, c_vp]),
+    'sso_kron_plan_run_at': (c_i32, [c_i64, c_vp, c_vp, c_i32, c_vp, c_i64, c_vp, c_i64, c_vp]),
     'sso_precond_plan_dev_bytes': (c_sz, [c_i32, c_vp, c_vp]),
     'sso_precond_plan_create': (c_i64, [c_i32] + [c_vp] * 8 + [c_sz, c_i32, c_vp, c_vp]),
     'sso_precond_plan_run': (c_i32, [c_i64, c_vp]),
@@ -903,6 +904,12 @@ def kron_plan_run(plan: Plan, damp_r: torch.Tensor, info: Optional[torch.Tensor]
                   do_std: bool):
     _check(lib().sso_kron_plan_run(plan.handle, _ptr(damp_r), _ptr(info), int(do_inverse), int(do_std),
                                    _stream()))
+
+
+def kron_plan_run_at(plan: Plan, damp_r: torch.Tensor, info: Optional[torch.Tensor], do_inverse: bool, src: torch.Tensor, out: torch.Tensor):
+    d = src.shape[0]
+    _check(lib().sso_kron_plan_run_at(plan.handle, _ptr(damp_r), _ptr(info), int(do_inverse), src.data_ptr(), max(d, src.stride(0)),
+                                      out.data_ptr(), max(d, out.stride(0)), _stream()))
 
 
 def precond_plan(dA, dG, A_inv, G_inv, gw, gb, tmp, device, host_only=False) -> Plan:

@@ -249,6 +249,33 @@ def test_kron_plan_with_std_runs_either_half(nat, pad):
             assert bool((sd[i]._base[:, d:] == 7.0).all()) and bool((dst[i]._base[:, d:] == 7.0).all())
 
 
+@pytest.mark.parametrize('d', [1, 5, 64, 129, 300])
+def test_inv_and_cholesky_read_the_matrix_where_it_lies(nat, d):
+    import torchsso
+    m = spd(d, d, d) + 0.1 * torch.eye(d, device='cuda')
+    wide = torch.full((d, d + 8), float('nan'), device='cuda')
+    views = [m, m.t(), m.double()]
+    for first in (0, 1, 4):
+        wide[:, first:first + d] = m
+        views.append(wide.clone()[:, first:first + d])
+    odd = torch.full((d, d + 3), float('nan'), device='cuda')
+    odd[:, :d] = m
+    views.append(odd[:, :d])
+    inverse = torch.linalg.inv(m.double())
+    upper = torch.linalg.cholesky(m.double(), upper=True)
+    for v in views:
+        before = v.clone()
+        i, u, low = torchsso.utils.inv(v), torchsso.utils.cholesky(v), torchsso.utils.cholesky(v, upper=False)
+        assert i.dtype == torch.float32 and i.is_contiguous() and rel(i, inverse) < 1e-5 and torch.equal(i, i.t())
+        assert rel(u, upper) < 1e-5 and torch.equal(u, u.triu()) and torch.equal(low, u.t())
+        assert torch.equal(v, before)
+    plan, zero, info = torchsso.utils.linalg._solo(d, m.device, False)[0], torch.zeros(1, device='cuda'), torch.zeros(2, dtype=torch.int32, device='cuda')
+    with pytest.raises(RuntimeError):
+        nat.kron_plan_run_at(plan, zero, info, True, m, m)
+    with pytest.raises(RuntimeError):
+        nat.kron_plan_run_at(plan, zero, info, False, m, torch.empty_like(m))      # a plan without factors
+
+
 @pytest.mark.parametrize('at', [0, 127, 128, 290])
 def test_kron_plan_reports_the_bad_pivot(nat, at):
     """One matrix of three is not positive definite: its pivot is named and the others are as they would be without it."""

@@ -162,6 +162,10 @@ class FactorPool:
         """acc <- scale*data (first) or acc + scale*data."""
         self._flat('data', 'acc', scale, 0.0 if first else 1.0, kron, diag)
 
+    def accumulate_last(self, scale: float, kron=None, diag=None):
+        """data <- acc + scale*data."""
+        self._flat('acc', 'data', 1.0, scale, kron, diag)
+
     def take_accumulated(self, kron=None, diag=None):
         """data <- acc."""
         self._flat('acc', 'data', 1.0, 0.0, kron, diag)

@@ -172,6 +172,7 @@ class SecondOrderOptimizer(Optimizer):
         self._grad_view = {p: self._grad_flat[o:o + n].view(p.shape) for p, (o, n) in views.items()}
         self._grad_slot = views
         self._acc_first = True
+        self._acc_in_place = False      # the sum of this step already lies where _take_accumulated puts it
 
     # ------------------------------------------------------------------ gradients
     @property
@@ -284,21 +285,30 @@ class SecondOrderOptimizer(Optimizer):
         if dsts:
             torch._foreach_copy_(dsts, srcs)
 
-    def _accumulate(self, scale: float):
-        if self._grad_acc is None:
-            self._grad_acc = torch.zeros_like(self._grad_flat)
+    def _accumulate(self, scale: float, last: bool = False):
+        """acc <- acc + scale * (this closure's gradients and curvature).  The last of a step's closures is added the
+        other way round, data <- acc + scale * data: the sum lands where it is used, two passes over the pool less."""
         first = self._acc_first
-        nat.axpby(self._grad_flat, self._grad_acc, scale, 0.0 if first else 1.0)
-        self.pool.accumulate(scale, first)
+        in_place = last and (not first or scale == 1.0)
+        if not in_place:
+            if self._grad_acc is None:
+                self._grad_acc = torch.zeros_like(self._grad_flat)
+            nat.axpby(self._grad_flat, self._grad_acc, scale, 0.0 if first else 1.0)
+            self.pool.accumulate(scale, first)
+        elif not first:
+            nat.axpby(self._grad_acc, self._grad_flat, 1.0, scale)
+            self.pool.accumulate_last(scale)
         for group in self.param_groups:
             curv = group['curv']
             if curv is not None and not _is_pooled(curv) and curv.data is not None:
                 group['acc_curv'].update(curv.data, scale=scale)
         self._acc_first = False
+        self._acc_in_place = in_place
 
     def _take_accumulated(self, target='params'):
-        nat.axpby(self._grad_acc, self._grad_flat, 1.0, 0.0)
-        self.pool.take_accumulated()
+        if not self._acc_in_place:
+            nat.axpby(self._grad_acc, self._grad_flat, 1.0, 0.0)
+            self.pool.take_accumulated()
         for group in self.param_groups:
             curv = group['curv']
             if curv is not None and not _is_pooled(curv):
@@ -306,6 +316,7 @@ class SecondOrderOptimizer(Optimizer):
                 if acc is not None:
                     curv.data = acc
         self._acc_first = True
+        self._acc_in_place = False
 
     # ------------------------------------------------------------------ step
     def step(self, closure=None):
@@ -318,7 +329,7 @@ class SecondOrderOptimizer(Optimizer):
             nat.join_curvature_stream(None)
             self._harvest_grads()
             if n > 1:
-                self._accumulate(1.0 / n)
+                self._accumulate(1.0 / n, last=self.optim_state['acc_step'] + 1 >= n)
             self.optim_state['acc_step'] += 1
             if self.optim_state['acc_step'] < n:
                 return loss

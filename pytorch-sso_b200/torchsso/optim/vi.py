@@ -196,14 +196,14 @@ class VIOptimizer(SecondOrderOptimizer):
         acc_prob = TensorAccumulator()
         self.set_random_seed()
 
-        for _ in range(m):
+        for i in range(m):
             self.sample_params()
             loss, output = closure()
             nat.join_curvature_stream(None)
             acc_loss.update(loss.detach(), scale=1 / m)
             acc_prob.update(_probabilities(output.detach()), scale=1 / n)
             self._harvest_grads()
-            self._accumulate(1 / m / n)
+            self._accumulate(1 / m / n, last=i == m - 1 and self.optim_state['acc_step'] + 1 >= n)
 
         loss, prob = acc_loss.get(), acc_prob.get()
         self.optim_state['acc_step'] += 1

@@ -152,6 +152,58 @@ __global__ void __launch_bounds__(256) split_kernel(const FactorParams p, uint32
   }
 }
 
+// The same for NCHW planes whose pixels come in aligned runs of four: a CTA turns 64 pixels x 64 channels, four 16-byte loads
+// per thread in flight.  Quad q of a channel's pixels lies at place q ^ (channel / 8), so that neither the 16-byte stores
+// nor the loads of eight channels of a pixel (lanes: octets, then four pixels) meet a bank conflict.
+__global__ void __launch_bounds__(256) split_planes_kernel(const FactorParams p, uint32_t pixels, int ones_at, int header_words, Parts out_a, Parts out_b) {
+  __shared__ __align__(16) float t[64 * 64];
+  begin_factor(p, header_words);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t px0 = blockIdx.x * 64u, hw = (uint32_t)(p.h * p.w);
+  const int c0 = blockIdx.y * 64;
+  {
+    const int q = tid & 15, c = tid >> 4;
+    const uint32_t px = px0 + 4 * q, n = px / hw;
+    const float* src = reinterpret_cast<const float*>(p.x) + n * p.sn + (px - n * hw) + (c0 + c) * p.sc;
+    float4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int ch = c0 + c + 16 * i;
+      const float fill = ch == ones_at ? 1.f : 0.f;
+      v[i] = make_float4(fill, fill, fill, fill);
+      if (px < pixels && ch < p.c) v[i] = __ldg(reinterpret_cast<const float4*>(src + 16 * i * p.sc));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int ch = c + 16 * i;
+      *reinterpret_cast<float4*>(&t[ch * 64 + ((q ^ (ch >> 3)) << 2)]) = v[i];
+    }
+  }
+  __syncthreads();
+  const int o = lane & 7;
+  if (c0 + 8 * o >= out_a.c8) return;
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const int r = it * 32 + warp * 4 + (lane >> 3);
+    const uint32_t px = px0 + r;
+    if (px >= pixels) return;
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = t[(8 * o + i) * 64 + (((r >> 2) ^ o) << 2) + (r & 3)];
+    const float w = p.weight ? p.weight[px / hw] : 1.f;
+    for (int side = 0; side < (p.weight ? 2 : 1); ++side) {
+      const float f = side == 0 ? w : 1.f;
+      uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) split2(f * v[2 * i], f * v[2 * i + 1], hi[i], mid[i], lo[i]);
+      __nv_bfloat16* d = const_cast<__nv_bfloat16*>(side == 0 ? out_a.a : out_b.b) + (int64_t)px * out_a.c8 + c0 + 8 * o;
+      *reinterpret_cast<uint4*>(d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(d + out_a.stride) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+      *reinterpret_cast<uint4*>(d + 2 * out_a.stride) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+  }
+}
+
 // The same where the channels are contiguous, 16-byte aligned and a multiple of four: a thread takes eight channels of
 // a pixel straight from global memory to global memory.
 __global__ void __launch_bounds__(256) split_direct_kernel(const FactorParams p, uint32_t pixels, int ones_at, int header_words, Parts out_a, Parts out_b) {
@@ -959,6 +1011,9 @@ int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, c
   q.ticket_tiles = s.tiles;
   const bool direct = !s.fold && p.sc == 1 && p.c % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 && p.sn % 4 == 0 &&
                       (p.h == 1 || p.sh % 4 == 0) && (p.w == 1 || p.sw % 4 == 0) && (int64_t)n_run * p.h * s.width * (s.c8 / 8) < ((int64_t)1 << 31);
+  // planes (of more than one pixel) that a thread reads four pixels at a time
+  const bool planes = !s.fold && !direct && p.sw == 1 && p.sh == p.w && p.h * p.w % 4 == 0 && p.sc % 4 == 0 && p.sn % 4 == 0 &&
+                      (reinterpret_cast<uintptr_t>(p.x) & 15) == 0;
   const int header_words = fused ? (int)(hdr / sizeof(int)) : 1;
   for (int r = 0, n0 = 0; r < runs; ++r, n0 += n_run) {
     const int n = std::min(n_run, p.n - n0);
@@ -971,6 +1026,8 @@ int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, c
     if (direct)
       f32::split_direct_kernel<<<(unsigned)ceil_div64(pixels * (s.c8 / 8), 256), 256, 0, st>>>(in, (uint32_t)pixels, ones_at,
                                                                                                             r == 0 ? header_words : 0, parts, parts);
+    else if (planes)
+      f32::split_planes_kernel<<<dim3((unsigned)ceil_div64(pixels, 64), ceil_div(s.c8, 64)), 256, 0, st>>>(in, (uint32_t)pixels, ones_at, r == 0 ? header_words : 0, parts, parts);
     else
       f32::split_kernel<<<dim3((unsigned)ceil_div64(pixels, 32), ceil_div(s.c8, 64)), 256, 0, st>>>(in, (uint32_t)pixels, s.width, s.fold, ones_at,
                                                                                                   r == 0 ? header_words : 0, parts, parts);

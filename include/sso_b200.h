@@ -317,7 +317,8 @@ typedef struct {
   int32_t lda, ldb, ldc, ldc2;
   int32_t m, n, k;
   uint32_t flags;     /* bit0: A transposed, bit1: B transposed, bit2: symmetric square tile (only
-                         its lower half is computed and it is mirrored inside the tile) */
+                         its lower half is computed and it is mirrored inside the tile),
+                         bit3: block of up to 256x256 (phases of kind 6) */
   float alpha, beta;
 } sso_tile_task;
 
@@ -350,7 +351,8 @@ typedef struct {
 
 typedef struct {
   int32_t kind;       /* 0 gemm64, 1 gemm128, 2 diag-block factor (<= 64), 3 copy, 4 gemm128 whose operands are both read along k,
-                         5 diag-block factor of a 128-column panel (same records as 2, size <= 128) */
+                         5 diag-block factor of a 128-column panel (same records as 2, size <= 128),
+                         6 gemm256 (as 4, blocks of 256x256, on the device only) */
   int32_t first;      /* first record of this phase in its table */
   int32_t count;      /* number of records (= CTAs) */
   int32_t reserved;

@@ -31,6 +31,7 @@ namespace sso {
 
 int launch_tile_tasks_tc(const sso_tile_task* tasks_dev, int count, int* status_dev, cudaStream_t st);
 int launch_tile_tasks_kc(const sso_tile_task* tasks_dev, int count, int* status_dev, cudaStream_t st);
+int launch_tile_pairs(const sso_tile_task* tasks_dev, const void* maps_dev, int count, int* status_dev, cudaStream_t st);
 int launch_tile_tasks_tma(const sso_tile_task* tasks_dev, const void* maps_dev, int count, int* status_dev, cudaStream_t st);
 decltype(&cuTensorMapEncodeTiled) tensor_map_encoder();
 bool tma_encode_f32_rows(void* out, const float* base, int64_t rows, int64_t cols, int64_t ld, int box_rows = 128);
@@ -447,6 +448,10 @@ static Plan* find_plan(int64_t h) {
 
 static size_t align_up(size_t v, size_t a = 256) { return (v + a - 1) / a * a; }
 
+struct KRange {      // of a block's operands
+  int first, count;
+};
+
 struct Builder {
   Plan& p;
   std::vector<sso_phase>* phases;
@@ -454,12 +459,12 @@ struct Builder {
   int task_begin() const { return (int)p.tasks.size(); }
   void gemm(const float* A, int lda, bool ta, const float* B, int ldb, bool tb, float* C, int ldc,
             int m, int n, int k, float alpha, float beta, float* C2 = nullptr, int ldc2 = 0,
-            bool symmetric = false) {
+            bool symmetric = false, int block = 128) {
     sso_tile_task t;
     t.A = A; t.B = B; t.C = C; t.C2 = C2;
     t.lda = lda; t.ldb = ldb; t.ldc = ldc; t.ldc2 = ldc2;
     t.m = m; t.n = n; t.k = k;
-    t.flags = (ta ? 1u : 0u) | (tb ? 2u : 0u) | (symmetric ? 4u : 0u);
+    t.flags = (ta ? 1u : 0u) | (tb ? 2u : 0u) | (symmetric ? 4u : 0u) | (block > 128 ? 8u : 0u);
     t.alpha = alpha; t.beta = beta;
     p.tasks.push_back(t);
   }
@@ -468,6 +473,21 @@ struct Builder {
   static bool k_contiguous(const sso_tile_task& t) {
     auto al = [](const void* p, int ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; };
     return (t.flags & 3u) == 2u && al(t.A, t.lda) && al(t.B, t.ldb);
+  }
+  // C <- alpha A[m x k] B[n x k]^T + beta C in blocks: 256x256 if `pairs` allows it and both sides are longer than 128, those at
+  // the edges too (four tiles of 128 take twice as long as one block; strips of tiles beside the blocks would be a launch
+  // of their own, 124 us for the last row of 4609), else 128x128.  The range of K of a block: k_of(i0, block).
+  template <typename K>
+  void blocks(const float* A, int lda, const float* B, int ldb, float* C, int ldc, int m, int n, bool pairs, float alpha, float beta, K k_of) {
+    sso_tile_task probe{};
+    probe.A = A; probe.lda = lda; probe.B = B; probe.ldb = ldb; probe.flags = 2u;
+    const int T = pairs && m > 128 && n > 128 && k_contiguous(probe) ? 256 : 128;
+    for (int i = 0; i < m; i += T) {
+      const KRange r = k_of(i, T);
+      for (int j = 0; j < n; j += T)
+        gemm(A + (int64_t)i * lda + r.first, lda, false, B + (int64_t)j * ldb + r.first, ldb, true, C + (int64_t)i * ldc + j, ldc,
+             std::min(T, m - i), std::min(T, n - j), r.count, alpha, beta, nullptr, 0, false, T);
+    }
   }
   void push_phase(int kind, int first, int count) {
     if (count <= 0) return;
@@ -478,8 +498,17 @@ struct Builder {
   void end_phase(int kind, int first, int count) {
     if (count <= 0) return;
     if (kind != 1) return push_phase(kind, first, count);
-    // the tasks of a phase are independent: run the k-contiguous ones (kind 4) and the rest
-    // (kind 1) as two launches
+    // the tasks of a phase are independent: run blocks of 256 (kind 6), the other k-contiguous ones (kind 4) and the rest
+    // (kind 1) as launches of their own
+    auto is_pair = [](const sso_tile_task& t) { return (t.flags & 8u) != 0; };
+    auto wide = std::stable_partition(p.tasks.begin() + first, p.tasks.begin() + first + count, is_pair);
+    const int npair = (int)(wide - (p.tasks.begin() + first));
+    if (g_phase_lpt)
+      std::stable_sort(p.tasks.begin() + first, wide, [](const sso_tile_task& a, const sso_tile_task& b) { return a.k > b.k; });
+    push_phase(6, first, npair);
+    first += npair;
+    count -= npair;
+    if (count <= 0) return;
     auto mid = std::stable_partition(p.tasks.begin() + first, p.tasks.begin() + first + count, k_contiguous);
     const int nfast = (int)(mid - (p.tasks.begin() + first));
     // CTAs are handed out in task order: longest K first keeps the tail of each launch short
@@ -697,7 +726,7 @@ static int upload(Plan& p, void* dev_mem, size_t dev_bytes) {
     std::vector<unsigned char> maps(p.tasks.size() * 256, 0);
     bool ok = true, any = false;
     auto encode_phase = [&](const sso_phase& ph) {
-      if (ph.kind != 4) return;
+      if (ph.kind != 4 && ph.kind != 6) return;
       for (int i = ph.first; i < ph.first + ph.count && ok; ++i) {
         const sso_tile_task& t = p.tasks[i];
         ok = tma_encode_f32_rows(&maps[(size_t)i * 256], t.A, t.m, t.k, t.lda) &&
@@ -751,6 +780,12 @@ static int run_phases(const Plan& p, const std::vector<sso_phase>& phases, int* 
         }
         tile_task_kernel<8><<<ph.count, 256, 0, st>>>(p.d_tasks + ph.first);
         break;
+      case 6: {
+        if (!p.have_maps) return fail(-5, "no tensor maps for blocks of 256");
+        const int rc = launch_tile_pairs(p.d_tasks + ph.first, p.d_maps + (size_t)ph.first * 256, ph.count, p.d_status, st);
+        if (rc) return rc;
+        continue;
+      }
       case 2: diag_block_kernel<<<ph.count, 256, 0, st>>>(p.d_diags + ph.first, info); break;
       case 5:
         SSO_ENSURE_SMEM((dpanel::diag_panel_kernel), dpanel::SMEM_BYTES);
@@ -1177,13 +1212,22 @@ int sso_kron_plan_run_at(int64_t plan, const float* damp_r_dev, int* info_dev, i
   return run_flow(*p, do_inverse ? p->flow_inv : p->flow_std, damp_r_dev, info_dev, 1, do_inverse != 0, !do_inverse, st, src, ld_src, out, ld_out);
 }
 
+// Whether products of these layers run in blocks of 256: with more than two rounds of 128x128 tiles on the GPU they halve the
+// traffic (ResNet-50: 1584 tiles a phase, VGG-16: 938); with fewer, half as many SMs would work (4608 x 512: 144 tiles, one round).
+static bool pairs_pay(int n, const int64_t* dA, const int64_t* dG) {
+  int64_t tiles = 0;
+  for (int l = 0; l < n; ++l) tiles += ((dA[l] + 127) / 128) * ((dG[l] + 127) / 128);
+  return tiles > 2 * 148 && g_engine_tma && g_engine_tc && tensor_map_encoder() != nullptr;
+}
+
 // ---- precondition --------------------------------------------------------------------------
 static Plan* build_precond(int n, const int64_t* dA, const int64_t* dG, float* const* A_inv,
                            float* const* G_inv, float* const* gw, float* const* gb, float* const* tmp,
-                           const int64_t* ldA, const int64_t* ldG) {
+                           const int64_t* ldA, const int64_t* ldG, bool on_device) {
   Plan* p = new Plan();
   Builder b(*p, &p->run_phases);
   constexpr int T = 128;
+  const bool pairs = on_device && pairs_pay(n, dA, dG);
   // Both factors are symmetric, which lets every operand be read along its contiguous
   // direction (the fast path of the tensor-core tasks):
   //   tmp = U^T = A_inv[:, :wc] * gw^T (+ A_inv[:, wc] * gb^T),   [gw | gb] = G_inv * U.
@@ -1194,10 +1238,7 @@ static Plan* build_precond(int n, const int64_t* dA, const int64_t* dG, float* c
     const int la = ldA ? (int)ldA[l] : a, lg = ldG ? (int)ldG[l] : g;
     const bool bias = gb && gb[l];
     const int wcols = bias ? a - 1 : a;
-    for (int i = 0; i < a; i += T)
-      for (int j = 0; j < g; j += T)
-        b.gemm(A_inv[l] + (int64_t)i * la, la, false, gw[l] + (int64_t)j * wcols, wcols, true,
-               tmp[l] + (int64_t)i * lg + j, lg, std::min(T, a - i), std::min(T, g - j), wcols, 1.f, 0.f);
+    b.blocks(A_inv[l], la, gw[l], wcols, tmp[l], lg, a, g, pairs, 1.f, 0.f, [&](int, int) { return KRange{0, wcols}; });
   }
   b.end_phase(1, first, b.task_begin() - first);
   first = b.task_begin();
@@ -1217,10 +1258,8 @@ static Plan* build_precond(int n, const int64_t* dA, const int64_t* dG, float* c
     const int lg = ldG ? (int)ldG[l] : g;
     const bool bias = gb && gb[l];
     const int wcols = bias ? a - 1 : a;
+    b.blocks(G_inv[l], lg, tmp[l], lg, gw[l], wcols, g, wcols, pairs, 1.f, 0.f, [&](int, int) { return KRange{0, g}; });
     for (int i = 0; i < g; i += T) {
-      for (int j = 0; j < wcols; j += T)
-        b.gemm(G_inv[l] + (int64_t)i * lg, lg, false, tmp[l] + (int64_t)j * lg, lg, true,
-               gw[l] + (int64_t)i * wcols + j, wcols, std::min(T, g - i), std::min(T, wcols - j), g, 1.f, 0.f);
       if (bias)
         b.gemm(G_inv[l] + (int64_t)i * lg, lg, false, tmp[l] + (int64_t)wcols * lg, lg, true,
                gb[l] + i, 1, std::min(T, g - i), 1, g, 1.f, 0.f);
@@ -1247,7 +1286,7 @@ int64_t sso_precond_plan_create(int n_layers, const int64_t* dA, const int64_t* 
   for (int l = 0; l < n_layers; ++l)
     SSO_CHECK_ARG(dA[l] > 0 && dG[l] > 0 && A_inv[l] && G_inv[l] && gw[l] && tmp[l],
                   "precond plan: bad layer %d", l);
-  Plan* p = build_precond(n_layers, dA, dG, A_inv, G_inv, gw, gb, tmp, ldA, ldG);
+  Plan* p = build_precond(n_layers, dA, dG, A_inv, G_inv, gw, gb, tmp, ldA, ldG, !host_only);
   p->host_only = host_only != 0;
   if (!p->host_only) {
     const int rc = upload(*p, dev_mem, dev_mem_bytes);
@@ -1329,6 +1368,7 @@ static Plan* build_sample_along_k(int n, const int64_t* dA, const int64_t* dG, f
   Builder b(*p, &p->run_phases);
   constexpr int T = 128;
   std::vector<float*> tt(n);
+  const bool pairs = pairs_pay(n, dA, dG);
   int first = b.task_begin();
   size_t at = 0;
   for (int l = 0; l < n; ++l) {
@@ -1349,10 +1389,8 @@ static Plan* build_sample_along_k(int n, const int64_t* dA, const int64_t* dG, f
       layout(e, copy, a, g, a, 0, g);
       e = copy;
     }
-    for (int j = 0; j < a; j += T)           // row block j of U_A^T ends with its diagonal block
-      for (int i = 0; i < g; i += T)
-        b.gemm(ut + (int64_t)j * la, la, false, e + (int64_t)i * la, la, true, tt[l] + (int64_t)j * lg + i, lg, std::min(T, a - j),
-               std::min(T, g - i), std::min(a, j + T), 1.f, 0.f);
+    // row block j of U_A^T ends with its diagonal block
+    b.blocks(ut, la, e, la, tt[l], lg, a, g, pairs, 1.f, 0.f, [&](int j, int block) { return KRange{0, std::min(a, j + block)}; });
   }
   b.end_phase(1, first, b.task_begin() - first);
   first = b.task_begin();
@@ -1361,14 +1399,10 @@ static Plan* build_sample_along_k(int n, const int64_t* dA, const int64_t* dG, f
     const int a = (int)dA[l], g = (int)dG[l], lg = padded_ld(g), ldu = ldG ? (int)ldG[l] : g;
     const bool bias = bvec && bvec[l];
     const int wcols = bias ? a - 1 : a;
-    for (int i = 0; i < g; i += T) {         // row block i of U_G starts with its diagonal block
-      const float* u = U_G[l] + (int64_t)i * ldu + i;
-      for (int j = 0; j < wcols; j += T)
-        b.gemm(u, ldu, false, tt[l] + (int64_t)j * lg + i, lg, true, w[l] + (int64_t)i * wcols + j, wcols, std::min(T, g - i),
-               std::min(T, wcols - j), g - i, 1.f, 1.f);
-      if (bias)
-        b.gemm(u, ldu, false, tt[l] + (int64_t)wcols * lg + i, lg, true, bvec[l] + i, 1, std::min(T, g - i), 1, g - i, 1.f, 1.f);
-    }
+    // row block i of U_G starts with its diagonal block
+    b.blocks(U_G[l], ldu, tt[l], lg, w[l], wcols, g, wcols, pairs, 1.f, 1.f, [&](int i, int) { return KRange{i, g - i}; });
+    for (int i = 0; bias && i < g; i += T)
+      b.gemm(U_G[l] + (int64_t)i * ldu + i, ldu, false, tt[l] + (int64_t)wcols * lg + i, lg, true, bvec[l] + i, 1, std::min(T, g - i), 1, g - i, 1.f, 1.f);
   }
   p->n_scaled_tasks = b.task_begin() - first;
   b.end_phase(1, first, b.task_begin() - first);
@@ -1434,6 +1468,11 @@ int64_t sso_sample_plan_create(int n_layers, const int64_t* dA, const int64_t* d
     char* mem = reinterpret_cast<char*>(align_up(reinterpret_cast<uintptr_t>(dev_mem)));
     Plan* p = build_sample_along_k(n_layers, dA, dG, U_A, U_G, noise, w, b, ldA, ldG, mem);
     p->d_layouts = reinterpret_cast<LayoutRec*>(mem + scratch - 256 - align_up(2 * (size_t)n_layers * sizeof(LayoutRec)));
+    // blocks of 256 read the 128x128 block above the diagonal of U_A^T too, which nothing ever writes
+    if (pairs_pay(n_layers, dA, dG) && cudaMemset(mem, 0, scratch - 256) != cudaSuccess) {
+      delete p;
+      return fail(-2, "sample plan: clearing the scratch matrices failed");
+    }
     int rc = upload(*p, mem + scratch - 256, dev_mem_bytes - scratch);
     if (rc == 0 && cudaMemcpy(p->d_layouts, p->layouts.data(), p->layouts.size() * sizeof(LayoutRec), cudaMemcpyHostToDevice) != cudaSuccess)
       rc = fail(-2, "sample plan: copy of the layout records failed");

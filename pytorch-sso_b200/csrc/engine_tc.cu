@@ -18,6 +18,7 @@
 // Every wait is bounded; a timeout sets *status and the task writes nothing.
 #include "common.cuh"
 #include "tc_common.cuh"
+#include "tc_pair.cuh"
 
 namespace sso {
 namespace etc {
@@ -516,7 +517,7 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_kc_kernel(const sso_tile
 // on the host when the plan is built, two per task), so the loads no longer pass through the
 // load/store units.  The load warps only split: A into tensor memory (hi and lo, a row per lane, which
 // takes its part of the operand traffic off shared memory), B's hi in place and lo into a second ring.
-// Bound: the MMAs for large tasks (4608 x 512 preconditioned in 152 us, 287 TFLOP/s), set-up, pipeline fill
+// Bound: the feed of the operands for large tasks (4608 x 512 preconditioned in 152 us, 159 TFLOP/s), set-up, pipeline fill
 // and store of a task (about 10 us) for small ones.  us, with A in shared memory and chunks split one by one / in
 // shared memory / in tensor memory: that layer 175 / 161 / 152, ResNet-50's preconditioning 1122 / 1037 / 1005.
 // ------------------------------------------------------------------------------------------
@@ -683,7 +684,210 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// Blocks of 256x256: a cluster of two CTAs computes one with tcgen05.mma.cta_group::2.  A CTA fetches and splits 128 rows of
+// either operand and its tensor core reads them for 256 columns, so that a stage brings in half the bytes per
+// multiplication of the 128x128 tasks, which are bound by that (32 KB per SM and 0.91 us, 5.2 TB/s over the chip).  Eight
+// accumulate warps (128 sums per thread), one that issues the MMAs (the leader's), one that issues the boxes, eight that
+// split in two groups of every other stage.  Bound: shared memory (224 KB of operand traffic a stage and SM).  us, tiles of
+// 128 / blocks of 256 and what tiles are left: preconditioning of ResNet-50's layers 1010 / 750, of VGG-16's 882 / 673, a
+// posterior draw of VGG-16's 555 / 482.
+// ------------------------------------------------------------------------------------------
+namespace pair {
+constexpr int RAW = 4, LO = 3, BLOCK = 256;
+// five warpgroups: 0-1 accumulate, 2 issues, 3-4 split; they share the block's 640 x 96 registers as 168 + 168 + 32 + 56 + 56
+constexpr int THREADS = 640, PROD_WARP = 9, SPLIT_WARP0 = 12, SPLIT_WARPS = 8;
+constexpr size_t SMEM = (RAW + LO) * PART + 1024;
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+tile_pair_kernel(const sso_tile_task* __restrict__ tasks, const TaskMaps* __restrict__ maps, int* status) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t bars[2 * RAW + 2 * LO + 4];
+  __shared__ uint32_t tmem_base_slot;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // uniform, for setmaxnreg
+  const uint32_t rank = cluster_ctarank();
+  const int task = blockIdx.x >> 1;
+  if (tid == 32 * PROD_WARP) {      // fetched while barriers and TMEM are set up
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(maps[task].a)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(maps[task].b)) : "memory");
+  }
+  const sso_tile_task t = tasks[task];
+  const int nstages = ceil_div(t.k, KS), nchunks = ceil_div(nstages, FLUSH);
+  const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t lo0 = smem0 + RAW * PART;
+  const uint32_t bar0 = smem_u32(bars);
+  auto rawfull = [&](int s) { return bar0 + 8u * s; };
+  auto rawfree = [&](int s) { return bar0 + 8u * (RAW + s); };
+  auto full = [&](int s) { return bar0 + 8u * (2 * RAW + s); };
+  auto lofree = [&](int s) { return bar0 + 8u * (2 * RAW + LO + s); };
+  const uint32_t accfull0 = bar0 + 8u * (2 * RAW + 2 * LO), accempty0 = accfull0 + 16u;
+  if (tid == 0) {
+    for (int s = 0; s < RAW; ++s) { mbar_init(rawfull(s), 1); mbar_init(rawfree(s), 1); }
+    for (int s = 0; s < LO; ++s) { mbar_init(full(s), SPLIT_WARPS); mbar_init(lofree(s), 1); }      // four warps of either CTA
+    for (int b = 0; b < 2; ++b) { mbar_init(accfull0 + 8u * b, 1); mbar_init(accempty0 + 8u * b, 2 * EPI_WARPS); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == MMA_WARP) tmem_alloc2(smem_u32(&tmem_base_slot), TMEM_COLS2);
+  tc_fence_before();
+  cluster_sync_all();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_slot;
+
+  if (warp < EPI_WARPS) {
+    // ------------------------------------------------------------------ accumulate and store
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+    const int q = warp & 3, half = warp >> 2;
+    const uint32_t leader_accempty0 = map_to_cta(accempty0, 0u);
+    float acc[128];
+#pragma unroll
+    for (int i = 0; i < 128; ++i) acc[i] = 0.f;
+    bool ok = true;
+    for (int c = 0; c < nchunks; ++c) {
+      const int b = c & 1;
+      if (!mbar_wait(accfull0 + 8u * b, (c >> 1) & 1, status, 53)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BLOCK + half * 128);
+#pragma unroll
+      for (int part = 0; part < 8; ++part) {
+        uint32_t v[16];
+        tmem_ld16(taddr + part * 16, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[part * 16 + i] += __uint_as_float(v[i]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(leader_accempty0 + 8u * b);
+    }
+    // A wait that gave up leaves the sums incomplete: the block is written all the same, as NaN.  The ring is free: every
+    // MMA has read its operands before the last accumulator was published.
+    const float nan = __int_as_float(0x7fc00000);
+    float* stg = reinterpret_cast<float*>(smem_raw + (smem0 - smem_u32(smem_raw))) + warp * 1024;
+    const int row0 = (int)rank * TILE + q * 32, rows = min(32, t.m - row0);
+#pragma unroll
+    for (int part = 0; part < 4; ++part) {
+      const int col0 = half * 128 + part * 32;
+      if (col0 >= t.n || !ok) break;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) stg[lane * 32 + (i ^ lane)] = t.alpha * acc[part * 32 + i];
+      __syncwarp();
+      const int c = col0 + lane;
+      float* o = t.C + (int64_t)row0 * t.ldc + c;
+      if (c < t.n) {
+        for (int r0 = 0; r0 < rows; r0 += 8) {
+          float old[8];
+          if (t.beta != 0.f) {        // eight rows in flight before the first store
+#pragma unroll
+            for (int j = 0; j < 8; ++j) old[j] = r0 + j < rows ? o[(int64_t)(r0 + j) * t.ldc] : 0.f;
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int r = r0 + j;
+            if (r >= rows) break;
+            const float v = stg[r * 32 + (lane ^ r)];
+            o[(int64_t)r * t.ldc] = t.beta != 0.f ? fmaf(t.beta, old[j], v) : v;
+          }
+        }
+      }
+      __syncwarp();
+    }
+    if (!ok)
+      for (int r = 0; r < rows; ++r)
+        for (int c = half * 128 + lane; c < min(half * 128 + 128, t.n); c += 32) t.C[(int64_t)(row0 + r) * t.ldc + c] = nan;
+  } else if (warp < SPLIT_WARP0) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");      // one instruction for the whole warpgroup
+    if (warp == MMA_WARP && lane == 0 && rank == 0) {
+      const uint32_t idesc = instr_desc_pair(2u, 0u);   // tf32, K-major
+      bool ok = true;
+      for (int s = 0; s < nstages; ++s) {
+        const int rs = s % RAW, ls = s % LO, c = s / FLUSH, b = c & 1;
+        const bool first_of_chunk = (s % FLUSH) == 0;
+        if (first_of_chunk && c >= 2) ok = mbar_wait(accempty0 + 8u * b, ((c >> 1) - 1) & 1, status, 52);
+        if (ok) ok = mbar_wait(full(ls), (s / LO) & 1, status, 51);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t ah = smem0 + rs * PART, bh = ah + OPB, al = lo0 + ls * PART, bl = al + OPB;
+        const uint32_t d_tmem = tmem_base + (uint32_t)(b * BLOCK);
+#pragma unroll
+        for (int ks = 0; ks < KS / 8; ++ks) {
+          const uint64_t adh = smem_desc_sw128_kmajor(ah + ks * 32u), adl = smem_desc_sw128_kmajor(al + ks * 32u);
+          const uint64_t bdh = smem_desc_sw128_kmajor(bh + ks * 32u), bdl = smem_desc_sw128_kmajor(bl + ks * 32u);
+          umma2<true>(d_tmem, adl, bdh, idesc, (first_of_chunk && ks == 0) ? 0u : 1u);
+          umma2<true>(d_tmem, adh, bdl, idesc, 1u);
+          umma2<true>(d_tmem, adh, bdh, idesc, 1u);
+        }
+        umma2_commit_both(rawfree(rs));
+        umma2_commit_both(lofree(ls));
+        if ((s % FLUSH) == FLUSH - 1 || s == nstages - 1) umma2_commit_both(accfull0 + 8u * b);
+      }
+    } else if (warp == PROD_WARP && lane == 0 && !g_inject_stall) {      // stalled: nothing is ever loaded
+      const uint64_t map_a = reinterpret_cast<uint64_t>(maps[task].a), map_b = reinterpret_cast<uint64_t>(maps[task].b);
+      const int row = (int)rank * TILE;
+      int s = 0;
+      for (; s < nstages; ++s) {
+        const int rs = s % RAW;
+        if (s >= RAW && !mbar_wait(rawfree(rs), ((s / RAW) - 1) & 1, status, 54)) break;
+        const uint32_t fb = rawfull(rs), dst = smem0 + rs * PART;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(PART) : "memory");
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(dst), "l"(map_a), "r"(s * KS), "r"(row), "r"(fb) : "memory");
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(dst + OPB), "l"(map_b), "r"(s * KS), "r"(row), "r"(fb) : "memory");
+      }
+      ring_landed<RAW>(s, rawfull, status, 57);
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ split warps
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    const int group = (warp - SPLIT_WARP0) >> 2;
+    const uint32_t at0 = sw_off(32 * (warp & 3) + lane, 0);      // a thread has this row of both operands; chunk j: bits 4 to 6 xor j
+    const uint32_t leader_full0 = map_to_cta(full(0), 0u);
+    for (int s = group; s < nstages; s += 2) {
+      const int rs = s % RAW, ls = s % LO;
+      if (!mbar_wait(rawfull(rs), (s / RAW) & 1, status, 56)) break;
+      if (s >= LO && !mbar_wait(lofree(ls), ((s / LO) - 1) & 1, status, 55)) break;
+#pragma unroll 1
+      for (int side = 0; side < 2; ++side) {
+        const uint32_t hi = smem0 + rs * PART + side * OPB + at0, lo = lo0 + ls * PART + side * OPB + at0;
+        // all loads before the first store: one chunk at a time, each would wait for the one before.  hi is rounded to
+        // nearest (see tile_task_tma_kernel)
+        float4 v[KS / 4];
+#pragma unroll
+        for (int j = 0; j < KS / 4; ++j)
+          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w) : "r"(hi ^ (j << 4)));
+#pragma unroll
+        for (int j = 0; j < KS / 4; ++j) {
+          const uint32_t h0 = rna_tf32(v[j].x), h1 = rna_tf32(v[j].y), h2 = rna_tf32(v[j].z), h3 = rna_tf32(v[j].w);
+          const uint32_t l0 = __float_as_uint(v[j].x - __uint_as_float(h0)), l1 = __float_as_uint(v[j].y - __uint_as_float(h1));
+          const uint32_t l2 = __float_as_uint(v[j].z - __uint_as_float(h2)), l3 = __float_as_uint(v[j].w - __uint_as_float(h3));
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(hi ^ (j << 4)), "r"(h0), "r"(h1), "r"(h2), "r"(h3) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(lo ^ (j << 4)), "r"(l0), "r"(l1), "r"(l2), "r"(l3) : "memory");
+        }
+      }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(leader_full0 + 8u * ls);
+    }
+  }
+  tc_fence_before();
+  cluster_sync_all();          // neither CTA leaves while its peer's MMAs may still read its shared memory
+  if (warp == MMA_WARP) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc2(tmem_base, TMEM_COLS2);
+  }
+}
+}  // namespace pair
+
 }  // namespace etc
+
+int launch_tile_pairs(const sso_tile_task* tasks_dev, const void* maps_dev, int count, int* status_dev, cudaStream_t st) {
+  SSO_ENSURE_SMEM(etc::pair::tile_pair_kernel, etc::pair::SMEM);
+  etc::pair::tile_pair_kernel<<<2 * count, etc::pair::THREADS, etc::pair::SMEM, st>>>(tasks_dev, reinterpret_cast<const etc::TaskMaps*>(maps_dev), status_dev);
+  SSO_LAUNCH_OK("tile_pair_kernel");
+  return 0;
+}
 
 int engine_tc_set_wait_controls(long long cycles, int stall) { return tc::set_wait_controls(cycles, stall); }
 

@@ -349,6 +349,41 @@ def test_sample_plan_along_k(nat, shapes, bias):
         assert rel(got, want[i]) < 2e-6
 
 
+# enough layers for blocks of 256 (more than two rounds of 128x128 tiles): strips of up to 128 rows or columns beside them,
+# blocks that are not full, layers without a block, rows that cannot be read with TMA
+WIDE = [(260, 260), (384, 129), (513, 640), (1152, 385), (2308, 1024), (516, 255), (128, 640), (2304, 513), (641, 300), (256, 256)]
+
+
+@pytest.mark.parametrize('bias', [False, True])
+def test_sample_plan_in_wide_blocks(nat, bias):
+    test_sample_plan_along_k(nat, WIDE, bias)
+
+
+@pytest.mark.parametrize('bias', [False, True])
+def test_precond_plan_in_wide_blocks(nat, bias):
+    shapes = [(a + int(bias), g) for a, g in WIDE]
+
+    def inverse(d, seed):
+        m = torch.full((d, (d + 3) // 4 * 4), float('nan'), device='cuda')
+        x = torch.randn(d, d, device='cuda')
+        m[:, :d] = x + x.t()
+        return m[:, :d]
+    A, G = [inverse(a, a) for a, _ in shapes], [inverse(g, g + 1) for _, g in shapes]
+    w = [torch.randn(g, a - int(bias), device='cuda') for a, g in shapes]
+    b = [torch.randn(g, device='cuda') if bias else None for _, g in shapes]
+    tmp = [torch.empty(a * max(m.stride(0), g), device='cuda') for (a, g), m in zip(shapes, G)]
+    want = []
+    for i in range(len(shapes)):
+        grad = w[i] if b[i] is None else torch.cat([w[i], b[i][:, None]], 1)
+        want.append(G[i].double() @ grad.double() @ A[i].double())
+    plan = nat.precond_plan([a for a, _ in shapes], [g for _, g in shapes], A, G, w, b, tmp, torch.device('cuda'))
+    nat.precond_plan_run(plan)
+    assert plan.status() == 0
+    for i in range(len(shapes)):
+        got = w[i] if b[i] is None else torch.cat([w[i], b[i][:, None]], 1)
+        assert rel(got, want[i]) < 2e-6, shapes[i]
+
+
 @pytest.mark.parametrize('cfg', [(128, 4096, 1, 1, (1, 1), (1, 1), (0, 0), (1, 1), True), (1, 300, 1, 1, (1, 1), (1, 1), (0, 0), (1, 1), False),
                                  (4, 512, 7, 7, (3, 3), (1, 1), (1, 1), (1, 1), True), (1, 256, 40, 40, (1, 1), (2, 2), (0, 0), (1, 1), False),
                                  (2, 4, 30, 30, (11, 11), (4, 4), (2, 2), (1, 1), True), (1, 64, 224, 224, (3, 3), (1, 1), (1, 1), (1, 1), False)])

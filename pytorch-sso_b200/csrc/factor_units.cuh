@@ -12,6 +12,8 @@
 // this one went by output rows and read each element of the lower triangle again for its mirror, four bytes at a time,
 // or scattered four-byte stores.  Whole factors, us: fp32 512 channels 3x3 on 4x4 (d 4609, 128 images) 375 -> 323, adding
 // to a running average 443 -> 356; bf16 512 channels 3x3 on 7x7 (d 4608, 32 images) 170 -> 123 and 234 -> 152.
+// Items taken apart by shifts and results written 16 bytes at a time: the finishing of VGG-16's factors (four samples)
+// 1508 -> 1238, of ResNet-50's 504 -> 427.
 #pragma once
 #include "common.cuh"
 #include "factor_params.cuh"
@@ -93,16 +95,42 @@ __device__ __forceinline__ float4 sum_splits(const float* __restrict__ src, int 
   return add4(a, b);
 }
 
-// One direction of a unit: rows x cols of the result from (row0, col0) on; at(r, c) gives an element's sum.
-template <typename At>
-__device__ __forceinline__ void write_block(const Problem& u, int row0, int col0, int rows, int cols, bool bad, At at) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+// One direction of a unit: rows x cols of the result from (row0, col0) on; an element's sum is s[r][c], or s[c][r] in the other
+// direction.  Four columns at a time where the result allows 16-byte accesses.
+template <bool TURNED>
+__device__ __forceinline__ void write_block(const Problem& u, int row0, int col0, int rows, int cols, float alpha, const float* __restrict__ s, int pitch) {
+  auto at = [&](int r, int c) { return TURNED ? s[c * pitch + r] : s[r * pitch + c]; };
   float* base = u.out + (int64_t)row0 * u.ldo + col0;
-  const float nanv = __int_as_float(0x7fc00000);
+  if (cols % 4 == 0 && u.ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0) {
+    const int quads = cols >> 2, dr = (int)blockDim.x / quads, dq = (int)blockDim.x - dr * quads;
+    int r = (int)threadIdx.x / quads, q = (int)threadIdx.x - r * quads;
+    while (r < rows) {
+      float4 old[4];
+      int rr[4], c[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {        // old values before the first store, so that the four are in flight together
+        rr[j] = r;
+        c[j] = 4 * q;
+        if (u.beta != 0.f && r < rows) old[j] = *reinterpret_cast<const float4*>(base + (int64_t)r * u.ldo + c[j]);
+        r += dr;
+        q += dq;
+        if (q >= quads) { q -= quads; ++r; }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (rr[j] >= rows) break;
+        float4 v = make_float4(alpha * at(rr[j], c[j]), alpha * at(rr[j], c[j] + 1), alpha * at(rr[j], c[j] + 2), alpha * at(rr[j], c[j] + 3));
+        if (u.beta != 0.f) v = make_float4(fmaf(u.beta, old[j].x, v.x), fmaf(u.beta, old[j].y, v.y), fmaf(u.beta, old[j].z, v.z), fmaf(u.beta, old[j].w, v.w));
+        *reinterpret_cast<float4*>(base + (int64_t)rr[j] * u.ldo + c[j]) = v;
+      }
+    }
+    return;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int r0 = warp; r0 < rows; r0 += 4 * nw) {
     for (int c = lane; c < cols; c += 32) {
       float old[4];
-      if (u.beta != 0.f) {        // before the first store, so that the four are in flight together
+      if (u.beta != 0.f) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) old[j] = r0 + j * nw < rows ? base[(int64_t)(r0 + j * nw) * u.ldo + c] : 0.f;
       }
@@ -110,8 +138,7 @@ __device__ __forceinline__ void write_block(const Problem& u, int row0, int col0
       for (int j = 0; j < 4; ++j) {
         const int r = r0 + j * nw;
         if (r >= rows) break;
-        float v = u.alpha * at(r, c);
-        if (bad) v = nanv;
+        const float v = alpha * at(r, c);
         base[(int64_t)r * u.ldo + c] = u.beta == 0.f ? v : fmaf(u.beta, old[j], v);
       }
     }
@@ -131,15 +158,18 @@ __device__ __forceinline__ void finish(const Problem& u, int unit, float* __rest
   };
   // lanes: rows (up to eight), then the lanes of a sum, then column groups, then the rest of the rows
   const int rbits = min(B < 8 ? 2 : 3, 5 - u.lanes), rsub = 1 << rbits, sub_n = 1 << u.lanes;
-  const int quads = B / 4, per_pair = quads * (B >> rbits), pairs = kk * kk;
-  const int n = (pairs * per_pair) << (rbits + u.lanes);
+  // a unit's side is a power of two, so that an item is taken apart by shifts; the pair of kernel positions (below 56 * 56)
+  // by a multiplication.  With divisions the kernel was bound by its instructions (69 % of the issue slots)
+  const int quad_bits = __ffs(B) - 3, pair_bits = quad_bits + __ffs(B) - 1 - rbits, pairs = kk * kk;
+  const uint32_t inv_kk = (1u << 20) / (uint32_t)kk + 1u;
+  const int n = pairs << (pair_bits + rbits + u.lanes);
   const int r_lo = tid & (rsub - 1), sub = (tid >> rbits) & (sub_n - 1);
 #pragma unroll 2
   for (int t0 = tid & ~31; t0 < n; t0 += nt) {
     const int w = (t0 + (tid & 31)) >> (rbits + u.lanes);
-    const int pair = w / per_pair, e = w - pair * per_pair;
-    const int q = e % quads, r = (e / quads) << rbits | r_lo;
-    int k1 = pair / kk, k2 = pair - k1 * kk;
+    const int pair = w >> pair_bits, e = w & ((1 << pair_bits) - 1);
+    const int q = e & ((1 << quad_bits) - 1), r = (e >> quad_bits) << rbits | r_lo;
+    const int k1 = (int)(((uint32_t)pair * inv_kk) >> 20), k2 = pair - k1 * kk;
     bool valid = pair < pairs && sub < u.splits && !(diag && k1 < k2);
     const bool below = k1 >= k2;
     const int ri = below ? k1 * u.c + I * B + r : k2 * u.c + J * B + r;
@@ -170,10 +200,11 @@ __device__ __forceinline__ void finish(const Problem& u, int unit, float* __rest
   }
   __syncthreads();
   const bool bad = status && *status != 0;
+  const float alpha = bad ? __int_as_float(0x7fc00000) : u.alpha;      // NaN in place of a result whose kernel gave up
   const int row0 = I * E, col0 = J * E, rows = min(E, u.pub * kk - row0), cols = min(E, u.pub * kk - col0);
-  write_block(u, row0, col0, rows, cols, bad, [&](int r, int c) { return s[r * pitch + c]; });
+  write_block<false>(u, row0, col0, rows, cols, alpha, s, pitch);
   if (!diag) {
-    write_block(u, col0, row0, cols, rows, bad, [&](int r, int c) { return s[c * pitch + r]; });
+    write_block<true>(u, col0, row0, cols, rows, alpha, s, pitch);
     return;
   }
   // the ones column of a k x k window: its row and column next to this block, and the corner
@@ -185,8 +216,7 @@ __device__ __forceinline__ void finish(const Problem& u, int unit, float* __rest
     const float* src = at(u.dcols, c);
     float v = 0.f;
     for (int sp = 0; sp < u.splits; ++sp) v += src[(int64_t)sp * (128 * 128)];
-    v *= u.alpha;
-    if (bad) v = __int_as_float(0x7fc00000);
+    v *= alpha;
     float* o1 = u.out + (int64_t)last * u.ldo + col;
     float* o2 = u.out + (int64_t)col * u.ldo + last;
     const float v1 = u.beta != 0.f ? fmaf(u.beta, *o1, v) : v, v2 = u.beta != 0.f ? fmaf(u.beta, *o2, v) : v;

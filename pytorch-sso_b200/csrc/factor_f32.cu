@@ -80,37 +80,21 @@ __device__ __forceinline__ void begin_factor(const FactorParams& p, int header_w
 }
 
 // A CTA turns 32 pixels x 64 channels: read with the lanes along whichever of the two is contiguous, staged in shared
-// memory, written as 16-byte chunks of eight channels.  With few channels the kernel's columns are folded into them:
-// channel kx*c + ch of pixel (y, ox) is x[ch][y][ox*stride + kx*dil - pad], so that three channels under a 7x7 window
-// are 7 x 24 columns and not 49 x 8.
-__global__ void __launch_bounds__(256) split_kernel(const FactorParams p, uint32_t pixels, int width, int fold, int ones_at, int header_words,
-                                                    Parts out_a, Parts out_b) {
+// memory, written as 16-byte chunks of eight channels.
+__global__ void __launch_bounds__(256) split_kernel(const FactorParams p, uint32_t pixels, int ones_at, int header_words, Parts out_a, Parts out_b) {
   __shared__ __align__(16) float t[32][68];
   begin_factor(p, header_words);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t px0 = blockIdx.x * 32u;
   const int c0 = blockIdx.y * 64;
   const float* x = reinterpret_cast<const float*>(p.x);
-  const int hw = p.h * width;      // pixels of an image
+  const int hw = p.h * p.w;        // pixels of an image
   auto offset = [&](uint32_t px) {
     const uint32_t n = px / (uint32_t)hw;
-    const int rem = (int)(px - n * hw), y = rem / width;
-    return n * p.sn + y * p.sh + (rem - y * width) * p.sw;
+    const int rem = (int)(px - n * hw), y = rem / p.w;
+    return n * p.sn + y * p.sh + (rem - y * p.w) * p.sw;
   };
-  if (fold) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const uint32_t px = px0 + lane;
-      const int cf = c0 + warp + 8 * i, kx = cf / p.c, ch = cf - kx * p.c;
-      float v = 0.f;
-      if (px < pixels && kx < fold) {
-        const uint32_t n = px / (uint32_t)hw;
-        const int rem = (int)(px - n * hw), y = rem / width, ix = (rem - y * width) * p.stride_w + kx * p.dil_w - p.pad_w;
-        if ((unsigned)ix < (unsigned)p.w) v = __ldg(x + n * p.sn + y * p.sh + ix * p.sw + ch * p.sc);
-      }
-      t[lane][warp + 8 * i] = v;
-    }
-  } else if (p.sc <= (p.w > 1 ? p.sw : p.h > 1 ? p.sh : p.sn)) {      // lanes along the channels
+  if (p.sc <= (p.w > 1 ? p.sw : p.h > 1 ? p.sh : p.sn)) {      // lanes along the channels
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const uint32_t px = px0 + warp + 8 * i;
@@ -146,6 +130,40 @@ __global__ void __launch_bounds__(256) split_kernel(const FactorParams p, uint32
       split2(f * v.z, f * v.w, hi[2 * i + 1], mid[2 * i + 1], lo[2 * i + 1]);
     }
     __nv_bfloat16* d = const_cast<__nv_bfloat16*>(side == 0 ? out_a.a : out_b.b) + (int64_t)px * out_a.c8 + c0 + o;
+    *reinterpret_cast<uint4*>(d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(d + out_a.stride) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+    *reinterpret_cast<uint4*>(d + 2 * out_a.stride) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+}
+
+// With few channels the kernel's columns are folded into them: channel kx*c + ch of pixel (y, ox) is
+// x[ch][y][ox*stride + kx*dil - pad], so that three channels under a 7x7 window are 7 x 24 columns and not 49 x 8.  A thread takes
+// eight of a pixel's folded channels from global memory to global memory; neighbouring pixels read the same lines
+// (staged in shared memory, 32 pixels x 64 channels per CTA, the stem of ResNet-50 left most threads without a channel).
+__global__ void __launch_bounds__(256) split_folded_kernel(const FactorParams p, uint32_t pixels, int width, int fold, int header_words, Parts out_a, Parts out_b) {
+  begin_factor(p, header_words);
+  const int oct = out_a.c8 / 8, hw = p.h * width;
+  const uint32_t i = blockIdx.x * 256u + threadIdx.x, px = i / (uint32_t)oct;
+  if (px >= pixels) return;
+  const int cf0 = (int)(i - px * oct) * 8;
+  const uint32_t n = px / (uint32_t)hw;
+  const int rem = (int)(px - n * hw), y = rem / width, x0 = (rem - y * width) * p.stride_w - p.pad_w;
+  const float* src = reinterpret_cast<const float*>(p.x) + n * p.sn + y * p.sh;
+  int kx = cf0 / p.c, ch = cf0 - kx * p.c;
+  float v[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int ix = x0 + kx * p.dil_w;
+    v[k] = kx < fold && (unsigned)ix < (unsigned)p.w ? __ldg(src + ix * p.sw + ch * p.sc) : 0.f;
+    if (++ch == p.c) { ch = 0; ++kx; }
+  }
+  const float w = p.weight ? p.weight[n] : 1.f;
+  for (int side = 0; side < (p.weight ? 2 : 1); ++side) {
+    const float f = side == 0 ? w : 1.f;
+    uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) split2(f * v[2 * k], f * v[2 * k + 1], hi[k], mid[k], lo[k]);
+    __nv_bfloat16* d = const_cast<__nv_bfloat16*>(side == 0 ? out_a.a : out_b.b) + (int64_t)px * out_a.c8 + cf0;
     *reinterpret_cast<uint4*>(d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<uint4*>(d + out_a.stride) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
     *reinterpret_cast<uint4*>(d + 2 * out_a.stride) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
@@ -1028,9 +1046,10 @@ int factor_f32_launch(FactorParams p, void* workspace, size_t workspace_bytes, c
                                                                                                             r == 0 ? header_words : 0, parts, parts);
     else if (planes)
       f32::split_planes_kernel<<<dim3((unsigned)ceil_div64(pixels, 64), ceil_div(s.c8, 64)), 256, 0, st>>>(in, (uint32_t)pixels, ones_at, r == 0 ? header_words : 0, parts, parts);
+    else if (s.fold)
+      f32::split_folded_kernel<<<(unsigned)ceil_div64(pixels * (s.c8 / 8), 256), 256, 0, st>>>(in, (uint32_t)pixels, s.width, s.fold, r == 0 ? header_words : 0, parts, parts);
     else
-      f32::split_kernel<<<dim3((unsigned)ceil_div64(pixels, 32), ceil_div(s.c8, 64)), 256, 0, st>>>(in, (uint32_t)pixels, s.width, s.fold, ones_at,
-                                                                                                  r == 0 ? header_words : 0, parts, parts);
+      f32::split_kernel<<<dim3((unsigned)ceil_div64(pixels, 32), ceil_div(s.c8, 64)), 256, 0, st>>>(in, (uint32_t)pixels, ones_at, r == 0 ? header_words : 0, parts, parts);
     SSO_LAUNCH_OK("split_kernel");
     q.n = n;
     q.weight = in.weight;

@@ -128,10 +128,13 @@ class VIOptimizer(SecondOrderOptimizer):
         drawn layer by layer in param_group order; all Kronecker layers are then transformed in
         one batched plan."""
         batches, diag = {}, {}
+        # copies of all layers go to the device together: one layer's parameters fill a quarter of the GPU
+        to, source = [], []
         for group in self.param_groups:
             params, mean, curv = group['params'], group['mean'], group['curv']
             if curv is None or curv.std is None:
-                torch._foreach_copy_([p.data for p in params], mean)
+                to += [p.data for p in params]
+                source += mean
                 continue
             fast = (isinstance(curv, (_KronFactors, _DiagSq, _DiagBatchNorm)) and _is_pooled(curv) and
                     all(p.data.is_contiguous() and p.dtype == torch.float32 for p in params))
@@ -148,14 +151,20 @@ class VIOptimizer(SecondOrderOptimizer):
                 u += curv.std
                 continue
             buf = self._noise_buf(group)
-            buf.copy_(torch.randn_like(buf))
-            torch._foreach_copy_([p.data for p in params], mean)
+            to.append(buf)
+            source.append(torch.randn_like(buf))
+            to += [p.data for p in params]
+            source += mean
             c, t, nz = batches.setdefault(float(group['std_scale']), ([], [], []))
             c.append(curv)
             t.append([p.data for p in params])
             nz.append(buf)
+        for p, m, _, _ in diag.values():
+            to += p
+            source += m
+        if to:
+            torch._foreach_copy_(to, source)
         for scale, (p, m, e, u) in diag.items():
-            torch._foreach_copy_(p, m)
             torch._foreach_addcmul_(p, e, u, value=scale)
         for scale, (c, t, nz) in batches.items():
             self.pool.sample(c, t, nz, scale)
@@ -215,8 +224,8 @@ class VIOptimizer(SecondOrderOptimizer):
         self.optim_state['step'] += 1
         groups = self.local_param_groups
         self._update_groups(groups, 'mean', True, lambda g: g['std_scale'] > 0)
-        for group in groups:
-            torch._foreach_copy_([p.data for p in group['params']], group['mean'])
+        if groups:
+            torch._foreach_copy_([p.data for group in groups for p in group['params']], [m for group in groups for m in group['mean']])
         self.adjust_kl_weighting()
         return loss, prob
 

@@ -1341,6 +1341,12 @@ __global__ void __launch_bounds__(256) layout_kernel(const LayoutRec* __restrict
     const int j = j0 + y + 4 * u;
     if (j < r.cols && i0 + x < r.rows) r.dst[(int64_t)j * r.ld_dst + i0 + x] = tile[x][y + 4 * u];
   }
+  if (bj != bi + 1 || (bi & 1)) return;      // across the diagonal of a block of 256: read by tile_pair_kernel, zero
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {
+    const int i = i0 + y + 4 * u;
+    if (i < r.rows && j0 + x < r.cols) r.dst[(int64_t)i * r.ld_dst + j0 + x] = 0.f;
+  }
 }
 
 // Scratch of a layer in the program below: U_A^T, the noise (if copied), (E U_A)^T.
@@ -1468,11 +1474,6 @@ int64_t sso_sample_plan_create(int n_layers, const int64_t* dA, const int64_t* d
     char* mem = reinterpret_cast<char*>(align_up(reinterpret_cast<uintptr_t>(dev_mem)));
     Plan* p = build_sample_along_k(n_layers, dA, dG, U_A, U_G, noise, w, b, ldA, ldG, mem);
     p->d_layouts = reinterpret_cast<LayoutRec*>(mem + scratch - 256 - align_up(2 * (size_t)n_layers * sizeof(LayoutRec)));
-    // blocks of 256 read the 128x128 block above the diagonal of U_A^T too, which nothing ever writes
-    if (pairs_pay(n_layers, dA, dG) && cudaMemset(mem, 0, scratch - 256) != cudaSuccess) {
-      delete p;
-      return fail(-2, "sample plan: clearing the scratch matrices failed");
-    }
     int rc = upload(*p, mem + scratch - 256, dev_mem_bytes - scratch);
     if (rc == 0 && cudaMemcpy(p->d_layouts, p->layouts.data(), p->layouts.size() * sizeof(LayoutRec), cudaMemcpyHostToDevice) != cudaSuccess)
       rc = fail(-2, "sample plan: copy of the layout records failed");

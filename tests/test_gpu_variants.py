@@ -355,8 +355,15 @@ WIDE = [(260, 260), (384, 129), (513, 640), (1152, 385), (2308, 1024), (516, 255
 
 
 @pytest.mark.parametrize('bias', [False, True])
-def test_sample_plan_in_wide_blocks(nat, bias):
-    test_sample_plan_along_k(nat, WIDE, bias)
+def test_sample_plan_in_wide_blocks(nat, bias, monkeypatch):
+    make = nat.sample_plan
+
+    def plan_of_nans(dA, *args):
+        plan = make(dA, *args)
+        plan._dev_mem[:dA[0] * ((dA[0] + 3) // 4 * 4) * 4].fill_(255)      # the first U_A^T: only what a run writes may be read
+        return plan
+    monkeypatch.setattr(nat, 'sample_plan', plan_of_nans)
+    test_sample_plan_along_k(nat, WIDE[4:5] + WIDE[:4] + WIDE[5:], bias)
 
 
 @pytest.mark.parametrize('bias', [False, True])

@@ -59,6 +59,22 @@ int ensure_dynamic_smem(const void* kernel, int bytes);
     if (rc__) return rc__;                                                               \
   } while (0)
 
+// A launch whose kernel may be set up while the one before it still runs; it waits for that one's end itself (griddepcontrol.wait).
+template <typename... Args>
+inline void launch_early(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <typename T>
 __device__ __forceinline__ float to_f32(T v);
 template <>

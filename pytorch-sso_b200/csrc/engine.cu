@@ -66,6 +66,8 @@ __global__ void __launch_bounds__(256) tile_task_kernel(const sso_tile_task* __r
   constexpr int PER = TILE * KT / 256;  // elements per thread per operand per stage
   __shared__ __align__(16) float As[KT * TILE];
   __shared__ __align__(16) float Bs[KT * TILE];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");      // a phase may be launched beside the one before (launch_early)
   const sso_tile_task t = tasks[blockIdx.x];
   const int tid = threadIdx.x;
   const bool ta = t.flags & 1u, tb = t.flags & 2u;
@@ -761,7 +763,7 @@ __global__ void fold_status_kernel(const int* __restrict__ status, int* __restri
 static int run_phases(const Plan& p, const std::vector<sso_phase>& phases, int* info, cudaStream_t st) {
   for (const sso_phase& ph : phases) {
     switch (ph.kind) {
-      case 0: tile_task_kernel<4><<<ph.count, 256, 0, st>>>(p.d_tasks + ph.first); break;
+      case 0: launch_early(tile_task_kernel<4>, dim3(ph.count), 256, 0, st, (const sso_tile_task*)(p.d_tasks + ph.first)); break;
       case 1:
         if (g_engine_tc) {
           const int rc = launch_tile_tasks_tc(p.d_tasks + ph.first, ph.count, p.d_status, st);

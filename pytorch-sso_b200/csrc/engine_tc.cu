@@ -537,6 +537,8 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(maps[blockIdx.x].a)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(maps[blockIdx.x].b)) : "memory");
   }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");      // launched beside the phase before: its results, and a scale in the tasks, are there
   const sso_tile_task t = tasks[blockIdx.x];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nstages = ceil_div(t.k, KS);
@@ -711,8 +713,6 @@ tile_pair_kernel(const sso_tile_task* __restrict__ tasks, const TaskMaps* __rest
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(maps[task].a)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(maps[task].b)) : "memory");
   }
-  const sso_tile_task t = tasks[task];
-  const int nstages = ceil_div(t.k, KS), nchunks = ceil_div(nstages, FLUSH);
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t lo0 = smem0 + RAW * PART;
   const uint32_t bar0 = smem_u32(bars);
@@ -732,6 +732,10 @@ tile_pair_kernel(const sso_tile_task* __restrict__ tasks, const TaskMaps* __rest
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");      // as in tile_task_tma_kernel
+  const sso_tile_task t = tasks[task];
+  const int nstages = ceil_div(t.k, KS), nchunks = ceil_div(nstages, FLUSH);
 
   if (warp < EPI_WARPS) {
     // ------------------------------------------------------------------ accumulate and store
@@ -884,7 +888,7 @@ tile_pair_kernel(const sso_tile_task* __restrict__ tasks, const TaskMaps* __rest
 
 int launch_tile_pairs(const sso_tile_task* tasks_dev, const void* maps_dev, int count, int* status_dev, cudaStream_t st) {
   SSO_ENSURE_SMEM(etc::pair::tile_pair_kernel, etc::pair::SMEM);
-  etc::pair::tile_pair_kernel<<<2 * count, etc::pair::THREADS, etc::pair::SMEM, st>>>(tasks_dev, reinterpret_cast<const etc::TaskMaps*>(maps_dev), status_dev);
+  launch_early(etc::pair::tile_pair_kernel, dim3(2 * count), etc::pair::THREADS, etc::pair::SMEM, st, tasks_dev, reinterpret_cast<const etc::TaskMaps*>(maps_dev), status_dev);
   SSO_LAUNCH_OK("tile_pair_kernel");
   return 0;
 }
@@ -895,7 +899,7 @@ int launch_tile_tasks_tma(const sso_tile_task* tasks_dev, const void* maps_dev, 
   constexpr int RAW = 5, LO = 3;
   const size_t smem = (size_t)RAW * etc::PART + (size_t)LO * etc::OPB + 1024;
   SSO_ENSURE_SMEM((etc::tile_task_tma_kernel<RAW, LO, 3>), smem);
-  etc::tile_task_tma_kernel<RAW, LO, 3><<<count, etc::THREADS, smem, st>>>(tasks_dev, reinterpret_cast<const etc::TaskMaps*>(maps_dev), status_dev);
+  launch_early(etc::tile_task_tma_kernel<RAW, LO, 3>, dim3(count), etc::THREADS, smem, st, tasks_dev, reinterpret_cast<const etc::TaskMaps*>(maps_dev), status_dev);
   SSO_LAUNCH_OK("tile_task_tma_kernel");
   return 0;
 }

@@ -423,22 +423,6 @@ int factor_tc_launch(FactorParams p, int dtype, void* workspace, size_t workspac
   return fail(-1, "unknown dtype %d", dtype);
 }
 
-// A finishing kernel may be set up while its producer still runs (it waits for the producer's end itself).
-template <typename... Args>
-static void launch_early(void (*kernel)(Args...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 int factor_tc_run_reduce(const FactorParams& p, int tiles, cudaStream_t st) {
   if (units::supported(p)) {
     const units::Problem u = units::plan(p, 148);

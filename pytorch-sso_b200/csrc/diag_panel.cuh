@@ -21,10 +21,10 @@
 // (non-positive, denormal or NaN) is recorded once per matrix (LAPACK numbering) and replaced by 1, like the 64-wide
 // kernel does for non-positive ones.
 // Measured: a 16x16 block in 1500 clocks (2280 with a reciprocal square root, a select and the scaling of the column on the
-// chain between two pivots, and with the entries above the diagonal cleared); 128 rows in 12.5 us before that (before the
-// elimination went in two steps of eight and took the next block from registers 14.4); a chain of four barriers per panel with all warps in step and the inverse by three levels of
-// doubling afterwards took 23.  Inside the dataflow kernel (1000 columns) 402 us with that one, 265 now; elimination and
-// products are straight-line code that issues an instruction in about four clocks.
+// chain between two pivots, and with the entries above the diagonal cleared), 128 rows in 22610 clocks (26270).  Before
+// the elimination went in two steps of eight and took the next block from registers 14.4 us; a chain of four barriers per
+// panel with all warps in step and the inverse by three levels of doubling afterwards took 23.  Elimination and products
+// are straight-line code that issues an instruction in three to four clocks.
 #pragma once
 #include "common.cuh"
 

@@ -537,3 +537,57 @@ def test_vi_step_at_fixed_draws(nat, monkeypatch):
         ia, ig = (m.double() for m in g['curv'].inv)
         raw = flat(grad_sum[2 * j:2 * j + 2]) + g['l2_reg'] * mean[j]
         assert rel(flat(g['mean']) - mean[j], -0.05 * ig @ raw @ ia) < 1e-3, j
+
+# ------------------------------------------------------------------------------------------- accumulation
+@pytest.mark.parametrize('numel,shift', [(3, 0), (4097, 0), (100003, 1)])
+@pytest.mark.parametrize('scale', [1 / 3, 1 / 6, 0.2, 0.5])
+def test_a_scaled_sum_is_rounded_once_whichever_side_it_lies_on(nat, numel, shift, scale):
+    terms, total = torch.randn(numel + shift, device='cuda')[shift:], torch.randn(numel + shift, device='cuda')[shift:]
+    want = total.clone()
+    nat.axpby(terms, want, scale, 1.0)
+    nat.axpby(total, terms, 1.0, scale)
+    assert torch.equal(terms, want)
+
+
+@pytest.mark.parametrize('samples,micro_steps', [(0, 3), (1, 1), (1, 3), (3, 1), (5, 2)])
+def test_the_closures_of_a_step_are_added_one_by_one(nat, monkeypatch, samples, micro_steps):
+    """Gradients and factors of a step against the fp64 sum over its closures (weight samples, micro-steps, both): one fused
+    multiply-add for each."""
+    import torch.nn as nn
+    import torch.nn.functional as F
+    import torchsso
+    model = nn.Sequential(nn.Linear(200, 300), nn.Tanh(), nn.Linear(300, 10)).cuda()
+    x, y = torch.randn(64, 200, device='cuda'), torch.randint(0, 10, (64,), device='cuda')
+    shapes, kw = {'Linear': 'Kron'}, {'ema_decay': 0.9, 'damping': 1e-2}
+    if samples:
+        opt = torchsso.optim.VIOptimizer(model, 500, 'Cov', shapes, kw, lr=1e-3, num_mc_samples=samples, acc_steps=micro_steps)
+    else:
+        opt = torchsso.optim.SecondOrderOptimizer(model, 'Cov', shapes, kw, lr=1e-3, acc_steps=micro_steps)
+    n = max(samples, 1) * micro_steps
+    scale = torch.tensor(1 / max(samples, 1) / micro_steps, dtype=torch.float32).double().item()      # the kernels' scale
+    terms, sums = [], []
+    accumulate, take = opt._accumulate, opt._take_accumulated
+
+    def both():
+        return torch.cat([opt._grad_flat, *(m.flatten() for g in opt.param_groups for m in g['curv'].data)])
+    monkeypatch.setattr(opt, '_accumulate', lambda *a, **k: (terms.append(both()), accumulate(*a, **k)))
+    monkeypatch.setattr(opt, '_take_accumulated', lambda *a, **k: (take(*a, **k), sums.append(both())))
+
+    def closure():
+        opt.zero_grad()
+        out = model(x[torch.randperm(64, device='cuda')[:32]])
+        loss = F.cross_entropy(out, y[:32])
+        loss.backward()
+        return loss, out
+    for step in range(2):
+        terms.clear()
+        sums.clear()
+        for _ in range(micro_steps):
+            opt.step(closure=closure)
+        assert len(terms) == n and len(sums) == 1
+        fused = (scale * terms[0].double()).float()
+        for t in terms[1:]:
+            fused = (scale * t.double() + fused.double()).float()
+        exact = sum(scale * t.double() for t in terms)
+        assert (sums[0] != fused).double().mean() < 1e-4      # but for what a second rounding of the emulation does
+        assert rel(sums[0], exact) < 1.01 * rel(fused, exact) + 1e-12

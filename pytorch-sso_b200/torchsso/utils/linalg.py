@@ -6,28 +6,38 @@ torchsso/utils/cholesky_cupy.py:9-14, executed by the tile-task engine of libsso
 Both are one-matrix conveniences; the optimizers invert all layers in one batched plan."""
 from __future__ import annotations
 
+from collections import OrderedDict
+
 import torch
 
 from .. import _native as nat
 
-_cache = {}
+_cache = OrderedDict()      # a plan for each size, device and direction, the one that was used longest ago first
+_LIMIT = 34                 # inverses and factors of 17 sizes
 
 
 def _solo(d: int, device, upper: bool):
     key = (d, device.index, upper)      # a plan that can factor inverts in reverse order, which an inverse alone need not pay for
     ent = _cache.get(key)
-    if ent is None:
-        src, dst = (torch.empty((d, d), dtype=torch.float32, device=device) for _ in range(2))
+    if ent is not None:
+        _cache.move_to_end(key)
+        return ent
+    zero = torch.zeros(1, dtype=torch.float32, device=device)
+    info = torch.zeros(2, dtype=torch.int32, device=device)
+    direct = not nat.kron_plan_uses_work()
+    src = dst = std = None
+    if direct:
+        # every run brings its matrix and its result (_run): the plan has none of its own, and these addresses are not used
+        none = [zero.data_ptr()]
+        plan = nat.kron_plan([d], none, none, None, none if upper else None, [-1], [0], device, lds=[d])
+    else:
+        src, dst, work = (torch.empty((d, d), dtype=torch.float32, device=device) for _ in range(3))
         std = torch.empty_like(src) if upper else None
-        direct = not nat.kron_plan_uses_work()
-        work = None if direct else [torch.empty_like(src)]
-        plan = nat.kron_plan([d], [src], [dst], work, [std] if upper else None, [-1], [0], device)
-        zero = torch.zeros(1, dtype=torch.float32, device=device)
-        info = torch.zeros(2, dtype=torch.int32, device=device)
-        ent = (plan, src, dst, std, zero, info, direct)
-        if len(_cache) > 16:
-            _cache.clear()
-        _cache[key] = ent
+        plan = nat.kron_plan([d], [src], [dst], [work], [std] if upper else None, [-1], [0], device)
+    ent = (plan, src, dst, std, zero, info, direct)
+    while len(_cache) >= _LIMIT:
+        _cache.popitem(last=False)
+    _cache[key] = ent
     return ent
 
 
@@ -41,8 +51,8 @@ def _run(m: torch.Tensor, upper: bool) -> torch.Tensor:
     # read where it lies, if the kernel can read it as fast as a copy
     aligned = m.data_ptr() % 16 == 0 and m.stride(0) % 4 == 0 or m.shape[0] % 4 != 0
     if m.dtype != torch.float32 or m.stride(1) != 1 or not m.shape[0] <= m.stride(0) < 1 << 31 or not aligned:
-        m = src.copy_(m)
-    out = torch.empty_like(src)
+        m = torch.empty(m.shape, dtype=torch.float32, device=m.device).copy_(m)
+    out = torch.empty(m.shape, dtype=torch.float32, device=m.device)
     nat.kron_plan_run_at(plan, zero, info, not upper, m, out)
     return out
 

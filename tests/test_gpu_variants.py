@@ -591,3 +591,25 @@ def test_the_closures_of_a_step_are_added_one_by_one(nat, monkeypatch, samples, 
         exact = sum(scale * t.double() for t in terms)
         assert (sums[0] != fused).double().mean() < 1e-4      # but for what a second rounding of the emulation does
         assert rel(sums[0], exact) < 1.01 * rel(fused, exact) + 1e-12
+
+# ------------------------------------------------------------------------------------------- one matrix
+def test_inv_and_cholesky_of_many_sizes_keep_their_plans(nat, monkeypatch):
+    """A dozen sizes, each inverted and factored: their plans are made once, and hold little beside their scratch."""
+    import torchsso
+    from torchsso.utils import linalg
+    made, make = [], nat.kron_plan
+    monkeypatch.setattr(nat, 'kron_plan', lambda dims, *a, **k: (made.append(dims[0]), make(dims, *a, **k))[1])
+    mats = [spd(d, d, d) + 0.1 * torch.eye(d, device='cuda') for d in range(200, 212)]
+    linalg._cache.clear()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    for _ in range(3):
+        for m in mats:
+            assert rel(torchsso.utils.inv(m), torch.linalg.inv(m.double())) < 1e-5
+            assert rel(torchsso.utils.cholesky(m), torch.linalg.cholesky(m.double(), upper=True)) < 1e-5
+    assert len(made) == 2 * len(mats), made
+    # two plans of a size: a scratch matrix, two diagonal blocks, tables
+    assert torch.cuda.memory_allocated() - before < sum(2 * (212 * 212 + 2 * 128 * 128) * 4 + (96 << 10) for _ in mats)
+    for d in range(300, 360):      # the cache has a limit
+        torchsso.utils.inv(torch.eye(d, device='cuda'))
+    assert len(linalg._cache) <= 40

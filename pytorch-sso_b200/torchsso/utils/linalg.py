@@ -50,7 +50,7 @@ def _run(m: torch.Tensor, upper: bool) -> torch.Tensor:
         return (std if upper else dst).clone()
     # read where it lies, if the kernel can read it as fast as a copy
     aligned = m.data_ptr() % 16 == 0 and m.stride(0) % 4 == 0 or m.shape[0] % 4 != 0
-    if m.dtype != torch.float32 or m.stride(1) != 1 or not m.shape[0] <= m.stride(0) < 1 << 31 or not aligned:
+    if m.dtype != torch.float32 or m.is_neg() or m.stride(1) != 1 or not m.shape[0] <= m.stride(0) < 1 << 31 or not aligned:
         m = torch.empty(m.shape, dtype=torch.float32, device=m.device).copy_(m)
     out = torch.empty(m.shape, dtype=torch.float32, device=m.device)
     nat.kron_plan_run_at(plan, zero, info, not upper, m, out)

@@ -613,3 +613,12 @@ def test_inv_and_cholesky_of_many_sizes_keep_their_plans(nat, monkeypatch):
     for d in range(300, 360):      # the cache has a limit
         torchsso.utils.inv(torch.eye(d, device='cuda'))
     assert len(linalg._cache) <= 40
+
+
+def test_inv_and_cholesky_of_a_negated_view(nat):
+    import torchsso
+    m = spd(130, 130, 0) + 0.1 * torch.eye(130, device='cuda')
+    v = torch._neg_view(-m)
+    assert v.is_neg() and torch.equal(v, m)
+    assert torch.equal(torchsso.utils.inv(v), torchsso.utils.inv(m))
+    assert torch.equal(torchsso.utils.cholesky(v), torchsso.utils.cholesky(m))

@@ -753,6 +753,12 @@ static int upload(Plan& p, void* dev_mem, size_t dev_bytes) {
   return 0;
 }
 
+// The copies of a plan's tables are on the default stream, its runs need not be: they start when the tables are there.
+static int tables_landed() {
+  SSO_CUDA_OK(cudaStreamSynchronize(cudaStreamLegacy));
+  return 0;
+}
+
 // A tensor-core tile task whose bounded wait gave up has set the plan's status word (and written NaN
 // tiles); surface it through the LAPACK-style info array the caller already reads: info[0] = -(1000 + code).
 __global__ void fold_status_kernel(const int* __restrict__ status, int* __restrict__ info) {
@@ -1149,6 +1155,7 @@ int64_t sso_kron_plan_create(int n_mats, const int64_t* dims, float* const* src,
       char* q = head + scratch - 256 + align_up(tables);
       if (!rc) rc = upload_flow(p->flow_inv, q);
       if (!rc && std_out) rc = upload_flow(p->flow_std, q);
+      if (!rc) rc = tables_landed();
       if (rc) { delete p; return rc; }
       return register_plan(p);
     }
@@ -1158,7 +1165,8 @@ int64_t sso_kron_plan_create(int n_mats, const int64_t* dims, float* const* src,
   Plan* p = build_kron(n_mats, dims, src, dst, work, std_out, partner, role, xb.data(), lds);
   p->host_only = host_only != 0;
   if (!p->host_only) {
-    const int rc = upload(*p, reinterpret_cast<char*>(dev_mem) + scratch, dev_mem_bytes - scratch);
+    int rc = upload(*p, reinterpret_cast<char*>(dev_mem) + scratch, dev_mem_bytes - scratch);
+    if (!rc) rc = tables_landed();
     if (rc != 0) { delete p; return rc; }
   }
   return register_plan(p);
@@ -1293,7 +1301,8 @@ int64_t sso_precond_plan_create(int n_layers, const int64_t* dA, const int64_t* 
   Plan* p = build_precond(n_layers, dA, dG, A_inv, G_inv, gw, gb, tmp, ldA, ldG, !host_only);
   p->host_only = host_only != 0;
   if (!p->host_only) {
-    const int rc = upload(*p, dev_mem, dev_mem_bytes);
+    int rc = upload(*p, dev_mem, dev_mem_bytes);
+    if (!rc) rc = tables_landed();
     if (rc != 0) { delete p; return rc; }
   }
   return register_plan(p);
@@ -1481,13 +1490,15 @@ int64_t sso_sample_plan_create(int n_layers, const int64_t* dA, const int64_t* d
     int rc = upload(*p, mem + scratch - 256, dev_mem_bytes - scratch);
     if (rc == 0 && cudaMemcpy(p->d_layouts, p->layouts.data(), p->layouts.size() * sizeof(LayoutRec), cudaMemcpyHostToDevice) != cudaSuccess)
       rc = fail(-2, "sample plan: copy of the layout records failed");
+    if (rc == 0) rc = tables_landed();
     if (rc != 0) { delete p; return rc; }
     return register_plan(p);
   }
   Plan* p = build_sample(n_layers, dA, dG, U_A, U_G, noise, w, b, tmp, ldA, ldG);
   p->host_only = host_only != 0;
   if (!p->host_only) {
-    const int rc = upload(*p, dev_mem, dev_mem_bytes);
+    int rc = upload(*p, dev_mem, dev_mem_bytes);
+    if (!rc) rc = tables_landed();
     if (rc != 0) { delete p; return rc; }
   }
   return register_plan(p);

@@ -872,6 +872,15 @@ def _lds(*lists):
     return _i64(out)
 
 
+def _plan_memory(nbytes: int, device) -> torch.Tensor:
+    """Memory of a plan.  Its tables are written by copies of the default stream: on another one, what is still queued
+    on this memory from its last owner would come behind them."""
+    mem = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
+    if _stream() and not torch.cuda.is_current_stream_capturing():
+        torch.cuda.current_stream().synchronize()
+    return mem
+
+
 def kron_plan_uses_work() -> bool:
     return bool(lib().sso_kron_plan_uses_work())
 
@@ -890,7 +899,7 @@ def kron_plan(dims, src, dst, work, std, partner, role, device, host_only=False,
         mem = None
         mem_ptr = host_mem.ctypes.data
     else:
-        mem = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
+        mem = _plan_memory(nbytes, device)
         mem_ptr = mem.data_ptr()
     h = L.sso_kron_plan_create(n, d, _ptrs(src), _ptrs(dst), None if work is None else _ptrs(work),
                                None if std is None else _ptrs(std), _i32(partner), _i32(role),
@@ -917,7 +926,7 @@ def precond_plan(dA, dG, A_inv, G_inv, gw, gb, tmp, device, host_only=False) -> 
     n = len(dA)
     a, g = _i64(dA), _i64(dG)
     nbytes = L.sso_precond_plan_dev_bytes(n, a, g)
-    mem = None if host_only else torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
+    mem = None if host_only else _plan_memory(nbytes, device)
     h = L.sso_precond_plan_create(n, a, g, _ptrs(A_inv), _ptrs(G_inv), _ptrs(gw), _ptrs(gb), _ptrs(tmp),
                                   _ptr(mem), nbytes, int(host_only), _lds(A_inv), _lds(G_inv))
     return Plan(h, mem, (A_inv, G_inv, gw, gb, tmp))
@@ -936,7 +945,7 @@ def sample_plan(dA, dG, U_A, U_G, noise, w, b, tmp, device, host_only=False) -> 
     n = len(dA)
     a, g = _i64(dA), _i64(dG)
     nbytes = L.sso_sample_plan_dev_bytes(n, a, g)
-    mem = None if host_only else torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
+    mem = None if host_only else _plan_memory(nbytes, device)
     h = L.sso_sample_plan_create(n, a, g, _ptrs(U_A), _ptrs(U_G), _ptrs(noise), _ptrs(w), _ptrs(b),
                                  None if tmp is None else _ptrs(tmp), _ptr(mem), nbytes, int(host_only), _lds(U_A), _lds(U_G))
     return Plan(h, mem, (U_A, U_G, noise, w, b, tmp))

@@ -622,3 +622,40 @@ def test_inv_and_cholesky_of_a_negated_view(nat):
     assert v.is_neg() and torch.equal(v, m)
     assert torch.equal(torchsso.utils.inv(v), torchsso.utils.inv(m))
     assert torch.equal(torchsso.utils.cholesky(v), torchsso.utils.cholesky(m))
+
+
+@pytest.mark.parametrize('kind', ['inverse', 'precondition', 'sample'])
+def test_a_plan_made_on_a_stream_of_its_own(nat, kind):
+    """Its memory was a tensor's before, whose last kernel is still queued on that stream: the tables come behind it."""
+    d = 640
+    a, g, e = spd(d, d, 0) + torch.eye(d, device='cuda'), spd(d, d, 1), torch.randn(d, d, device='cuda')
+    dims, device, zero = nat._i64([d]), torch.device('cuda'), torch.zeros(1, device='cuda')
+    ua, ug, w, out, tmp = a.triu(), g.triu(), torch.zeros(d, d, device='cuda'), torch.empty(d, d, device='cuda'), torch.empty(d * d, device='cuda')
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        nbytes = (nat.lib().sso_kron_plan_dev_bytes(1, dims, 0) if kind == 'inverse' else
+                  nat.lib().sso_precond_plan_dev_bytes(1, dims, dims) if kind == 'precondition' else
+                  nat.lib().sso_sample_plan_dev_bytes(1, dims, dims))
+        before = torch.empty(nbytes, dtype=torch.uint8, device='cuda')
+        address = before.data_ptr()
+        torch.cuda._sleep(40000000)
+        before.fill_(255)
+        del before
+        if kind == 'inverse':
+            plan = nat.kron_plan([d], [a], [out], [tmp.view(d, d)], None, [-1], [0], device)
+            nat.kron_plan_run(plan, zero, None, True, False)
+        elif kind == 'precondition':
+            w.copy_(e)
+            plan = nat.precond_plan([d], [d], [a], [g], [w], [None], [tmp], device)
+            nat.precond_plan_run(plan)
+        else:
+            plan = nat.sample_plan([d], [d], [ua], [ug], [e], [w], [None], [tmp] if nat.sample_plan_uses_tmp() else None, device)
+            nat.sample_plan_run(plan, 0.5)
+    assert plan._dev_mem.data_ptr() == address      # the case that is meant
+    stream.synchronize()
+    a, g, e, ua, ug = (t.double() for t in (a, g, e, ua, ug))
+    if kind == 'inverse':
+        assert rel(out, torch.linalg.inv(a)) < 1e-5
+    else:
+        assert rel(w, g @ e @ a if kind == 'precondition' else 0.5 * ug @ e @ ua) < 2e-6

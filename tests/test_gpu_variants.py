@@ -659,3 +659,58 @@ def test_a_plan_made_on_a_stream_of_its_own(nat, kind):
         assert rel(out, torch.linalg.inv(a)) < 1e-5
     else:
         assert rel(w, g @ e @ a if kind == 'precondition' else 0.5 * ug @ e @ ua) < 2e-6
+
+
+@pytest.mark.parametrize('threads', [False, True])
+@pytest.mark.parametrize('d', [64, 500])
+def test_inv_and_cholesky_on_several_streams(nat, d, threads):
+    """Different matrices of one size on two streams at a time, issued by one thread or by one for each."""
+    import threading
+    import torchsso
+    mats = [spd(d, d, i) + (0.1 + i) * torch.eye(d, device='cuda') for i in range(4)]
+    want = [(torchsso.utils.inv(m), torchsso.utils.cholesky(m)) for m in mats]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream(), torch.cuda.Stream()], {}
+
+    def work(s, repeats):
+        with torch.cuda.stream(streams[s]):
+            for r in range(repeats):
+                for i in (s, s + 2):
+                    got[s, r, i] = torchsso.utils.inv(mats[i]), torchsso.utils.cholesky(mats[i])
+    if threads:
+        workers = [threading.Thread(target=work, args=(s, 25)) for s in range(2)]
+        for t in workers:
+            t.start()
+        for t in workers:
+            t.join()
+    else:
+        for r in range(25):
+            for s in range(2):
+                work(s, 1)
+                got.update({(s, r + 1, i): got[s, 0, i] for i in (s, s + 2)})
+    torch.cuda.synchronize()
+    assert len(got) >= 100
+    for (s, r, i), (a, u) in got.items():
+        assert torch.equal(a, want[i][0]) and torch.equal(u, want[i][1])
+
+
+def test_inv_in_a_graph_keeps_its_plan(nat):
+    """Replayed after other sizes have been through the cache, and beside calls of the same size."""
+    import torchsso
+    from torchsso.utils import linalg
+    d = 150
+    m = spd(d, d, 0) + 0.1 * torch.eye(d, device='cuda')
+    torchsso.utils.inv(m)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = torchsso.utils.inv(m)
+    for size in range(400, 400 + linalg._LIMIT + 1):
+        torchsso.utils.inv(torch.eye(size, device='cuda'))
+    for i in range(3):
+        fresh = spd(d, d, i) + 0.1 * torch.eye(d, device='cuda')
+        m.copy_(fresh)
+        graph.replay()
+        other = torchsso.utils.inv(2 * fresh)
+        want = torch.linalg.inv(fresh.double())
+        assert rel(out, want) < 1e-5 and rel(other, want / 2) < 1e-5
+    assert (d, m.device.index, False) in linalg._cache and (d, m.device.index, False) in linalg._captured

@@ -361,6 +361,7 @@ typedef struct {
 /* Batched pi-damped SPD inverse (and optional upper Cholesky factor of the result).
  *   for matrix i:  M_i = src_i + v_i * I,  v_i = r_i * pi  (role 0, "A")  or  r_i / pi  (role 1, "G")
  *                  pi  = sqrt( (tr A / d_A) / (tr G / d_G) ) of the pair (i, partner_i); partner -1 => pi = 1
+ *                  of src_i only the lower triangle is read
  *                  dst_i <- M_i^-1 (both triangles);   std_i <- U with U^T U = dst_i (upper), if requested
  * Replaces: torchsso/curv/curvature.py:302-312 and :334-340 (pi, add_value_to_diagonal),
  *           torchsso/utils/inv_cupy.py:27-132 (cuSOLVER potrf + potrs against identity),

@@ -364,30 +364,22 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
         const int gr = r0 + row, gc = c0 + col0;
         const float* const src = g.src ? g.src : m.src;
         const int ld_src = g.src ? g.ld_src : m.ld_src;
-        const bool vec = ld_src % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && gc + 64 <= d;
         if (REV) {
-          // row and column d - 1 - i; the padding rows come first and are those of an identity
-          const int row_p = d - 1 - gr;
-          if (row_p >= m.pub) {
+          // element (d - 1 - gc - i, d - 1 - gr), which lies in the lower triangle as (gr, gc + i) does: a row of it for the lanes
+          // of a warp; the padding rows come first and are those of an identity
+          const int col_p = d - 1 - gr;
+          if (col_p >= m.pub) {
 #pragma unroll
             for (int i = 0; i < 64; ++i) acc[i] = gc + i == gr ? 1.f : 0.f;
-          } else if (row_p >= 0) {
-            const float* p = src + (int64_t)row_p * ld_src + (d - 1 - gc);
-            if (vec && (gc > 0 || d == m.pub)) {
+          } else if (col_p >= 0) {
+            const float* p = src + (int64_t)(d - 1 - gc) * ld_src + col_p;
 #pragma unroll
-              for (int i = 0; i < 64; i += 4) {
-                const float4 v = __ldcg(reinterpret_cast<const float4*>(p - i - 3));
-                acc[i] = v.w; acc[i + 1] = v.z; acc[i + 2] = v.y; acc[i + 3] = v.x;
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 64; ++i)
-                if (gc + i < d && d - 1 - gc - i < m.pub) acc[i] = __ldcg(p - i);
-            }
+            for (int i = 0; i < 64; ++i, p -= ld_src)
+              if (gc + i < d && d - 1 - gc - i < m.pub) acc[i] = __ldcg(p);
           }
         } else if (gr < d) {
           const float* p = src + (int64_t)gr * ld_src + gc;
-          if (vec) {
+          if (ld_src % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && gc + 64 <= d) {
 #pragma unroll
             for (int i = 0; i < 64; i += 4) {
               const float4 v = __ldcg(reinterpret_cast<const float4*>(p + i));

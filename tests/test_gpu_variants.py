@@ -714,3 +714,36 @@ def test_inv_in_a_graph_keeps_its_plan(nat):
         want = torch.linalg.inv(fresh.double())
         assert rel(out, want) < 1e-5 and rel(other, want / 2) < 1e-5
     assert (d, m.device.index, False) in linalg._cache and (d, m.device.index, False) in linalg._captured
+
+
+@pytest.mark.parametrize('flow', [1, 0])
+@pytest.mark.parametrize('std', [False, True])
+@pytest.mark.parametrize('pad', [0, 1, 4])
+def test_kron_plan_reads_the_lower_triangle(nat, std, pad, flow):
+    """Nothing above the diagonal is looked at, with sampling factors (in reverse order) or without."""
+    nat.configure('flow', flow)
+    try:
+        _lower_triangle(nat, std, pad)
+    finally:
+        nat.configure('flow', 1)
+
+
+def _lower_triangle(nat, std, pad):
+    dims = [1, 2, 5, 16, 66, 127, 129, 130, 257, 400]
+    full = [spd(d, d + pad, i) for i, d in enumerate(dims)]
+    src = []
+    for m, d in zip(full, dims):
+        lower = torch.full((d, d + pad), float('nan'), device='cuda')[:, :d]
+        i, j = torch.tril_indices(d, d, device='cuda')
+        lower[i, j] = m[i, j]
+        src.append(lower)
+    dst, work, sd = ([torch.full((d, d + pad), 7.0, device='cuda')[:, :d] for d in dims] for _ in range(3))
+    plan = nat.kron_plan(dims, src, dst, work, sd if std else None, [-1] * len(dims), [0] * len(dims), torch.device('cuda'))
+    info = torch.zeros(2 * len(dims), dtype=torch.int32, device='cuda')
+    nat.kron_plan_run(plan, torch.full((len(dims),), 0.1, device='cuda'), info, True, std)
+    assert not info.any()
+    for i, d in enumerate(dims):
+        want = torch.linalg.inv(full[i].double() + 0.1 * torch.eye(d, device='cuda', dtype=torch.float64))
+        assert rel(dst[i], want) < 1e-5, d
+        if std:
+            assert rel(sd[i], torch.linalg.cholesky(want, upper=True)) < 1e-5, d

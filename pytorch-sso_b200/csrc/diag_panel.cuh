@@ -43,7 +43,7 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// MUFU.RCP alone (1 ulp); the same
+// MUFU.RCP alone (1 ulp); the same, but that it gives 0 above 2^126 (eliminate_large)
 __device__ __forceinline__ float rcp_approx(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -140,6 +140,32 @@ constexpr Schedule make_schedule() {
 }
 static __constant__ Schedule c_schedule = make_schedule();
 
+// A 16x16 block with an element above 2^125 on its diagonal, whose reciprocal may be no normal number: columns are scaled by
+// reciprocal square roots before they are subtracted.  In shared memory and slow, for matrices near the largest float only.  D: the
+// block, then L; V: L^-1.  Returns the bad pivots, a bit each.
+__device__ __forceinline__ uint32_t eliminate_large(float* __restrict__ D, float* __restrict__ V, int lane) {
+  const int l = lane & 15, h = lane >> 4;
+  float* const row = h ? V + l : D + l * PP;      // as in eliminate: a row of the block, or a column of the inverse
+  const int step = h ? PP : 1;
+#pragma unroll 1
+  for (int c = 0; h && c < PK; ++c) row[c * step] = c == l ? 1.f : 0.f;
+  uint32_t bad_pivots = 0;
+#pragma unroll 1
+  for (int j = 0; j < PK; ++j) {
+    __syncwarp();
+    const float pv = D[j * PP + j];
+    const bool bad = !(pv >= 1.17549435e-38f);
+    if (bad) bad_pivots |= 1u << j;
+    const float pivot = bad ? 1.f : pv, x = (lane == j ? pivot : row[j * step]) * rsqrt_approx(pivot);
+    __syncwarp();
+    row[j * step] = x;
+    __syncwarp();
+#pragma unroll 1
+    for (int c = j + 1; c < PK; ++c) row[c * step] = fmaf(-x, D[c * PP + j], row[c * step]);
+  }
+  return bad_pivots;
+}
+
 // The elimination of panel k's diagonal block by one warp.  The block's entries above the diagonal are not looked at.
 __device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restrict__ V, int k, int n, int* __restrict__ info, int first, int dir, int lane) {
   const int l = lane & 15, h = lane >> 4, c0 = PK * k;
@@ -152,10 +178,20 @@ __device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restri
 #pragma unroll
     for (int i = 0; i < 4; ++i) v[q + i] = h ? (q + i == l ? 1.f : 0.f) : d[i];
   }
+  auto report = [&](uint32_t bad_pivots) {
+    if (!bad_pivots || lane != 0 || !info) return;
+    const int bad = __ffs(bad_pivots) - 1;
+    if (c0 + bad < n) atomicCAS(info, 0, first + dir * (c0 + bad));
+  };
+  const bool large = __any_sync(0xffffffffu, D[l * PP + l] > 0x1p125f);      // no pivot is larger than what it began as
   uint32_t bad_pivots = 0;
 #pragma unroll
   for (int j0 = 0; j0 < PK; j0 += 8) {
     if (j0 > 0) {
+      if (large) {      // asked here, when the answer has long been there; nothing has been stored yet
+        report(eliminate_large(D, V + c0 * PP + c0, lane));
+        return;
+      }
       // the first eight columns from the other eight, all at once: rows 8 to 15 of them by way of shared memory (a
       // shuffle costs more than four cycles, 64 of them more than the sixteen loads)
       if (lane >= 8 && lane < 16) {
@@ -205,10 +241,7 @@ __device__ __forceinline__ void eliminate(float* __restrict__ S, float* __restri
 #pragma unroll
     for (int q = 0; q < PK; q += 4) st4(D + l * PP + q, v[q], v[q + 1], v[q + 2], v[q + 3]);
   }
-  if (bad_pivots && lane == 0 && info) {
-    const int bad = __ffs(bad_pivots) - 1;
-    if (c0 + bad < n) atomicCAS(info, 0, first + dir * (c0 + bad));
-  }
+  report(bad_pivots);
 }
 
 // The factorisation itself, by 256 threads (barriers 1 and 2).  S holds the lower triangle on entry, visible to all of

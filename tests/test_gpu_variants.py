@@ -747,3 +747,17 @@ def _lower_triangle(nat, std, pad):
         assert rel(dst[i], want) < 1e-5, d
         if std:
             assert rel(sd[i], torch.linalg.cholesky(want, upper=True)) < 1e-5, d
+
+
+@pytest.mark.parametrize('d', [1, 8, 9, 17, 130, 300])
+@pytest.mark.parametrize('top', [126.0, 127.5])
+def test_factors_of_a_matrix_near_the_largest_float(nat, d, top):
+    """Pivots above 2^126, whose reciprocals are no normal numbers, among others of 2^-20."""
+    import torchsso
+    scale = torch.where(torch.arange(d, device='cuda') % 3 == 1, 2.0 ** -10, 2.0 ** (top / 2)).double()
+    m = (spd(d, d, d) + torch.eye(d, device='cuda')).double()
+    m = m / m.diagonal().max()
+    m = (scale[:, None] * m * scale).float()
+    got, want = torchsso.utils.cholesky(m), torch.linalg.cholesky(m.double(), upper=True)
+    assert bool(got.isfinite().all())
+    assert rel(got.double() / scale, want / scale) < 1e-5      # column by column: U diag(1 / scale)

@@ -384,8 +384,9 @@ int64_t sso_kron_plan_create(int n_mats, const int64_t* dims, float* const* src,
                              void* dev_mem, size_t dev_mem_bytes, int host_only,
                              const int64_t* lds /* nullable: leading dimensions of src/dst/work/std, default dims */);
 /* damp_r_dev: per-matrix r = sqrt(damping); info_dev: per-matrix status (2 ints: inverse, std): 0, or the 1-based row of
- * the first pivot that is not positive.  A plan with std_out takes the matrices of its inverses from the last row to the
- * first (the factor comes with the inverse then, and with do_inverse only the first of the two statuses is used). */
+ * the first pivot that is not positive.  Where the dataflow kernel runs the plan (sso_kron_plan_uses_work() == 0) and it has
+ * std_out, its inverses take their matrices from the last row to the first: the factor comes with the inverse, and with do_inverse
+ * only the first of the two statuses is used.  Everything else goes from the first row on, with a status for each pass. */
 int sso_kron_plan_run(int64_t plan, const float* damp_r_dev, int* info_dev,
                       int do_inverse, int do_std, void* stream);
 /* The inverse (do_inverse) or else the upper Cholesky factor of a matrix that is not the plan's own: `src` instead of src_0 (or

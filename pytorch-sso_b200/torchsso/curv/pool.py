@@ -74,6 +74,7 @@ class FactorPool:
         self._mats = {}
         self._ranges = {}
         self.last_info: Optional[torch.Tensor] = None
+        self._last_reversed = False
         for c in list(kron) + list(diag):
             c._pool = self
 
@@ -224,6 +225,8 @@ class FactorPool:
             self._damp[key] = r
         nat.kron_plan_run(plan, damp, info, do_inverse, with_std)
         self.last_info = info
+        # an inverse with sampling factors goes from the last row to the first, in the kernel that needs no work matrices
+        self._last_reversed = with_std and do_inverse and not nat.kron_plan_uses_work()
 
     def _trim_plans(self, limit: int = 32):
         """Plans bake buffer addresses in; callers with unstable addresses would grow the cache."""
@@ -249,8 +252,9 @@ class FactorPool:
         bad = torch.nonzero(info).flatten()
         if bad.numel():
             i = int(bad[0])
-            raise RuntimeError('curvature matrix %d (%s pass) is not positive definite at row %d'
-                               % (i // 2, 'inverse' if i % 2 == 0 else 'cholesky', int(info[i])))
+            raise RuntimeError('curvature matrix %d (%s pass) is not positive definite at row %d%s'
+                               % (i // 2, 'inverse' if i % 2 == 0 else 'cholesky', int(info[i]),
+                                  ', taken from the last row to the first' if self._last_reversed else ''))
 
     def precondition(self, curvs: Sequence, grads: Sequence[Sequence[torch.Tensor]]):
         """grads[i] = [dW (, db)] of layer i, fp32 contiguous; replaced by G^-1 [dW|db] A^-1."""

@@ -192,6 +192,30 @@ def test_pool_ranges_without_a_neighbour(no_collection, monkeypatch):
     assert spans == [pool.k_total]
 
 
+@pytest.mark.parametrize('uses_work', [False, True])
+@pytest.mark.parametrize('std,inverse', [(False, True), (True, True), (True, False)])
+def test_a_bad_pivot_is_counted_from_where_the_pass_began(monkeypatch, std, inverse, uses_work):
+    """The dataflow kernel takes the matrices of an inverse with sampling factors from the last row on; every other pass
+    goes from the first."""
+    class NoPlan:
+        def status(self):
+            return 0
+
+    def run(plan, damp, info, do_inverse, do_std):
+        info[2 + (not do_inverse)] = 7
+    monkeypatch.setattr(nat, 'kron_plan_uses_work', lambda: uses_work)
+    monkeypatch.setattr(nat, 'kron_plan', lambda *a, **k: NoPlan())
+    monkeypatch.setattr(nat, 'kron_plan_run', run)
+    opt = make()
+    pool = opt.pool
+    pool.update_inv(with_std=False)
+    with pytest.raises(RuntimeError, match=r'matrix 1 \(inverse pass\) is not positive definite at row 7$'):
+        pool.check_info()
+    pool.update_inv(with_std=std, do_inverse=inverse)
+    with pytest.raises(RuntimeError, match='from the last row to the first' if std and inverse and not uses_work else 'at row 7$'):
+        pool.check_info()
+
+
 # ------------------------------------------------------------------------------------------- prepared calls
 def on_meta(t):
     return torch.empty_strided(t.shape, t.stride(), dtype=t.dtype, device='meta')

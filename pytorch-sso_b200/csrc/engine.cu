@@ -60,8 +60,10 @@ struct MatRec {       // per-matrix data for the trace / pi kernel
 // ------------------------------------------------------------------------------------------
 // tile GEMM kernel
 // ------------------------------------------------------------------------------------------
+// Launched beside the phase before, whose results it reads after its wait: tasks and operands come by ordinary loads, as the
+// non-coherent ones are for memory that nobody writes while the kernel lives.
 template <int MT>
-__global__ void __launch_bounds__(256) tile_task_kernel(const sso_tile_task* __restrict__ tasks) {
+__global__ void __launch_bounds__(256) tile_task_kernel(const sso_tile_task* tasks) {
   constexpr int TILE = 16 * MT;
   constexpr int PER = TILE * KT / 256;  // elements per thread per operand per stage
   __shared__ __align__(16) float As[KT * TILE];
@@ -75,7 +77,7 @@ __global__ void __launch_bounds__(256) tile_task_kernel(const sso_tile_task* __r
   const bool a_kcontig = !ta, b_kcontig = tb;
 
   float ra[PER], rb[PER];
-  auto load_op = [&](const float* __restrict__ P, int ld, bool kcontig, int lim, int k0, float (&r)[PER]) {
+  auto load_op = [&](const float* P, int ld, bool kcontig, int lim, int k0, float (&r)[PER]) {
     if (kcontig) {
       const int k = k0 + (tid & 31), g = tid >> 5;
       const bool kok = k < t.k;
@@ -84,7 +86,7 @@ __global__ void __launch_bounds__(256) tile_task_kernel(const sso_tile_task* __r
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int idx = g * 4 + 32 * i + q;
-          r[i * 4 + q] = (kok && idx < lim) ? __ldg(P + (int64_t)idx * ld + k) : 0.f;
+          r[i * 4 + q] = (kok && idx < lim) ? P[(int64_t)idx * ld + k] : 0.f;
         }
     } else {
       const int idx = tid % TILE, kb = tid / TILE;
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(256) tile_task_kernel(const sso_tile_task* __r
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
         const int k = k0 + kb + (256 / TILE) * i;
-        r[i] = (iok && k < t.k) ? __ldg(P + (int64_t)k * ld + idx) : 0.f;
+        r[i] = (iok && k < t.k) ? P[(int64_t)k * ld + idx] : 0.f;
       }
     }
   };

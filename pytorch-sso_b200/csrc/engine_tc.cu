@@ -527,7 +527,7 @@ struct alignas(128) TaskMaps {
 };
 
 template <int RAW_SLOTS, int LO_SLOTS, int PREFETCH>
-__global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_tile_task* __restrict__ tasks,
+__global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_tile_task* tasks,      // written by the launches before: no non-coherent loads
                                                                     const TaskMaps* __restrict__ maps, int* status) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * RAW_SLOTS + 2 * LO_SLOTS + 4];
@@ -702,7 +702,7 @@ constexpr int THREADS = 640, PROD_WARP = 9, SPLIT_WARP0 = 12, SPLIT_WARPS = 8;
 constexpr size_t SMEM = (RAW + LO) * PART + 1024;
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
-tile_pair_kernel(const sso_tile_task* __restrict__ tasks, const TaskMaps* __restrict__ maps, int* status) {
+tile_pair_kernel(const sso_tile_task* tasks, const TaskMaps* __restrict__ maps, int* status) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * RAW + 2 * LO + 4];
   __shared__ uint32_t tmem_base_slot;

@@ -761,3 +761,30 @@ def test_factors_of_a_matrix_near_the_largest_float(nat, d, top):
     got, want = torchsso.utils.cholesky(m), torch.linalg.cholesky(m.double(), upper=True)
     assert bool(got.isfinite().all())
     assert rel(got.double() / scale, want / scale) < 1e-5      # column by column: U diag(1 / scale)
+
+
+def test_phases_launched_early_see_the_phase_before(nat):
+    """The factorisation by launches, where 64-wide products follow one another on the same matrix: the same bits every time."""
+    dims = [1100, 700, 321, 65]
+    src = [spd(d, d, i) for i, d in enumerate(dims)]
+    dst, work, sd = ([torch.empty(d, d, device='cuda') for d in dims] for _ in range(3))
+    nat.configure('flow', 0)
+    nat.configure('chol_panel', 0)      # diagonal blocks by 64-wide halves
+    try:
+        plan = nat.kron_plan(dims, src, dst, work, sd, [-1] * 4, [0] * 4, torch.device('cuda'))
+        kinds = [k for k, _, _ in plan.phases()]
+        assert any(a == b == 0 for a, b in zip(kinds, kinds[1:]))
+        damp, info, first = torch.full((4,), 0.1, device='cuda'), torch.zeros(8, dtype=torch.int32, device='cuda'), None
+        for _ in range(20):
+            for m in work:
+                m.fill_(float('nan'))
+            nat.kron_plan_run(plan, damp, info, True, True)
+            got = [m.clone() for m in dst + sd]
+            first = first or got
+            assert all(torch.equal(a, b) for a, b in zip(got, first))
+    finally:
+        nat.configure('flow', 1)
+        nat.configure('chol_panel', 1)
+    for m, d, a, u in zip(src, dims, dst, sd):
+        want = torch.linalg.inv(m.double() + 0.1 * torch.eye(d, device='cuda', dtype=torch.float64))
+        assert rel(a, want) < 1e-5 and rel(u, torch.linalg.cholesky(want, upper=True)) < 1e-5

@@ -352,7 +352,7 @@ typedef struct {
 typedef struct {
   int32_t kind;       /* 0 gemm64, 1 gemm128, 2 diag-block factor (<= 64), 3 copy, 4 gemm128 whose operands are both read along k,
                          5 diag-block factor of a 128-column panel (same records as 2, size <= 128),
-                         6 gemm256 (as 4, blocks of 256x256, on the device only) */
+                         6 gemm256 (as 4, blocks of up to 256x256) */
   int32_t first;      /* first record of this phase in its table */
   int32_t count;      /* number of records (= CTAs) */
   int32_t reserved;

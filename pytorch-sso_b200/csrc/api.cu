@@ -77,7 +77,7 @@ static int g_tma_auto = 1;   // whether SSO_IMPL_AUTO may pick the TMA-fed tcgen
 
 using namespace sso;
 
-namespace sso { extern int g_flow; extern int g_engine_tma; extern int g_chol_ksplit; extern int g_phase_lpt; extern int g_chol_panel; }
+namespace sso { extern int g_flow; extern int g_engine_tma; extern int g_chol_ksplit; extern int g_phase_lpt; extern int g_chol_panel; extern int g_inject_no_maps; }
 
 extern "C" {
 
@@ -105,6 +105,7 @@ int sso_configure(const char* key, int value) {
   // tile-task kernels issue no loads, so that the waits of their consumers run out
   if (k == "wait_kcycles") { g_wait_kcycles = value < 0 ? 0 : value; return apply_wait_controls(); }
   if (k == "inject_stall") { g_stall = value != 0; return apply_wait_controls(); }
+  if (k == "inject_no_maps") { g_inject_no_maps = value != 0; return 0; }      // tensor maps of the tile products cannot be made
   if (k == "tc_flush") { factor_tc_set_flush(value); return 0; }
   return fail(-1, "configure: unknown key %s", key);
 }

@@ -16,6 +16,7 @@
 //       Y   = L_21 * Inv_11          (into scratch)      Inv_21 = - Inv_22 * Y
 //   Inverse:  M^-1 = Linv^T * Linv   (lower tiles computed, mirrored into the upper triangle)
 #include <algorithm>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <queue>
@@ -1231,17 +1232,29 @@ static bool pairs_pay(int n, const int64_t* dA, const int64_t* dG) {
   int64_t tiles = 0;
   for (int l = 0; l < n; ++l)
     if (dA[l] > 128 && dG[l] > 128) tiles += ((dA[l] + 127) / 128) * ((dG[l] + 127) / 128);
-  return tiles > 2 * 148 && g_engine_tma && g_engine_tc && tensor_map_encoder() != nullptr;
+  return tiles > 2 * 148 && g_engine_tma && g_engine_tc;
+}
+
+// Builds a plan of products and brings it to the device.  Blocks of 256 have no kernel without tensor maps: where one cannot
+// be made, the plan is built again with 128x128 tiles alone, which have.
+static Plan* create_products(bool pairs, void* mem, size_t bytes, int& rc, const std::function<Plan*(bool)>& build) {
+  for (;; pairs = false) {
+    Plan* p = build(pairs);
+    rc = upload(*p, mem, bytes);
+    const bool blocks = std::any_of(p->run_phases.begin(), p->run_phases.end(), [](const sso_phase& ph) { return ph.kind == 6; });
+    if (rc == 0 && (p->have_maps || !blocks)) return p;
+    delete p;
+    if (rc != 0) return nullptr;
+  }
 }
 
 // ---- precondition --------------------------------------------------------------------------
 static Plan* build_precond(int n, const int64_t* dA, const int64_t* dG, float* const* A_inv,
                            float* const* G_inv, float* const* gw, float* const* gb, float* const* tmp,
-                           const int64_t* ldA, const int64_t* ldG, bool on_device) {
+                           const int64_t* ldA, const int64_t* ldG, bool pairs) {
   Plan* p = new Plan();
   Builder b(*p, &p->run_phases);
   constexpr int T = 128;
-  const bool pairs = on_device && pairs_pay(n, dA, dG);
   // Both factors are symmetric, which lets every operand be read along its contiguous
   // direction (the fast path of the tensor-core tasks):
   //   tmp = U^T = A_inv[:, :wc] * gw^T (+ A_inv[:, wc] * gb^T),   [gw | gb] = G_inv * U.
@@ -1300,13 +1313,17 @@ int64_t sso_precond_plan_create(int n_layers, const int64_t* dA, const int64_t* 
   for (int l = 0; l < n_layers; ++l)
     SSO_CHECK_ARG(dA[l] > 0 && dG[l] > 0 && A_inv[l] && G_inv[l] && gw[l] && tmp[l],
                   "precond plan: bad layer %d", l);
-  Plan* p = build_precond(n_layers, dA, dG, A_inv, G_inv, gw, gb, tmp, ldA, ldG, !host_only);
-  p->host_only = host_only != 0;
-  if (!p->host_only) {
-    int rc = upload(*p, dev_mem, dev_mem_bytes);
-    if (!rc) rc = tables_landed();
-    if (rc != 0) { delete p; return rc; }
+  auto build = [&](bool pairs) { return build_precond(n_layers, dA, dG, A_inv, G_inv, gw, gb, tmp, ldA, ldG, pairs); };
+  const bool pairs = pairs_pay(n_layers, dA, dG);
+  if (host_only) {
+    Plan* p = build(pairs);
+    p->host_only = true;
+    return register_plan(p);
   }
+  int rc = 0;
+  Plan* p = create_products(pairs, dev_mem, dev_mem_bytes, rc, build);
+  if (!rc) rc = tables_landed();
+  if (rc != 0) { delete p; return rc; }
   return register_plan(p);
 }
 
@@ -1384,12 +1401,11 @@ static size_t sample_scratch_bytes(int n, const int64_t* dA, const int64_t* dG) 
 
 // [w | b] += s * U_G (E U_A) with every operand along k:  tt = (E U_A)^T = U_A^T E^T, then U_G tt^T.
 static Plan* build_sample_along_k(int n, const int64_t* dA, const int64_t* dG, float* const* U_A, float* const* U_G, float* const* noise,
-                                  float* const* w, float* const* bvec, const int64_t* ldA, const int64_t* ldG, char* mem) {
+                                  float* const* w, float* const* bvec, const int64_t* ldA, const int64_t* ldG, char* mem, bool pairs) {
   Plan* p = new Plan();
   Builder b(*p, &p->run_phases);
   constexpr int T = 128;
   std::vector<float*> tt(n);
-  const bool pairs = pairs_pay(n, dA, dG);
   int first = b.task_begin();
   size_t at = 0;
   for (int l = 0; l < n; ++l) {
@@ -1487,9 +1503,11 @@ int64_t sso_sample_plan_create(int n_layers, const int64_t* dA, const int64_t* d
     const size_t scratch = sample_scratch_bytes(n_layers, dA, dG);
     SSO_CHECK_ARG(dev_mem != nullptr && dev_mem_bytes >= scratch, "sample plan: plan memory too small");
     char* mem = reinterpret_cast<char*>(align_up(reinterpret_cast<uintptr_t>(dev_mem)));
-    Plan* p = build_sample_along_k(n_layers, dA, dG, U_A, U_G, noise, w, b, ldA, ldG, mem);
-    p->d_layouts = reinterpret_cast<LayoutRec*>(mem + scratch - 256 - align_up(2 * (size_t)n_layers * sizeof(LayoutRec)));
-    int rc = upload(*p, mem + scratch - 256, dev_mem_bytes - scratch);
+    int rc = 0;
+    Plan* p = create_products(pairs_pay(n_layers, dA, dG), mem + scratch - 256, dev_mem_bytes - scratch, rc, [&](bool pairs) {
+      return build_sample_along_k(n_layers, dA, dG, U_A, U_G, noise, w, b, ldA, ldG, mem, pairs);
+    });
+    if (p) p->d_layouts = reinterpret_cast<LayoutRec*>(mem + scratch - 256 - align_up(2 * (size_t)n_layers * sizeof(LayoutRec)));
     if (rc == 0 && cudaMemcpy(p->d_layouts, p->layouts.data(), p->layouts.size() * sizeof(LayoutRec), cudaMemcpyHostToDevice) != cudaSuccess)
       rc = fail(-2, "sample plan: copy of the layout records failed");
     if (rc == 0) rc = tables_landed();

@@ -349,8 +349,8 @@ def test_sample_plan_along_k(nat, shapes, bias):
         assert rel(got, want[i]) < 2e-6
 
 
-# enough layers for blocks of 256 (more than two rounds of 128x128 tiles): strips of up to 128 rows or columns beside them,
-# blocks that are not full, layers without a block, rows that cannot be read with TMA
+# enough layers for blocks of 256 (more than two rounds of 128x128 tiles): blocks that are not full, down to a row or a column
+# beyond the last whole one, layers without a block, rows that cannot be read with TMA
 WIDE = [(260, 260), (384, 129), (513, 640), (1152, 385), (2308, 1024), (516, 255), (128, 640), (2304, 513), (641, 300), (256, 256)]
 
 
@@ -361,6 +361,7 @@ def test_sample_plan_in_wide_blocks(nat, bias, monkeypatch):
     def plan_of_nans(dA, *args):
         plan = make(dA, *args)
         plan._dev_mem[:dA[0] * ((dA[0] + 3) // 4 * 4) * 4].fill_(255)      # the first U_A^T: only what a run writes may be read
+        assert any(k == 6 for k, _, _ in plan.phases())
         return plan
     monkeypatch.setattr(nat, 'sample_plan', plan_of_nans)
     test_sample_plan_along_k(nat, WIDE[4:5] + WIDE[:4] + WIDE[5:], bias)
@@ -368,6 +369,10 @@ def test_sample_plan_in_wide_blocks(nat, bias, monkeypatch):
 
 @pytest.mark.parametrize('bias', [False, True])
 def test_precond_plan_in_wide_blocks(nat, bias):
+    assert any(k == 6 for k, _, _ in precond_in_wide_blocks(nat, bias).phases())
+
+
+def precond_in_wide_blocks(nat, bias):
     shapes = [(a + int(bias), g) for a, g in WIDE]
 
     def inverse(d, seed):
@@ -389,6 +394,21 @@ def test_precond_plan_in_wide_blocks(nat, bias):
     for i in range(len(shapes)):
         got = w[i] if b[i] is None else torch.cat([w[i], b[i][:, None]], 1)
         assert rel(got, want[i]) < 2e-6, shapes[i]
+    return plan
+
+
+@pytest.mark.parametrize('bias', [False, True])
+def test_plans_in_wide_blocks_without_tensor_maps(nat, bias, monkeypatch):
+    """Where the driver makes no map, such a plan runs in 128x128 tiles."""
+    plans, make = [], nat.sample_plan
+    monkeypatch.setattr(nat, 'sample_plan', lambda *a: (plans.append(make(*a)), plans[-1])[1])
+    nat.configure('inject_no_maps', 1)
+    try:
+        plans.append(precond_in_wide_blocks(nat, bias))
+        test_sample_plan_along_k(nat, WIDE, bias)
+    finally:
+        nat.configure('inject_no_maps', 0)
+    assert len(plans) == 2 and not any(k == 6 for plan in plans for k, _, _ in plan.phases())
 
 
 @pytest.mark.parametrize('cfg', [(128, 4096, 1, 1, (1, 1), (1, 1), (0, 0), (1, 1), True), (1, 300, 1, 1, (1, 1), (1, 1), (0, 0), (1, 1), False),

@@ -41,8 +41,8 @@ def run_program(plan, mem, shift=None, scale_alpha=None):
     copies, _ = plan.copy_recs()
     info = {}
     for kind, first, count in plan.phases():
-        if kind in (0, 1, 4):
-            tile = 64 if kind == 0 else 128
+        if kind in (0, 1, 4, 6):
+            tile = {0: 64, 6: 256}.get(kind, 128)
             results = []
             for t in [tasks[i] for i in range(first, first + count)]:
                 assert 0 < t.m <= tile and 0 < t.n <= tile and t.k > 0
@@ -236,6 +236,59 @@ def test_precondition_program(dA, dG, bias):
     if bias:
         got = np.concatenate([got, gb.reshape(dG, 1)], axis=1)
     assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < 1e-5
+
+
+@pytest.mark.parametrize('bias', [False, True])
+def test_precondition_program_in_wide_blocks(bias):
+    """More than two rounds of 128x128 tiles: layers with both sides above 128 in blocks of 256, the others as they were."""
+    shapes = [(2308 + bias, 1025), (1152 + bias, 385), (2304 + bias, 513), (128 + bias, 300), (641, 257), (260, 128), (512 + bias, 700)]
+    mem, rng = Mem(), np.random.default_rng(7)
+
+    def aligned(n):      # rows on 16 bytes, as those of the device are
+        raw = mem.new(n + 4)
+        at = (-raw.ctypes.data % 16) // 4
+        return raw[at:at + n]
+
+    def padded(d, seed):
+        ld = (d + 3) // 4 * 4
+        buf = aligned(d * ld)
+        m = np.lib.stride_tricks.as_strided(buf, shape=(d, d), strides=(4 * ld, 4))
+        x = np.random.default_rng(seed).standard_normal((d, d)).astype(np.float32)
+        m[...] = x + x.T
+        return buf, m
+    A, G, w, b, tmp, want = [], [], [], [], [], []
+    for i, (a, g) in enumerate(shapes):
+        wc = a - bias
+        A.append(padded(a, 2 * i))
+        G.append(padded(g, 2 * i + 1))
+        w.append(aligned(g * wc))
+        b.append(aligned(g) if bias else None)
+        tmp.append(aligned(a * ((g + 3) // 4 * 4)))
+        grad = rng.standard_normal((g, a)).astype(np.float32)
+        w[-1].reshape(g, wc)[...] = grad[:, :wc]
+        if bias:
+            b[-1][:] = grad[:, wc]
+        want.append(G[-1][1].astype(np.float64) @ grad @ A[-1][1].astype(np.float64))
+
+    def address(bufs):
+        return [None if x is None else x.ctypes.data for x in bufs]
+    dA, dG = [a for a, _ in shapes], [g for _, g in shapes]
+    L, n = nat.lib(), len(shapes)
+    lds = [nat._i64([(d + 3) // 4 * 4 for d in dims]) for dims in (dA, dG)]
+    h = L.sso_precond_plan_create(n, nat._i64(dA), nat._i64(dG), nat._ptrs(address(x for x, _ in A)), nat._ptrs(address(x for x, _ in G)),
+                                  nat._ptrs(address(w)), nat._ptrs(address(b)), nat._ptrs(address(tmp)), None, 0, 1, *lds)
+    plan = nat.Plan(h, None, None)
+    assert {k for k, _, _ in plan.phases()} >= {4, 6}
+    tasks, _ = plan.tasks()
+    for kind, first, count in plan.phases():
+        for t in tasks[first:first + count]:
+            assert kind != 6 or t.lda % 4 == t.ldb % 4 == t.A % 16 == t.B % 16 == 0
+    run_program(plan, mem)
+    for (a, g), x, y, ref in zip(shapes, w, b, want):
+        got = x.reshape(g, a - bias)
+        if bias:
+            got = np.concatenate([got, y.reshape(g, 1)], axis=1)
+        assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < 1e-6
 
 
 @pytest.mark.parametrize('dA,dG,bias', [(21, 16, True), (200, 150, True), (129, 130, False)])

@@ -250,7 +250,8 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tc_kernel(const sso_tile
     if (lane == 0) {
       const uint32_t idesc = instr_desc(2u, 0u);   // tf32, K-major
       bool ok = true;
-      for (int s = 0; s < nstages && ok; ++s) {
+      int s = 0;
+      for (; s < nstages && ok; ++s) {
         const int slot = s % STAGES, c = s / FLUSH, b = c & 1;
         const bool first_of_chunk = (s % FLUSH) == 0;
         if (first_of_chunk && c >= 2) ok = mbar_wait(accempty_bar(b), ((c >> 1) - 1) & 1, status, 12);
@@ -273,6 +274,7 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tc_kernel(const sso_tile
         umma_commit(empty_bar(slot));
         if ((s % FLUSH) == FLUSH - 1 || s == nstages - 1) umma_commit(accfull_bar(b));
       }
+      mmas_done<STAGES>(s, empty_bar, status, 18);
     }
   } else {
     // ------------------------------------------------------------------ load warps
@@ -414,7 +416,8 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_kc_kernel(const sso_tile
     if (lane == 0) {
       const uint32_t idesc = instr_desc(2u, 0u);   // tf32, K-major
       bool ok = true;
-      for (int s = 0; s < nstages && ok; ++s) {
+      int s = 0;
+      for (; s < nstages && ok; ++s) {
         const int rs = s % RAW_SLOTS, ls = s % LO_SLOTS, c = s / FLUSH, b = c & 1;
         const bool first_of_chunk = (s % FLUSH) == 0;
         if (first_of_chunk && c >= 2) ok = mbar_wait(accempty0 + 8u * b, ((c >> 1) - 1) & 1, status, 22);
@@ -436,6 +439,7 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_kc_kernel(const sso_tile
         umma_commit(lofree_bar(ls));
         if ((s % FLUSH) == FLUSH - 1 || s == nstages - 1) umma_commit(accfull0 + 8u * b);
       }
+      mmas_done<LO_SLOTS>(s, lofree_bar, status, 28);
     }
   } else {
     // ------------------------------------------------------------------ load + split warps
@@ -580,7 +584,8 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
     if (lane == 0) {
       const uint32_t idesc = instr_desc(2u, 0u);   // tf32, K-major
       bool ok = true;
-      for (int s = 0; s < nstages && ok; ++s) {
+      int s = 0;
+      for (; s < nstages && ok; ++s) {
         const int rs = s % RAW_SLOTS, ls = s % LO_SLOTS, c = s / FLUSH, b = c & 1;
         const bool first_of_chunk = (s % FLUSH) == 0;
         if (first_of_chunk && c >= 2) ok = mbar_wait(accempty0 + 8u * b, ((c >> 1) - 1) & 1, status, 42);
@@ -602,6 +607,7 @@ __global__ void __launch_bounds__(THREADS, 1) tile_task_tma_kernel(const sso_til
         umma_commit(lofree_bar(ls));
         if ((s % FLUSH) == FLUSH - 1 || s == nstages - 1) umma_commit(accfull0 + 8u * b);
       }
+      mmas_done<LO_SLOTS>(s, lofree_bar, status, 48);
     }
   } else {
     // ------------------------------------------------------------------ producer thread + split warps
@@ -803,7 +809,8 @@ tile_pair_kernel(const sso_tile_task* tasks, const TaskMaps* __restrict__ maps, 
     if (warp == MMA_WARP && lane == 0 && rank == 0) {
       const uint32_t idesc = instr_desc_pair(2u, 0u);   // tf32, K-major
       bool ok = true;
-      for (int s = 0; s < nstages; ++s) {
+      int s = 0;
+      for (; s < nstages; ++s) {
         const int rs = s % RAW, ls = s % LO, c = s / FLUSH, b = c & 1;
         const bool first_of_chunk = (s % FLUSH) == 0;
         if (first_of_chunk && c >= 2) ok = mbar_wait(accempty0 + 8u * b, ((c >> 1) - 1) & 1, status, 52);
@@ -824,6 +831,7 @@ tile_pair_kernel(const sso_tile_task* tasks, const TaskMaps* __restrict__ maps, 
         umma2_commit_both(lofree(ls));
         if ((s % FLUSH) == FLUSH - 1 || s == nstages - 1) umma2_commit_both(accfull0 + 8u * b);
       }
+      mmas_done<LO>(s, lofree, status, 58);
     } else if (warp == PROD_WARP && lane == 0 && !g_inject_stall) {      // stalled: nothing is ever loaded
       const uint64_t map_a = reinterpret_cast<uint64_t>(maps[task].a), map_b = reinterpret_cast<uint64_t>(maps[task].b);
       const int row = (int)rank * TILE;

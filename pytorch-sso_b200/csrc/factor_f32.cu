@@ -493,7 +493,8 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
       const uint32_t idesc = PAIR ? (instr_desc_pair(1u, 1u) & ~(0x3Fu << 17)) | ((uint32_t)((ragged ? last_n : 256) >> 3) << 17)
                                   : ((instr_desc(1u, 1u) & ~(0x3Fu << 17)) | ((uint32_t)(n_cols >> 3) << 17));
       bool ok = true;
-      for (int s = 0; s < nstages && ok; ++s) {
+      int s = 0;
+      for (; s < nstages && ok; ++s) {
         const int slot = s % STAGES, c = s / FLUSH, b = c & 1;
         const bool first_of_chunk = (s % FLUSH) == 0;
         if (first_of_chunk && c >= 2) ok = mbar_wait(accempty_bar(b), ((c >> 1) - 1) & 1, status, 62);
@@ -524,6 +525,7 @@ __global__ void __launch_bounds__(THREADS, 1) factor_f32_kernel(const FactorPara
           if (publish) umma_commit(accfull_bar(b));
         }
       }
+      mmas_done<STAGES>(s, empty_bar, status, 68);
     }
     __syncwarp();
     asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");
@@ -791,6 +793,7 @@ __global__ void __launch_bounds__(THREADS, 1) narrow_kernel(const FactorParams p
           }
         }
       }
+      mmas_done<2>(c, accfull_bar, status, 78);      // a chunk is begun only when its accumulator is free
     }
   } else if (warp >= LOAD_WARP0) {
     const int w = warp - LOAD_WARP0;

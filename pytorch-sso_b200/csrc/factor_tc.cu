@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
     if (lane == 0) {
       const uint32_t idesc = instr_desc(C::FMT, C::MAJOR);
       bool ok = true;
-      for (int s = 0; s < nstages && ok; ++s) {
+      int s = 0;
+      for (; s < nstages && ok; ++s) {
         const int slot = s % STAGES, c = s / flush, b = c & 1;
         const bool first_of_chunk = (s % flush) == 0;
         if (first_of_chunk && c >= 2) ok = mbar_wait(accempty_bar(b), ((c >> 1) - 1) & 1, status, 2);
@@ -158,6 +159,7 @@ __global__ void __launch_bounds__(THREADS, 1) factor_tc_kernel(const FactorParam
         umma_commit(empty_bar(slot));
         if ((s % flush) == flush - 1 || s == nstages - 1) umma_commit(accfull_bar(b));
       }
+      mmas_done<STAGES>(s, empty_bar, status, 8);
     }
   } else {
     // ------------------------------------------------------------------ gather warps

@@ -277,6 +277,7 @@ __global__ void __launch_bounds__(THREADS, 1) flow_kernel(const Args g) {
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) { dead = 1; break; }
     }
+    if (warp == MMA_WARP && lane == 0) mmas_done<LO>((int)stage, lofree, status, 98);
   } else if (warp >= SPLIT_WARP0) {
     // ------------------------------------------------------------------ split warps
     asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");

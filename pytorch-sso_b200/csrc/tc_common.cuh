@@ -62,6 +62,12 @@ template <int SLOTS, typename Bar>
 __device__ __forceinline__ void ring_landed(int issued, Bar full_bar, int* status, int code) {
   for (int s = issued > SLOTS ? issued - SLOTS : 0; s < issued; ++s) mbar_wait(full_bar(s % SLOTS), (s / SLOTS) & 1, status, code);
 }
+// The same for the MMAs of the `issued` stages so far, by the thread that issued and committed them: when an accumulate warp gave
+// up, nobody else waits for these, and they must not read shared memory or write tensor memory that has been given back.
+template <int SLOTS, typename Bar>
+__device__ __forceinline__ void mmas_done(int issued, Bar free_bar, int* status, int code) {
+  if (issued > 0) mbar_wait(free_bar((issued - 1) % SLOTS), ((issued - 1) / SLOTS) & 1, status, code);
+}
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }

@@ -179,3 +179,80 @@ def test_inverse_of_many_small_matrices_wait_runs_out(nat):
         nat.configure('wait_kcycles', 0)
     assert plan.status() != 0 and int(info[0]) == -(1000 + plan.status())
     assert bool(torch.isnan(torch.stack(dst)).all())
+
+
+@pytest.mark.parametrize('bias', [False, True])
+def test_blocks_of_256_wait_runs_out(nat, bias):
+    """A preconditioning plan of CTA pairs: each pair answers its block with NaN, at the edges of the matrix too, and leaves."""
+    shapes = [(2308 + bias, 1025), (1152 + bias, 388), (2304 + bias, 513), (513 + bias, 640), (260 + bias, 257)]
+    A = [torch.randn(a, (a + 3) // 4 * 4, device='cuda')[:, :a] for a, _ in shapes]
+    G = [torch.randn(g, (g + 3) // 4 * 4, device='cuda')[:, :g] for _, g in shapes]
+    A, G = [[torch.empty_like(m._base)[:, :m.shape[0]].copy_(m + m.t()) for m in ms] for ms in (A, G)]
+    grads = [torch.randn(g, a, device='cuda') for a, g in shapes]
+
+    def run(stall):
+        w = [x[:, :x.shape[1] - bias].contiguous() for x in grads]
+        b = [x[:, -1].contiguous() if bias else None for x in grads]
+        around = [torch.full((x.numel() + 64,), 7.0, device='cuda') for x in w]      # what lies next to the results
+        w = [r[32:-32].view_as(x).copy_(x) for r, x in zip(around, w)]
+        tmp = [torch.empty(a * g.stride(0), device='cuda') for (a, _), g in zip(shapes, G)]
+        plan = nat.precond_plan([a for a, _ in shapes], [g for _, g in shapes], A, G, w, b, tmp, torch.device('cuda'))
+        assert any(k == 6 for k, _, _ in plan.phases())
+        if stall:
+            nat.configure('wait_kcycles', 2000)
+            nat.configure('inject_stall', 1)
+        try:
+            nat.precond_plan_run(plan)
+            torch.cuda.synchronize()
+        finally:
+            nat.configure('inject_stall', 0)
+            nat.configure('wait_kcycles', 0)
+        assert all(bool((r[:32] == 7.0).all() and (r[-32:] == 7.0).all()) for r in around)
+        return plan.status(), w, b
+
+    status, w, b = run(True)
+    assert status != 0
+    assert all(bool(torch.isnan(x).all()) for x in w)
+    status, w, b = run(False)
+    assert status == 0
+    for i, (x, y) in enumerate(zip(w, b)):
+        got = torch.cat([x, y[:, None]], 1) if bias else x
+        assert _rel(got, (G[i].double() @ grads[i].double() @ A[i].double()).cpu()) < 2e-6, shapes[i]
+
+
+def test_inverse_with_sampling_factors_wait_runs_out(nat):
+    """In reverse order and padded to rows of four: the inverses are NaN, the factors where their blocks were not reached, and
+    nothing outside of the matrices is written."""
+    dims, pad = [1, 5, 126, 130, 257, 389], 3
+    n = len(dims)
+    src = []
+    for i, d in enumerate(dims):
+        x = cases.make_normal((2 * d + 8, d), i).cuda()
+        src.append(torch.full((d, d + pad), 7.0, device='cuda')[:, :d].copy_(x.t() @ x / x.shape[0]))
+    damp = torch.full((n,), 0.1, device='cuda')
+
+    def run(stall):
+        dst, std = ([torch.full((d, d + pad), 7.0, device='cuda')[:, :d] for d in dims] for _ in range(2))
+        plan = nat.kron_plan(dims, src, dst, None, std, [-1] * n, [0] * n, torch.device('cuda'))
+        info = torch.zeros(2 * n, dtype=torch.int32, device='cuda')
+        if stall:
+            nat.configure('wait_kcycles', 2000)
+            nat.configure('inject_stall', 1)
+        try:
+            nat.kron_plan_run(plan, damp, info, True, True)
+            torch.cuda.synchronize()
+        finally:
+            nat.configure('inject_stall', 0)
+            nat.configure('wait_kcycles', 0)
+        assert all(bool((m._base[:, d:] == 7.0).all()) for ms in (dst, std) for m, d in zip(ms, dims))
+        return plan.status(), info, dst, std
+
+    status, info, dst, std = run(True)
+    assert status != 0 and int(info[0]) == -(1000 + status)
+    assert all(bool(torch.isnan(m).all()) for m in dst)
+    assert all(bool(torch.isnan(u[0, -1])) for u, d in zip(std, dims) if d > 128)
+    status, info, dst, std = run(False)
+    assert status == 0 and not info.any()
+    for m, a, u, d in zip(src, dst, std, dims):
+        want = torch.linalg.inv(m.double().cpu() + 0.1 * torch.eye(d, dtype=torch.float64))
+        assert _rel(a, want) < 1e-5 and _rel(u, torch.linalg.cholesky(want, upper=True)) < 1e-5

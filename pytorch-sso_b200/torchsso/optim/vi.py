@@ -29,6 +29,15 @@ def _probabilities(output):
     raise ValueError(f'Invalid ndim {output.ndim}')
 
 
+def _copy_all(to, source):
+    """to[i] <- source[i], in one launch for the tensors of a type: one of another type would send the whole list through
+    copies of their own."""
+    kinds = {(t.dtype, s.dtype) for t, s in zip(to, source)}
+    for kind in kinds:
+        pairs = [(t, s) for t, s in zip(to, source) if (t.dtype, s.dtype) == kind] if len(kinds) > 1 else None
+        torch._foreach_copy_(*([t for t, _ in pairs], [s for _, s in pairs]) if pairs else (to, source))
+
+
 class VIOptimizer(SecondOrderOptimizer):
     r"""Variational-inference optimizer.  Arguments as in the reference class: ``dataset_size``
     scales the KL term (l2_reg = kl_weighting / dataset_size / prior_variance, sampling scale
@@ -128,8 +137,9 @@ class VIOptimizer(SecondOrderOptimizer):
         drawn layer by layer in param_group order; all Kronecker layers are then transformed in
         one batched plan."""
         batches, diag = {}, {}
-        # copies of all layers go to the device together: one layer's parameters fill a quarter of the GPU
-        to, source = [], []
+        # copies of all layers go to the device together: one layer's parameters fill a quarter of the GPU.  Noise that waits for
+        # its copy is no more than 32 MB, or than one layer's (no more than the largest layer's: 0.45 ms more for VGG-16's four draws)
+        to, source, waiting = [], [], 0
         for group in self.param_groups:
             params, mean, curv = group['params'], group['mean'], group['curv']
             if curv is None or curv.std is None:
@@ -151,8 +161,12 @@ class VIOptimizer(SecondOrderOptimizer):
                 u += curv.std
                 continue
             buf = self._noise_buf(group)
+            if waiting and waiting + buf.numel() > 8 << 20:
+                _copy_all(to, source)
+                to, source, waiting = [], [], 0
             to.append(buf)
             source.append(torch.randn_like(buf))
+            waiting += buf.numel()
             to += [p.data for p in params]
             source += mean
             c, t, nz = batches.setdefault(float(group['std_scale']), ([], [], []))
@@ -162,8 +176,7 @@ class VIOptimizer(SecondOrderOptimizer):
         for p, m, _, _ in diag.values():
             to += p
             source += m
-        if to:
-            torch._foreach_copy_(to, source)
+        _copy_all(to, source)
         for scale, (p, m, e, u) in diag.items():
             torch._foreach_addcmul_(p, e, u, value=scale)
         for scale, (c, t, nz) in batches.items():
@@ -224,8 +237,7 @@ class VIOptimizer(SecondOrderOptimizer):
         self.optim_state['step'] += 1
         groups = self.local_param_groups
         self._update_groups(groups, 'mean', True, lambda g: g['std_scale'] > 0)
-        if groups:
-            torch._foreach_copy_([p.data for group in groups for p in group['params']], [m for group in groups for m in group['mean']])
+        _copy_all([p.data for group in groups for p in group['params']], [m for group in groups for m in group['mean']])
         self.adjust_kl_weighting()
         return loss, prob
 

@@ -808,3 +808,45 @@ def test_phases_launched_early_see_the_phase_before(nat):
     for m, d, a, u in zip(src, dims, dst, sd):
         want = torch.linalg.inv(m.double() + 0.1 * torch.eye(d, device='cuda', dtype=torch.float64))
         assert rel(a, want) < 1e-5 and rel(u, torch.linalg.cholesky(want, upper=True)) < 1e-5
+
+
+def test_weight_samples_hold_the_noise_of_some_layers(nat):
+    """What a draw allocates is 32 MB of noise on its way to where it is kept: two of these five layers."""
+    import torch.nn as nn
+    import torch.nn.functional as F
+    import torchsso
+    model = nn.Sequential(*[nn.Linear(2000, 2000, bias=i % 2 == 0) for i in range(5)], nn.Linear(2000, 10)).cuda()
+    x, y = torch.randn(32, 2000, device='cuda'), torch.randint(0, 10, (32,), device='cuda')
+    opt = torchsso.optim.VIOptimizer(model, 500, 'Cov', {'Linear': 'Kron'}, {'ema_decay': 0.9, 'damping': 1e-2}, lr=1e-3, num_mc_samples=1)
+
+    def closure():
+        opt.zero_grad()
+        out = model(x)
+        loss = F.cross_entropy(out, y)
+        loss.backward()
+        return loss, out
+    opt.step(closure=closure)
+    opt.sample_params()
+    torch.manual_seed(3)
+    opt.sample_params()
+    drawn = [p.clone() for p in model.parameters()]
+    torch.manual_seed(3)
+    want = [torch.randn_like(opt._noise_buf(g)) for g in opt.param_groups]
+    torch.manual_seed(3)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    opt.sample_params()
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - before < 36 << 20      # blocks of the allocator may be larger; all layers: 80 MB
+    assert all(torch.equal(p, q) for p, q in zip(model.parameters(), drawn))
+    assert all(torch.equal(opt._noise_buf(g), e) for g, e in zip(opt.param_groups, want))
+
+
+def test_copies_of_tensors_of_several_types(nat):
+    from torchsso.optim.vi import _copy_all
+    source = [torch.randn(n, device='cuda').to(t) for n, t in ((5, torch.float32), (3, torch.bfloat16), (7, torch.float32), (1, torch.float64))]
+    to = [torch.zeros(s.shape, device='cuda', dtype=t) for s, t in zip(source, (torch.float32, torch.bfloat16, torch.bfloat16, torch.float32))]
+    _copy_all(to, source)
+    _copy_all([], [])
+    assert all(torch.equal(t, s.to(t.dtype)) for t, s in zip(to, source))

@@ -19,7 +19,7 @@
 // Bound: for one large matrix the chain of diagonal blocks, for many the shared-memory traffic of the 3xTF32 stages
 // (as tile_task_tma_kernel).  Against one launch per phase (us): 577+64 508 -> 180, 1000 637 -> 265, six factors of a
 // 784-1000-1000-10 network 1196 -> 296, 4608+512 3363 -> 1424, the 106 factors of ResNet-50 8970 -> 3600, those of VGG-16
-// with sampling factors 19416 -> 7440, with these out of the same factorisation 6440 -> 4620.
+// with sampling factors 19416 -> 6440, and 4290 with these out of the same factorisation.
 // Sampling factors: with J the reversal of rows and columns and J M J = L L^T, the lower Cholesky factor of M^-1 is J L^-T J.  A
 // matrix whose factor is wanted is therefore read, and its results are written, in reverse; in between nothing differs.
 // Every wait is bounded; a CTA whose wait gives up sets the status word and writes NaN for this and all further tasks.
